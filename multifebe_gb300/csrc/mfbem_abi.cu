@@ -28,6 +28,7 @@
 #include "mfbem_assemble.cuh"
 #include "mfbem_internal.cuh"
 #include "mfbem_hbie.cuh"
+#include "mfbem_radial.cuh"
 #include "mfbem_lu.cuh"
 #include "mfbem_tc.cuh"
 #include "mfbem_oz.cuh"
@@ -115,6 +116,10 @@ struct mfbem_handle {
   bool ms_built[2] = {false, false};
   long long mb_pts[3] = {0, 0, 0}, ms_pts[2][3] = {{0, 0, 0}, {0, 0, 0}};
   DevBuf parh;  // HarParH per frequency of the last harmonic assembly
+  // radial tables of the last harmonic call and a bound of the distance
+  // between any two points of the mesh's elements
+  DevBuf rad;
+  double rmax = 0.0;
 };
 
 // ---------------------------------------------------------------------------
@@ -586,6 +591,19 @@ static int upload_impl(const mfbem_mesh_desc* d, const mfbem_dual_desc* dual, mf
         dcv[2 * dof] = cv[6 * s + 2 * k];
         dcv[2 * dof + 1] = cv[6 * s + 2 * k + 1];
       }
+  // per element, for the flush of the mixed pair kernels (face 1 of a
+  // crack-like element: those kernels do not take such regions)
+  std::vector<int> emask(ne, 0), enz(ne, 0);
+  for (int e = 0; e < ne; ++e) {
+    const int ck = rev[e] >> 1;
+    for (int kn = 0; kn < 8; ++kn)
+      for (int k = 0; k < 3; ++k) {
+        const int dof = edof[8 * e + kn] + (k << ck), bit = 1 << (3 * kn + k);
+        if (dct[dof] == 1) emask[e] |= bit;
+        if (dcv[2 * dof] != 0.0 || dcv[2 * dof + 1] != 0.0) enz[e] |= bit;
+      }
+    if (rev[e] & 1) emask[e] |= 1 << 24;
+  }
   // formulation per node: 0 SBIE, 1 HBIE alone, 2 Burton & Miller at common points,
   // 3 crack-like node (dual BEM), 4 Burton & Miller with the SBIE at its own point
   std::vector<int> form(nn, 0);
@@ -679,12 +697,33 @@ static int upload_impl(const mfbem_mesh_desc* d, const mfbem_dual_desc* dual, mf
       for (int v : inc[node_of_dn[c.dn]]) inc_el.push_back(v);
     inc_start[i + 1] = (int)inc_el.size();
   }
+  // points of an element stay within 3 times (the largest sum of |phi| of the
+  // quad8 shape functions) its nodes' distance from their mean
+  {
+    double lo[3] = {HUGE_VAL, HUGE_VAL, HUGE_VAL}, hi[3] = {-HUGE_VAL, -HUGE_VAL, -HUGE_VAL};
+    for (int e = 0; e < ne; ++e) {
+      const double* X = d->x_gn + 24 * (size_t)e;
+      double c[3] = {0, 0, 0}, R = 0.0;
+      for (int k = 0; k < 8; ++k)
+        for (int q = 0; q < 3; ++q) c[q] += 0.125 * X[3 * k + q];
+      for (int k = 0; k < 8; ++k)
+        R = std::max(R, std::sqrt((X[3 * k] - c[0]) * (X[3 * k] - c[0]) + (X[3 * k + 1] - c[1]) * (X[3 * k + 1] - c[1]) +
+                                  (X[3 * k + 2] - c[2]) * (X[3 * k + 2] - c[2])));
+      for (int q = 0; q < 3; ++q) {
+        lo[q] = std::min(lo[q], c[q] - 3.0 * R);
+        hi[q] = std::max(hi[q], c[q] + 3.0 * R);
+      }
+    }
+    h->rmax = std::sqrt((hi[0] - lo[0]) * (hi[0] - lo[0]) + (hi[1] - lo[1]) * (hi[1] - lo[1]) +
+                        (hi[2] - lo[2]) * (hi[2] - lo[2]));
+  }
   // --- device arrays
   double *ex, *cl, *ball, *dcvd, *cpxd, *cpxid, *ngn, *tbp;
-  int *gln, *revd, *edofd, *dctd, *cpdn, *cpk, *cpe, *cpkn, *dncp, *incs, *ince;
+  int *gln, *revd, *edofd, *emaskd, *enzd, *dctd, *cpdn, *cpk, *cpe, *cpkn, *dncp, *incs, *ince;
   if ((rc = dupload(h, &ex, d->x_gn, 24 * (size_t)ne)) || (rc = dupload(h, &cl, d->csize, (size_t)ne)) ||
       (rc = dupload(h, &gln, d->n_phi, (size_t)ne)) || (rc = dupload(h, &ball, d->bball, 4 * (size_t)ne)) ||
       (rc = dupload(h, &revd, rev.data(), rev.size())) || (rc = dupload(h, &edofd, edof.data(), edof.size())) ||
+      (rc = dupload(h, &emaskd, emask.data(), emask.size())) || (rc = dupload(h, &enzd, enz.data(), enz.size())) ||
       (rc = dupload(h, &dctd, dct.data(), dct.size())) || (rc = dupload(h, &dcvd, dcv.data(), dcv.size())) ||
       (rc = dupload(h, &cpxd, cpx.data(), cpx.size())) || (rc = dupload(h, &cpxid, cpxi.data(), cpxi.size())) ||
       (rc = dupload(h, &cpdn, cp_dn.data(), cp_dn.size())) || (rc = dupload(h, &cpk, cp_kind.data(), cp_kind.size())) ||
@@ -714,6 +753,7 @@ static int upload_impl(const mfbem_mesh_desc* d, const mfbem_dual_desc* dual, mf
     }
   }
   m.ex = ex; m.cl = cl; m.gln_far = gln; m.ball = ball; m.rev = revd; m.edof = edofd;
+  m.emask = emaskd; m.enz = enzd;
   m.dct = dctd; m.dcv = dcvd; m.cpx = cpxd; m.cp_xi = cpxid; m.cp_dn = cpdn; m.cp_kind = cpk;
   m.cp_elem = cpe; m.cp_kn = cpkn; m.dn_cp = dncp; m.inc_start = incs; m.inc_el = ince;
   m.n_gn = ngn; m.tbp_gn = tbp;
@@ -830,7 +870,7 @@ extern "C" int mfbem_mesh_release(mfbem_handle* h) {
     cudaDeviceSynchronize();
     for (auto& o : h->owned) pool_give(o.first, o.second, h->dev);
     for (DevBuf* b : {&h->A, &h->b, &h->A32, &h->x, &h->r, &h->work, &h->ipiv, &h->info, &h->par, &h->nu, &h->parf,
-                      &h->pphi_f, &h->geo_f, &h->gm, &h->parh})
+                      &h->pphi_f, &h->geo_f, &h->gm, &h->parh, &h->rad})
       pool_give(b->p, b->bytes, b->dev);
     if (h->st) {
       std::lock_guard<std::mutex> lk(g_pool_mu);
@@ -988,6 +1028,53 @@ struct AsmTimes {
   }
 };
 
+// Radial tables (dev_radial.cuh) of a harmonic call's nf frequencies, rebuilt
+// on every call: q [nf][6] (lambda, mu, rho, omega; host), dpar / dparh their
+// device parameter blocks (dparh: HBIE points only), mixed: the double-float
+// rows too. t->n = 0 (the kernels evaluate E_n directly) where the tables do
+// not apply: a wavenumber of zero or not finite, or more intervals than
+// kRadMaxN.
+static int radial_prepare(mfbem_handle* h, const double* q, int nf, const HarParD* dpar, const HarParH* dparh,
+                          bool mixed, RadTab* t) {
+  *t = RadTab();
+  std::vector<double> hl(nf);
+  double most = 0.0;
+  for (int f = 0; f < nf; ++f) {
+    const double* v = q + 6 * f;
+    const std::complex<double> lam(v[0], v[1]), mu(v[2], v[3]);
+    const double k1 = std::abs(v[5] / std::sqrt((lam + 2.0 * mu) / v[4])), k2 = std::abs(v[5] / std::sqrt(mu / v[4]));
+    const double k = std::max(k1, k2);
+    if (!(std::isfinite(k1) && std::isfinite(k2) && k > 0.0 && h->rmax > 0.0)) return 0;
+    // no longer than the mesh: the samples stay at distances that occur
+    hl[f] = std::min(kRadKh / k, h->rmax);
+    most = std::max(most, h->rmax / hl[f]);
+  }
+  if (!(most < kRadMaxN)) return 0;
+  const int n = (int)std::ceil(most) + 1, nfun = dparh ? 10 : 5;
+  const size_t rows = (size_t)nf * n, bc = rows * nfun * kRadC * sizeof(double2),
+               bf = mixed ? rows * 5 * kRadRowF * sizeof(float4) : 0, bs = sizeof(RadF) * nf, bsf = sizeof(RadFF) * nf;
+  int rc;
+  if ((rc = ensure(h->rad, bc + bf + bs + bsf + sizeof(double) * nf))) return rc;
+  char* p = (char*)h->rad.p;
+  double2* c = (double2*)p;
+  float4* cf4 = mixed ? (float4*)(p + bc) : nullptr;
+  RadF* rf = (RadF*)(p + bc + bf);
+  RadFF* rff = (RadFF*)(p + bc + bf + bs);
+  double* dh = (double*)(p + bc + bf + bs + bsf);
+  CK(cudaMemcpyAsync(dh, hl.data(), sizeof(double) * nf, cudaMemcpyHostToDevice, h->st));
+  if (dparh) k_radial<10><<<dim3(n, nf), 32, 0, h->st>>>(dpar, dparh, dh, n, c, cf4, rf, mixed ? rff : nullptr);
+  else k_radial<5><<<dim3(n, nf), 32, 0, h->st>>>(dpar, nullptr, dh, n, c, cf4, rf, mixed ? rff : nullptr);
+  ++g_launches;
+  CK(cudaGetLastError());
+  t->c = c;
+  t->cf4 = cf4;
+  t->f = rf;
+  t->ff_ = rff;
+  t->n = n;
+  t->nfun = nfun;
+  return 0;
+}
+
 template <class POL>
 static int launch_assembly(mfbem_handle* h, const POL& pol, const double* d_nu, int nf, double* A, size_t lda,
                            size_t astride, double* b, size_t bstride, AsmTimes* tm = nullptr,
@@ -1012,8 +1099,11 @@ static int launch_assembly(mfbem_handle* h, const POL& pol, const double* d_nu, 
   if (h->has_bm && !bm) return fail(MFBEM_EARG, "Burton & Miller pair lists not prepared");
   const DMesh& mb = h->mb;
   const DMesh& msv = h->ms[kStatic ? 0 : 1];
-  typedef typename std::conditional<kStatic, PolHbieStatic, PolHbieHarmonic>::type PolH;
-  typedef typename std::conditional<kStatic, HsStatic, HsHarmonic>::type HsK;
+  constexpr bool kRad = std::is_same<POL, PolHarmonicRad>::value;
+  typedef typename std::conditional<kStatic, PolHbieStatic,
+                                    typename std::conditional<kRad, PolHbieHarmonicRad, PolHbieHarmonic>::type>::type PolH;
+  typedef typename std::conditional<kStatic, HsStatic,
+                                    typename std::conditional<kRad, HsHarmonicRad, HsHarmonic>::type>::type HsK;
   PolH phb{};
   HsK hsk{};
   if (hb) {
@@ -1023,9 +1113,14 @@ static int launch_assembly(mfbem_handle* h, const POL& pol, const double* d_nu, 
       hsk.ctes1 = phb.ctes1; hsk.ctes2 = phb.ctes2; hsk.ctes3 = phb.ctes3;
     } else {
       if (!pol.ph) return fail(MFBEM_EARG, "HBIE points need the d* / s* parameters");
-      phb.p = pol.p;
+      if constexpr (kRad) {
+        phb.t = pol.t;
+        hsk.t = pol.t;
+      } else {
+        phb.p = pol.p;
+        hsk.p = pol.p;
+      }
       phb.ph = pol.ph;
-      hsk.p = pol.p;
       hsk.ph = pol.ph;
     }
     phb.cpn = mb.cp_n;
@@ -1043,13 +1138,15 @@ static int launch_assembly(mfbem_handle* h, const POL& pol, const double* d_nu, 
     phs.c = h->hs_c;
     phs.nu = pol.nu;
   }
+  RadTab rt;
+  if constexpr (kRad) rt = pol.t;
   CK(cudaMemsetAsync(h->d_err, 0, sizeof(int), h->st));
   if (tm) cudaEventRecord(tm->ev[0], h->st);
   if (m.nreg > 0) {
-    if constexpr (std::is_same<POL, PolHarmonic>::value) {
+    if constexpr (!kStatic) {
       if (mixed && pf && dsf) {
-        k_mixed<MIX_REG, WPB><<<g, WPB * 32, 0, h->st>>>(m, pf, dsf, nullptr, nf, (double2*)A, lda, astride / 2, b,
-                                                         bstride);
+        k_mixed<MIX_REG, 2, kRad><<<nblk(nw, 2), 64, 0, h->st>>>(m, rt, pf, dsf, nullptr, nf, (double2*)A, lda,
+                                                               astride / 2, b, bstride);
       } else {
         k_reg<POL, WPB><<<g, WPB * 32, 0, h->st>>>(m, pol, nf, A, lda, astride, b, bstride);
       }
@@ -1075,7 +1172,8 @@ static int launch_assembly(mfbem_handle* h, const POL& pol, const double* d_nu, 
   if (tm) cudaEventRecord(tm->ev[1], h->st);
   if (m.nadp > 0) {
     if (mixed && lgf)
-      k_mixed<MIX_ADP, WPB><<<g, WPB * 32, 0, h->st>>>(m, pf, dsf, lgf, nf, (double2*)A, lda, astride / 2, b, bstride);
+      k_mixed<MIX_ADP, 2, kRad><<<nblk(nw, 2), 64, 0, h->st>>>(m, rt, pf, dsf, lgf, nf, (double2*)A, lda, astride / 2, b,
+                                                             bstride);
     else k_adp<POL, WPB><<<g, WPB * 32, 0, h->st>>>(m, pol, nf, A, lda, astride, b, bstride);
     ++g_launches;
   }
@@ -1097,7 +1195,8 @@ static int launch_assembly(mfbem_handle* h, const POL& pol, const double* d_nu, 
   // the singular kernels keep two combo sets per point: 2 warps per block
   if (m.nsing > 0) {
     if (mixed && sgf)
-      k_mixed<MIX_SING, 2><<<nblk(nw, 2), 64, 0, h->st>>>(m, pf, dsf, sgf, nf, (double2*)A, lda, astride / 2, b, bstride);
+      k_mixed<MIX_SING, 2, kRad><<<nblk(nw, 2), 64, 0, h->st>>>(m, rt, pf, dsf, sgf, nf, (double2*)A, lda, astride / 2, b,
+                                                                bstride);
     else k_sing<POL, 2><<<nblk(nw, 2), 64, 0, h->st>>>(m, pol, nf, A, lda, astride, b, bstride);
     ++g_launches;
   }
@@ -1143,9 +1242,10 @@ static int copy_mat(void* dst, size_t dpitch, const void* src, size_t spitch, si
   return 0;
 }
 
-template <bool CPLX>
-static int assemble_common(mfbem_handle* h, const void* polp, const double* nu_host, double* A, int lda, double* b,
+template <class POL>
+static int assemble_common(mfbem_handle* h, const POL& pol, const double* nu_host, double* A, int lda, double* b,
                            int flags) {
+  constexpr bool CPLX = !std::is_same<POL, PolStatic>::value;
   const int n = h->ndof;
   if (lda < n) return fail(MFBEM_EARG, "lda < n_dof");
   if (int rd = check_dev(h)) return rd;
@@ -1184,8 +1284,7 @@ static int assemble_common(mfbem_handle* h, const void* polp, const double* nu_h
   cudaEventRecord(e0, h->st);
   AsmTimes tm;
   long long l0 = g_launches;
-  if (CPLX) rc = launch_assembly(h, *(const PolHarmonic*)polp, (const double*)h->nu.p, 1, dA, dlda, 0, db, 0, &tm);
-  else rc = launch_assembly(h, *(const PolStatic*)polp, (const double*)h->nu.p, 1, dA, dlda, 0, db, 0, &tm);
+  rc = launch_assembly(h, pol, (const double*)h->nu.p, 1, dA, dlda, 0, db, 0, &tm);
   cudaEventRecord(e1, h->st);
   if (rc) return rc;
   if (!dev) {
@@ -1215,7 +1314,7 @@ extern "C" int mfbem_assemble_staela(mfbem_handle* h, double mu, double nu, doub
   pol.nu = nu;
   pol.mu = mu;
   double nuv[2] = {nu, 0.0};
-  return assemble_common<false>(h, &pol, nuv, A, lda, b, flags);
+  return assemble_common(h, pol, nuv, A, lda, b, flags);
 }
 
 // d* / s* parameters per frequency (HarParH) from q [nf][6] (lambda, mu, rho,
@@ -1242,10 +1341,14 @@ extern "C" int mfbem_assemble_harela(mfbem_handle* h, const double lambda[2], co
   CK(cudaMemcpyAsync(dq, q, sizeof(q), cudaMemcpyHostToDevice, h->st));
   k_harpar<<<1, 32, 0, h->st>>>(dq, 1, (HarParD*)h->par.p, zexp_thresholds()); ++g_launches;
   if ((rc = bm_prepare(h, 1))) return rc;
+  PolHarmonicRad pr;
+  pr.p = (const HarParD*)h->par.p;
+  if ((rc = hbie_params(h, dq, 1, &pr.ph)) || (rc = radial_prepare(h, q, 1, pr.p, pr.ph, false, &pr.t))) return rc;
+  if (pr.t.n > 0) return assemble_common(h, pr, nu, A, lda, b, flags);
   PolHarmonic pol;
-  pol.p = (const HarParD*)h->par.p;
-  if ((rc = hbie_params(h, dq, 1, &pol.ph))) return rc;
-  return assemble_common<true>(h, &pol, nu, A, lda, b, flags);
+  pol.p = pr.p;
+  pol.ph = pr.ph;
+  return assemble_common(h, pol, nu, A, lda, b, flags);
 }
 
 // ---------------------------------------------------------------------------
@@ -1519,6 +1622,83 @@ extern "C" int mfbem_internal_zexp(int32_t n, const double* z, double* e64, doub
   cudaFree(d2.p);
   if (e != cudaSuccess) return fail(MFBEM_ECUDA, std::string("zexp check: ") + cudaGetErrorString(e));
   return 0;
+}
+
+// ---------------------------------------------------------------------------
+// Test hook: the radial functions of one material and frequency (q: lambda,
+// mu, rho, omega) at n distances r <= rmax: psi, chi (times cte_u), TT1..TT3
+// (cte_t) and S1..S5 (cte_s), complete, from the table in binary64 (tab
+// [n][10][2]), from the double-float table (tabf [n][5][2]) and by the direct
+// evaluation (dir [n][10][2]).
+// ---------------------------------------------------------------------------
+__global__ void k_radial_check(RadTab t, const HarParD* p, const HarParH* ph, const double* rr, int n, double* tab,
+                               double* tabf, double* dir) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double r = rr[i], d1 = 1.0 / r;
+  double x;
+  const RadF& q = t.f[0];
+  const double2* w = rad_row(t, 0, q, r, x);
+  cd X[10], Y[10];
+  X[0] = rad_eval(w, x) + q.s[0] * d1;
+  X[1] = rad_eval(w + kRadC, x) + q.s[1] * d1;
+  HbieCoefH c;
+  hbie_coef_rad(t, 0, r, d1, true, c);
+  X[2] = c.TT1; X[3] = c.TT2; X[4] = c.TT3; X[5] = c.S1; X[6] = c.S2; X[7] = c.S3; X[8] = c.S4; X[9] = c.S5;
+  double d1r1, d1r2;
+  harela_coeffs(*p, r, Y[0], Y[1], Y[2], Y[3], Y[4], d1r1, d1r2, true);
+  hbie_coef_h(*p, *ph, r, true, c);
+  Y[5] = c.S1; Y[6] = c.S2; Y[7] = c.S3; Y[8] = c.S4; Y[9] = c.S5;
+  for (int k = 0; k < 10; ++k) {
+    Y[k] = (k < 2 ? p->cte_u : (k < 5 ? p->cte_t : ph->cte_s)) * Y[k];
+    tab[20 * i + 2 * k] = X[k].re;
+    tab[20 * i + 2 * k + 1] = X[k].im;
+    dir[20 * i + 2 * k] = Y[k].re;
+    dir[20 * i + 2 * k + 1] = Y[k].im;
+  }
+  c2 F[5];
+  const ff rf = ff_from(r), df = ff_rcp(rf);
+  rad_eval_ff<false>(t, 0, t.ff_[0], rf, df, ff_mul(df, df), F);
+  for (int k = 0; k < 5; ++k) {
+    const cf v = c2_to(F[k]);
+    tabf[10 * i + 2 * k] = ff_to(v.re);
+    tabf[10 * i + 2 * k + 1] = ff_to(v.im);
+  }
+}
+extern "C" int mfbem_internal_radial(const double* q, double rmax, int32_t n, const double* r, double* tab,
+                                     double* tabf, double* dir) {
+  g_err.clear();
+  if (!q || !(rmax > 0.0) || n <= 0 || !r || !tab || !tabf || !dir) return fail(MFBEM_EARG, "invalid argument");
+  int rc = init_tables();
+  if (rc) return rc;
+  mfbem_handle h;  // the default stream; only its table buffer and extent are used
+  h.rmax = rmax;
+  const size_t nb[6] = {sizeof(HarParD), sizeof(HarParH), 6 * sizeof(double), 8 * (size_t)n, 160 * (size_t)n, 80 * (size_t)n};
+  DevBuf d[7];
+  for (int i = 0; i < 7; ++i)
+    if ((rc = ensure(d[i], i < 6 ? nb[i] : nb[4]))) return rc;
+  HarParD* p = (HarParD*)d[0].p;
+  HarParH* ph = (HarParH*)d[1].p;
+  auto run = [&]() -> int {
+    CK(cudaMemcpy(d[2].p, q, nb[2], cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(d[3].p, r, nb[3], cudaMemcpyHostToDevice));
+    k_harpar<<<1, 32>>>((const double*)d[2].p, 1, p, zexp_thresholds()); ++g_launches;
+    k_harparh<<<1, 32>>>((const double*)d[2].p, 1, ph); ++g_launches;
+    RadTab t;
+    if (int e = radial_prepare(&h, q, 1, p, ph, true, &t)) return e;
+    if (t.n == 0) return fail(MFBEM_EARG, "no table for these parameters");
+    k_radial_check<<<nblk(n, 64), 64>>>(t, p, ph, (const double*)d[3].p, n, (double*)d[4].p, (double*)d[5].p,
+                                        (double*)d[6].p); ++g_launches;
+    CK(cudaGetLastError());
+    CK(cudaMemcpy(tab, d[4].p, nb[4], cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(tabf, d[5].p, nb[5], cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(dir, d[6].p, nb[4], cudaMemcpyDeviceToHost));
+    return 0;
+  };
+  rc = run();
+  for (auto& b : d) pool_give(b.p, b.bytes, b.dev);
+  pool_give(h.rad.p, h.rad.bytes, h.rad.dev);
+  return rc;
 }
 
 #include "mfbem_solve.cuh"

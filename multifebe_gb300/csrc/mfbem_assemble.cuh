@@ -18,6 +18,7 @@
 #include "dev_point.cuh"
 #include "mfbem_dev.h"
 #include "dev_df64.cuh"
+#include "dev_radial.cuh"
 
 namespace mfb {
 
@@ -45,6 +46,7 @@ __device__ __forceinline__ void addA(double* A, size_t idx, cd v) {
 struct PolStatic {
   typedef double T;
   static constexpr int NG = 6;  // independent components of g per node (u* symmetric)
+  static constexpr bool kScaled = false;  // point() leaves cte_u / cte_t to the flush
   StaelaP k;
   double nu = 0.0, mu = 0.0;
   __device__ T cte_t(int) const { return k.ctet1; }
@@ -72,6 +74,7 @@ struct HarParH;
 struct PolHarmonic {
   typedef cd T;
   static constexpr int NG = 6;
+  static constexpr bool kScaled = false;
   const HarParD* p;  // one parameter block per frequency
   const HarParH* ph = nullptr;  // d* / s* parameters per frequency (HBIE points only)
   __device__ T cte_t(int f) const { return p[f].cte_t; }
@@ -105,6 +108,66 @@ struct PolHarmonic {
       }
   }
 };
+// The same kernels with the radial functions read from the call's table
+// (dev_radial.cuh); cte_u and cte_t are in the table. t*(l, k) is formed as
+// dr_l P_k + n_l Q_k (+ TT2 dr/dn on the diagonal) with P_k = TT1 dr/dn dr_k +
+// TT3 n_k, Q_k = TT2 dr_k: 60 instead of 96 real multiply-adds. k_reg of the
+// 8x8 cube is bound by the FP64 pipe (two lanes per cycle and SM): about 1260
+// FP64 operations a point with E_n evaluated directly, 500 here, 240 of them
+// the weighting by the eight shape functions. Four systems of the cube: regular
+// pairs 51.7 -> 28.5 ms, singular pairs 20.9 -> 12.1 ms.
+struct PolHarmonicRad {
+  typedef cd T;
+  static constexpr int NG = 6;
+  static constexpr bool kScaled = true;
+  RadTab t;
+  const HarParD* p;
+  const HarParH* ph = nullptr;
+  __device__ T cte_t(int) const { return mk(1.0); }
+  __device__ T cte_u(int) const { return mk(1.0); }
+  __device__ T cpv(int f) const { return t.f[f].s[3]; }
+  template <bool SING>
+  __device__ __forceinline__ void eval(int f, const double rv[3], const double n[3], T fu[9], T ft[9], T* fc) const {
+    const RadF& q = t.f[f];
+    const double r2 = rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2];
+    double d1 = rsqrt(r2), r = r2 * d1;
+    r = fma(0.5 * d1, fma(-r, r, r2), r);
+    d1 = fma(d1, fma(-r, d1, 1.0), d1);
+    const double d2 = d1 * d1;
+    double x;
+    const double2* c = rad_row(t, f, q, r, x);
+    const cd psi = rad_eval(c, x) + q.s[0] * d1, chi = rad_eval(c + kRadC, x) + q.s[1] * d1;
+    const cd T1 = rad_eval(c + 2 * kRadC, x) + q.s[2] * d2;
+    cd T2 = rad_eval(c + 3 * kRadC, x), T3 = rad_eval(c + 4 * kRadC, x), A2;
+    const cd c2 = q.s[3] * d2;
+    A2 = T2 + c2;
+    if (!SING) {
+      T2 = A2;
+      T3 = T3 + q.s[4] * d2;
+    }
+    const double dr[3] = {rv[0] * d1, rv[1] * d1, rv[2] * d1};
+    const double drdn = dr[0] * n[0] + dr[1] * n[1] + dr[2] * n[2];
+    const cd a = T1 * drdn, d0 = A2 * drdn;
+#pragma unroll
+    for (int ik = 0; ik < 3; ++ik) {
+      const cd P = a * dr[ik] + T3 * n[ik], Q = T2 * dr[ik], X = -(chi * dr[ik]);
+#pragma unroll
+      for (int il = 0; il < 3; ++il) {
+        cd v = P * dr[il] + Q * n[il];
+        if (il == ik) v = v + d0;
+        ft[3 * il + ik] = v;
+        fu[3 * il + ik] = il == ik ? X * dr[il] + psi : X * dr[il];
+        if (SING) fc[3 * il + ik] = il == ik ? mk(0.0) : c2 * (n[il] * dr[ik] - n[ik] * dr[il]);
+      }
+    }
+  }
+  __device__ void point(int f, int, const double rv[3], const double n[3], T fu[9], T ft[9]) const {
+    eval<false>(f, rv, n, fu, ft, nullptr);
+  }
+  __device__ void point_sing(int f, int, const double rv[3], const double n[3], T fu[9], T ft[9], T fc[9]) const {
+    eval<true>(f, rv, n, fu, ft, fc);
+  }
+};
 
 // Half-space complementary kernel (static, traction-free surface x3 = xp):
 // the pair lists of these policies are classified on the images of the
@@ -113,6 +176,7 @@ struct PolHarmonic {
 struct PolHsc {
   typedef double T;
   static constexpr int NG = 9;
+  static constexpr bool kScaled = false;
   StaelaP k;
   const double* c;  // [ncp]
   double xp, nu;
@@ -132,6 +196,7 @@ struct PolHsc {
 struct PolHscSing {
   typedef double T;
   static constexpr int NG = 9;
+  static constexpr bool kScaled = false;
   StaelaP k;
   const double* c;
   double nu;
@@ -188,7 +253,7 @@ __device__ __forceinline__ void flush_pair(const DMesh& m, const POL& pol, int f
     if (o < 72) {
       int kn = o / 9, il = (o % 9) / 3, ik = o % 3;
       if (hli_phi) v = v + hli_phi[9 + kn] * pol.cpv(f) * hli_phi[3 * il + ik];
-      v = v * pol.cte_t(f);
+      if constexpr (!POL::kScaled) v = v * pol.cte_t(f);
       if (rev) v = -v;
       const size_t row = dn_row(m, dn, il);
       for (int fc = 0; fc <= ck; ++fc, v = -v) {
@@ -199,7 +264,7 @@ __device__ __forceinline__ void flush_pair(const DMesh& m, const POL& pol, int f
     } else {
       int q = o - 72, kn = q / NG, sidx = q % NG;
       int il = NG == 6 ? sym_il(sidx) : sidx / 3, ik = NG == 6 ? sym_ik(sidx) : sidx % 3;
-      v = v * pol.cte_u(f);
+      if constexpr (!POL::kScaled) v = v * pol.cte_u(f);
       for (int t = 0; t < (il == ik || NG == 9 ? 1 : 2); ++t) {
         int r_ = t ? ik : il, c_ = t ? il : ik;
         const size_t row = dn_row(m, dn, r_);
@@ -819,69 +884,104 @@ __device__ __forceinline__ void harela_point_ff(const HarParF& q, const ff rv[3]
   }
 }
 
-template <bool SING> struct alignas(16) ComboF;
-template <> struct alignas(16) ComboF<false> {
-  cf fu[6], ft[9];
-  ff w[8];
-  int pair;
+// Quadrature-point record of the mixed kernels in shared memory: the nine t*
+// components, the six of u* (16 bytes each: re.hi, im.hi, re.lo, im.lo), for
+// singular pairs the three of the antisymmetric CPV integrand ((0,1), (0,2),
+// (1,2)), then the eight weights phi J w (hi, hi, lo, lo) and for singular
+// pairs (phi - phi_i) J w. The record is an odd number of 16-byte units long,
+// so the 128-bit stores of 32 lanes' records meet no bank conflict.
+template <bool SING> struct PtRec;
+template <> struct PtRec<false> {
+  static constexpr int kFc = 240, kW = 240, kWd = 0, kSize = 368;
 };
-template <> struct alignas(16) ComboF<true> {
-  cf fu[6], ft[9], fc[9];
-  ff w[8], wd[8];
-  int pair;
+template <> struct PtRec<true> {
+  static constexpr int kFc = 240, kW = 288, kWd = 416, kSize = 560;
 };
-
-__device__ __forceinline__ cf cf_sub(cf a, cf b) { return cf_add(a, cf_neg(b)); }
-__device__ __forceinline__ cf cval_f(const ff* dcv_f, int dof) { return cf{dcv_f[2 * (size_t)dof], dcv_f[2 * (size_t)dof + 1]}; }
-// df64 complex entry {re.hi, re.lo, im.hi, im.lo} += v
-// A(idx) += v: the pair's double-float sum rounded once to binary64
-__device__ __forceinline__ void addAc(double2* A, size_t idx, cf v) {
-  double2 a = A[idx];
-  a.x += ff_to(v.re);
-  a.y += ff_to(v.im);
-  A[idx] = a;
+__device__ __forceinline__ void rec_put(char* r, int comp, c2 v) {
+  *reinterpret_cast<ulonglong2*>(r + 16 * comp) = make_ulonglong2(v.h, v.l);
 }
-__device__ __forceinline__ void add3(cf bc[3], int i, cf v) {
-  if (i == 0) bc[0] = cf_add(bc[0], v);
-  else if (i == 1) bc[1] = cf_add(bc[1], v);
-  else bc[2] = cf_add(bc[2], v);
+__device__ __forceinline__ c2 rec_get(const char* r) {
+  const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(r);
+  return c2{v.x, v.y};
 }
 
-// scale, reverse and scatter this lane's outputs of one pair (the scatter of
-// flush_pair in double-float; rows 3 dn + il: never used on a region with
-// crack-like boundaries): A entries added to the binary64 system,
-// prescribed values into the lane's b partial sums bc. hp (singular pairs only): static
-// line integrals hli[9] and phi_i[8] of the pair; their CPV part
-// T2[0] hli(il,ik) phi_i(kn) is added to the h outputs.
-__device__ __forceinline__ void flush_pair_ff(const DMesh& m, const HarParF& q, const ff* dcv_f, int dn, int e,
-                                              const cf acc[kAcc], double2* Ac, size_t lda, cf bc[3], const ff* hp) {
-  const int lane = threadIdx.x & 31;
-  const bool rev = (m.rev[e] & 1) != 0;
-#pragma unroll 1
-  for (int j = 0; j < kAcc; ++j) {
-    const int o = lane + 32 * j;
-    if (o >= kOut) break;
-    cf aj = cf_norm(sel4(acc[0], acc[1], acc[2], acc[3], j));
-    if (o < 72) {
-      const int kn = o / 9, il = (o % 9) / 3, ik = o % 3;
-      if (hp) aj = cf_add(aj, cf_scale(q.c0[3], ff_mul(hp[9 + kn], hp[3 * il + ik])));
-      cf v = cf_mul(aj, q.cte_t);
-      if (rev) v = cf_neg(v);
-      const int dof = m.edof[8 * e + kn] + ik;
-      if (m.dct[dof] == 1) addAc(Ac, (size_t)dof * lda + 3 * (size_t)dn + il, v);
-      else add3(bc, il, cf_neg(cf_mul(v, cval_f(dcv_f, dof))));
-    } else {
-      const int qq = o - 72, kn = qq / 6, sidx = qq % 6, il = sym_il(sidx), ik = sym_ik(sidx);
-      const cf v = cf_mul(aj, q.cte_u);
-      for (int t = 0; t < (il == ik ? 1 : 2); ++t) {
-        const int r_ = t ? ik : il, c_ = t ? il : ik;
-        const int dof = m.edof[8 * e + kn] + c_;
-        if (m.dct[dof] == 0) addAc(Ac, (size_t)dof * lda + 3 * (size_t)dn + r_, cf_neg(v));
-        else add3(bc, r_, cf_mul(v, cval_f(dcv_f, dof)));
+// X_t(r) of one frequency from its double-float table row, entire part plus
+// singular part (SING: without the 1/r^2 parts of TT2, TT3): the terms up to
+// x^kRadDF by compensated accumulation, the rest -- at most 1e-8 of X on an
+// interval with |k| h / 2 = 1/16 -- in FP32 (6e-16 of X).
+template <bool SING>
+__device__ __forceinline__ void rad_eval_ff(const RadTab& tb, int f, const RadFF& q, ff r, ff d1r1, ff d1r2, c2 X[5]) {
+  const ff s = ff_mul(r, q.inv2h);
+  const int i = min(max((int)(0.5f * s.hi), 0), tb.n - 1);
+  const ff x = ff_add(s, ff{-(float)(2 * i + 1), 0.0f});
+  const ff x2 = ff_mul(x, x), x3 = ff_mul(x2, x), x4 = ff_mul(x2, x2);
+  const u64f2 x5 = f2_dup(__fmul_rn(x4.hi, x.hi)), x1 = f2_dup(x.hi);
+  const float4* c = tb.cf4 + ((size_t)f * tb.n + i) * (5 * kRadRowF);
+  const r2 xp[4] = {r2_from(x), r2_from(x2), r2_from(x3), r2_from(x4)};
+  const r2 d1 = r2_from(d1r1), d2 = r2_from(d1r2);
+#pragma unroll
+  for (int t = 0; t < 5; ++t, c += kRadRowF) {
+    c2 a = c2_from(__ldg(c));
+#pragma unroll
+    for (int m = 1; m <= kRadDF; ++m) c2_mac(a, c2_from(__ldg(c + m)), xp[m - 1]);
+    const c2 v = c2_from(__ldg(c + kRadDF + 1)), u = c2_from(__ldg(c + kRadDF + 2));
+    a.l = f2_fma(x5, f2_fma(x1, f2_fma(x1, u.h, v.l), v.h), a.l);
+    if (!SING || t < 3) c2_mac(a, c2_from(q.s[t]), t < 2 ? d1 : d2);
+    X[t] = c2_norm(a);
+  }
+}
+// u*, t* (and the CPV integrand of a singular pair) at one point with the
+// radial functions from the table; constants included, t* as in PolHarmonicRad
+template <bool SING>
+__device__ __forceinline__ void harela_point_rad_ff(const RadTab& tb, int f, const RadFF& q, const ff rv[3],
+                                                    const ff n[3], char* rec) {
+  const ff rq = ff_add(ff_add(ff_mul(rv[0], rv[0]), ff_mul(rv[1], rv[1])), ff_mul(rv[2], rv[2]));
+  const ff r = ff_sqrt(rq);
+  const ff d1r1 = ff_rcp(r), d1r2 = ff_mul(d1r1, d1r1);
+  c2 X[5];
+  rad_eval_ff<SING>(tb, f, q, r, d1r1, d1r2, X);
+  const ff dr[3] = {ff_mul(rv[0], d1r1), ff_mul(rv[1], d1r1), ff_mul(rv[2], d1r1)};
+  const ff drdn = ff_add(ff_add(ff_mul(dr[0], n[0]), ff_mul(dr[1], n[1])), ff_mul(dr[2], n[2]));
+  const r2 dn2 = r2_from(drdn);
+  const r2 drp[3] = {r2_from(dr[0]), r2_from(dr[1]), r2_from(dr[2])};
+  const r2 np[3] = {r2_from(n[0]), r2_from(n[1]), r2_from(n[2])};
+  const c2 a = c2_scale(X[2], dn2);
+  c2 d0;
+  if constexpr (SING) {
+    const c2 cc = c2_scale(c2_from(q.s[3]), r2_from(d1r2));
+    d0 = c2_scale(c2_add(X[3], cc), dn2);
+    const ff f01 = ff_sub(ff_mul(n[0], dr[1]), ff_mul(n[1], dr[0]));
+    const ff f02 = ff_sub(ff_mul(n[0], dr[2]), ff_mul(n[2], dr[0]));
+    const ff f12 = ff_sub(ff_mul(n[1], dr[2]), ff_mul(n[2], dr[1]));
+    rec_put(rec + PtRec<SING>::kFc, 0, c2_scale(cc, r2_from(f01)));
+    rec_put(rec + PtRec<SING>::kFc, 1, c2_scale(cc, r2_from(f02)));
+    rec_put(rec + PtRec<SING>::kFc, 2, c2_scale(cc, r2_from(f12)));
+  } else {
+    d0 = c2_scale(X[3], dn2);
+  }
+#pragma unroll
+  for (int ik = 0; ik < 3; ++ik) {
+    c2 P = c2_zero();
+    c2_mac(P, a, drp[ik]);
+    c2_mac(P, X[4], np[ik]);
+    P = c2_norm(P);
+    const c2 Q = c2_scale(X[3], drp[ik]), Xc = c2_neg(c2_scale(X[1], drp[ik]));
+#pragma unroll
+    for (int il = 0; il < 3; ++il) {
+      c2 v = il == ik ? d0 : c2_zero();
+      c2_mac(v, P, drp[il]);
+      c2_mac(v, Q, np[il]);
+      rec_put(rec, 3 * il + ik, c2_norm(v));
+      if (ik >= il) {
+        c2 u = c2_scale(Xc, drp[il]);
+        if (il == ik) u = c2_add(u, X[0]);
+        rec_put(rec, 9 + ik + (il == 1 ? 2 : (il == 2 ? 3 : 0)), u);
       }
     }
   }
 }
+__device__ __forceinline__ cf cf_sub(cf a, cf b) { return cf_add(a, cf_neg(b)); }
+__device__ __forceinline__ cf cval_f(const ff* dcv_f, int dof) { return cf{dcv_f[2 * (size_t)dof], dcv_f[2 * (size_t)dof + 1]}; }
 
 // Singular (polar) points: the regular parts of u*, t* and the CPV integrand
 // (PolHarmonic::point_sing) in double-float. TT2, TT3 without their 1/r^2
@@ -937,6 +1037,101 @@ __device__ __forceinline__ void harela_point_sing_ff(const HarParF& q, const ff 
   }
 }
 
+// the direct evaluation into a record: constants multiplied in
+template <bool SING>
+__device__ __forceinline__ void harela_point_direct_ff(const HarParF& q, const ff rv[3], const ff n[3], char* rec) {
+  cf fu[6], ft[9];
+  if constexpr (SING) {
+    cf fc[9];
+    harela_point_sing_ff(q, rv, n, fu, ft, fc);
+    rec_put(rec + PtRec<SING>::kFc, 0, c2_from(cf_mul(fc[1], q.cte_t)));
+    rec_put(rec + PtRec<SING>::kFc, 1, c2_from(cf_mul(fc[2], q.cte_t)));
+    rec_put(rec + PtRec<SING>::kFc, 2, c2_from(cf_mul(fc[5], q.cte_t)));
+  } else {
+    harela_point_ff(q, rv, n, fu, ft);
+  }
+#pragma unroll 1
+  for (int c = 0; c < 15; ++c) rec_put(rec, c, c2_from(c < 9 ? cf_mul(ft[c], q.cte_t) : cf_mul(fu[c - 9], q.cte_u)));
+}
+
+// One pair's sums into the system: normalise, add a singular pair's CPV sums
+// (acd: component lane / 8, node lane % 8) and line-integral part cpv hli(il,ik)
+// phi_i(kn) (hp: hli[9], phi_i[8]), reverse, and scatter as flush_pair does
+// (rows 3 dn + il: never used on a region with crack-like boundaries). A's
+// entry (row il, column direction ik of node kn) is h where the traction is
+// known there and -g where the displacement is (bit 3 kn + ik of the element's
+// mask), so every one of the 24 x 3 entries gets one value: they are staged
+// and added to A one real per lane and round. Products with the prescribed
+// values (none where the value is zero) go to bc0 / bc1.
+template <bool SG>
+__device__ __forceinline__ void flush_pair_ff(const DMesh& m, const cf& cpv, const ff* dcv_f, int e, c2 acc[4], c2 acd,
+                                              double* Arow, size_t lda, int comp, int half, int cil, int cik, cf& bc0,
+                                              cf& bc1, float4* stage, const ff* hp) {
+  const int lane = threadIdx.x & 31;
+  const int mask = m.emask[e], nz = m.enz[e];
+  const int* ed = m.edof + 8 * (size_t)e;
+  const bool isg = comp >= 9, live = (lane & 15) < 15;
+  if constexpr (SG) {
+    const c2 dn = c2_norm(acd);
+    const int src = 8 * max(cil + cik - 1, 0) + 4 * half;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      c2 d;
+      d.h = __shfl_sync(0xffffffffu, dn.h, min(src + k, 31));
+      d.l = __shfl_sync(0xffffffffu, dn.l, min(src + k, 31));
+      acc[k] = c2_norm(acc[k]);
+      if (!isg) {
+        if (cil != cik) acc[k] = c2_add(acc[k], cil < cik ? d : c2_neg(d));
+        acc[k] = c2_add(acc[k], c2_scale(c2_from(cpv), r2_from(ff_mul(hp[9 + 4 * half + k], hp[3 * cil + cik]))));
+      }
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) acc[k] = c2_norm(acc[k]);
+  }
+  if (!isg && (mask >> 24)) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) acc[k] = c2_neg(acc[k]);
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int kn = 4 * half + k, o = 9 * kn;
+    const bool t1 = (mask >> (3 * kn + cik)) & 1, t2 = (mask >> (3 * kn + cil)) & 1;
+    c2 v = acc[k];
+    if (isg) v = c2_neg(v);
+    if (live) {
+      if (isg != t1) *reinterpret_cast<ulonglong2*>(stage + o + 3 * cik + cil) = make_ulonglong2(v.h, v.l);
+      if (isg && !t2 && cil != cik) *reinterpret_cast<ulonglong2*>(stage + o + 3 * cil + cik) = make_ulonglong2(v.h, v.l);
+    }
+  }
+  if (nz) {
+#pragma unroll 1
+    for (int k = 0; k < 4; ++k) {
+      const int kn = 4 * half + k;
+      const int b1 = 3 * kn + cik, b2 = 3 * kn + cil;
+      const cf v = c2_to(k == 0 ? acc[0] : (k == 1 ? acc[1] : (k == 2 ? acc[2] : acc[3])));
+      if (((nz >> b1) & 1) && isg == (((mask >> b1) & 1) != 0)) {
+        const cf p = cf_mul(v, cval_f(dcv_f, ed[kn] + cik));
+        bc0 = cf_add(bc0, isg ? p : cf_neg(p));
+      }
+      if (isg && cil != cik && ((nz >> b2) & 1) && ((mask >> b2) & 1))
+        bc1 = cf_add(bc1, cf_mul(v, cval_f(dcv_f, ed[kn] + cil)));
+    }
+  }
+  __syncwarp();
+  const float* sf = reinterpret_cast<const float*>(stage);
+#pragma unroll
+  for (int j = 0; j < 5; ++j) {
+    const int q = lane + 32 * j;
+    if (q < 144) {
+      const int o = q >> 1, part = q & 1, col = o / 3, il = o - 3 * col, kn = col / 3, ik = col - 3 * kn;
+      double* p = Arow + 2 * ((size_t)(ed[kn] + ik) * lda + il) + part;
+      *p += (double)sf[4 * o + part] + (double)sf[4 * o + 2 + part];
+    }
+  }
+  __syncwarp();
+}
+
 // Pair lists walked by the mixed kernels: regular pairs (precalculated element
 // datasets), adaptive pairs (subdivision leaves) and singular pairs (polar points).
 enum MixKind { MIX_REG = 0, MIX_ADP = 1, MIX_SING = 2 };
@@ -945,39 +1140,55 @@ enum MixKind { MIX_REG = 0, MIX_ADP = 1, MIX_SING = 2 };
 // frequency), the two-phase scheme of k_reg, all arithmetic after x - x_i in
 // double-float; each pair's sums are rounded once to binary64 and added to
 // the system Ac (complex entries, stride astride_e per frequency; the warp
-// owns its node's rows, so no other warp writes them). dsf: df64 copies of phi*J*w [ne][ptot][8], unit
-// normals [ne][ptot][3] and prescribed values [ndof][2]; gf: df64 copy of the
-// frequency-independent point geometry (leaf_geo for adaptive, sing_geo for
-// singular pairs), component-major.
-template <int KIND, int WPB>
-__global__ void __launch_bounds__(WPB * 32, 4) k_mixed(DMesh m, const HarParF* pf, const ff* dsf, const ff* gf, int nf,
-                                                       double2* Ac, size_t lda, size_t astride_e, double* b,
-                                                       size_t bstride) {
+// owns its node's rows, so no other warp writes them). dsf: df64 copies of
+// phi*J*w [ne][ptot][8], unit normals [ne][ptot][3] and prescribed values
+// [ndof][2]; gf: df64 copy of the frequency-independent point geometry
+// (leaf_geo for adaptive, sing_geo for singular pairs), component-major. TAB:
+// radial functions from the call's table (dev_radial.cuh), else E_n directly.
+//
+// Batches: 32 points of the collocation point's list at a time. The pairs (or
+// leaves) of a batch come from one coalesced read of the next 32 list offsets
+// and a warp-wide OR of their start bits: no search per point, and phase 2 runs
+// over whole segments of a pair. Phase 2: lane = 16 * half + component, the 15
+// components' sums over the nodes 4 half .. 4 half + 3 in four accumulators, so
+// a point costs a lane one component and four weight loads for four
+// multiply-adds (the earlier layout, outputs dealt out 32 at a time, loaded
+// a component and a weight for each). Flush: the sums go through shared memory
+// so that the 144 reals of A's 24 columns x 3 rows, whose binary64 conversions
+// and additions run at two lanes per cycle, fill the warp.
+// Bound by issue slots and latency (45 % of slots, FP64 pipe 34 %, FP32 pipe
+// 24 % at 2 frequencies of the 8x8 cube; 174 warp instructions a regular
+// point). Against direct E_n evaluation with scalar double-float and outputs
+// dealt out 32 at a time (497 instructions a point), the 20-frequency sweep of
+// the cube: regular pairs 73 -> 35 ms, singular pairs 26 -> 11.3 ms.
+template <int KIND, int WPB, bool TAB>
+__global__ void __launch_bounds__(WPB * 32, KIND == MIX_SING ? 5 : 8) k_mixed(DMesh m, RadTab rt, const HarParF* pf, const ff* dsf,
+                                                       const ff* gf, int nf, double2* Ac, size_t lda, size_t astride_e,
+                                                       double* b, size_t bstride) {
   constexpr bool SG = KIND == MIX_SING;
-  __shared__ ComboF<SG> sm[WPB][32];
+  typedef PtRec<SG> R;
+  __shared__ __align__(16) char sm[WPB][32 * R::kSize];
+  __shared__ float4 stg[WPB][72];
   __shared__ ff hps[WPB][SG ? 17 : 1];
   const int lane = threadIdx.x & 31, w = threadIdx.x / 32;
   const long long gw = blockIdx.x * (long long)WPB + w;
   if (gw >= (long long)m.ndn * nf) return;
   const int dn = (int)(gw % m.ndn), f = (int)(gw / m.ndn);
-  ComboF<SG>* S = sm[w];
-  const HarParF& Q = pf[f];
+  char* S = sm[w];
+  char* my = S + lane * R::kSize;
   const ff* pphi_f = dsf;
   const ff* pn_f = dsf + 8LL * m.ne * m.ptot;
   const ff* dcv_f = pn_f + 3LL * m.ne * m.ptot;
-  double2* Acf = Ac + astride_e * f;
-  cf bc[3] = {cf_zero(), cf_zero(), cf_zero()};
-  // this lane's output slots: byte offset of its kernel value in the point's
-  // ComboF (t* or u* component) << 4 | element node; -1 past the 120 outputs.
-  // One path for both kinds, so no slot diverges between t* and u* lanes.
-  int slot[kAcc];
-#pragma unroll
-  for (int j = 0; j < kAcc; ++j) {
-    const int o = lane + 32 * j;
-    if (o < 72) slot[j] = (int)((offsetof(ComboF<SG>, ft) + sizeof(cf) * (o % 9)) << 4) | (o / 9);
-    else if (o < kOut) slot[j] = (int)((offsetof(ComboF<SG>, fu) + sizeof(cf) * ((o - 72) % 6)) << 4) | ((o - 72) / 6);
-    else slot[j] = -1;
-  }
+  double* Arow = reinterpret_cast<double*>(Ac + astride_e * f + 3 * (size_t)dn);
+  // phase 2 layout: component comp (t* 0..8, u* 9..14; the 16th lane of a half
+  // repeats the 15th) and nodes 4 half .. 4 half + 3
+  const int half = lane >> 4, comp = min(lane & 15, 14);
+  const int dcomp = min(lane >> 3, 2);  // singular: CPV component and node lane & 7
+  // (row, column direction) of this lane's component for the b sums
+  const int cil = comp < 9 ? comp / 3 : sym_il(comp - 9), cik = comp < 9 ? comp % 3 : sym_ik(comp - 9);
+  cf cpv = cf_zero();
+  if constexpr (SG) cpv = TAB ? rt.ff_[f].s[3] : cf_mul(pf[f].c0[3], pf[f].cte_t);
+  cf bc0 = cf_zero(), bc1 = cf_zero();  // rows cil and (u* off the diagonal) cik
   for (int cp = m.dn_cp[dn]; cp < m.dn_cp[dn + 1]; ++cp) {
     int s0, s1;
     const long long* pts;
@@ -992,25 +1203,40 @@ __global__ void __launch_bounds__(WPB * 32, 4) k_mixed(DMesh m, const HarParF* p
     }
     if (s0 == s1) continue;
     const double* xi = m.cpx + 3 * (size_t)cp;
-    const long long P0 = pts[s0], Qn = pts[s1] - P0;
-    int cur = -1;
-    cf acc[kAcc];
-    for (int j = 0; j < kAcc; ++j) acc[j] = cf_zero();
-    for (long long base = 0; base < Qn; base += 32) {
-      const long long c = base + lane;
+    const long long P0 = pts[s0];
+    const int Qn = (int)(pts[s1] - P0);
+    int cur = -1;  // pair whose sums are open
+    c2 acc[4], acd;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) acc[k] = c2_zero();
+    acd = c2_zero();
+    int jw = s0;  // list entry of the batch's first point, before its own start bits
+    for (int base = 0; base < Qn; base += 32) {
+      // starts of the list entries after jw inside this batch
+      const int jn = jw + 1 + lane;
+      const long long bd = jn < s1 ? pts[jn] - P0 - base : 32;
+      const unsigned starts = __reduce_or_sync(0xffffffffu, bd < 32 ? 1u << (int)bd : 0u);
+      const int jl = jw + __popc(starts & (0xffffffffu >> (31 - lane)));
+      const int c = base + lane;
+      int pid = -1;  // pair of this lane's point
       if (c < Qn) {
-        const int jl = find_le(pts, s0, s1, P0 + c);
         ff rv[3], n[3];
         if (KIND == MIX_REG) {
           const int pr = m.reg_pair[jl];
           const int e = pr & 0xFFFFFF, ps = pr >> 24;
-          const size_t pt = (size_t)e * m.ptot + m.ps_off[ps] + (size_t)(P0 + c - m.reg_pt[jl]);
+          const size_t pt = (size_t)e * m.ptot + m.ps_off[ps] + (size_t)(P0 + c - pts[jl]);
           rv[0] = ff_from(m.px[3 * pt] - xi[0]);
           rv[1] = ff_from(m.px[3 * pt + 1] - xi[1]);
           rv[2] = ff_from(m.px[3 * pt + 2] - xi[2]);
           n[0] = pn_f[3 * pt]; n[1] = pn_f[3 * pt + 1]; n[2] = pn_f[3 * pt + 2];
-          for (int k = 0; k < 8; ++k) S[lane].w[k] = pphi_f[8 * pt + k];
-          S[lane].pair = jl;
+          const float4* w4 = reinterpret_cast<const float4*>(pphi_f + 8 * pt);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float4 v = __ldg(w4 + k);
+            rec_put(my + R::kW, 2 * k, c2{f2_dup(v.x), f2_dup(v.y)});
+            rec_put(my + R::kW, 2 * k + 1, c2{f2_dup(v.z), f2_dup(v.w)});
+          }
+          pid = jl;
         } else {
           const long long g = P0 + c, np = SG ? m.nsing_pts : m.nleaf_pts;
 #pragma unroll
@@ -1018,63 +1244,81 @@ __global__ void __launch_bounds__(WPB * 32, 4) k_mixed(DMesh m, const HarParF* p
             rv[k] = gf[k * np + g];
             n[k] = gf[(3 + k) * np + g];
           }
-          for (int k = 0; k < 8; ++k) S[lane].w[k] = gf[(6 + k) * np + g];
-          if constexpr (SG) {
-            for (int k = 0; k < 8; ++k) S[lane].wd[k] = gf[(14 + k) * np + g];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            const ff v = gf[(6 + k) * np + g];
+            rec_put(my + R::kW, k, c2{f2_dup(v.hi), f2_dup(v.lo)});
           }
-          S[lane].pair = SG ? jl : m.leaf_pair[jl];
+          if constexpr (SG) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              const ff v = gf[(14 + k) * np + g];
+              rec_put(my + R::kWd, k, c2{f2_dup(v.hi), f2_dup(v.lo)});
+            }
+          }
+          pid = SG ? jl : m.leaf_pair[jl];
         }
-        if constexpr (SG) harela_point_sing_ff(Q, rv, n, S[lane].fu, S[lane].ft, S[lane].fc);
-        else harela_point_ff(Q, rv, n, S[lane].fu, S[lane].ft);
+        if constexpr (TAB) harela_point_rad_ff<SG>(rt, f, rt.ff_[f], rv, n, my);
+        else harela_point_direct_ff<SG>(pf[f], rv, n, my);
       }
       __syncwarp();
-      const int nt = (int)min((long long)32, Qn - base);
-      // one extra step after the last point flushes the last pair (single call site)
-      const int tend = (base + 32 >= Qn) ? nt + 1 : nt;
+      const int nt = min(32, Qn - base);
+      int t = 0;
 #pragma unroll 1
-      for (int t = 0; t < tend; ++t) {
-        const int jp = t < nt ? S[t].pair : -1;
-        if (jp != cur) {
+      while (true) {
+        // the next point's pair; past the list's end -1 (flushes the last one)
+        const bool end = t >= nt;
+        if (end && base + 32 < Qn) break;
+        const int pr = end ? -1 : __shfl_sync(0xffffffffu, pid, t);
+        if (pr != cur) {
           if (cur >= 0) {
             const int e = KIND == MIX_REG ? (m.reg_pair[cur] & 0xFFFFFF) : (KIND == MIX_ADP ? m.adp_e[cur] : m.sing_e[cur]);
-            flush_pair_ff(m, Q, dcv_f, dn, e, acc, Acf, lda, bc, SG ? hps[w] : nullptr);
+            flush_pair_ff<SG>(m, cpv, dcv_f, e, acc, acd, Arow, lda, comp, half, cil, cik, bc0, bc1, stg[w], hps[w]);
           }
-          cur = jp;
-          for (int j = 0; j < kAcc; ++j) acc[j] = cf_zero();
+          cur = pr;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) acc[k] = c2_zero();
+          acd = c2_zero();
           if constexpr (SG) {
             __syncwarp();
-            if (jp >= 0 && lane < 17) {
-              const double* D = m.sing_d + (size_t)jp * SING_D;
+            if (pr >= 0 && lane < 17) {
+              const double* D = m.sing_d + (size_t)pr * SING_D;
               hps[w][lane] = ff_from(lane < 9 ? D[13 + lane] : D[5 + lane - 9]);
             }
             __syncwarp();
           }
         }
-        if (t < nt) {
-          const char* St = reinterpret_cast<const char*>(&S[t]);
+        if (end) break;
+        // points of the same list entry: up to the next start bit
+        const unsigned rest = t < 31 ? starts >> (t + 1) : 0u;
+        const int te = min(nt, rest ? t + __ffs(rest) : 32);
+        const char* rec = S + t * R::kSize;
+#pragma unroll 1
+        for (; t < te; ++t, rec += R::kSize) {
+          const c2 a = rec_get(rec + 16 * comp), na = c2_neg(a);
+          const char* rw = rec + R::kW + 64 * half;
 #pragma unroll
-          for (int j = 0; j < kAcc; ++j) {
-            const int sl = slot[j];
-            if (sl >= 0) {
-              // compensated accumulation (lo unnormalised until the flush)
-              const int kn = sl & 15;
-              acc_cmac_r(acc[j], *reinterpret_cast<const cf*>(St + (sl >> 4)), S[t].w[kn]);
-              if constexpr (SG) {
-                const int o = lane + 32 * j;
-                if (o < 72) acc_cmac_r(acc[j], S[t].fc[o % 9], S[t].wd[kn]);
-              }
-            }
+          for (int k = 0; k < 4; ++k) {
+            const c2 v = rec_get(rw + 16 * k);
+            c2_mac_n(acc[k], a, na, v.h, v.l);
+          }
+          if constexpr (SG) {
+            const c2 d = rec_get(rec + R::kFc + 16 * dcomp), v = rec_get(rec + R::kWd + 16 * (lane & 7));
+            c2_mac_n(acd, d, c2_neg(d), v.h, v.l);
           }
         }
       }
+      jw += __popc(starts);
       __syncwarp();
     }
   }
-  // b: one warp reduction per DOF node
+  // b: one warp reduction per row of the node
   double* bf = b + bstride * f;
+  const bool live = (lane & 15) < 15;
 #pragma unroll 1
   for (int il = 0; il < 3; ++il) {
-    cf v = il == 0 ? bc[0] : (il == 1 ? bc[1] : bc[2]);
+    cf v = live && cil == il ? bc0 : cf_zero();
+    if (live && comp >= 9 && cik != cil && cik == il) v = cf_add(v, bc1);
 #pragma unroll 1
     for (int o = 16; o > 0; o >>= 1) {
       cf u;

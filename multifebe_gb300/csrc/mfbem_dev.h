@@ -45,6 +45,8 @@ struct DMesh {
   const double* ball;
   const int* rev;
   const int* edof;
+  const int* emask;      // [ne] bit 3 kn + k: traction known at node kn, direction k; bit 24: reversed
+  const int* enz;        // [ne] bit 3 kn + k: the prescribed value there is not zero
   // dofs
   const int* dct;
   const double* dcv;

@@ -91,14 +91,27 @@ __device__ __forceinline__ void hbie_coef_h(const HarParD& q, const HarParH& s, 
          s.S5[7] * a[5] + s.S5[8] * b[5] + s.S5[9] * a[6] + s.S5[10] * b[6];
 }
 
-// Harmonic d* and s* at one point for the collocation normal ni (constants
-// cte_d, cte_s applied by the flush).
-__device__ __forceinline__ void hbie_point_h(const HarParD& q, const HarParH& s, const double rv[3], const double n[3],
+// The same from the call's radial table (dev_radial.cuh), the constants cte_d
+// (in TT1..TT3) and cte_s (in S1..S5) included: eight Horner sums of degree 7
+// in place of the two decomposed exponentials and their 75 combinations.
+__device__ __forceinline__ void hbie_coef_rad(const RadTab& t, int f, double r, double d1r1, bool full, HbieCoefH& c) {
+  const RadF& q = t.f[f];
+  const double d2 = d1r1 * d1r1, f2 = full ? d2 : 0.0, f3 = full ? d2 * d1r1 : 0.0;
+  double x;
+  const double2* w = rad_row(t, f, q, r, x) + 2 * kRadC;
+  c.TT1 = rad_eval(w, x) + q.s[2] * f2;
+  c.TT2 = rad_eval(w + kRadC, x) + q.s[3] * f2;
+  c.TT3 = rad_eval(w + 2 * kRadC, x) + q.s[4] * f2;
+  cd S[5];
+#pragma unroll
+  for (int j = 0; j < 5; ++j) S[j] = rad_eval(w + (3 + j) * kRadC, x) + q.s1[j] * d1r1 + q.s3[j] * f3;
+  c.S1 = S[0]; c.S2 = S[1]; c.S3 = S[2]; c.S4 = S[3]; c.S5 = S[4];
+}
+
+// Harmonic d* and s* at one point for the collocation normal ni from their
+// coefficients (constants cte_d, cte_s as the coefficients have them).
+__device__ __forceinline__ void hbie_point_h(const HbieCoefH& c, double d1r, const double rv[3], const double n[3],
                                              const double ni[3], cd fd[9], cd fs[9]) {
-  const double r = sqrt(rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2]);
-  HbieCoefH c;
-  hbie_coef_h(q, s, r, true, c);
-  const double d1r = 1.0 / r;
   const double dr[3] = {rv[0] * d1r, rv[1] * d1r, rv[2] * d1r};
   const double drdn = dr[0] * n[0] + dr[1] * n[1] + dr[2] * n[2];
   const double drdni = -(dr[0] * ni[0] + dr[1] * ni[1] + dr[2] * ni[2]);
@@ -122,6 +135,7 @@ __device__ __forceinline__ void hbie_point_h(const HarParD& q, const HarParH& s,
 struct PolHbieStatic {
   typedef double T;
   static constexpr int NG = 9;
+  static constexpr bool kScaled = false;
   double nu, cted1, cted2, ctes1, ctes2, ctes3;
   const double* cpn;    // [ncp][3] collocation normals
   const double* cpa;    // [ncp] Burton & Miller alpha
@@ -144,6 +158,7 @@ struct PolHbieStatic {
 struct PolHbieHarmonic {
   typedef cd T;
   static constexpr int NG = 9;
+  static constexpr bool kScaled = false;
   const HarParD* p;
   const HarParH* ph;
   const double* cpn;
@@ -153,7 +168,10 @@ struct PolHbieHarmonic {
   __device__ T cte_u(int f) const { return ph[f].cte_d; }
   __device__ T cpv(int) const { return mk(0.0); }
   __device__ void point(int f, int cp, const double rv[3], const double n[3], T fu[9], T ft[9]) const {
-    hbie_point_h(p[f], ph[f], rv, n, cpn + 3 * (size_t)cp, fu, ft);
+    const double r = sqrt(rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2]);
+    HbieCoefH c;
+    hbie_coef_h(p[f], ph[f], r, true, c);
+    hbie_point_h(c, 1.0 / r, rv, n, cpn + 3 * (size_t)cp, fu, ft);
     if (hbie_weighted(cpk[cp])) {
       const cd b = cpa[cp] * ph[f].ic2;
 #pragma unroll
@@ -162,6 +180,31 @@ struct PolHbieHarmonic {
         ft[q] = b * ft[q];
       }
     }
+  }
+};
+struct PolHbieHarmonicRad {
+  typedef cd T;
+  static constexpr int NG = 9;
+  static constexpr bool kScaled = true;
+  RadTab t;
+  const HarParH* ph;
+  const double* cpn;
+  const double* cpa;
+  const int* cpk;
+  __device__ T cte_t(int) const { return mk(1.0); }
+  __device__ T cte_u(int) const { return mk(1.0); }
+  __device__ T cpv(int) const { return mk(0.0); }
+  __device__ void point(int f, int cp, const double rv[3], const double n[3], T fu[9], T ft[9]) const {
+    const double r = sqrt(rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2]), d1 = 1.0 / r;
+    HbieCoefH c;
+    hbie_coef_rad(t, f, r, d1, true, c);
+    // beta on the eight coefficients instead of the eighteen components
+    if (hbie_weighted(cpk[cp])) {
+      const cd b = cpa[cp] * ph[f].ic2;
+      c.TT1 = b * c.TT1; c.TT2 = b * c.TT2; c.TT3 = b * c.TT3;
+      c.S1 = b * c.S1; c.S2 = b * c.S2; c.S3 = b * c.S3; c.S4 = b * c.S4; c.S5 = b * c.S5;
+    }
+    hbie_point_h(c, d1, rv, n, cpn + 3 * (size_t)cp, fu, ft);
   }
 };
 __host__ __device__ inline PolHbieStatic hbie_static_policy(double mu, double nu) {
@@ -215,6 +258,17 @@ struct HsHarmonic {
     return HsCoef<cd>{q.T1[0], q.T2[0], s.S1[0], s.S2[0], s.S3[0], s.S4[0], s.S5[0], s.cte_d, s.cte_s, s.ic2};
   }
   __device__ void dyn(int f, double r, HbieCoefH& c) const { hbie_coef_h(p[f], ph[f], r, false, c); }
+};
+struct HsHarmonicRad {
+  typedef cd T;
+  static constexpr bool kDyn = true;
+  RadTab t;
+  const HarParH* ph;
+  __device__ HsCoef<cd> coef(int f) const {
+    const RadF& q = t.f[f];
+    return HsCoef<cd>{q.s[2], q.s[3], q.s3[0], q.s3[1], q.s3[2], q.s3[3], q.s3[4], mk(1.0), mk(1.0), ph[f].ic2};
+  }
+  __device__ void dyn(int f, double r, HbieCoefH& c) const { hbie_coef_rad(t, f, r, 1.0 / r, false, c); }
 };
 
 template <typename T>

@@ -1585,9 +1585,14 @@ extern "C" int mfbem_sweep_harela(mfbem_handle* h, const double lambda[2], const
   CK(cudaMemsetAsync(A, 0, sizeof(double2) * nn * n_freq, h->st));
   CK(cudaMemsetAsync(b, 0, sizeof(double2) * (size_t)n * n_freq, h->st));
   if ((rc = bm_prepare(h, 1))) return rc;
+  PolHarmonicRad pr;
+  pr.p = dpar;
+  if ((rc = hbie_params(h, dq, n_freq, &pr.ph)) ||
+      (rc = radial_prepare(h, q.data(), n_freq, dpar, pr.ph, precision >= 1, &pr.t)))
+    return rc;
   PolHarmonic pol;
   pol.p = dpar;
-  if ((rc = hbie_params(h, dq, n_freq, &pol.ph))) return rc;
+  pol.ph = pr.ph;
   AsmTimes tm;
   long long l0 = g_launches;
   const HarParF* pf = nullptr;
@@ -1619,9 +1624,11 @@ extern "C" int mfbem_sweep_harela(mfbem_handle* h, const double lambda[2], const
     pf = (const HarParF*)h->parf.p;
     dsf = (const ff*)h->pphi_f.p;
   }
-  if ((rc = launch_assembly(h, pol, dnu, n_freq, (double*)A, n, 2 * nn, (double*)b, 2 * (size_t)n, &tm, pf, dsf,
-                            precision >= 1, sgf, lgf)))
-    return rc;
+  rc = pr.t.n > 0 ? launch_assembly(h, pr, dnu, n_freq, (double*)A, n, 2 * nn, (double*)b, 2 * (size_t)n, &tm, pf, dsf,
+                                    precision >= 1, sgf, lgf)
+                  : launch_assembly(h, pol, dnu, n_freq, (double*)A, n, 2 * nn, (double*)b, 2 * (size_t)n, &tm, pf, dsf,
+                                    precision >= 1, sgf, lgf);
+  if (rc) return rc;
   cudaEventRecord(a1, h->st);
   if ((rc = check_err(h))) return rc;
   float ams = 0;
