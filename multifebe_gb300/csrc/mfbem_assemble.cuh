@@ -33,13 +33,14 @@ __device__ __forceinline__ double shfl_x(double v, int o) { return __shfl_xor_sy
 __device__ __forceinline__ cd shfl_x(cd v, int o) { return mk(shfl_x(v.re, o), shfl_x(v.im, o)); }
 __device__ __forceinline__ double cval(const double* dcv, int dof, double) { return dcv[2 * (size_t)dof]; }
 __device__ __forceinline__ cd cval(const double* dcv, int dof, cd) { return mk(dcv[2 * (size_t)dof], dcv[2 * (size_t)dof + 1]); }
-__device__ __forceinline__ void addA(double* A, size_t idx, double v) { A[idx] += v; }
+// A(idx) += v as a reduction performed at the L2 (the result is not used): the
+// flush of a pair does not wait for A to arrive. The rows belong to one warp, so
+// each entry's additions keep their order: they come from one thread, or from
+// threads ordered by the warp barriers between two flushes.
+__device__ __forceinline__ void addA(double* A, size_t idx, double v) { atomicAdd(A + idx, v); }
 __device__ __forceinline__ void addA(double* A, size_t idx, cd v) {
-  double2* p = reinterpret_cast<double2*>(A) + idx;
-  double2 a = *p;
-  a.x += v.re;
-  a.y += v.im;
-  *p = a;
+  atomicAdd(A + 2 * idx, v.re);
+  atomicAdd(A + 2 * idx + 1, v.im);
 }
 
 // Kernel family policies -----------------------------------------------------
@@ -1126,7 +1127,7 @@ __device__ __forceinline__ void flush_pair_ff(const DMesh& m, const cf& cpv, con
     if (q < 144) {
       const int o = q >> 1, part = q & 1, col = o / 3, il = o - 3 * col, kn = col / 3, ik = col - 3 * kn;
       double* p = Arow + 2 * ((size_t)(ed[kn] + ik) * lda + il) + part;
-      *p += (double)sf[4 * o + part] + (double)sf[4 * o + 2 + part];
+      atomicAdd(p, (double)sf[4 * o + part] + (double)sf[4 * o + 2 + part]);
     }
   }
   __syncwarp();
