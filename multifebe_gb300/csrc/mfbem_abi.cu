@@ -26,8 +26,8 @@
 #include "mfbem_host.h"
 #include "mfbem_precompute.cuh"
 #include "mfbem_assemble.cuh"
-#include "mfbem_internal.cuh"
 #include "mfbem_hbie.cuh"
+#include "mfbem_internal.cuh"
 #include "mfbem_radial.cuh"
 #include "mfbem_lu.cuh"
 #include "mfbem_tc.cuh"
@@ -120,6 +120,10 @@ struct mfbem_handle {
   // between any two points of the mesh's elements
   DevBuf rad;
   double rmax = 0.0;
+  double box_lo[3] = {0, 0, 0}, box_hi[3] = {0, 0, 0};  // box that holds every element
+  // work buffers of the internal points, in the order of their use (grown as
+  // needed, released with the handle)
+  std::vector<DevBuf> ip_ws;
 };
 
 // ---------------------------------------------------------------------------
@@ -716,6 +720,8 @@ static int upload_impl(const mfbem_mesh_desc* d, const mfbem_dual_desc* dual, mf
     }
     h->rmax = std::sqrt((hi[0] - lo[0]) * (hi[0] - lo[0]) + (hi[1] - lo[1]) * (hi[1] - lo[1]) +
                         (hi[2] - lo[2]) * (hi[2] - lo[2]));
+    std::copy(lo, lo + 3, h->box_lo);
+    std::copy(hi, hi + 3, h->box_hi);
   }
   // --- device arrays
   double *ex, *cl, *ball, *dcvd, *cpxd, *cpxid, *ngn, *tbp;
@@ -872,6 +878,7 @@ extern "C" int mfbem_mesh_release(mfbem_handle* h) {
     for (DevBuf* b : {&h->A, &h->b, &h->A32, &h->x, &h->r, &h->work, &h->ipiv, &h->info, &h->par, &h->nu, &h->parf,
                       &h->pphi_f, &h->geo_f, &h->gm, &h->parh, &h->rad})
       pool_give(b->p, b->bytes, b->dev);
+    for (DevBuf& b : h->ip_ws) pool_give(b.p, b.bytes, b.dev);
     if (h->st) {
       std::lock_guard<std::mutex> lk(g_pool_mu);
       g_ctx_pool.emplace_back(h->dev, h->st);
@@ -1028,13 +1035,13 @@ struct AsmTimes {
   }
 };
 
-// Radial tables (dev_radial.cuh) of a harmonic call's nf frequencies, rebuilt
-// on every call: q [nf][6] (lambda, mu, rho, omega; host), dpar / dparh their
+// Radial tables (dev_radial.cuh) of a harmonic call's nf frequencies for
+// distances up to rmax, rebuilt on every call: q [nf][6] (lambda, mu, rho, omega; host), dpar / dparh their
 // device parameter blocks (dparh: HBIE points only), mixed: the double-float
 // rows too. t->n = 0 (the kernels evaluate E_n directly) where the tables do
 // not apply: a wavenumber of zero or not finite, or more intervals than
 // kRadMaxN.
-static int radial_prepare(mfbem_handle* h, const double* q, int nf, const HarParD* dpar, const HarParH* dparh,
+static int radial_prepare(mfbem_handle* h, double rmax, const double* q, int nf, const HarParD* dpar, const HarParH* dparh,
                           bool mixed, RadTab* t) {
   *t = RadTab();
   std::vector<double> hl(nf);
@@ -1044,10 +1051,10 @@ static int radial_prepare(mfbem_handle* h, const double* q, int nf, const HarPar
     const std::complex<double> lam(v[0], v[1]), mu(v[2], v[3]);
     const double k1 = std::abs(v[5] / std::sqrt((lam + 2.0 * mu) / v[4])), k2 = std::abs(v[5] / std::sqrt(mu / v[4]));
     const double k = std::max(k1, k2);
-    if (!(std::isfinite(k1) && std::isfinite(k2) && k > 0.0 && h->rmax > 0.0)) return 0;
+    if (!(std::isfinite(k1) && std::isfinite(k2) && k > 0.0 && rmax > 0.0)) return 0;
     // no longer than the mesh: the samples stay at distances that occur
-    hl[f] = std::min(kRadKh / k, h->rmax);
-    most = std::max(most, h->rmax / hl[f]);
+    hl[f] = std::min(kRadKh / k, rmax);
+    most = std::max(most, rmax / hl[f]);
   }
   if (!(most < kRadMaxN)) return 0;
   const int n = (int)std::ceil(most) + 1, nfun = dparh ? 10 : 5;
@@ -1343,7 +1350,7 @@ extern "C" int mfbem_assemble_harela(mfbem_handle* h, const double lambda[2], co
   if ((rc = bm_prepare(h, 1))) return rc;
   PolHarmonicRad pr;
   pr.p = (const HarParD*)h->par.p;
-  if ((rc = hbie_params(h, dq, 1, &pr.ph)) || (rc = radial_prepare(h, q, 1, pr.p, pr.ph, false, &pr.t))) return rc;
+  if ((rc = hbie_params(h, dq, 1, &pr.ph)) || (rc = radial_prepare(h, h->rmax, q, 1, pr.p, pr.ph, false, &pr.t))) return rc;
   if (pr.t.n > 0) return assemble_common(h, pr, nu, A, lda, b, flags);
   PolHarmonic pol;
   pol.p = pr.p;
@@ -1354,17 +1361,16 @@ extern "C" int mfbem_assemble_harela(mfbem_handle* h, const double lambda[2], co
 // ---------------------------------------------------------------------------
 // Internal points (calculate_internal_points_mechanics_bem_{staela,harela})
 // ---------------------------------------------------------------------------
+// work buffers of one call: the handle's ip_ws in order of use
 struct TmpBufs {
-  std::vector<void*> v;
-  ~TmpBufs() {
-    for (void* p : v) cudaFree(p);
-  }
+  mfbem_handle* h;
+  size_t used = 0;
+  explicit TmpBufs(mfbem_handle* h_) : h(h_) {}
   int get(void** p, size_t bytes) {
-    if (cudaMalloc(p, std::max<size_t>(bytes, 16)) != cudaSuccess) {
-      cudaGetLastError();
-      return fail(MFBEM_ENOMEM, "cudaMalloc (internal points)");
-    }
-    v.push_back(*p);
+    if (used == h->ip_ws.size()) h->ip_ws.emplace_back();
+    DevBuf& b = h->ip_ws[used++];
+    if (int rc = ensure(b, std::max<size_t>(bytes, 16))) return rc;
+    *p = b.p;
     return 0;
   }
 };
@@ -1380,8 +1386,14 @@ static int ip_pass(mfbem_handle* h, IpArgs a, const POL& pol, TmpBufs& tb, std::
   int rc;
   if ((rc = tb.get((void**)&a.cls_s, (size_t)n_ip * ne)) || (rc = tb.get((void**)&a.cls_h, (size_t)n_ip * ne)) ||
       (rc = tb.get((void**)&a.npair, sizeof(int) * n_ip)) || (rc = tb.get((void**)&a.poff, sizeof(int) * (n_ip + 1))) ||
-      (rc = tb.get((void**)&a.err, sizeof(int))) || (rc = tb.get(&a.out, ob)))
+      (rc = tb.get((void**)&a.err, sizeof(int))) || (rc = tb.get(&a.out, ob)) ||
+      (rc = tb.get(&a.uw, sizeof(T) * 6 * (size_t)ne * m.ptot * nf)))
     return rc;
+  // warps for the GPU (152 SMs x 64) from the points, then from groups of 32 elements
+  const int groups = (ne + 31) / 32, want = (int)((152LL * 64 + (long long)n_ip * nf - 1) / ((long long)n_ip * nf));
+  a.gpc = (groups + std::min(groups, want) - 1) / std::min(groups, want);
+  a.nch = (groups + a.gpc - 1) / a.gpc;
+  if ((rc = tb.get(&a.part, sizeof(T) * 9 * (size_t)a.nch * n_ip * nf))) return rc;
   cudaStream_t st = h->st;
   const int big = INT_MAX;
   CK(cudaMemcpyAsync(a.err, &big, sizeof(int), cudaMemcpyHostToDevice, st));
@@ -1393,14 +1405,16 @@ static int ip_pass(mfbem_handle* h, IpArgs a, const POL& pol, TmpBufs& tb, std::
   CK(cudaStreamSynchronize(st));
   a.npairs = np;
   if ((rc = tb.get((void**)&a.pair_e, sizeof(int) * (size_t)np)) || (rc = tb.get((void**)&a.pair_ip, sizeof(int) * (size_t)np)) ||
-      (rc = tb.get(&a.slot, sizeof(T) * 12 * (size_t)np * nf)))
+      (rc = tb.get(&a.slot, sizeof(T) * 9 * (size_t)np * nf)))
     return rc;
   k_ip_fill<<<nblk(n_ip, 8), 256, 0, st>>>(m, a); ++g_launches;
   if (np > 0) {
     k_ip_adp<POL><<<nblk((long long)np * nf, 64), 64, 0, st>>>(m, a, pol, h->d_qs); ++g_launches;
   }
   constexpr int WPB = 4;
-  k_ip_reg<POL, WPB><<<nblk((long long)n_ip * nf, WPB), WPB * 32, 0, st>>>(m, a, pol); ++g_launches;
+  k_ip_weights<T><<<nblk((long long)ne * m.ptot * nf, 128), 128, 0, st>>>(m, a); ++g_launches;
+  k_ip_reg<POL, WPB><<<nblk((long long)n_ip * nf * a.nch, WPB), WPB * 32, 0, st>>>(m, a, pol); ++g_launches;
+  k_ip_sum<T><<<nblk(9LL * n_ip * nf, 128), 128, 0, st>>>(a); ++g_launches;
   CK(cudaGetLastError());
   out.assign(12 * (size_t)n_ip * nf, T{});
   int err = 0;
@@ -1416,7 +1430,7 @@ static int ip_pass(mfbem_handle* h, IpArgs a, const POL& pol, TmpBufs& tb, std::
 }
 
 template <class POL>
-static int internal_points_run(mfbem_handle* h, const POL& pol, int nf, int32_t n_ip, const double* x_ip,
+static int internal_points_run(mfbem_handle* h, TmpBufs& tb, const POL& pol, int nf, int32_t n_ip, const double* x_ip,
                                const double* u_nodes, const double* t_nodes, const double* u2_nodes,
                                const double* t2_nodes, double* u_ip, double* sigma_ip) {
   typedef typename POL::T T;
@@ -1444,7 +1458,6 @@ static int internal_points_run(mfbem_handle* h, const POL& pol, int nf, int32_t 
     u_nodes = (const double*)ueff.data();
     t_nodes = (const double*)teff.data();
   }
-  TmpBufs tb;
   IpArgs a{};
   a.nip = n_ip;
   a.nf = nf;
@@ -1461,7 +1474,7 @@ static int internal_points_run(mfbem_handle* h, const POL& pol, int nf, int32_t 
   CK(cudaMemcpyAsync((void*)a.xip, x_ip, sizeof(double) * 3 * (size_t)n_ip, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync((void*)a.uval, u_nodes, vb, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync((void*)a.tval, t_nodes, vb, cudaMemcpyHostToDevice, st));
-  k_ip_onnode<<<nblk(n_ip, 128), 128, 0, st>>>(a); ++g_launches;
+  k_ip_onnode<<<nblk(n_ip, 4), 128, 0, st>>>(a); ++g_launches;
   std::vector<T> out;
   if ((rc = ip_pass(h, a, pol, tb, out))) return rc;
   // static half-space: the complementary kernels from the points' images
@@ -1523,7 +1536,8 @@ static int internal_points_staela(mfbem_handle* h, double mu, double nu, int32_t
   pol.ctes1 = mu / (4.0 * kPi * (1.0 - nu));
   pol.ctes2 = 1.0 - 2.0 * nu;
   pol.ctes3 = 1.0 - 4.0 * nu;
-  return internal_points_run(h, pol, 1, n_ip, x_ip, u_nodes, t_nodes, u2_nodes, t2_nodes, u_ip, sigma_ip);
+  TmpBufs tb(h);
+  return internal_points_run(h, tb, pol, 1, n_ip, x_ip, u_nodes, t_nodes, u2_nodes, t2_nodes, u_ip, sigma_ip);
 }
 extern "C" int mfbem_internal_points_staela(mfbem_handle* h, double mu, double nu, int32_t n_ip, const double* x_ip,
                                             const double* u_nodes, const double* t_nodes, double* u_ip,
@@ -1547,7 +1561,7 @@ static int internal_points_harela(mfbem_handle* h, const double lambda[2], const
     return fail(MFBEM_EARG, "invalid argument");
   if (int rd = check_dev(h)) return rd;
   if (n_ip == 0) return 0;
-  TmpBufs tb;
+  TmpBufs tb(h);
   HarParD* pd;
   HarParH* ph;
   double* dq;
@@ -1559,10 +1573,24 @@ static int internal_points_harela(mfbem_handle* h, const double lambda[2], const
   CK(cudaMemcpyAsync(dq, q, sizeof(q), cudaMemcpyHostToDevice, h->st));
   k_harpar<<<1, 32, 0, h->st>>>(dq, 1, pd, zexp_thresholds()); ++g_launches;
   k_harparh<<<1, 32, 0, h->st>>>(dq, 1, ph); ++g_launches;
+  // distances to the points, which need not lie within the mesh's extent
+  double ext = 0.0;
+  for (int c = 0; c < 3; ++c) {
+    double lo = h->box_lo[c], hi = h->box_hi[c];
+    for (int ip = 0; ip < n_ip; ++ip) {
+      lo = std::min(lo, x_ip[3 * (size_t)ip + c]);
+      hi = std::max(hi, x_ip[3 * (size_t)ip + c]);
+    }
+    ext += (hi - lo) * (hi - lo);
+  }
+  IpHarmonicRad pr;
+  if ((rc = radial_prepare(h, std::sqrt(ext), q, 1, pd, ph, false, &pr.t))) return rc;
+  if (pr.t.n > 0)
+    return internal_points_run(h, tb, pr, 1, n_ip, x_ip, u_nodes, t_nodes, u2_nodes, t2_nodes, u_ip, sigma_ip);
   IpHarmonic pol;
   pol.p = pd;
   pol.ph = ph;
-  return internal_points_run(h, pol, 1, n_ip, x_ip, u_nodes, t_nodes, u2_nodes, t2_nodes, u_ip, sigma_ip);
+  return internal_points_run(h, tb, pol, 1, n_ip, x_ip, u_nodes, t_nodes, u2_nodes, t2_nodes, u_ip, sigma_ip);
 }
 extern "C" int mfbem_internal_points_harela(mfbem_handle* h, const double lambda[2], const double mu[2], double rho,
                                             double omega, int32_t n_ip, const double* x_ip, const double* u_nodes,
@@ -1671,8 +1699,7 @@ extern "C" int mfbem_internal_radial(const double* q, double rmax, int32_t n, co
   if (!q || !(rmax > 0.0) || n <= 0 || !r || !tab || !tabf || !dir) return fail(MFBEM_EARG, "invalid argument");
   int rc = init_tables();
   if (rc) return rc;
-  mfbem_handle h;  // the default stream; only its table buffer and extent are used
-  h.rmax = rmax;
+  mfbem_handle h;  // the default stream; only its table buffer is used
   const size_t nb[6] = {sizeof(HarParD), sizeof(HarParH), 6 * sizeof(double), 8 * (size_t)n, 160 * (size_t)n, 80 * (size_t)n};
   DevBuf d[7];
   for (int i = 0; i < 7; ++i)
@@ -1685,7 +1712,7 @@ extern "C" int mfbem_internal_radial(const double* q, double rmax, int32_t n, co
     k_harpar<<<1, 32>>>((const double*)d[2].p, 1, p, zexp_thresholds()); ++g_launches;
     k_harparh<<<1, 32>>>((const double*)d[2].p, 1, ph); ++g_launches;
     RadTab t;
-    if (int e = radial_prepare(&h, q, 1, p, ph, true, &t)) return e;
+    if (int e = radial_prepare(&h, rmax, q, 1, p, ph, true, &t)) return e;
     if (t.n == 0) return fail(MFBEM_EARG, "no table for these parameters");
     k_radial_check<<<nblk(n, 64), 64>>>(t, p, ph, (const double*)d[3].p, n, (double*)d[4].p, (double*)d[5].p,
                                         (double*)d[6].p); ++g_launches;

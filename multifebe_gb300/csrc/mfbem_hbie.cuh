@@ -25,6 +25,113 @@
 
 namespace mfb {
 
+// d* / s* coefficients of fbem_bem_harela3d_calculate_parameters (bem_harela3d.f90:219-283)
+// (ic2 = i / c2, the Burton & Miller factor of the harmonic builder)
+struct HarParH {
+  cd S1[11], S2[11], S3[12], S4[10], S5[11];
+  cd cte_d, cte_s, ic2;
+};
+__host__ __device__ inline HarParH harela_hbie_params(cd lambda, cd mu, double rho, double omega) {
+  HarParH p;
+  const cd I = mk(0.0, 1.0);
+  cd c1 = csqrt_((lambda + 2.0 * mu) / rho), c2 = csqrt_(mu / rho);
+  cd k1 = omega / c1, k2 = omega / c2;
+  cd c1p2 = c1 * c1, c2p2 = c2 * c2, c1p3 = c1p2 * c1, c1p4 = c1p2 * c1p2, c1p5 = c1p4 * c1, c2p3 = c2p2 * c2;
+  cd k1p2 = k1 * k1, k2p2 = k2 * k2, q = k1p2 / k2p2;
+  cd ik1 = I * k1, ik2 = I * k2, ik1p2 = ik1 * ik1, ik2p2 = ik2 * ik2;
+  cd r = c2p2 / c1p2;
+  const double om2 = omega * omega, om3 = om2 * omega;
+  p.S1[0] = 3.0 * (1.0 - 2.0 * r);
+  p.S1[1] = -0.5 * c2p2 / c1p4 * om2;
+  p.S1[2] = k2p2;
+  p.S1[3] = 4.0 * I * k1 * q;
+  p.S1[4] = -7.0 * I * k2;
+  p.S1[5] = 24.0 * q;
+  p.S1[6] = mk(-27.0);
+  p.S1[7] = 60.0 * q / ik1;
+  p.S1[8] = -60.0 / ik2;
+  p.S1[9] = 60.0 * q / ik1p2;
+  p.S1[10] = -60.0 / ik2p2;
+  p.S2[0] = 6.0 * r;
+  p.S2[1] = (0.5 / c2p2 + 1.5 * c2p2 / c1p4 - 1.0 / c1p2) * om2;
+  p.S2[2] = 2.0 * c2p2 / c1p4 * (c1p2 / c2p2 - 2.0) * om2;
+  p.S2[3] = 2.0 * I * c2p2 / c1p3 * (8.0 - 3.0 * c1p2 / c2p2) * omega;
+  p.S2[4] = -4.0 * I * k2;
+  p.S2[5] = 6.0 * r * (6.0 - c1p2 / c2p2);
+  p.S2[6] = mk(-24.0);
+  p.S2[7] = r * 60.0 / ik1;
+  p.S2[8] = -60.0 / ik2;
+  p.S2[9] = 60.0 / ik2p2;
+  p.S2[10] = -60.0 / ik2p2;
+  p.S3[0] = 30.0 * (1.0 - r);
+  p.S3[1] = 1.5 * (1.0 / c2p2 - c2p2 / c1p4) * om2;
+  p.S3[2] = -4.0 * r * k1p2;
+  p.S3[3] = 4.0 * k2p2;
+  p.S3[4] = 40.0 * r * I * k1;
+  p.S3[5] = -40.0 * I * k2;
+  p.S3[6] = 180.0 * r;
+  p.S3[7] = mk(-180.0);
+  p.S3[8] = 420.0 * r / ik1;
+  p.S3[9] = -420.0 / ik2;
+  p.S3[10] = 420.0 / ik2p2;
+  p.S3[11] = -420.0 / ik2p2;
+  p.S4[0] = 2.0 * r;
+  p.S4[1] = 0.5 * (c2p2 / c1p4 + 1.0 / c2p2) * om2;
+  p.S4[2] = -2.0 / 5.0 * (1.0 / c2p3 + 2.0 / 3.0 * c2p2 / c1p5) * I * om3;
+  p.S4[3] = 2.0 * I * k2;
+  p.S4[4] = -4.0 * r;
+  p.S4[5] = mk(6.0);
+  p.S4[6] = -12.0 * r / ik1;
+  p.S4[7] = 12.0 / ik2;
+  p.S4[8] = -12.0 / ik2p2;
+  p.S4[9] = 12.0 / ik2p2;
+  p.S5[0] = 2.0 * (1.0 - 3.0 * r);
+  p.S5[1] = (-2.0 / c1p2 + 0.5 / c2p2 + 0.5 * c2p2 / c1p4) * om2;
+  p.S5[2] = (8.0 / 3.0 / c1p3 + 4.0 / 15.0 / c2p3 - 1.0 / c1 / c2p2 - 24.0 / 15.0 * c2p2 / c1p5) * I * om3;
+  p.S5[3] = (-4.0 / c1p2 + 1.0 / c2p2 + 4.0 * c2p2 / c1p4) * om2;
+  p.S5[4] = 4.0 * I * (1.0 / c1 - 2.0 * c2p2 / c1p3) * omega;
+  p.S5[5] = 4.0 * (1.0 - 3.0 * r);
+  p.S5[6] = mk(4.0);
+  p.S5[7] = 12.0 * I * k1 / k2p2;
+  p.S5[8] = -12.0 * I / k2;
+  p.S5[9] = 12.0 / k2p2;
+  p.S5[10] = -12.0 / k2p2;
+  p.cte_d = mk(k1_4Pi);
+  p.cte_s = k1_4Pi * mu;
+  p.ic2 = I / c2;
+  return p;
+}
+
+// E_2..E_6 of z (numerical.f90:1258-1331), as zexp_2to5 plus E_6
+__device__ __forceinline__ void zexp_2to6(const ZexpSteps& steps, cd z, cd E[7]) {
+  const double az2 = z.re * z.re + z.im * z.im;
+  cd z2 = z * z, z3 = z2 * z, z4 = z3 * z, z5 = z4 * z;
+  if (az2 <= 1.0) {
+    const int N = zexp_nterms(steps, az2) + 6;
+    cd t = mk(1.0);
+    for (int k = N; k >= 7; --k) t = 1.0 + t * z * (1.0 / (double)k);
+    E[6] = ((z5 * z) * (1.0 / 720.0)) * t;
+    E[5] = E[6] + z5 * (1.0 / 120.0);
+    E[4] = E[5] + z4 * (1.0 / 24.0);
+    E[3] = E[4] + z3 * (1.0 / 6.0);
+    E[2] = E[3] + z2 * 0.5;
+  } else {
+    E[2] = (cexp_(z) - 1.0) - z;
+    E[3] = E[2] - 0.5 * z2;
+    E[4] = E[3] - (1.0 / 6.0) * z3;
+    E[5] = E[4] - (1.0 / 24.0) * z4;
+    E[6] = E[5] - (1.0 / 120.0) * z5;
+  }
+}
+
+// q: [nf][6] = lambda (re, im), mu (re, im), rho, omega
+__global__ void k_harparh(const double* q, int nf, HarParH* out) {
+  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  if (f >= nf) return;
+  const double* v = q + 6 * f;
+  out[f] = harela_hbie_params(mk(v[0], v[1]), mk(v[2], v[3]), v[4], v[5]);
+}
+
 // HBIE points weighted by the Burton & Miller factor beta alpha: kind 3
 // ('dual_bm_same') and 5 ('dual_bm_mixed'); kinds 2 ('hbie') and 4
 // (crack-like node) take weight 1.

@@ -14,239 +14,159 @@
 //
 // Layout of the work: the shape-function weights of every quadrature point are
 // contracted with the element's nodal values first (t_w = sum_kn phi_kn J w t_kn,
-// the same for u), so no 8x3x3 kernel block is formed; one warp per (point,
-// frequency) walks the elements with the precalculated rules, and one thread per
-// quasi-singular (point, element) pair walks the subdivision tree, writing its
-// 12 sums to a slot that the warp adds in element order (deterministic). FP64:
-// this runs once per solution, not per sweep step.
+// the same for u), so no 8x3x3 kernel block is formed; for the precalculated
+// rules that is done once per call and dataset point (k_ip_weights), since it
+// does not depend on the internal point. Kernel and nodal vectors are
+// contracted before the tensors are formed: sigma is symmetric, and with
+// a = dr.T, b = dr.U, w = n.U, d = dr/dn its six components take about 150
+// multiply-adds a point instead of the 1350 of 3 x 9 components of d* and s*.
+// One warp per (point, frequency, 32 elements) spreads the quadrature points of
+// its elements over the lanes (elements with a 2 x 2 rule no longer leave 28
+// lanes idle), one thread per quasi-singular (point, element) pair walks the
+// subdivision tree; partial sums are added per point in element order
+// (deterministic). FP64. 300 points in a harmonic 6 x 6 cube, the
+// whole call: 27.5 ms with one warp per point and lanes on one element's points,
+// 2.7 ms here (0.7 ms of it the classification).
 #pragma once
 
 namespace mfb {
 
-// d* / s* coefficients of fbem_bem_harela3d_calculate_parameters (bem_harela3d.f90:219-283)
-// (ic2 = i / c2, the Burton & Miller factor of the harmonic builder)
-struct HarParH {
-  cd S1[11], S2[11], S3[12], S4[10], S5[11];
-  cd cte_d, cte_s, ic2;
+// Contraction of one quadrature point with t_w (T) and u_w (U): the u-part
+// (SBIE) and the sigma-part (HBIE with the three unit normals; six components,
+// (0,0) (0,1) (0,2) (1,1) (1,2) (2,2)). rs = -1 for a reversed element. With
+//   g = psi I - chi dr dr^T, h = TT1 d dr dr^T + TT2 (n dr^T + d I) + TT3 dr n^T
+//   d*, s* of hbie_point_s / hbie_point_h with n_i = e_c
+// and the constants of u*, t*, d*, s* in the coefficients.
+template <typename T>
+struct IpCoef {
+  T psi, chi, TT1, TT2, TT3, S1, S2, S3, S4, S5;
 };
-__host__ __device__ inline HarParH harela_hbie_params(cd lambda, cd mu, double rho, double omega) {
-  HarParH p;
-  const cd I = mk(0.0, 1.0);
-  cd c1 = csqrt_((lambda + 2.0 * mu) / rho), c2 = csqrt_(mu / rho);
-  cd k1 = omega / c1, k2 = omega / c2;
-  cd c1p2 = c1 * c1, c2p2 = c2 * c2, c1p3 = c1p2 * c1, c1p4 = c1p2 * c1p2, c1p5 = c1p4 * c1, c2p3 = c2p2 * c2;
-  cd k1p2 = k1 * k1, k2p2 = k2 * k2, q = k1p2 / k2p2;
-  cd ik1 = I * k1, ik2 = I * k2, ik1p2 = ik1 * ik1, ik2p2 = ik2 * ik2;
-  cd r = c2p2 / c1p2;
-  const double om2 = omega * omega, om3 = om2 * omega;
-  p.S1[0] = 3.0 * (1.0 - 2.0 * r);
-  p.S1[1] = -0.5 * c2p2 / c1p4 * om2;
-  p.S1[2] = k2p2;
-  p.S1[3] = 4.0 * I * k1 * q;
-  p.S1[4] = -7.0 * I * k2;
-  p.S1[5] = 24.0 * q;
-  p.S1[6] = mk(-27.0);
-  p.S1[7] = 60.0 * q / ik1;
-  p.S1[8] = -60.0 / ik2;
-  p.S1[9] = 60.0 * q / ik1p2;
-  p.S1[10] = -60.0 / ik2p2;
-  p.S2[0] = 6.0 * r;
-  p.S2[1] = (0.5 / c2p2 + 1.5 * c2p2 / c1p4 - 1.0 / c1p2) * om2;
-  p.S2[2] = 2.0 * c2p2 / c1p4 * (c1p2 / c2p2 - 2.0) * om2;
-  p.S2[3] = 2.0 * I * c2p2 / c1p3 * (8.0 - 3.0 * c1p2 / c2p2) * omega;
-  p.S2[4] = -4.0 * I * k2;
-  p.S2[5] = 6.0 * r * (6.0 - c1p2 / c2p2);
-  p.S2[6] = mk(-24.0);
-  p.S2[7] = r * 60.0 / ik1;
-  p.S2[8] = -60.0 / ik2;
-  p.S2[9] = 60.0 / ik2p2;
-  p.S2[10] = -60.0 / ik2p2;
-  p.S3[0] = 30.0 * (1.0 - r);
-  p.S3[1] = 1.5 * (1.0 / c2p2 - c2p2 / c1p4) * om2;
-  p.S3[2] = -4.0 * r * k1p2;
-  p.S3[3] = 4.0 * k2p2;
-  p.S3[4] = 40.0 * r * I * k1;
-  p.S3[5] = -40.0 * I * k2;
-  p.S3[6] = 180.0 * r;
-  p.S3[7] = mk(-180.0);
-  p.S3[8] = 420.0 * r / ik1;
-  p.S3[9] = -420.0 / ik2;
-  p.S3[10] = 420.0 / ik2p2;
-  p.S3[11] = -420.0 / ik2p2;
-  p.S4[0] = 2.0 * r;
-  p.S4[1] = 0.5 * (c2p2 / c1p4 + 1.0 / c2p2) * om2;
-  p.S4[2] = -2.0 / 5.0 * (1.0 / c2p3 + 2.0 / 3.0 * c2p2 / c1p5) * I * om3;
-  p.S4[3] = 2.0 * I * k2;
-  p.S4[4] = -4.0 * r;
-  p.S4[5] = mk(6.0);
-  p.S4[6] = -12.0 * r / ik1;
-  p.S4[7] = 12.0 / ik2;
-  p.S4[8] = -12.0 / ik2p2;
-  p.S4[9] = 12.0 / ik2p2;
-  p.S5[0] = 2.0 * (1.0 - 3.0 * r);
-  p.S5[1] = (-2.0 / c1p2 + 0.5 / c2p2 + 0.5 * c2p2 / c1p4) * om2;
-  p.S5[2] = (8.0 / 3.0 / c1p3 + 4.0 / 15.0 / c2p3 - 1.0 / c1 / c2p2 - 24.0 / 15.0 * c2p2 / c1p5) * I * om3;
-  p.S5[3] = (-4.0 / c1p2 + 1.0 / c2p2 + 4.0 * c2p2 / c1p4) * om2;
-  p.S5[4] = 4.0 * I * (1.0 / c1 - 2.0 * c2p2 / c1p3) * omega;
-  p.S5[5] = 4.0 * (1.0 - 3.0 * r);
-  p.S5[6] = mk(4.0);
-  p.S5[7] = 12.0 * I * k1 / k2p2;
-  p.S5[8] = -12.0 * I / k2;
-  p.S5[9] = 12.0 / k2p2;
-  p.S5[10] = -12.0 / k2p2;
-  p.cte_d = mk(k1_4Pi);
-  p.cte_s = k1_4Pi * mu;
-  p.ic2 = I / c2;
-  return p;
+template <typename T>
+__device__ __forceinline__ void ip_sbie(const IpCoef<T>& c, const double dr[3], const double n[3], double d, const T ut[3],
+                                        const T uu[3], double rs, T du[3]) {
+  const T a = ut[0] * dr[0] + ut[1] * dr[1] + ut[2] * dr[2], b = uu[0] * dr[0] + uu[1] * dr[1] + uu[2] * dr[2];
+  const T w = uu[0] * n[0] + uu[1] * n[1] + uu[2] * n[2];
+  const T A = -(c.chi * a) - (c.TT1 * (b * d) + c.TT3 * w) * rs;
+  const T h2 = c.TT2 * rs;
+#pragma unroll
+  for (int l = 0; l < 3; ++l) du[l] = du[l] + c.psi * ut[l] + A * dr[l] - h2 * (b * n[l] + uu[l] * d);
 }
-
-// E_2..E_6 of z (numerical.f90:1258-1331), as zexp_2to5 plus E_6
-__device__ __forceinline__ void zexp_2to6(const ZexpSteps& steps, cd z, cd E[7]) {
-  const double az2 = z.re * z.re + z.im * z.im;
-  cd z2 = z * z, z3 = z2 * z, z4 = z3 * z, z5 = z4 * z;
-  if (az2 <= 1.0) {
-    const int N = zexp_nterms(steps, az2) + 6;
-    cd t = mk(1.0);
-    for (int k = N; k >= 7; --k) t = 1.0 + t * z * (1.0 / (double)k);
-    E[6] = ((z5 * z) * (1.0 / 720.0)) * t;
-    E[5] = E[6] + z5 * (1.0 / 120.0);
-    E[4] = E[5] + z4 * (1.0 / 24.0);
-    E[3] = E[4] + z3 * (1.0 / 6.0);
-    E[2] = E[3] + z2 * 0.5;
-  } else {
-    E[2] = (cexp_(z) - 1.0) - z;
-    E[3] = E[2] - 0.5 * z2;
-    E[4] = E[3] - (1.0 / 6.0) * z3;
-    E[5] = E[4] - (1.0 / 24.0) * z4;
-    E[6] = E[5] - (1.0 / 120.0) * z5;
+template <typename T>
+__device__ __forceinline__ void ip_hbie(const IpCoef<T>& c, const double dr[3], const double n[3], double d, const T ut[3],
+                                        const T uu[3], double rs, T sg[6]) {
+  const T a = ut[0] * dr[0] + ut[1] * dr[1] + ut[2] * dr[2], b = uu[0] * dr[0] + uu[1] * dr[1] + uu[2] * dr[2];
+  const T w = uu[0] * n[0] + uu[1] * n[1] + uu[2] * n[2];
+  const T bd = b * d;
+  const T A = -(c.TT1 * a) - (c.S2 * w - c.S3 * bd) * rs, D = -(c.TT3 * a) - (c.S2 * bd + c.S5 * w) * rs;
+  const T s1 = c.S1 * (-rs), s4 = c.S4 * (-rs);
+  T V[3], W[3];
+#pragma unroll
+  for (int l = 0; l < 3; ++l) {
+    V[l] = s1 * (uu[l] * d + b * n[l]) - c.TT2 * ut[l];
+    W[l] = s4 * uu[l];
   }
+  int q = 0;
+#pragma unroll
+  for (int l = 0; l < 3; ++l)
+#pragma unroll
+    for (int k = l; k < 3; ++k, ++q) {
+      T v = A * (dr[l] * dr[k]) + V[l] * dr[k] + V[k] * dr[l] + W[l] * n[k] + W[k] * n[l];
+      if (l == k) v = v + D;
+      sg[q] = sg[q] + v;
+    }
+}
+__device__ __forceinline__ double ip_geo(const double rv[3], const double n[3], double dr[3], double& d1r, double& drdn) {
+  const double r = sqrt(rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2]);
+  d1r = 1.0 / r;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) dr[c] = rv[c] * d1r;
+  drdn = dr[0] * n[0] + dr[1] * n[1] + dr[2] * n[2];
+  return r;
 }
 
-// The contraction of one quadrature point: u-part (SBIE) and sigma-part (HBIE
-// with the three unit normals), already multiplied by the nodal values' weighted
-// sums ut (tractions) and uu (displacements). rs = -1 for a reversed element.
 struct IpStatic {
   typedef double T;
   StaelaP k;
   double nu, cted1, cted2, ctes1, ctes2, ctes3, mu = 0.0;
   __device__ void sbie(int, const double*, const double rv[3], const double n[3], const T ut[3], const T uu[3], double rs,
                        T du[3]) const {
-    double fu[9], ft[9];
-    staela_point(k, rv, n, fu, ft);
-#pragma unroll
-    for (int il = 0; il < 3; ++il) {
-      double g = 0.0, h = 0.0;
-#pragma unroll
-      for (int ik = 0; ik < 3; ++ik) {
-        g += fu[3 * il + ik] * ut[ik];
-        h += ft[3 * il + ik] * uu[ik];
-      }
-      du[il] += k.cteu1 * g - rs * k.ctet1 * h;
-    }
+    double dr[3], d1r, d;
+    ip_geo(rv, n, dr, d1r, d);
+    const double cu = k.cteu1 * d1r, ct = k.ctet1 * d1r * d1r;
+    IpCoef<double> c;
+    c.psi = cu * k.cteu2; c.chi = -cu; c.TT1 = 3.0 * ct; c.TT2 = k.ctet2 * ct; c.TT3 = -c.TT2;
+    ip_sbie(c, dr, n, d, ut, uu, rs, du);
   }
   __device__ void hbie(int, const double*, const double rv[3], const double n[3], const T ut[3], const T uu[3], double rs,
-                       T sg[3][3]) const {
-    const double r = sqrt(rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2]);
-    const double d1r = 1.0 / r, d1r2 = d1r * d1r, d1r3 = d1r2 * d1r;
-    const double dr[3] = {rv[0] * d1r, rv[1] * d1r, rv[2] * d1r};
-    const double drdn = dr[0] * n[0] + dr[1] * n[1] + dr[2] * n[2];
-#pragma unroll 1
-    for (int kc = 0; kc < 3; ++kc) {
-      const double drdni = -dr[kc], nni = n[kc];
-#pragma unroll
-      for (int il = 0; il < 3; ++il) {
-        double l = 0.0, m = 0.0;
-#pragma unroll
-        for (int ik = 0; ik < 3; ++ik) {
-          const double dk = il == ik ? 1.0 : 0.0, nil = il == kc ? 1.0 : 0.0, nik = ik == kc ? 1.0 : 0.0;
-          const double fd = d1r2 * ((cted2 * dk + 3.0 * dr[il] * dr[ik]) * drdni + cted2 * (nil * dr[ik] - nik * dr[il]));
-          const double fs = d1r3 * (3.0 * (5.0 * dr[il] * dr[ik] - nu * dk) * drdn * drdni +
-                                    3.0 * ctes2 * (dr[ik] * nil * drdn - dr[il] * n[ik] * drdni) +
-                                    3.0 * nu * (dr[il] * nik * drdn - dr[ik] * n[il] * drdni) +
-                                    (3.0 * nu * dr[il] * dr[ik] + ctes2 * dk) * nni + ctes2 * n[il] * nik -
-                                    ctes3 * n[ik] * nil);
-          l += fd * ut[ik];
-          m += fs * uu[ik];
-        }
-        sg[il][kc] += cted1 * l - rs * ctes1 * m;
-      }
-    }
+                       T sg[6]) const {
+    double dr[3], d1r, d;
+    ip_geo(rv, n, dr, d1r, d);
+    const double cd_ = cted1 * d1r * d1r, cs = ctes1 * d1r * d1r * d1r;
+    IpCoef<double> c;
+    c.TT1 = 3.0 * cd_; c.TT2 = cted2 * cd_; c.TT3 = -c.TT2;
+    c.S1 = 3.0 * nu * cs; c.S2 = 3.0 * ctes2 * cs; c.S3 = 15.0 * cs; c.S4 = ctes2 * cs; c.S5 = -ctes3 * cs;
+    ip_hbie(c, dr, n, d, ut, uu, rs, sg);
   }
 };
 
+// E_n evaluated directly (wavenumbers or distances beyond the radial table)
 struct IpHarmonic {
   typedef cd T;
   const HarParD* p;
   const HarParH* ph;
   __device__ void sbie(int f, const double*, const double rv[3], const double n[3], const T ut[3], const T uu[3], double rs,
                        T du[3]) const {
-    cd fu[9], ft[9];
-    harela_point(p[f], rv, n, fu, ft);
-#pragma unroll
-    for (int il = 0; il < 3; ++il) {
-      cd g = mk(0.0), h = mk(0.0);
-#pragma unroll
-      for (int ik = 0; ik < 3; ++ik) {
-        g = g + fu[3 * il + ik] * ut[ik];
-        h = h + ft[3 * il + ik] * uu[ik];
-      }
-      du[il] = du[il] + p[f].cte_u * g - (rs * p[f].cte_t) * h;
-    }
+    double dr[3], d1r, d, d1, d2;
+    const HarParD& q = p[f];
+    const double r = ip_geo(rv, n, dr, d1r, d);
+    IpCoef<cd> c;
+    harela_coeffs(q, r, c.psi, c.chi, c.TT1, c.TT2, c.TT3, d1, d2, true);
+    c.psi = q.cte_u * c.psi; c.chi = q.cte_u * c.chi;
+    c.TT1 = q.cte_t * c.TT1; c.TT2 = q.cte_t * c.TT2; c.TT3 = q.cte_t * c.TT3;
+    ip_sbie(c, dr, n, d, ut, uu, rs, du);
   }
   __device__ void hbie(int f, const double*, const double rv[3], const double n[3], const T ut[3], const T uu[3], double rs,
-                       T sg[3][3]) const {
-    const HarParD& q = p[f];
-    const HarParH& s = ph[f];
-    const double r = sqrt(rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2]);
-    const double d1r1 = 1.0 / r, d1r2 = d1r1 * d1r1, d1r3 = d1r2 * d1r1, d1r4 = d1r3 * d1r1, d1r5 = d1r4 * d1r1;
-    const double dr[3] = {rv[0] * d1r1, rv[1] * d1r1, rv[2] * d1r1};
-    const double drdn = dr[0] * n[0] + dr[1] * n[1] + dr[2] * n[2];
-    cd a[7], b[7];
-    zexp_2to6(q.steps, mk(q.k1.im * r, -q.k1.re * r), a);
-    zexp_2to6(q.steps, mk(q.k2.im * r, -q.k2.re * r), b);
-    const double sc[7] = {0.0, 0.0, d1r1, d1r2, d1r3, d1r4, d1r5};
-#pragma unroll
-    for (int j = 2; j < 7; ++j) {
-      a[j] = a[j] * sc[j];
-      b[j] = b[j] * sc[j];
-    }
-    const cd TT1 = q.T1[0] * d1r2 + q.T1[1] + q.T1[2] * a[2] + q.T1[3] * b[2] + q.T1[4] * a[3] + q.T1[5] * b[3] +
-                   q.T1[6] * a[4] + q.T1[7] * b[4] + q.T1[8] * a[5] + q.T1[9] * b[5];
-    const cd TT2 = q.T2[0] * d1r2 + q.T2[1] + q.T2[2] * b[2] + q.T2[3] * a[3] + q.T2[4] * b[3] + q.T2[5] * a[4] +
-                   q.T2[6] * b[4] + q.T2[7] * a[5] + q.T2[8] * b[5];
-    const cd TT3 = q.T3[0] * d1r2 + q.T3[1] + q.T3[2] * a[2] + q.T3[3] * a[3] + q.T3[4] * b[3] + q.T3[5] * a[4] +
-                   q.T3[6] * b[4] + q.T3[7] * a[5] + q.T3[8] * b[5];
-    const cd S1 = s.S1[0] * d1r3 + s.S1[1] * d1r1 + s.S1[2] * b[2] + s.S1[3] * a[3] + s.S1[4] * b[3] +
-                  s.S1[5] * a[4] + s.S1[6] * b[4] + s.S1[7] * a[5] + s.S1[8] * b[5] + s.S1[9] * a[6] + s.S1[10] * b[6];
-    const cd S2 = s.S2[0] * d1r3 + s.S2[1] * d1r1 + s.S2[2] * a[2] + s.S2[3] * a[3] + s.S2[4] * b[3] +
-                  s.S2[5] * a[4] + s.S2[6] * b[4] + s.S2[7] * a[5] + s.S2[8] * b[5] + s.S2[9] * a[6] + s.S2[10] * b[6];
-    const cd S3 = s.S3[0] * d1r3 + s.S3[1] * d1r1 + s.S3[2] * a[2] + s.S3[3] * b[2] + s.S3[4] * a[3] +
-                  s.S3[5] * b[3] + s.S3[6] * a[4] + s.S3[7] * b[4] + s.S3[8] * a[5] + s.S3[9] * b[5] +
-                  s.S3[10] * a[6] + s.S3[11] * b[6];
-    const cd S4 = s.S4[0] * d1r3 + s.S4[1] * d1r1 + s.S4[2] + s.S4[3] * b[3] + s.S4[4] * a[4] + s.S4[5] * b[4] +
-                  s.S4[6] * a[5] + s.S4[7] * b[5] + s.S4[8] * a[6] + s.S4[9] * b[6];
-    const cd S5 = s.S5[0] * d1r3 + s.S5[1] * d1r1 + s.S5[2] + s.S5[3] * a[2] + s.S5[4] * a[3] + s.S5[5] * a[4] +
-                  s.S5[6] * b[4] + s.S5[7] * a[5] + s.S5[8] * b[5] + s.S5[9] * a[6] + s.S5[10] * b[6];
-    const cd cl = s.cte_d, cm = rs * s.cte_s;
-#pragma unroll 1
-    for (int kc = 0; kc < 3; ++kc) {
-      const double drdni = -dr[kc], nni = n[kc];
-#pragma unroll
-      for (int il = 0; il < 3; ++il) {
-        cd l = mk(0.0), m = mk(0.0);
-#pragma unroll
-        for (int ik = 0; ik < 3; ++ik) {
-          const double dk = il == ik ? 1.0 : 0.0, nil = il == kc ? 1.0 : 0.0, nik = ik == kc ? 1.0 : 0.0;
-          const cd fd = TT1 * (dr[il] * dr[ik] * drdni) - TT2 * (-drdni * dk + dr[il] * nik) - TT3 * (dr[ik] * nil);
-          const cd fs = S1 * (dr[il] * nik * drdn - dr[ik] * n[il] * drdni - dk * drdn * drdni + dr[il] * dr[ik] * nni) +
-                        S2 * (dr[ik] * nil * drdn - dr[il] * n[ik] * drdni) + S3 * (dr[il] * dr[ik] * drdn * drdni) +
-                        S4 * (dk * nni + nik * n[il]) + S5 * (n[ik] * nil);
-          l = l + fd * ut[ik];
-          m = m + fs * uu[ik];
-        }
-        sg[il][kc] = sg[il][kc] + cl * l - cm * m;
-      }
-    }
+                       T sg[6]) const {
+    double dr[3], d1r, d;
+    const double r = ip_geo(rv, n, dr, d1r, d);
+    HbieCoefH k;
+    hbie_coef_h(p[f], ph[f], r, true, k);
+    const cd cl = ph[f].cte_d, cm = ph[f].cte_s;
+    IpCoef<cd> c;
+    c.TT1 = cl * k.TT1; c.TT2 = cl * k.TT2; c.TT3 = cl * k.TT3;
+    c.S1 = cm * k.S1; c.S2 = cm * k.S2; c.S3 = cm * k.S3; c.S4 = cm * k.S4; c.S5 = cm * k.S5;
+    ip_hbie(c, dr, n, d, ut, uu, rs, sg);
+  }
+};
+// the same from the call's radial table
+struct IpHarmonicRad {
+  typedef cd T;
+  RadTab t;
+  __device__ void sbie(int f, const double*, const double rv[3], const double n[3], const T ut[3], const T uu[3], double rs,
+                       T du[3]) const {
+    double dr[3], d1r, d, x;
+    const double r = ip_geo(rv, n, dr, d1r, d);
+    const RadF& q = t.f[f];
+    const double2* w = rad_row(t, f, q, r, x);
+    const double d2 = d1r * d1r;
+    IpCoef<cd> c;
+    c.psi = rad_eval(w, x) + q.s[0] * d1r;
+    c.chi = rad_eval(w + kRadC, x) + q.s[1] * d1r;
+    c.TT1 = rad_eval(w + 2 * kRadC, x) + q.s[2] * d2;
+    c.TT2 = rad_eval(w + 3 * kRadC, x) + q.s[3] * d2;
+    c.TT3 = rad_eval(w + 4 * kRadC, x) + q.s[4] * d2;
+    ip_sbie(c, dr, n, d, ut, uu, rs, du);
+  }
+  __device__ void hbie(int f, const double*, const double rv[3], const double n[3], const T ut[3], const T uu[3], double rs,
+                       T sg[6]) const {
+    double dr[3], d1r, d;
+    const double r = ip_geo(rv, n, dr, d1r, d);
+    HbieCoefH k;
+    hbie_coef_rad(t, f, r, d1r, true, k);
+    IpCoef<cd> c;
+    c.TT1 = k.TT1; c.TT2 = k.TT2; c.TT3 = k.TT3;
+    c.S1 = k.S1; c.S2 = k.S2; c.S3 = k.S3; c.S4 = k.S4; c.S5 = k.S5;
+    ip_hbie(c, dr, n, d, ut, uu, rs, sg);
   }
 };
 
@@ -377,7 +297,7 @@ struct IpHsc {
     }
   }
   __device__ void hbie(int, const double* xi, const double rv[3], const double n[3], const T ut[3], const T uu[3],
-                       double rs, T sg[3][3]) const {
+                       double rs, T sg[6]) const {
     // x = image + rv
     const double xq[3] = {xi[0] + rv[0], xi[1] + rv[1], 2.0 * xp - xi[2] + rv[2]};
     HJet xj[3], ij[3];
@@ -408,11 +328,12 @@ struct IpHsc {
           }
           dt[l][k][p] = Ku * v;
         }
-    // d*_lkp, s*_lkp contracted with n_i = e_kc: sg(:, kc) += d ut - rs s uu
+    // d*_lkp, s*_lkp contracted with n_i = e_kc: sg(l, kc) += d ut - rs s uu,
+    // symmetric in (l, kc)
 #pragma unroll 1
-    for (int kc = 0; kc < 3; ++kc)
+    for (int l = 0; l < 3; ++l)
 #pragma unroll 1
-      for (int l = 0; l < 3; ++l) {
+      for (int kc = l; kc < 3; ++kc) {
         double acc = 0.0;
         for (int k = 0; k < 3; ++k) {
           double dl = mu * Ku * (u[l][k].gi[kc] + u[kc][k].gi[l]);
@@ -423,18 +344,10 @@ struct IpHsc {
           }
           acc += dl * ut[k] - rs * sl * uu[k];
         }
-        sg[l][kc] += acc;
+        sg[kc + (l == 1 ? 2 : (l == 2 ? 3 : 0))] += acc;
       }
   }
 };
-
-// q: [nf][6] = lambda (re, im), mu (re, im), rho, omega
-__global__ void k_harparh(const double* q, int nf, HarParH* out) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= nf) return;
-  const double* v = q + 6 * f;
-  out[f] = harela_hbie_params(mk(v[0], v[1]), mk(v[2], v[3]), v[4], v[5]);
-}
 
 // inputs of the internal-point kernels
 struct IpArgs {
@@ -454,8 +367,11 @@ struct IpArgs {
   int* pair_e;           // [npairs]
   int* pair_ip;
   int* err;              // first point (1-based) on an element away from its nodes, 0 if none
-  void* slot;            // [nf][npairs][12] T
+  void* slot;            // [nf][npairs][9] T: u (3), sigma (6)
   int npairs;
+  void* uw;              // [nf][ne ptot][6] T: u_w, t_w at the dataset points
+  void* part;            // [nf][nip][nch][9] T: partial sums of gpc groups of 32 elements each
+  int nch, gpc;
   void* out;             // [nf][nip][12] T: u(3), then sigma(:, kc) for kc = 0..2
   // image pass of a half-space region: pairs classified and integrated from
   // the image (x_i1, x_i2, 2 xp - x_i3) of each point; points at a node add 0
@@ -469,18 +385,20 @@ __device__ __forceinline__ void ip_ref(const IpArgs& a, const double* xi, double
   xr[2] = a.image ? 2.0 * a.hs_xp - xi[2] : xi[2];
 }
 
-// point at a node: the last node (in node order) within 1e-12 csize
+// point at a node: the last node (in node order) within 1e-12 csize; one warp
+// per point
 __global__ void k_ip_onnode(IpArgs a) {
-  const int ip = blockIdx.x * blockDim.x + threadIdx.x;
+  const int ip = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (ip >= a.nip) return;
   const double* x = a.xip + 3 * (size_t)ip;
   int last = -1;
-  for (int s = 0; s < a.nn; ++s) {
+  for (int s = threadIdx.x & 31; s < a.nn; s += 32) {
     if (a.nodecl[s] <= 0.0) continue;  // node of no element
     const double r0 = x[0] - a.nodex[3 * s], r1 = x[1] - a.nodex[3 * s + 1], r2 = x[2] - a.nodex[3 * s + 2];
     if (sqrt(r0 * r0 + r1 * r1 + r2 * r2) / a.nodecl[s] < 1e-12) last = s;
   }
-  a.onnode[ip] = last;
+  last = __reduce_max_sync(0xffffffffu, last);
+  if ((threadIdx.x & 31) == 0) a.onnode[ip] = last;
 }
 
 // sbie_auto / hbie_auto classification of every (point, element) pair
@@ -610,11 +528,9 @@ __global__ void k_ip_adp(DMesh m, IpArgs a, POL pol, const QsCurves* __restrict_
     }
   }
   const double rs = (m.rev[e] & 1) ? -1.0 : 1.0;
-  T du[3], sg[3][3];
-  for (int c = 0; c < 3; ++c) {
-    du[c] = VT<T>::zero();
-    for (int k = 0; k < 3; ++k) sg[c][k] = VT<T>::zero();
-  }
+  T du[3], sg[6];
+  for (int c = 0; c < 3; ++c) du[c] = VT<T>::zero();
+  for (int c = 0; c < 6; ++c) sg[c] = VT<T>::zero();
   const size_t cid = (size_t)ip * m.ne + e;
 #pragma unroll 1
   for (int h = 0; h < 2; ++h) {
@@ -699,82 +615,138 @@ __global__ void k_ip_adp(DMesh m, IpArgs a, POL pol, const QsCurves* __restrict_
       }
     }
   }
-  // the layout of out: u, then sigma(:, kc) for kc = 0..2
-  T* sl = (T*)a.slot + ((size_t)f * a.npairs + pr) * 12;
-  for (int c = 0; c < 3; ++c) {
-    sl[c] = du[c];
-    for (int k = 0; k < 3; ++k) sl[3 + 3 * k + c] = sg[c][k];
-  }
+  T* sl = (T*)a.slot + ((size_t)f * a.npairs + pr) * 9;
+  for (int c = 0; c < 3; ++c) sl[c] = du[c];
+  for (int c = 0; c < 6; ++c) sl[3 + c] = sg[c];
 }
 
-// One warp per (point, frequency): the precalculated-rule pairs of every
-// element on the lanes, then the point's quasi-singular slots in element order.
+// u_w, t_w at every dataset point (all precalculated rules) of every element
+template <typename T>
+__global__ void k_ip_weights(DMesh m, IpArgs a) {
+  const long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x, np = (long long)m.ne * m.ptot;
+  if (id >= np * a.nf) return;
+  const int f = (int)(id / np);
+  const long long pt = id - f * np;
+  const int e = (int)(pt / m.ptot);
+  const T* uv = (const T*)a.uval + (size_t)f * a.nn * 3;
+  const T* tv = (const T*)a.tval + (size_t)f * a.nn * 3;
+  T un[24], tn[24];
+  double w[8];
+#pragma unroll
+  for (int kn = 0; kn < 8; ++kn) {
+    const int s = a.enode[8 * e + kn];
+    w[kn] = m.pphi[8 * pt + kn];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      un[3 * kn + c] = uv[3 * s + c];
+      tn[3 * kn + c] = tv[3 * s + c];
+    }
+  }
+  T* o = (T*)a.uw + 6 * id;
+  ip_weights<T>(un, tn, w, o, o + 3);
+}
+
+// One warp per (gpc groups of 32 elements, point, frequency): the
+// precalculated-rule pairs. gpc is 1 until the points alone fill the GPU.
+// A lane looks up one element's rule; a scan of the point counts then deals the
+// quadrature points of all 32 out to the lanes.
 template <class POL, int WPB>
 __global__ void __launch_bounds__(WPB * 32) k_ip_reg(DMesh m, IpArgs a, POL pol) {
   typedef typename POL::T T;
-  __shared__ T nv[WPB][48];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const long long gw = blockIdx.x * (long long)WPB + w;
-  if (gw >= (long long)a.nip * a.nf) return;
-  const int ip = (int)(gw % a.nip), f = (int)(gw / a.nip);
-  T* o = (T*)a.out + ((size_t)f * a.nip + ip) * 12;
-  const T* uv = (const T*)a.uval + (size_t)f * a.nn * 3;
-  const T* tv = (const T*)a.tval + (size_t)f * a.nn * 3;
-  const int on = a.onnode[ip];
-  if (on >= 0) {
-    if (lane < 12) o[lane] = (lane < 3 && !a.image) ? uv[3 * on + lane] : VT<T>::zero();
-    return;
-  }
+  const int lane = threadIdx.x & 31;
+  const long long gw = blockIdx.x * (long long)WPB + (threadIdx.x >> 5);
+  if (gw >= (long long)a.nip * a.nf * a.nch) return;
+  const int ch = (int)(gw % a.nch), ip = (int)((gw / a.nch) % a.nip), f = (int)(gw / a.nch / a.nip);
+  if (a.onnode[ip] >= 0) return;
   const double* xi = a.xip + 3 * (size_t)ip;
   double xr[3];
   ip_ref(a, xi, xr);
-  T du[3], sg[3][3];
-  for (int c = 0; c < 3; ++c) {
-    du[c] = VT<T>::zero();
-    for (int k = 0; k < 3; ++k) sg[c][k] = VT<T>::zero();
-  }
-  for (int e = 0; e < m.ne; ++e) {
-    const size_t cid = (size_t)ip * m.ne + e;
-    const uint8_t cs = a.cls_s[cid], ch = a.cls_h[cid];
-    if (cs == CLS_SING || ch == CLS_SING) continue;
-    if (cs >= CLS_ADP && ch >= CLS_ADP) continue;
-    __syncwarp();
-    for (int j = lane; j < 48; j += 32) {
-      const int kn = (j % 24) / 3, c = j % 3, s = a.enode[8 * e + kn];
-      nv[w][j] = j < 24 ? uv[3 * s + c] : tv[3 * s + c];
-    }
-    __syncwarp();
-    const double rs = (m.rev[e] & 1) ? -1.0 : 1.0;
+  const T* uw = (const T*)a.uw + (size_t)f * m.ne * m.ptot * 6;
+  T du[3], sg[6];
+  for (int c = 0; c < 3; ++c) du[c] = VT<T>::zero();
+  for (int c = 0; c < 6; ++c) sg[c] = VT<T>::zero();
+  unsigned revs = 0;
+  int cls_s = CLS_SING, cls_h = CLS_SING, e = 0;
+  const int g0 = ch * a.gpc, g1 = min(g0 + a.gpc, (m.ne + 31) / 32);
 #pragma unroll 1
-    for (int h = 0; h < 2; ++h) {
-      const uint8_t c = h ? ch : cs;
-      if (c >= CLS_ADP) continue;
-      const int P = m.ps_gln[c] * m.ps_gln[c];
-      for (int k = lane; k < P; k += 32) {
-        const size_t pt = (size_t)e * m.ptot + m.ps_off[c] + k;
-        const double rv[3] = {m.px[3 * pt] - xr[0], m.px[3 * pt + 1] - xr[1], m.px[3 * pt + 2] - xr[2]};
-        const double n[3] = {m.pn[3 * pt], m.pn[3 * pt + 1], m.pn[3 * pt + 2]};
-        double wq[8];
-        for (int q = 0; q < 8; ++q) wq[q] = m.pphi[8 * pt + q];
-        T uu[3], ut[3];
-        ip_weights<T>(nv[w], nv[w] + 24, wq, uu, ut);
+  for (int hg = 2 * g0; hg < 2 * g1; ++hg) {
+    const int h = hg & 1;
+    if (h == 0) {
+      e = 16 * hg + lane;
+      int rev = 0;
+      cls_s = cls_h = CLS_SING;
+      if (e < m.ne) {
+        const size_t cid = (size_t)ip * m.ne + e;
+        cls_s = a.cls_s[cid];
+        cls_h = a.cls_h[cid];
+        rev = m.rev[e] & 1;
+        if (cls_s == CLS_SING || cls_h == CLS_SING) cls_s = cls_h = CLS_SING;
+      }
+      revs = __ballot_sync(0xffffffffu, rev);
+    }
+    const int c = h ? cls_h : cls_s, P = c >= CLS_ADP ? 0 : m.ps_gln[c] * m.ps_gln[c];
+    int end = P;  // inclusive scan
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, end, o);
+      if (lane >= o) end += v;
+    }
+    const int total = __shfl_sync(0xffffffffu, end, 31);
+    // dataset index of scan position q of this lane's element: first + q
+    const int first = P > 0 ? e * m.ptot + m.ps_off[c] - (end - P) : 0;
+#pragma unroll 1
+    for (int base = 0; base < total; base += 32) {
+      const int q = base + lane;
+      int j = 0;  // lanes whose range ends at or before q
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+        if (__shfl_sync(0xffffffffu, end, j + o - 1) <= q) j += o;
+      j = min(j, 31);
+      const int pt = __shfl_sync(0xffffffffu, first, j) + q;
+      if (q < total) {
+        const double rs = (revs >> j) & 1 ? -1.0 : 1.0;
+        const double rv[3] = {m.px[3 * (size_t)pt] - xr[0], m.px[3 * (size_t)pt + 1] - xr[1], m.px[3 * (size_t)pt + 2] - xr[2]};
+        const double n[3] = {m.pn[3 * (size_t)pt], m.pn[3 * (size_t)pt + 1], m.pn[3 * (size_t)pt + 2]};
+        const T* v = uw + 6 * (size_t)pt;
+        const T uu[3] = {v[0], v[1], v[2]}, ut[3] = {v[3], v[4], v[5]};
         if (h) pol.hbie(f, xi, rv, n, ut, uu, rs, sg);
         else pol.sbie(f, xi, rv, n, ut, uu, rs, du);
       }
     }
   }
-  T acc[12];
-  for (int c = 0; c < 3; ++c) {
-    acc[c] = du[c];
-    for (int k = 0; k < 3; ++k) acc[3 + 3 * k + c] = sg[c][k];
+  T* o = (T*)a.part + 9 * (size_t)(((size_t)f * a.nip + ip) * a.nch + ch);
+#pragma unroll
+  for (int j = 0; j < 9; ++j) {
+    T v = j < 3 ? du[j < 3 ? j : 0] : sg[j < 3 ? 0 : j - 3];
+    for (int off = 16; off > 0; off >>= 1) v = v + shfl_x(v, off);
+    if (lane == 0) o[j] = v;
   }
-  for (int j = 0; j < 12; ++j)
-    for (int off = 16; off > 0; off >>= 1) acc[j] = acc[j] + shfl_x(acc[j], off);
-  if (lane == 0) {
+}
+
+// Sums of a point: its element groups, then its quasi-singular slots, in
+// order; one thread per (component, point, frequency)
+template <typename T>
+__global__ void k_ip_sum(IpArgs a) {
+  const long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (id >= 9LL * a.nip * a.nf) return;
+  const int j = (int)(id % 9), ip = (int)((id / 9) % a.nip), f = (int)(id / 9 / a.nip);
+  const int on = a.onnode[ip];
+  T v = VT<T>::zero();
+  if (on >= 0) {
+    if (j < 3 && !a.image) v = ((const T*)a.uval)[((size_t)f * a.nn + on) * 3 + j];
+  } else {
+    const T* p = (const T*)a.part + 9 * (size_t)(((size_t)f * a.nip + ip) * a.nch);
+    for (int ch = 0; ch < a.nch; ++ch) v = v + p[9 * ch + j];
     const T* sl = (const T*)a.slot;
-    for (int pr = a.poff[ip]; pr < a.poff[ip + 1]; ++pr)
-      for (int j = 0; j < 12; ++j) acc[j] = acc[j] + sl[((size_t)f * a.npairs + pr) * 12 + j];
-    for (int j = 0; j < 12; ++j) o[j] = acc[j];
+    for (int pr = a.poff[ip]; pr < a.poff[ip + 1]; ++pr) v = v + sl[((size_t)f * a.npairs + pr) * 9 + j];
+  }
+  T* o = (T*)a.out + ((size_t)f * a.nip + ip) * 12;
+  if (j < 3) {
+    o[j] = v;
+  } else {
+    const int l = sym_il(j - 3), k = sym_ik(j - 3);
+    o[3 + 3 * k + l] = v;
+    o[3 + 3 * l + k] = v;
   }
 }
 

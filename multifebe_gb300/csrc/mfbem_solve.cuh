@@ -1588,7 +1588,7 @@ extern "C" int mfbem_sweep_harela(mfbem_handle* h, const double lambda[2], const
   PolHarmonicRad pr;
   pr.p = dpar;
   if ((rc = hbie_params(h, dq, n_freq, &pr.ph)) ||
-      (rc = radial_prepare(h, q.data(), n_freq, dpar, pr.ph, precision >= 1, &pr.t)))
+      (rc = radial_prepare(h, h->rmax, q.data(), n_freq, dpar, pr.ph, precision >= 1, &pr.t)))
     return rc;
   PolHarmonic pol;
   pol.p = dpar;
