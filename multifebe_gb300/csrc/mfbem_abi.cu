@@ -1812,11 +1812,11 @@ extern "C" int mfbem_internal_f64_gemm(int32_t cplx, int32_t m, int32_t n, int32
     if (!rc) rc = oz_err_check(0);
   } else {
     if (cplx)
-      k_gemm_simt<double2><<<dim3(nblk(m, 64), nblk(n, 64), 1), 256>>>((const double2*)dA.p, m, 0,
+      k_gemm_simt<double2, 4><<<dim3(nblk(m, 64), nblk(n, 64), 1), 256>>>((const double2*)dA.p, m, 0,
                                                                         (const double2*)dB.p, k, 0, (double2*)dC.p, m,
                                                                         0, m, n, k);
     else
-      k_gemm_simt<double><<<dim3(nblk(m, 64), nblk(n, 64), 1), 256>>>((const double*)dA.p, m, 0, (const double*)dB.p,
+      k_gemm_simt<double, 4><<<dim3(nblk(m, 64), nblk(n, 64), 1), 256>>>((const double*)dA.p, m, 0, (const double*)dB.p,
                                                                        k, 0, (double*)dC.p, m, 0, m, n, k);
     ++g_launches;
     rc = cudaGetLastError() == cudaSuccess ? 0 : fail(MFBEM_ECUDA, "f64 gemm launch");

@@ -61,7 +61,15 @@ template <> struct Sc<double2> {
     cd q = mk(a.x, a.y) / mk(b.x, b.y);
     return make_double2(q.re, q.im);
   }
-  __device__ static double2 rcp(double2 a) { return div(one(), a); }
+  // Smith's scaled reciprocal, two divisions
+  __device__ static double2 rcp(double2 a) {
+    if (fabs(a.x) >= fabs(a.y)) {
+      const double r = a.y / a.x, d = 1.0 / (a.x + a.y * r);
+      return make_double2(d, -r * d);
+    }
+    const double r = a.x / a.y, d = 1.0 / (a.y + a.x * r);
+    return make_double2(r * d, -d);
+  }
   __device__ static bool iszero(double2 a) { return a.x == 0.0 && a.y == 0.0; }
   __device__ static double2 conj(double2 a) { return make_double2(a.x, -a.y); }
   __device__ static double2 from(double v) { return make_double2(v, 0.0); }
@@ -89,6 +97,17 @@ template <> struct Sc<float2> {
   __device__ static float2 from(double v) { return make_float2((float)v, 0.f); }
   __device__ static float re(float2 a) { return a.x; }
 };
+
+// a value of another lane
+template <typename S> __device__ __forceinline__ S shfl_s(S v, int src);
+template <> __device__ __forceinline__ float2 shfl_s(float2 v, int src) {
+  return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+}
+template <> __device__ __forceinline__ double2 shfl_s(double2 v, int src) {
+  return make_double2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+}
+template <> __device__ __forceinline__ float shfl_s(float v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+template <> __device__ __forceinline__ double shfl_s(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
 
 // ---------------------------------------------------------------------------
 // Panel factorisation, one CTA per matrix (used where the panel's arithmetic
@@ -387,30 +406,95 @@ __global__ void __launch_bounds__(NT) k_panel_coop(S* A, long long strideA, int 
 }
 
 // ---------------------------------------------------------------------------
-// Cluster panel: the same algorithm as k_panel_coop with the G CTAs of a
-// matrix forming one thread-block cluster (cluster rank = row chunk): the
-// per-column exchange goes through distributed shared memory and the
-// hardware cluster barrier instead of global memory and a spin on a counter.
-// Candidate slots are double-buffered by column parity, so one cluster
-// barrier per column suffices: a slot written at column j + 2 is read by
-// everyone before the barrier of column j + 1.
+// Cluster panel: the same pivoting as k_panel_coop with the G CTAs of a matrix
+// forming one thread-block cluster (cluster rank = row chunk). Per column each
+// CTA pushes its candidate (|a| as an ordered integer key, row, the row's kb
+// values, the reciprocal of its pivot) into every CTA's shared memory, one
+// hardware cluster barrier follows, and each warp picks the winner from local
+// memory: no remote read and no block barrier lies between the cluster barrier
+// and the update. The candidate of the next column is taken while its values
+// are updated. Slots are double-buffered by column parity: a slot of column
+// j + 2 is written after the barrier of column j + 1, which every CTA enters
+// after its last read of column j's.
+//
+// GB300's binary64 pipe takes 16 cycles per warp instruction whatever the
+// number of active lanes, so binary64 operations outside the rank-1 update
+// decide the time of a small panel: the reciprocal of the pivot is formed by
+// one warp per CTA, while the others push the rows, instead of by every thread
+// (30 to 100 operations each); the pivot search compares integers (redux);
+// complex updates use four FMAs. A column of an 870-row real panel takes 4800
+// cycles (barriers and exchange 1600, reciprocal and pushes 1500, update 1400),
+// 7600 before; 217 panels of four complex 3462-row systems 32.1 -> 12 ms with
+// 16 CTAs per matrix.
+// A NaN counts as zero in the search; the row jj itself is then taken.
 // ---------------------------------------------------------------------------
+// |a| ordered as an unsigned integer, 0 for NaN
+__device__ __forceinline__ unsigned long long piv_key(double v) {
+  const unsigned long long k = (unsigned long long)__double_as_longlong(v);
+  return k > 0x7ff0000000000000ull ? 0ull : k;
+}
+__device__ __forceinline__ unsigned long long piv_key(float v) {
+  const unsigned k = __float_as_uint(v);
+  return k > 0x7f800000u ? 0ull : (unsigned long long)k;
+}
+// the warp's largest key and, among its holders, the smallest row (key + 1 and
+// row as unsigned; no candidate: key1 = 0, row = ~0u)
+__device__ __forceinline__ void piv_reduce(unsigned long long& key1, unsigned& row) {
+  const unsigned hi = (unsigned)(key1 >> 32), lo = (unsigned)key1;
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+  row = __reduce_min_sync(0xffffffffu, hi == mh && lo == ml ? row : 0xffffffffu);
+  key1 = ((unsigned long long)mh << 32) | ml;
+}
+// 1 / d by two Newton steps from the binary32 reciprocal (2^-23 -> 2^-46 -> the
+// rounding of the last step) where d and 1 / d are well inside binary32's
+// range: on the chain of every column, where a dependent binary64 operation
+// takes 63 cycles and more
+__device__ __forceinline__ double piv_rcp(double d) {
+  const float f = fabsf((float)d);
+  if (!(f > 1e-36f && f < 1e36f)) return 1.0 / d;
+  double y = (double)__frcp_rn((float)d);
+  y = fma(y, fma(-d, y, 1.0), y);
+  return fma(y, fma(-d, y, 1.0), y);
+}
+// conj(d) / |d|^2 where |d|^2 stays within that range, else Smith's form
+__device__ __forceinline__ double2 piv_rcp(double2 d) {
+  const double q = fma(d.x, d.x, d.y * d.y);
+  const float f = (float)q;
+  if (!(f > 1e-36f && f < 1e36f)) return Sc<double2>::rcp(d);
+  const double y = piv_rcp(q);
+  return make_double2(d.x * y, -d.y * y);
+}
+__device__ __forceinline__ float piv_rcp(float d) { return 1.0f / d; }
+__device__ __forceinline__ float2 piv_rcp(float2 d) { return Sc<float2>::rcp(d); }
+// a - l p
+__device__ __forceinline__ double lu_fnma(double l, double p, double a) { return fma(-l, p, a); }
+__device__ __forceinline__ float lu_fnma(float l, float p, float a) { return fmaf(-l, p, a); }
+__device__ __forceinline__ double2 lu_fnma(double2 l, double2 p, double2 a) {
+  return make_double2(fma(-l.x, p.x, fma(l.y, p.y, a.x)), fma(-l.x, p.y, fma(-l.y, p.x, a.y)));
+}
+__device__ __forceinline__ float2 lu_fnma(float2 l, float2 p, float2 a) {
+  return make_float2(fmaf(-l.x, p.x, fmaf(l.y, p.y, a.x)), fmaf(-l.x, p.y, fmaf(-l.y, p.x, a.y)));
+}
+// bytes of dynamic shared memory of k_panel_cluster
+template <typename S>
+inline size_t panel_cluster_smem(int G, int kb, int chunk) {
+  return sizeof(S) * (((size_t)kb * chunk + 3) / 4 * 4 + 2 * (size_t)G * (kb + 1) + 2 * (size_t)kb) + 2 * (size_t)G * 16 + 32;
+}
 template <typename S, int NT>
 __global__ void __launch_bounds__(NT) k_panel_cluster(S* A, long long strideA, int lda, int n, int k, int kb,
                                                       int chunk, int* ipiv, int* info) {
   namespace cg = cooperative_groups;
-  typedef typename Sc<S>::R R;
   cg::cluster_group cl = cg::this_cluster();
   const int G = (int)cl.num_blocks(), g = (int)cl.block_rank();
   extern __shared__ __align__(16) unsigned char smraw[];
-  S* pan = reinterpret_cast<S*>(smraw);  // [kb][chunk]
-  S* prow = pan + (size_t)kb * chunk;     // [kb] pivot row
-  S* xrow = prow + 32;                    // [2][2][32]: slot parity x {candidate row, row jj}
-  R* xval = reinterpret_cast<R*>(xrow + 2 * 2 * 32);  // [2]
-  int* xidx = reinterpret_cast<int*>(xval + 2);        // [2]
-  __shared__ R sv[NT / 32];
-  __shared__ int si[NT / 32];
-  __shared__ int s_p;
+  S* pan = reinterpret_cast<S*>(smraw);          // [kb][chunk]
+  S* cand = pan + ((size_t)kb * chunk + 3) / 4 * 4;  // [2][G][kb + 1]: candidate row, reciprocal of its pivot
+  S* rowj = cand + 2 * (size_t)G * (kb + 1);     // [2][kb]: row jj before the interchange
+  unsigned long long* ckey = reinterpret_cast<unsigned long long*>(rowj + 2 * (size_t)kb);  // [2][G] key + 1
+  unsigned* crow = reinterpret_cast<unsigned*>(ckey + 2 * (size_t)G);                      // [2][G]
+  __shared__ unsigned long long wkey[NT / 32];
+  __shared__ unsigned wrow[NT / 32];
   const int mat = blockIdx.x / G;
   const int lane = threadIdx.x & 31, wid = threadIdx.x / 32;
   S* M = A + strideA * mat;
@@ -421,93 +505,209 @@ __global__ void __launch_bounds__(NT) k_panel_cluster(S* A, long long strideA, i
     pan[(size_t)c * chunk + i] = M[(size_t)(k + c) * lda + r0 + i];
   }
   __syncthreads();
+  unsigned long long bk = 0;  // this thread's candidate: key + 1, row
+  unsigned br = 0xffffffffu;
+  for (int i = threadIdx.x; i < nr; i += NT) {
+    const unsigned long long q = piv_key(Sc<S>::abs1(pan[i])) + 1;
+    if (q > bk) { bk = q; br = (unsigned)(r0 + i); }
+  }
+  cl.sync();  // every CTA of the cluster runs before the first push
   for (int j = 0; j < kb; ++j) {
     const int jj = k + j, slot = j & 1;
-    R best = -1;
-    int bi = -1;
-    for (int i = max(jj, r0) - r0 + threadIdx.x; i < nr; i += NT) {
-      const R v = Sc<S>::abs1(pan[(size_t)j * chunk + i]);
-      if (v > best) { best = v; bi = r0 + i; }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      const R ov = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ov > best || (ov == best && oi >= 0 && (bi < 0 || oi < bi))) { best = ov; bi = oi; }
-    }
-    if (lane == 0) { sv[wid] = best; si[wid] = bi; }
+    piv_reduce(bk, br);
+    if (lane == 0) { wkey[wid] = bk; wrow[wid] = br; }
     __syncthreads();
-    // the CTA's candidate: warp 0 reduces the warps' (larger |a|, then the
-    // smaller row; no row = -1 loses), then stages it and row jj
-    if (wid == 0) {
-      R v = lane < NT / 32 ? sv[lane] : (R)-1;
-      int ix = lane < NT / 32 ? si[lane] : -1;
-      for (int o = 16; o > 0; o >>= 1) {
-        const R ov = __shfl_xor_sync(0xffffffffu, v, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, ix, o);
-        if (oi >= 0 && (ix < 0 || ov > v || (ov == v && oi < ix))) { v = ov; ix = oi; }
-      }
-      if (lane == 0) {
-        xval[slot] = v;
-        xidx[slot] = ix;
-      }
-      if (lane < kb) {
-        if (ix >= 0) xrow[(slot * 2 + 0) * 32 + lane] = pan[(size_t)lane * chunk + (ix - r0)];
-        if (jj >= r0 && jj < r1) xrow[(slot * 2 + 1) * 32 + lane] = pan[(size_t)lane * chunk + (jj - r0)];
+    {
+      // every warp finds the CTA's candidate; warp 0 pushes its key and the
+      // reciprocal of its pivot, the others its row (and row jj)
+      unsigned long long q = lane < NT / 32 ? wkey[lane] : 0ull;
+      unsigned r = lane < NT / 32 ? wrow[lane] : 0xffffffffu;
+      piv_reduce(q, r);
+      const bool have = q != 0ull, own = jj >= r0 && jj < r1;
+      const int ix = have ? (int)r - r0 : 0;
+      if (wid == 0) {
+        if (have) {
+          const S d = pan[(size_t)j * chunk + ix];
+          const S rc = q == 1ull && Sc<S>::iszero(d) ? d : piv_rcp(d);
+          if (lane < G) cl.map_shared_rank(cand, lane)[((size_t)slot * G + g) * (kb + 1) + kb] = rc;
+        }
+        if (lane < G) {
+          cl.map_shared_rank(ckey, lane)[slot * G + g] = q;
+          cl.map_shared_rank(crow, lane)[slot * G + g] = r;
+        }
+      } else if (lane < kb) {
+        const S v = pan[(size_t)lane * chunk + ix], vj = own ? pan[(size_t)lane * chunk + (jj - r0)] : v;
+        for (int rk = wid - 1; rk < G; rk += NT / 32 - 1) {
+          if (have) cl.map_shared_rank(cand, rk)[((size_t)slot * G + g) * (kb + 1) + lane] = v;
+          if (own) cl.map_shared_rank(rowj, rk)[slot * kb + lane] = vj;
+        }
       }
     }
     cl.sync();
-    // winner over the cluster's candidates: warp 0 reads the G ranks' slots of
-    // distributed shared memory in parallel (one lane each), reduces with the
-    // same order, fetches the pivot row and interchanges rows p and jj
-    if (wid == 0) {
-      R v = (R)-1;
-      int ix = -1, gq = lane;
-      if (lane < G) {
-        v = cl.map_shared_rank(xval, lane)[slot];
-        ix = cl.map_shared_rank(xidx, lane)[slot];
-      }
-      for (int o = 16; o > 0; o >>= 1) {
-        const R ov = __shfl_xor_sync(0xffffffffu, v, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, ix, o);
-        const int og = __shfl_xor_sync(0xffffffffu, gq, o);
-        if (oi >= 0 && (ix < 0 || ov > v || (ov == v && oi < ix))) { v = ov; ix = oi; gq = og; }
-      }
-      const int own = (jj - k) / chunk;  // rank owning row jj
-      if (lane < kb) {
-        const S pr = cl.map_shared_rank(xrow, gq)[(slot * 2 + 0) * 32 + lane];
-        prow[lane] = pr;
-        if (ix != jj) {
-          if (ix >= r0 && ix < r1)
-            pan[(size_t)lane * chunk + (ix - r0)] = cl.map_shared_rank(xrow, own)[(slot * 2 + 1) * 32 + lane];
-          if (jj >= r0 && jj < r1) pan[(size_t)lane * chunk + (jj - r0)] = pr;
-        }
-      }
-      if (lane == 0) s_p = ix;
-    }
-    __syncthreads();
-    const int p = s_p;
+    unsigned long long q = lane < G ? ckey[slot * G + lane] : 0ull;
+    const unsigned long long q0 = q;
+    unsigned r = lane < G ? crow[slot * G + lane] : 0xffffffffu;
+    const unsigned rr = r;
+    piv_reduce(q, r);
+    const int win = __ffs(__ballot_sync(0xffffffffu, lane < G && q0 == q && rr == r)) - 1;
+    const int p = (int)r;
+    const S* pr = cand + ((size_t)slot * G + win) * (kb + 1);
+    const S* oj = rowj + slot * kb;
+    const bool zero = q == 1ull && Sc<S>::iszero(pr[j]);  // key 0: zero or NaN
     if (g == 0 && threadIdx.x == 0) {
       piv[jj] = p + 1;
-      if (Sc<S>::iszero(prow[j]) && info[mat] == 0) info[mat] = jj + 1;
+      if (zero && info[mat] == 0) info[mat] = jj + 1;
     }
-    const S dj = prow[j];
-    if (!Sc<S>::iszero(dj)) {
-      const S rcp = Sc<S>::rcp(dj);
-      for (int i = max(jj + 1, r0) - r0 + threadIdx.x; i < nr; i += NT) {
-        const S l = Sc<S>::mul(pan[(size_t)j * chunk + i], rcp);
-        pan[(size_t)j * chunk + i] = l;
-        for (int c = j + 1; c < kb; ++c)
-          pan[(size_t)c * chunk + i] = Sc<S>::sub(pan[(size_t)c * chunk + i], Sc<S>::mul(l, prow[c]));
+    if (jj >= r0 && jj < r1 && p != jj && (int)threadIdx.x < kb)
+      pan[(size_t)threadIdx.x * chunk + (jj - r0)] = pr[threadIdx.x];
+    const S rcp = pr[kb];
+    bk = 0;
+    br = 0xffffffffu;
+    for (int i = max(jj + 1, r0) - r0 + threadIdx.x; i < nr; i += NT) {
+      S* x = pan + i;
+      if (r0 + i == p) {  // takes row jj's place in the interchange
+        for (int c = 0; c < kb; ++c) x[(size_t)c * chunk] = oj[c];
+      }
+      if (!zero) {
+        const S l = Sc<S>::mul(x[(size_t)j * chunk], rcp);
+        x[(size_t)j * chunk] = l;
+#pragma unroll 5
+        for (int c = j + 1; c < kb; ++c) x[(size_t)c * chunk] = lu_fnma(l, pr[c], x[(size_t)c * chunk]);
+      }
+      if (j + 1 < kb) {
+        const unsigned long long qn = piv_key(Sc<S>::abs1(x[(size_t)(j + 1) * chunk])) + 1;
+        if (qn > bk) { bk = qn; br = (unsigned)(r0 + i); }
       }
     }
-    __syncthreads();
   }
+  __syncthreads();
   for (int t = threadIdx.x; t < kb * nr; t += NT) {
     const int c = t / nr, i = t - c * nr;
     M[(size_t)(k + c) * lda + r0 + i] = pan[(size_t)c * chunk + i];
   }
-  // no CTA may exit while others can still read its shared memory
-  cl.sync();
+}
+
+// ---------------------------------------------------------------------------
+// Interchanges of a 16-column panel applied to every column outside it and, for
+// the columns [k + kb, ce), U12 = inv(L11) A12 in the same pass (one launch in
+// place of k_laswp and k_trsm_cols). A warp composes the up to 16 interchanges
+// into "position R_q takes the entry of C_q" for at most 32 positions (lanes 0..
+// 15: the panel's rows, the others: rows below it), so a thread's loads of its
+// column are independent instead of a chain of 16 exchanges through memory;
+// the substitution runs on registers. One column per thread, 32 per CTA.
+// ---------------------------------------------------------------------------
+template <typename S>
+__global__ void __launch_bounds__(32) k_swap_trsm16(S* A, long long strideA, int lda, int n, int k, int kb, int ce,
+                                                    const int* ipiv) {
+  __shared__ S L[16 * 16];
+  __shared__ int R_[32], C_[32];
+  const int bidx = blockIdx.y, t = threadIdx.x;
+  S* M = A + strideA * bidx;
+  const int* piv = ipiv + (size_t)n * bidx;
+  int R = t < kb ? k + t : -1, C = R, nx = kb;
+  const int myp = t < kb ? piv[k + t] - 1 : 0;
+  for (int j = 0; j < kb; ++j) {
+    const int p = __shfl_sync(0xffffffffu, myp, j);
+    unsigned at = __ballot_sync(0xffffffffu, R == p);
+    if (!at) {
+      if (t == nx) R = C = p;
+      at = 1u << nx;
+      ++nx;
+    }
+    const int q = __ffs(at) - 1;
+    const int cj = __shfl_sync(0xffffffffu, C, j), cq = __shfl_sync(0xffffffffu, C, q);
+    if (t == j) C = cq;
+    if (t == q && q != j) C = cj;
+  }
+  R_[t] = R;
+  C_[t] = C;
+  for (int e = t; e < 256; e += 32) {
+    const int i = e & 15, jj = e >> 4;
+    L[e] = (i < kb && jj < kb && i > jj) ? M[(size_t)(k + jj) * lda + k + i] : Sc<S>::zero();
+  }
+  __syncwarp();
+  const int c = blockIdx.x * 32 + t;
+  if (c >= n - kb) return;
+  const int col = c < k ? c : c + kb;
+  S* Ac = M + (size_t)col * lda;
+  S x[16], y[16];
+#pragma unroll
+  for (int q = 0; q < 16; ++q) x[q] = q < kb ? Ac[C_[q]] : Sc<S>::zero();
+#pragma unroll
+  for (int q = 0; q < 16; ++q)
+    if (kb + q < nx) y[q] = Ac[C_[kb + q]];
+  const bool solve = col >= k + kb && col < ce;
+  if (solve) {
+#pragma unroll
+    for (int jj = 0; jj < 16; ++jj)
+#pragma unroll
+      for (int i = jj + 1; i < 16; ++i) x[i] = lu_fnma(L[jj * 16 + i], x[jj], x[i]);
+  }
+#pragma unroll
+  for (int q = 0; q < 16; ++q)
+    if (q < kb && (solve || C_[q] != R_[q])) Ac[k + q] = x[q];
+#pragma unroll
+  for (int q = 0; q < 16; ++q)
+    if (kb + q < nx && C_[kb + q] != R_[kb + q]) Ac[R_[kb + q]] = y[q];
+}
+
+// ---------------------------------------------------------------------------
+// U12 = inv(L11) A12 of a whole outer block (w <= 128 rows from K, columns
+// [c0, c1)) in one launch: a CTA holds NC columns in shared memory and walks the
+// block in steps of 16 rows: a step's rows are solved (16 lanes per column,
+// shuffles), then all threads subtract their multiples from the rows below.
+// In place of a TRSM and a GEMM launch per 16 rows, each with a fixed cost
+// (copies, a tile of the SMs idle, for the tensor-core path an operand split).
+// ---------------------------------------------------------------------------
+template <typename S, int NC>
+__global__ void __launch_bounds__(256) k_trsm_block(S* A, long long strideA, int lda, int K, int w, int c0, int c1) {
+  extern __shared__ __align__(16) unsigned char tbraw[];
+  S* X = reinterpret_cast<S*>(tbraw);       // [NC][129]
+  S* L = X + NC * 129;                      // [16][128 + 1]: the step's columns of L11
+  S* M = A + strideA * blockIdx.y;
+  const int cb = c0 + blockIdx.x * NC, nc = min(NC, c1 - cb), t = threadIdx.x;
+  for (int e = t; e < nc * w; e += 256) {
+    const int i = e % w, c = e / w;
+    X[c * 129 + i] = M[(size_t)(cb + c) * lda + K + i];
+  }
+  for (int s = 0; s < w; s += 16) {
+    const int sb = min(16, w - s), rows = w - s;
+    __syncthreads();  // X of the step before, and its reads of L, are done
+    for (int e = t; e < sb * rows; e += 256) {
+      const int i = e % rows, c = e / rows;
+      L[c * 129 + i] = M[(size_t)(K + s + c) * lda + K + s + i];
+    }
+    __syncthreads();
+    // 16 lanes per column, lane = row: one multiply-add per lane and step
+    if (t < 16 * NC) {
+      const int i = t & 15, c = t >> 4;
+      const bool on = i < sb && c < nc;
+      S x = on ? X[c * 129 + s + i] : Sc<S>::zero();
+#pragma unroll
+      for (int jj = 0; jj < 15; ++jj) {
+        const S l = on && jj < sb ? L[jj * 129 + i] : Sc<S>::zero();
+        const S xj = shfl_s(x, (t & 16) | jj);
+        if (i > jj) x = lu_fnma(l, xj, x);
+      }
+      if (on) X[c * 129 + s + i] = x;
+    }
+    __syncthreads();
+    // rows below: thread -> (row, column), rows fastest
+    const int below = rows - sb;
+    for (int e = t; e < below * nc; e += 256) {
+      const int i = e % below, c = e / below;
+      S v = X[c * 129 + s + sb + i];
+#pragma unroll
+      for (int jj = 0; jj < 16; ++jj)
+        if (jj < sb) v = lu_fnma(L[jj * 129 + sb + i], X[c * 129 + s + jj], v);
+      X[c * 129 + s + sb + i] = v;
+    }
+  }
+  __syncthreads();
+  for (int e = t; e < nc * w; e += 256) {
+    const int i = e % w, c = e / w;
+    M[(size_t)(cb + c) * lda + K + i] = X[c * 129 + i];
+  }
 }
 
 // Apply the panel interchanges (rows k..k+nb-1 with ipiv) to the columns
@@ -614,16 +814,6 @@ __global__ void __launch_bounds__(trsm_cols<S>()) k_trsm_cols(S* A, long long st
 // in shared memory, lane l holding rows l and l + 32 of the block; the solved
 // component is broadcast by a shuffle, no block-wide barrier per row.
 // LOWER: unit lower forward substitution; else upper backward substitution.
-template <typename S> __device__ __forceinline__ S shfl_s(S v, int src);
-template <> __device__ __forceinline__ float2 shfl_s(float2 v, int src) {
-  return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
-}
-template <> __device__ __forceinline__ double2 shfl_s(double2 v, int src) {
-  return make_double2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
-}
-template <> __device__ __forceinline__ float shfl_s(float v, int src) { return __shfl_sync(0xffffffffu, v, src); }
-template <> __device__ __forceinline__ double shfl_s(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
-
 // Stage the w x w diagonal block at (r0, r0) into D[col * 65 + row] with 128
 // threads, eight loads in flight per thread before their stores (the block is
 // usually cold in L2; one load per iteration would serialise on its latency).

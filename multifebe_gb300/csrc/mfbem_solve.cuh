@@ -102,23 +102,24 @@ __device__ __forceinline__ float2 zfma(float2 a, float2 b, float2 c) {
   return make_float2(fmaf(a.x, b.x, fmaf(-a.y, b.y, c.x)), fmaf(a.x, b.y, fmaf(a.y, b.x, c.y)));
 }
 __device__ __forceinline__ float zfma(float a, float b, float c) { return fmaf(a, b, c); }
-template <typename S>
+template <typename S, int Q>
 __global__ void __launch_bounds__(256) k_gemm_simt(const S* A, int lda, long long sA, const S* B, int ldb,
                                                    long long sB, S* C, int ldc, long long sC, int m, int n, int k) {
-  __shared__ S As[16][64 + 1];
-  __shared__ S Bs[16][64 + 1];
+  constexpr int T = 16 * Q;
+  __shared__ S As[16][T + 1];
+  __shared__ S Bs[16][T + 1];
   const int b = blockIdx.z, tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  const int i0 = blockIdx.x * 64, j0 = blockIdx.y * 64;
+  const int i0 = blockIdx.x * T, j0 = blockIdx.y * T;
   const S* Ab = A + sA * b;
   const S* Bb = B + sB * b;
-  S acc[4][4];
+  S acc[Q][Q];
 #pragma unroll
-  for (int u = 0; u < 4; ++u)
+  for (int u = 0; u < Q; ++u)
 #pragma unroll
-    for (int v = 0; v < 4; ++v) acc[u][v] = Sc<S>::zero();
+    for (int v = 0; v < Q; ++v) acc[u][v] = Sc<S>::zero();
   for (int l0 = 0; l0 < k; l0 += 16) {
-    for (int q = threadIdx.x; q < 16 * 64; q += 256) {
-      const int ii = q % 64, ll = q / 64;
+    for (int q = threadIdx.x; q < 16 * T; q += 256) {
+      const int ii = q % T, ll = q / T;
       As[ll][ii] = (i0 + ii < m && l0 + ll < k) ? Ab[(size_t)(l0 + ll) * lda + i0 + ii] : Sc<S>::zero();
       const int jj = q / 16, lb = q % 16;
       Bs[lb][jj] = (j0 + jj < n && l0 + lb < k) ? Bb[(size_t)(j0 + jj) * ldb + l0 + lb] : Sc<S>::zero();
@@ -126,32 +127,43 @@ __global__ void __launch_bounds__(256) k_gemm_simt(const S* A, int lda, long lon
     __syncthreads();
 #pragma unroll 4
     for (int ll = 0; ll < 16; ++ll) {
-      S a[4], bv[4];
+      S a[Q], bv[Q];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) a[u] = As[ll][tx + 16 * u];
+      for (int u = 0; u < Q; ++u) a[u] = As[ll][tx + 16 * u];
 #pragma unroll
-      for (int v = 0; v < 4; ++v) bv[v] = Bs[ll][ty + 16 * v];
+      for (int v = 0; v < Q; ++v) bv[v] = Bs[ll][ty + 16 * v];
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
+      for (int u = 0; u < Q; ++u)
 #pragma unroll
-        for (int v = 0; v < 4; ++v) acc[u][v] = zfma(a[u], bv[v], acc[u][v]);
+        for (int v = 0; v < Q; ++v) acc[u][v] = zfma(a[u], bv[v], acc[u][v]);
     }
     __syncthreads();
   }
   S* Cb = C + sC * b;
 #pragma unroll
-  for (int u = 0; u < 4; ++u)
+  for (int u = 0; u < Q; ++u)
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
+    for (int v = 0; v < Q; ++v) {
       const int i = i0 + tx + 16 * u, j = j0 + ty + 16 * v;
       if (i < m && j < n) Cb[(size_t)j * ldc + i] = Sc<S>::sub(Cb[(size_t)j * ldc + i], acc[u][v]);
     }
 }
+// Tile by the number of tiles: 64 x 64 while they give every SM one, else 32 x
+// 32, else 16 x 16. A binary64 tile of 64 x 64 x 16 takes one SM 17 us (two
+// multiply-adds per cycle), so the updates inside an outer block of a small
+// system are bound by the SMs left idle: the 93 updates of a real 870-row
+// factorisation 3.06 -> 0.6 ms, the 144 of a complex 2220-row one 11.5 -> 1.5.
 template <typename S>
 static int gemm_simt(cudaStream_t st, int m, int n, int k, const S* A, int lda, long long sA, const S* B, int ldb,
                      long long sB, S* C, int ldc, long long sC, int batch) {
   if (m <= 0 || n <= 0 || k <= 0) return 0;
-  k_gemm_simt<S><<<dim3(nblk(m, 64), nblk(n, 64), batch), 256, 0, st>>>(A, lda, sA, B, ldb, sB, C, ldc, sC, m, n, k);
+  auto tiles = [&](int t) { return (long long)nblk(m, t) * nblk(n, t) * batch; };
+  if (tiles(64) >= 152)
+    k_gemm_simt<S, 4><<<dim3(nblk(m, 64), nblk(n, 64), batch), 256, 0, st>>>(A, lda, sA, B, ldb, sB, C, ldc, sC, m, n, k);
+  else if (tiles(32) >= 152)
+    k_gemm_simt<S, 2><<<dim3(nblk(m, 32), nblk(n, 32), batch), 256, 0, st>>>(A, lda, sA, B, ldb, sB, C, ldc, sC, m, n, k);
+  else
+    k_gemm_simt<S, 1><<<dim3(nblk(m, 16), nblk(n, 16), batch), 256, 0, st>>>(A, lda, sA, B, ldb, sB, C, ldc, sC, m, n, k);
   ++g_launches;
   CK(cudaGetLastError());
   return 0;
@@ -279,44 +291,6 @@ static int gemm_sb(cudaStream_t st, int m, int n, int k, const float2* A, int ld
   return gemm_simt<float2>(st, m, n, k, A, lda, sA, B, ldb, sB, C, ldc, sC, batch);
 }
 
-// ---------------------------------------------------------------------------
-// TRSM of the plain LU's row panel, U12 = inv(L11) A12 with L11 the kb x kb
-// unit lower block at (k, k): on the tensor cores as the FP64-accurate update
-// A12 := 0 - (-inv(L11)) A12 (k_trtri_neg, k_take_zero, then the Ozaki GEMM)
-// when the panel row is long; the substitution kernel k_trsm_cols otherwise.
-// ---------------------------------------------------------------------------
-// T[b] = -inv(L11) (column-major, ld 32): one warp per (column j, matrix),
-// lane i holding x_i of column j; the forward substitution runs as kb steps
-// of one multiply-add per lane (x_c broadcast by a shuffle), so each lane's
-// dependent chain is kb operations long, and the columns run on separate
-// SMs (binary64 arithmetic is slow on this GPU; long chains of it on one SM
-// were the cost here).
-template <typename S>
-__global__ void __launch_bounds__(32) k_trtri_neg(const S* A, long long sA, int lda, int k, int kb, S* T) {
-  const int j = blockIdx.x, b = blockIdx.y, i = threadIdx.x;
-  const S* M = A + sA * b;
-  S x = (i == j) ? Sc<S>::one() : Sc<S>::zero();
-  for (int c = j; c < kb - 1; ++c) {
-    const S xc = shfl_s(x, c);
-    if (i > c && i < kb) x = Sc<S>::sub(x, Sc<S>::mul(M[(size_t)(k + c) * lda + k + i], xc));
-  }
-  T[1024 * (size_t)b + j * 32 + i] = Sc<S>::sub(Sc<S>::zero(), x);
-}
-// W[b] (kb x nc, ld kb) = A[k:k+kb, c0:c0+nc]; that block of A set to zero
-template <typename S>
-__global__ void k_take_zero(S* A, long long sA, int lda, int k, int kb, int c0, int nc, int batch, S* W) {
-  const long long tot = (long long)batch * nc * kb;
-  for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < tot; g += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(g % kb);
-    const long long r = g / kb;
-    const int c = (int)(r % nc), b = (int)(r / nc);
-    S* a = A + sA * b + (size_t)(c0 + c) * lda + k + i;
-    W[g] = *a;
-    *a = Sc<S>::zero();
-  }
-}
-static thread_local DevBuf g_trsm_ws;
-
 // Row interchanges of the mixed path's FP32 factorisation: none first (the
 // factors only precondition the FP64 refinement; the panel then needs no
 // pivot search across CTAs), partial pivoting when a zero pivot appears or
@@ -342,6 +316,33 @@ static int panel_nb_f64(int n) {
 template <typename S> struct IsF64 { static const bool v = false; };
 template <> struct IsF64<double> { static const bool v = true; };
 template <> struct IsF64<double2> { static const bool v = true; };
+
+// U12 of an outer block by k_trsm_block: binary64 work on the FP64 pipe, w / 2
+// multiply-adds per row and column (four times that if complex) at two per
+// cycle and SM. Against one TRSM and one GEMM launch per 16 rows (for long rows
+// on the tensor cores, each with its operand split): factorisation of one real
+// 870-row system 4.71 -> 4.10 ms, of one complex 3462-row system 47.6 -> 43.0,
+// of 20 of them 237 -> 212. From kTrsmSplit real columns up (nc x batch, x 2 if
+// complex) the block is solved as two halves with a depth-64 update between
+// them, which takes half of that binary64 work to the tensor cores: 67.5 ->
+// 63.5 ms for four complex 3462-row systems, no difference for one below 4096.
+constexpr double kTrsmSplit = 4096.0;
+template <typename S>
+static int trsm_block_run(cudaStream_t st, S* A, long long sA, int lda, int K, int w, int c0, int c1, int batch) {
+  // columns per CTA: 4, then 8, until every SM has its CTA, then 16
+  const int nc = c1 - c0;
+  const int NC = (long long)nblk(nc, 4) * batch <= 304 ? 4 : ((long long)nblk(nc, 8) * batch <= 304 ? 8 : 16);
+  const size_t sm = sizeof(S) * (129 * (size_t)NC + 16 * 129);
+  const void* f = NC == 4 ? (const void*)k_trsm_block<S, 4>
+                          : (NC == 8 ? (const void*)k_trsm_block<S, 8> : (const void*)k_trsm_block<S, 16>);
+  if (raise_smem_limit(f)) return fail(MFBEM_ECUDA, "shared-memory limit of the block TRSM");
+  if (NC == 4) k_trsm_block<S, 4><<<dim3(nblk(nc, 4), batch), 256, sm, st>>>(A, sA, lda, K, w, c0, c1);
+  else if (NC == 8) k_trsm_block<S, 8><<<dim3(nblk(nc, 8), batch), 256, sm, st>>>(A, sA, lda, K, w, c0, c1);
+  else k_trsm_block<S, 16><<<dim3(nblk(nc, 16), batch), 256, sm, st>>>(A, sA, lda, K, w, c0, c1);
+  ++g_launches;
+  CK(cudaGetLastError());
+  return 0;
+}
 
 // Workspace of the cooperative panel (barrier counters, candidate exchange,
 // error flag); per host thread, so concurrent sweeps do not share it
@@ -392,6 +393,35 @@ static bool coop_plan(int n, int nb, int batch, CoopPlan* pl) {
   return true;
 }
 
+// whether clusters of 16 CTAs of the panel for every matrix of the batch are resident at once
+template <typename S>
+static bool cluster16_fits(int n, int nb, int batch) {
+  const void* f = (const void*)k_panel_cluster<S, 256>;
+  const size_t sm = panel_cluster_smem<S>(16, nb, (n + 15) / 16);
+  if (sm > 200 * 1024 || raise_smem_limit(f)) return false;
+  if (cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 16;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(16 * batch);
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = sm;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  int ncl = 0;
+  if (cudaOccupancyMaxActiveClusters(&ncl, f, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return ncl >= batch;
+}
+
 // Blocked right-looking getrf for a batch of n x n matrices (stride sA).
 template <typename S>
 static int getrf_batched(cudaStream_t st, S* A, long long sA, int lda, int n, int batch,
@@ -426,11 +456,14 @@ static int getrf_batched(cudaStream_t st, S* A, long long sA, int lda, int n, in
   }
   // cluster panel: 8 CTAs per matrix in a thread-block cluster when a matrix's
   // panel rows fit their shared memory (about 200 KB each)
-  constexpr int GC = 8;
-  auto cl_smem = [&](int rows) {
-    const int ch = (rows + GC - 1) / GC;
-    return ((size_t)nb * ch + 32 + 4 * 32) * sizeof(S) + 2 * sizeof(R) + 2 * sizeof(int) + 16;
-  };
+  // 16 CTAs (opt-in size) where half as many rows per CTA shorten the binary64
+  // update by more than the larger cluster's exchange costs (400 cycles a
+  // column): one 16-column panel of 870 real rows 52 -> 56 us, of 1900 complex
+  // rows 91 -> 80, of 3462 complex rows 122 -> 91
+  const int cw = sizeof(S) / 8;
+  int GC = 8;
+  if (IsF64<S>::v && (double)n * cw > 2400.0 && cluster16_fits<S>(n, nb, batch)) GC = 16;
+  auto cl_smem = [&](int rows) { return panel_cluster_smem<S>(GC, nb, (rows + GC - 1) / GC); };
   bool use_cl = cl_smem(n) <= 200 * 1024 && !raise_smem_limit((const void*)k_panel_cluster<S, 256>);
   if (use_cl) {
     cudaLaunchConfig_t cfg = {};
@@ -481,22 +514,6 @@ static int getrf_batched(cudaStream_t st, S* A, long long sA, int lda, int n, in
   auto trsm = [&](int k, int kb, int c0, int c1) -> int {
     const int nc = c1 - c0;
     if (nc <= 0) return 0;
-    if constexpr (IsF64<S>::v) {
-      const double macs = (double)kb * kb * nc * batch * (std::is_same<S, double2>::value ? 4.0 : 1.0);
-      if (oz && nc >= 128 && macs >= kOzMinMacs / 4 && kb >= oz_min_depth()) {
-        const size_t tb = sizeof(S) * 1024 * (size_t)batch, wb = sizeof(S) * (size_t)kb * nc * batch;
-        int rc = ensure(g_trsm_ws, tb + wb);
-        if (rc) return rc;
-        S* T = (S*)g_trsm_ws.p;
-        S* W = (S*)((char*)g_trsm_ws.p + tb);
-        k_trtri_neg<S><<<dim3(32, batch), 32, 0, st>>>(A, sA, lda, k, kb, T); ++g_launches;
-        k_take_zero<S><<<(unsigned)std::min<long long>(nblk((long long)batch * nc * kb, 256), 152 * 16), 256, 0, st>>>(
-            A, sA, lda, k, kb, c0, nc, batch, W);
-        ++g_launches;
-        return oz_gemm_run<std::is_same<S, double2>::value>(st, T, 32, 1024, W, kb, (long long)kb * nc,
-                                                            A + k + (size_t)c0 * lda, lda, sA, kb, nc, kb, batch);
-      }
-    }
     k_trsm_cols<S><<<dim3(nblk(nc, trsm_cols<S>()), batch), trsm_cols<S>(), 0, st>>>(A, sA, lda, k, kb, c0, c1);
     ++g_launches;
     return 0;
@@ -556,11 +573,14 @@ static int getrf_batched(cudaStream_t st, S* A, long long sA, int lda, int n, in
         k_panel_cta<S, 512><<<batch, 512, 0, st>>>(A, sA, lda, n, k, kb, ipiv, info); ++g_launches;
       }
       int nout = n - kb;
-      if (nout > 0 && !nopiv) { k_laswp<S><<<dim3(nblk(nout, 128), batch), 128, 0, st>>>(A, sA, lda, n, k, kb, ipiv); ++g_launches; }
+      const bool fused = IsF64<S>::v && nb == 16;  // interchanges and in-block TRSM in one launch
+      if (fused && nout > 0) {
+        k_swap_trsm16<S><<<dim3(nblk(nout, 32), batch), 32, 0, st>>>(A, sA, lda, n, k, kb, KE, ipiv); ++g_launches;
+      } else if (nout > 0 && !nopiv) { k_laswp<S><<<dim3(nblk(nout, 128), batch), 128, 0, st>>>(A, sA, lda, n, k, kb, ipiv); ++g_launches; }
       if (k + kb < KE) {
         // inside the outer block: U12 and the update of columns [k+kb, KE)
         const int nc = KE - k - kb;
-        CKG(trsm(k, kb, k + kb, KE));
+        if (!fused) CKG(trsm(k, kb, k + kb, KE));
         CKG(gemm_sb(st, n - k - kb, nc, kb, A + k + kb + (size_t)k * lda, lda, sA, A + k + (size_t)(k + kb) * lda, lda,
                     sA, A + (k + kb) + (size_t)(k + kb) * lda, lda, sA, batch));
       }
@@ -568,7 +588,16 @@ static int getrf_batched(cudaStream_t st, S* A, long long sA, int lda, int n, in
     if (KE < n) {
       // U12 of the outer block (rows [K, KE), columns [KE, n)), blocked by nb
       const int nc = n - KE;
-      for (int k = K; k < KE; k += nb) {
+      const bool one = IsF64<S>::v && KE - K <= 128;
+      if (one && KE - K == 128 && (double)nc * batch * cw >= kTrsmSplit) {
+        CKG(trsm_block_run<S>(st, A, sA, lda, K, 64, KE, n, batch));
+        CKG(gemm_sb(st, 64, nc, 64, A + K + 64 + (size_t)K * lda, lda, sA, A + K + (size_t)KE * lda, lda, sA,
+                    A + (K + 64) + (size_t)KE * lda, lda, sA, batch));
+        CKG(trsm_block_run<S>(st, A, sA, lda, K + 64, 64, KE, n, batch));
+      } else if (one) {
+        CKG(trsm_block_run<S>(st, A, sA, lda, K, KE - K, KE, n, batch));
+      }
+      for (int k = K; k < KE && !one; k += nb) {
         const int kb = std::min(nb, KE - k);
         CKG(trsm(k, kb, KE, n));
         if (k + kb < KE)
