@@ -25,72 +25,12 @@
 
 namespace mfb {
 
-// ---------------------------------------------------------------------------
-// Conjugate-transposed triangular solves with the LU factors: U^H forward
-// (lower, non-unit) and L^H backward (upper, unit), blocked by 64 rows like
-// getrs_batched's solves.
-// ---------------------------------------------------------------------------
-template <typename S, bool LH>
-__global__ void __launch_bounds__(128) k_trsv_diag64_h(const S* A, long long strideA, int lda, S* b,
-                                                       long long strideb, int r0, int w) {
-  const S* M = A + strideA * blockIdx.x;
-  S* xg = b + strideb * blockIdx.x;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  S* D = reinterpret_cast<S*>(smraw);  // D[col * 65 + row] = A(r0 + row, r0 + col)
-  stage_diag64(M, lda, r0, w, D);
-  __syncthreads();
-  if (threadIdx.x >= 32) return;
-  const int l = threadIdx.x;
-  S x0 = l < w ? xg[r0 + l] : Sc<S>::zero();
-  S x1 = l + 32 < w ? xg[r0 + l + 32] : Sc<S>::zero();
-  if (!LH) {
-    // x_j /= conj(U_jj); x_i -= conj(U_ji) x_j for i > j (U_ji = D[i * 65 + j])
-    for (int j = 0; j < w; ++j) {
-      if (j < 32) { if (l == j) x0 = Sc<S>::div(x0, Sc<S>::conj(D[j * 65 + j])); }
-      else { if (l + 32 == j) x1 = Sc<S>::div(x1, Sc<S>::conj(D[j * 65 + j])); }
-      const S xj = shfl_s(j < 32 ? x0 : x1, j & 31);
-      if (l > j && l < w) x0 = Sc<S>::sub(x0, Sc<S>::mul(Sc<S>::conj(D[l * 65 + j]), xj));
-      if (l + 32 > j && l + 32 < w) x1 = Sc<S>::sub(x1, Sc<S>::mul(Sc<S>::conj(D[(l + 32) * 65 + j]), xj));
-    }
-  } else {
-    // unit diagonal; x_i -= conj(L_ji) x_j for i < j
-    for (int j = w - 1; j >= 0; --j) {
-      const S xj = shfl_s(j < 32 ? x0 : x1, j & 31);
-      if (l < j) x0 = Sc<S>::sub(x0, Sc<S>::mul(Sc<S>::conj(D[l * 65 + j]), xj));
-      if (l + 32 < j) x1 = Sc<S>::sub(x1, Sc<S>::mul(Sc<S>::conj(D[(l + 32) * 65 + j]), xj));
-    }
-  }
-  if (l < w) xg[r0 + l] = x0;
-  if (l + 32 < w) xg[r0 + l + 32] = x1;
-}
-
-// rows [i0, i1): x_i -= sum_j conj(A(r0 + j, i)) x_{r0 + j}; one warp per row,
-// reading column i's block rows contiguously
-template <typename S>
-__global__ void k_trsv_update_h(const S* A, long long strideA, int lda, S* b, long long strideb, int r0, int w,
-                                int i0, int i1) {
-  const S* M = A + strideA * blockIdx.y;
-  S* x = b + strideb * blockIdx.y;
-  __shared__ S xs[64];
-  if ((int)threadIdx.x < w) xs[threadIdx.x] = x[r0 + threadIdx.x];
-  __syncthreads();
-  const int l = threadIdx.x & 31;
-  const int i = i0 + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (i >= i1) return;
-  const S* col = M + (size_t)i * lda + r0;
-  S acc = Sc<S>::zero();
-  if (l < w) acc = Sc<S>::mul(Sc<S>::conj(col[l]), xs[l]);
-  if (l + 32 < w) acc = Sc<S>::add(acc, Sc<S>::mul(Sc<S>::conj(col[l + 32]), xs[l + 32]));
-  for (int o = 16; o > 0; o >>= 1) acc = Sc<S>::add(acc, shfl_s(acc, l ^ o));
-  if (l == 0) x[i] = Sc<S>::sub(x[i], acc);
-}
-
 // inverse of the getrs row permutation: out[perm[i]] = x[i]
 template <typename S>
 __global__ void k_scatter_perm(const S* x, long long sx, const int* perm, int n, S* out) {
   const int bi = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  out[(size_t)n * bi + perm[(size_t)n * bi + i]] = x[sx * bi + i];
+  out[(size_t)n * bi + perm[i]] = x[sx * bi + i];
 }
 // the interchanges in reverse order (one thread per right-hand side), for n
 // too large for k_perm's shared-memory index array
@@ -110,55 +50,29 @@ __global__ void k_rhs_swap_rev(S* b, long long sb, int n, const int* ipiv, long 
   }
 }
 
-enum TrOp { TR_L = 0, TR_U = 1, TR_UH = 2, TR_LH = 3 };
-
-// one triangular solve with the factors in A (no permutation)
+// one triangular solve with the factors in A (no permutation), batch
+// right-hand sides of one matrix
 template <typename S>
-static int trsv_op(cudaStream_t st, const S* A, long long sA, int lda, int n, S* b, long long sb, int batch, int op) {
-  const int TB = 64;
-  const size_t dsm = (size_t)TB * 65 * sizeof(S);
-  const void* kd = op == TR_L ? (const void*)k_trsv_diag64<S, true>
-                   : op == TR_U ? (const void*)k_trsv_diag64<S, false>
-                   : op == TR_UH ? (const void*)k_trsv_diag64_h<S, false> : (const void*)k_trsv_diag64_h<S, true>;
-  if (raise_smem_limit(kd)) return fail(MFBEM_ECUDA, "shared-memory limit of the triangular solve");
-  const int last = ((n - 1) / TB) * TB;
-  const bool fwd = op == TR_L || op == TR_UH;
-  for (int k = 0; k < n; k += TB) {
-    const int r0 = fwd ? k : last - k;
-    const int w = std::min(TB, n - r0);
-    const int i0 = fwd ? r0 + w : 0, i1 = fwd ? n : r0;
-    switch (op) {
-      case TR_L: k_trsv_diag64<S, true><<<batch, 128, dsm, st>>>(A, sA, lda, b, sb, r0, w); break;
-      case TR_U: k_trsv_diag64<S, false><<<batch, 128, dsm, st>>>(A, sA, lda, b, sb, r0, w); break;
-      case TR_UH: k_trsv_diag64_h<S, false><<<batch, 128, dsm, st>>>(A, sA, lda, b, sb, r0, w); break;
-      default: k_trsv_diag64_h<S, true><<<batch, 128, dsm, st>>>(A, sA, lda, b, sb, r0, w); break;
-    }
-    ++g_launches;
-    if (i1 > i0) {
-      if (op <= TR_U)
-        k_trsv_update<S><<<dim3(nblk(i1 - i0, 256), batch), 256, 0, st>>>(A, sA, lda, b, sb, r0, w, i0, i1);
-      else
-        k_trsv_update_h<S><<<dim3(nblk(i1 - i0, 8), batch), 256, 0, st>>>(A, sA, lda, b, sb, r0, w, i0, i1);
-      ++g_launches;
-    }
+static int trsv_op(cudaStream_t st, const S* A, int lda, int n, S* b, long long sb, int batch, int op) {
+  switch (op) {
+    case TR_L: return trsv_sf_run<S, TR_L>(st, A, 0, lda, n, b, sb, batch);
+    case TR_U: return trsv_sf_run<S, TR_U>(st, A, 0, lda, n, b, sb, batch);
+    case TR_UH: return trsv_sf_run<S, TR_UH>(st, A, 0, lda, n, b, sb, batch);
+    default: return trsv_sf_run<S, TR_LH>(st, A, 0, lda, n, b, sb, batch);
   }
-  CK(cudaGetLastError());
-  return 0;
 }
 
-// getrs with trans = 'C' (complex) / 'T' (real): x = P^T L^-H U^-H b
+// getrs with trans = 'C' (complex) / 'T' (real): x = P^T L^-H U^-H b; perm as
+// in getrs_batched
 template <typename S>
-static int getrs_conj(cudaStream_t st, const S* A, int lda, int n, const int* ipiv, S* b, long long sb, int batch) {
-  int rc = trsv_op<S>(st, A, 0, lda, n, b, sb, batch, TR_UH);
-  if (!rc) rc = trsv_op<S>(st, A, 0, lda, n, b, sb, batch, TR_LH);
+static int getrs_conj(cudaStream_t st, const S* A, int lda, int n, const int* ipiv, S* b, long long sb, int batch,
+                      const int* perm) {
+  int rc = trsv_op<S>(st, A, lda, n, b, sb, batch, TR_UH);
+  if (!rc) rc = trsv_op<S>(st, A, lda, n, b, sb, batch, TR_LH);
   if (rc) return rc;
-  const size_t psm = (size_t)n * sizeof(int);
-  if (psm <= 200 * 1024) {
+  if (perm) {
     if ((rc = ensure(g_rs_ws, (size_t)batch * n * (sizeof(int) + sizeof(S)) + 256))) return rc;
-    if (psm > 48 * 1024 && raise_smem_limit((const void*)k_perm)) return fail(MFBEM_ECUDA, "shared-memory limit of the row permutation");
-    int* perm = (int*)g_rs_ws.p;
     S* tmp = (S*)((char*)g_rs_ws.p + ((size_t)batch * n * sizeof(int) + 255) / 256 * 256);
-    k_perm<<<batch, 256, psm, st>>>(ipiv, 0, n, perm); ++g_launches;
     k_scatter_perm<S><<<dim3(nblk(n, 256), batch), 256, 0, st>>>(b, sb, perm, n, tmp); ++g_launches;
     k_scatter_back<S><<<dim3(nblk(n, 256), batch), 256, 0, st>>>(tmp, n, b, sb); ++g_launches;
   } else {
@@ -409,15 +323,6 @@ struct LseWork {
   int* flag;    // device int [2]
 };
 
-template <typename S>
-static int vstats(const LseWork& w, const S* x, int n, int q, int mode, double h[4]) {
-  if (mode) k_vstats<S, 1><<<1, 1024, 0, w.st>>>(x, n, q, w.red);
-  else k_vstats<S, 0><<<1, 1024, 0, w.st>>>(x, n, q, w.red);
-  ++g_launches;
-  CK(cudaMemcpyAsync(h, w.red, 4 * sizeof(double), cudaMemcpyDeviceToHost, w.st));
-  CK(cudaStreamSynchronize(w.st));
-  return 0;
-}
 template <typename S> static void vsign(const LseWork& w, S* x, int* isgn, int n);
 template <> void vsign<double2>(const LseWork& w, double2* x, int*, int n) {
   k_vsign_c<<<nblk(n, 256), 256, 0, w.st>>>(x, n); ++g_launches;
@@ -426,63 +331,129 @@ template <> void vsign<double>(const LseWork& w, double* x, int* isgn, int n) {
   k_vsign_r<<<nblk(n, 256), 256, 0, w.st>>>(x, isgn, n, 1, w.flag); ++g_launches;
 }
 
-// ?lacn2 with the reverse communication unrolled: apply(kase, x) overwrites x
-// by A x (kase 1) or A^H x (kase 2); est receives the estimate of ||A||_1.
-// x, v: n-vectors, isgn: n ints (real case).
-template <typename S, class F>
-static int lacn2(const LseWork& w, int n, S* x, S* v, int* isgn, F apply, double* est) {
-  const bool cplx = sizeof(S) == 16;
-  const unsigned g = nblk(n, 256);
-  double h[4];
-  int rc;
-  k_vfill<S><<<g, 256, 0, w.st>>>(x, n, 1.0 / n); ++g_launches;
-  if ((rc = apply(1, x))) return rc;
-  if (n == 1) {
-    if ((rc = vstats<S>(w, x, n, 0, 0, h))) return rc;
-    *est = h[0];
+// ?lacn2 for several estimates in step: each call of step() takes one estimate
+// from the result of its last application to its next one (kase 1: A x, 2:
+// A^H x; 0: done, est holds ||A||_1's estimate). The estimates share a matrix,
+// so the caller applies it to all that want the same kase at once, and their
+// scalars (stat: {sum, max, index, value at q}, flag: sign vector changed)
+// come back in one copy.
+template <typename S>
+struct Lacn2 {
+  int n = 0;
+  S *x = nullptr, *v = nullptr;
+  int* isgn = nullptr;
+  int kase = 0, phase = 0, j = 0, iter = 2, q = -1;
+  double e = 0.0, est = 0.0;
+  void begin(const LseWork& w, int n_, S* x_, S* v_, int* isgn_) {
+    n = n_; x = x_; v = v_; isgn = isgn_;
+    k_vfill<S><<<nblk(n, 256), 256, 0, w.st>>>(x, n, 1.0 / n); ++g_launches;
+    kase = 1;
+    phase = 1;
+    q = n == 1 ? 0 : -1;
+  }
+  // device work that the next step's decision needs (after the application)
+  int stats(const LseWork& w, double* stat, int* flag) {
+    k_vstats<S, 0><<<1, 1024, 0, w.st>>>(x, n, q, stat); ++g_launches;
+    if (phase == 3 && sizeof(S) == 8) {
+      CK(cudaMemsetAsync(flag, 0, sizeof(int), w.st));
+      k_vsign_r<<<nblk(n, 256), 256, 0, w.st>>>((double*)x, isgn, n, 0, flag); ++g_launches;
+    }
     return 0;
   }
-  if ((rc = vstats<S>(w, x, n, -1, 0, h))) return rc;
-  double e = h[0];
-  vsign<S>(w, x, isgn, n);
-  if ((rc = apply(2, x)) || (rc = vstats<S>(w, x, n, -1, 0, h))) return rc;
-  int j = (int)h[2], iter = 2;
+  int unit(const LseWork& w) {
+    k_vunit<S><<<nblk(n, 256), 256, 0, w.st>>>(x, n, j); ++g_launches;
+    kase = 1;
+    phase = 3;
+    q = -1;
+    return 0;
+  }
+  int step(const LseWork& w, const double* h, int flag) {
+    bool alt = false;
+    switch (phase) {
+      case 1:
+        if (n == 1) {
+          est = h[0];
+          kase = 0;
+          return 0;
+        }
+        e = h[0];
+        vsign<S>(w, x, isgn, n);
+        kase = 2;
+        phase = 2;
+        q = -1;
+        return 0;
+      case 2:
+        j = (int)h[2];
+        iter = 2;
+        return unit(w);
+      case 3: {
+        CK(cudaMemcpyAsync(v, x, sizeof(S) * n, cudaMemcpyDeviceToDevice, w.st));
+        const double eold = e;
+        e = h[0];
+        // real: a repeated sign vector means convergence
+        if ((sizeof(S) == 8 && !flag) || e <= eold) {
+          alt = true;
+          break;
+        }
+        vsign<S>(w, x, isgn, n);
+        kase = 2;
+        phase = 4;
+        q = j;
+        return 0;
+      }
+      case 4:
+        j = (int)h[2];
+        if (h[3] != h[1] && iter < 5) {
+          ++iter;
+          return unit(w);
+        }
+        alt = true;
+        break;
+      default: {
+        const double temp = 2.0 * (h[0] / (3.0 * n));
+        if (temp > e) {
+          CK(cudaMemcpyAsync(v, x, sizeof(S) * n, cudaMemcpyDeviceToDevice, w.st));
+          e = temp;
+        }
+        est = e;
+        kase = 0;
+        return 0;
+      }
+    }
+    if (alt) {
+      k_valt<S><<<nblk(n, 256), 256, 0, w.st>>>(x, n); ++g_launches;
+      kase = 1;
+      phase = 5;
+      q = -1;
+    }
+    return 0;
+  }
+};
+// Runs the estimates L until all are done. apply(kase, idx) applies the matrix
+// (kase 1) or its conjugate transpose (2) to the x of every estimate in idx.
+// stat (4 doubles) and flag (one int) per estimate: device.
+template <typename S, class F>
+static int lacn2_run(const LseWork& w, std::vector<Lacn2<S>>& L, double* stat, int* flag, F apply) {
+  std::vector<double> h(4 * L.size());
+  std::vector<int> f(L.size(), 0);
   for (;;) {
-    k_vunit<S><<<g, 256, 0, w.st>>>(x, n, j); ++g_launches;
-    if ((rc = apply(1, x))) return rc;
-    CK(cudaMemcpyAsync(v, x, sizeof(S) * n, cudaMemcpyDeviceToDevice, w.st));
-    const double eold = e;
-    if ((rc = vstats<S>(w, x, n, -1, 0, h))) return rc;
-    e = h[0];
-    if (!cplx) {  // repeated sign vector: converged
-      int f = 0;
-      CK(cudaMemsetAsync(w.flag, 0, sizeof(int), w.st));
-      k_vsign_r<<<g, 256, 0, w.st>>>((double*)x, isgn, n, 0, w.flag); ++g_launches;
-      CK(cudaMemcpyAsync(&f, w.flag, sizeof(int), cudaMemcpyDeviceToHost, w.st));
-      CK(cudaStreamSynchronize(w.st));
-      if (!f) break;
+    std::vector<int> k[3];
+    for (size_t i = 0; i < L.size(); ++i) k[L[i].kase].push_back((int)i);
+    if (k[1].empty() && k[2].empty()) return 0;
+    int rc;
+    for (int ks = 1; ks <= 2; ++ks) {
+      if (k[ks].empty()) continue;
+      if ((rc = apply(ks, k[ks]))) return rc;
+      for (int i : k[ks])
+        if ((rc = L[i].stats(w, stat + 4 * i, flag + i))) return rc;
     }
-    if (e <= eold) break;
-    vsign<S>(w, x, isgn, n);
-    if ((rc = apply(2, x))) return rc;
-    const int jlast = j;
-    if ((rc = vstats<S>(w, x, n, jlast, 0, h))) return rc;
-    j = (int)h[2];
-    if (h[3] != h[1] && iter < 5) {
-      ++iter;
-      continue;
-    }
-    break;
+    CK(cudaMemcpyAsync(h.data(), stat, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, w.st));
+    CK(cudaMemcpyAsync(f.data(), flag, sizeof(int) * f.size(), cudaMemcpyDeviceToHost, w.st));
+    CK(cudaStreamSynchronize(w.st));
+    for (int ks = 1; ks <= 2; ++ks)
+      for (int i : k[ks])
+        if ((rc = L[i].step(w, &h[4 * i], f[i]))) return rc;
   }
-  k_valt<S><<<g, 256, 0, w.st>>>(x, n); ++g_launches;
-  if ((rc = apply(1, x)) || (rc = vstats<S>(w, x, n, -1, 0, h))) return rc;
-  const double temp = 2.0 * (h[0] / (3.0 * n));
-  if (temp > e) {
-    CK(cudaMemcpyAsync(v, x, sizeof(S) * n, cudaMemcpyDeviceToDevice, w.st));
-    e = temp;
-  }
-  *est = e;
-  return 0;
 }
 
 // ?geequ + ?laqge on the device matrix A; r, c (device) receive the factors.
@@ -537,63 +508,104 @@ static int gecon1(const LseWork& w, const S* Ao, const S* LU, int n, S* x, S* v,
   *rcond = 0.0;
   if (n == 0) { *rcond = 1.0; return 0; }
   if (anorm == 0.0) return 0;
-  auto apply = [&](int kase, S* y) -> int {
-    int rc = trsv_op<S>(w.st, LU, 0, n, n, y, n, 1, kase == 1 ? TR_L : TR_UH);
-    if (!rc) rc = trsv_op<S>(w.st, LU, 0, n, n, y, n, 1, kase == 1 ? TR_U : TR_LH);
-    return rc;
-  };
-  double ainv = 0.0;
-  int rc = lacn2<S>(w, n, x, v, isgn, apply, &ainv);
+  std::vector<Lacn2<S>> L(1);
+  L[0].begin(w, n, x, v, isgn);
+  int rc = lacn2_run<S>(w, L, w.red, w.flag, [&](int kase, const std::vector<int>&) -> int {
+    int r = trsv_op<S>(w.st, LU, n, n, x, n, 1, kase == 1 ? TR_L : TR_UH);
+    return r ? r : trsv_op<S>(w.st, LU, n, n, x, n, 1, kase == 1 ? TR_U : TR_LH);
+  });
   if (rc) return rc;
+  const double ainv = L[0].est;
   if (ainv != 0.0) *rcond = (1.0 / ainv) / anorm;
   return 0;
 }
 
-// ?gerfs (no transpose) for one right-hand side: X refined in place,
-// ferr / berr as LAPACK returns them. Work: R, y, v (n each), wts, part
-// (64 n doubles), isgn (n ints).
+// ?gerfs (no transpose): X refined in place, ferr / berr as LAPACK returns
+// them. All right-hand sides go through the corrections and the norm estimates
+// in step, so a triangular solve -- a chain of n / 64 blocks whatever their
+// number -- serves all that need it. Work per right-hand side: R, y, v, p (n
+// each), wts (n), isgn (n ints), stat (4), flag; part (64 n) shared.
 template <typename S>
-static int gerfs1(const LseWork& w, const S* Ao, const S* LU, const int* ipiv, int n, const S* B, S* X, S* R, S* y,
-                  S* v, int* isgn, double* wts, double* part, double* ferr, double* berr) {
+struct GerfsWork {
+  S *R, *y, *v, *pack;
+  int* isgn;
+  double *wts, *part, *stat;
+  int* flag;
+};
+template <typename S>
+static int gerfs(const LseWork& w, const S* Ao, const S* LU, const int* ipiv, const int* perm, int n, int nrhs,
+                 const S* B, S* X, const GerfsWork<S>& g, double* ferr, double* berr) {
   const double nz = n + 1, safe1 = nz * kSafeMin, safe2 = safe1 / kEps;
   const int ch = 64, cpc = (n + ch - 1) / ch;
-  const unsigned g = nblk(n, 256);
-  double lstres = 3.0, h[4];
-  int count = 1, rc;
-  for (;;) {
-    CK(cudaMemcpyAsync(R, B, sizeof(S) * n, cudaMemcpyDeviceToDevice, w.st));
-    if ((rc = gemv_res<S>(w.st, n, Ao, n, 0, X, 0, R, 0, 1))) return rc;
-    k_absAx<S><<<dim3(g, ch), 256, 0, w.st>>>(Ao, n, n, X, cpc, part); ++g_launches;
-    k_berr<S><<<1, 1024, 0, w.st>>>(R, B, part, ch, n, safe1, safe2, wts, w.red); ++g_launches;
-    CK(cudaMemcpyAsync(h, w.red, sizeof(double), cudaMemcpyDeviceToHost, w.st));
-    CK(cudaStreamSynchronize(w.st));
-    *berr = h[0];
-    if (h[0] > kEps && 2.0 * h[0] <= lstres && count <= 5) {
-      CK(cudaMemcpyAsync(y, R, sizeof(S) * n, cudaMemcpyDeviceToDevice, w.st));
-      if ((rc = getrs_batched<S>(w.st, LU, 0, n, n, ipiv, 0, y, n, 1))) return rc;
-      k_vaxpy<S><<<g, 256, 0, w.st>>>(X, y, n); ++g_launches;
-      lstres = h[0];
-      ++count;
-      continue;
-    }
-    break;
-  }
-  k_ferr_w<S><<<g, 256, 0, w.st>>>(R, wts, n, nz * kEps, safe1, safe2); ++g_launches;
-  auto apply = [&](int kase, S* z) -> int {
-    int rc2 = 0;
-    if (kase == 1) {
-      rc2 = getrs_conj<S>(w.st, LU, n, n, ipiv, z, n, 1);
-      k_vmulw<S><<<g, 256, 0, w.st>>>(z, wts, n); ++g_launches;
-    } else {
-      k_vmulw<S><<<g, 256, 0, w.st>>>(z, wts, n); ++g_launches;
-      rc2 = getrs_batched<S>(w.st, LU, 0, n, n, ipiv, 0, z, n, 1);
-    }
-    return rc2;
+  const unsigned gr = nblk(n, 256);
+  const size_t vb = sizeof(S) * (size_t)n;
+  int rc;
+  // f(packed vectors, count) on the vectors base + n idx
+  auto packed = [&](S* base, const std::vector<int>& idx, auto f) -> int {
+    const int m = (int)idx.size();
+    if (m == nrhs) return f(base, m);
+    for (int i = 0; i < m; ++i)
+      CK(cudaMemcpyAsync(g.pack + (size_t)i * n, base + (size_t)idx[i] * n, vb, cudaMemcpyDeviceToDevice, w.st));
+    if (int r = f(g.pack, m)) return r;
+    for (int i = 0; i < m; ++i)
+      CK(cudaMemcpyAsync(base + (size_t)idx[i] * n, g.pack + (size_t)i * n, vb, cudaMemcpyDeviceToDevice, w.st));
+    return 0;
   };
-  double f = 0.0;
-  if ((rc = lacn2<S>(w, n, y, v, isgn, apply, &f))) return rc;
-  if ((rc = vstats<S>(w, X, n, -1, 1, h))) return rc;
-  *ferr = h[1] != 0.0 ? f / h[1] : f;
+  std::vector<double> lstres(nrhs, 3.0), h(4 * (size_t)nrhs);
+  std::vector<int> act(nrhs);
+  for (int j = 0; j < nrhs; ++j) act[j] = j;
+  // a right-hand side takes at most five corrections
+  for (int count = 1; !act.empty(); ++count) {
+    for (int j : act) {
+      const size_t o = (size_t)j * n;
+      CK(cudaMemcpyAsync(g.R + o, B + o, vb, cudaMemcpyDeviceToDevice, w.st));
+      if ((rc = gemv_res<S>(w.st, n, Ao, n, 0, X + o, 0, g.R + o, 0, 1))) return rc;
+      k_absAx<S><<<dim3(gr, ch), 256, 0, w.st>>>(Ao, n, n, X + o, cpc, g.part); ++g_launches;
+      k_berr<S><<<1, 1024, 0, w.st>>>(g.R + o, B + o, g.part, ch, n, safe1, safe2, g.wts + o, g.stat + 4 * j); ++g_launches;
+    }
+    CK(cudaMemcpyAsync(h.data(), g.stat, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, w.st));
+    CK(cudaStreamSynchronize(w.st));
+    std::vector<int> next;
+    for (int j : act) {
+      berr[j] = h[4 * j];
+      if (h[4 * j] > kEps && 2.0 * h[4 * j] <= lstres[j] && count <= 5) {
+        CK(cudaMemcpyAsync(g.y + (size_t)j * n, g.R + (size_t)j * n, vb, cudaMemcpyDeviceToDevice, w.st));
+        lstres[j] = h[4 * j];
+        next.push_back(j);
+      }
+    }
+    if (!next.empty()) {
+      if ((rc = packed(g.y, next, [&](S* z, int m) { return getrs_batched<S>(w.st, LU, 0, n, n, ipiv, 0, z, n, m, false, perm); })))
+        return rc;
+      for (int j : next) { k_vaxpy<S><<<gr, 256, 0, w.st>>>(X + (size_t)j * n, g.y + (size_t)j * n, n); ++g_launches; }
+    }
+    act = next;
+  }
+  std::vector<Lacn2<S>> L(nrhs);
+  for (int j = 0; j < nrhs; ++j) {
+    const size_t o = (size_t)j * n;
+    k_ferr_w<S><<<gr, 256, 0, w.st>>>(g.R + o, g.wts + o, n, nz * kEps, safe1, safe2); ++g_launches;
+    L[j].begin(w, n, g.y + o, g.v + o, g.isgn + o);
+  }
+  auto weigh = [&](const std::vector<int>& idx) {
+    for (int j : idx) { k_vmulw<S><<<gr, 256, 0, w.st>>>(g.y + (size_t)j * n, g.wts + (size_t)j * n, n); ++g_launches; }
+  };
+  rc = lacn2_run<S>(w, L, g.stat, g.flag, [&](int kase, const std::vector<int>& idx) -> int {
+    int r;
+    if (kase == 1) {
+      r = packed(g.y, idx, [&](S* z, int m) { return getrs_conj<S>(w.st, LU, n, n, ipiv, z, n, m, perm); });
+      if (!r) weigh(idx);
+    } else {
+      weigh(idx);
+      r = packed(g.y, idx, [&](S* z, int m) { return getrs_batched<S>(w.st, LU, 0, n, n, ipiv, 0, z, n, m, false, perm); });
+    }
+    return r;
+  });
+  if (rc) return rc;
+  for (int j = 0; j < nrhs; ++j) { k_vstats<S, 1><<<1, 1024, 0, w.st>>>(X + (size_t)j * n, n, -1, g.stat + 4 * j); ++g_launches; }
+  CK(cudaMemcpyAsync(h.data(), g.stat, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, w.st));
+  CK(cudaStreamSynchronize(w.st));
+  for (int j = 0; j < nrhs; ++j) ferr[j] = h[4 * j + 1] != 0.0 ? L[j].est / h[4 * j + 1] : L[j].est;
   return 0;
 }
 
@@ -660,9 +672,12 @@ static int solve_dropin(int32_t n, double* A, int32_t* ipiv, int32_t aodim, doub
   std::lock_guard<std::mutex> lk(g_solve_mu);
   const size_t es = sizeof(S), nn = (size_t)n * n, nr = (size_t)std::max(1, n_rhs);
   const bool keep_ao = condition || refine;
-  // vector work: x, v, R, y (n S each), r, c, wts (n doubles), part (64 n),
-  // bits (n u64), isgn (n ints), scalars
-  const size_t wbytes = 4 * n * es + (3 + 64) * (size_t)n * 8 + (size_t)n * 8 + (size_t)n * 4 + 256;
+  // vector work: x, v (n S each), r, c (n doubles), bits (n u64), isgn, perm (n
+  // ints), scalars; refine, per right-hand side: R, y, v, pack (n S), wts (n
+  // doubles), stat (4), isgn (n ints), flag; part (64 n doubles)
+  const size_t np = (size_t)n;
+  const size_t wbytes = 2 * np * es + 3 * np * 8 + 2 * np * 4 + 256 +
+                        (refine ? nr * (4 * np * es + np * 8 + 4 * 8 + np * 4 + 4) + 64 * np * 8 + 64 : 0);
   if ((rc = ensure(cx->A, nn * es)) || (rc = ensure(cx->b, (size_t)n * nr * es)) ||
       (rc = ensure(cx->ipiv, sizeof(int) * n)) || (rc = ensure(cx->info, sizeof(int) * 4)) ||
       (rc = ensure(cx->wv, wbytes)) || (keep_ao && (rc = ensure(cx->Ao, nn * es))) ||
@@ -674,14 +689,33 @@ static int solve_dropin(int32_t n, double* A, int32_t* ipiv, int32_t aodim, doub
   int* dp = (int*)cx->ipiv.p;
   int* di = (int*)cx->info.p;
   char* wp = (char*)cx->wv.p;
-  S* vx = (S*)wp; S* vv = vx + n; S* vR = vv + n; S* vy = vR + n;
-  double* dr = (double*)(vy + n);
-  double* dc = dr + n;
-  double* wts = dc + n;
-  double* part = wts + n;
-  unsigned long long* bits = (unsigned long long*)(part + 64 * (size_t)n);
-  int* isgn = (int*)(bits + n);
-  double* red = (double*)(((uintptr_t)(isgn + n) + 63) / 64 * 64);
+  // 16-byte entries first, then doubles, then ints
+  S* vx = (S*)wp;
+  S* vv = vx + np;
+  GerfsWork<S> gw{};
+  double* dr = (double*)(vv + np);
+  if (refine) {
+    gw.R = vv + np;
+    gw.y = gw.R + nr * np;
+    gw.v = gw.y + nr * np;
+    gw.pack = gw.v + nr * np;
+    dr = (double*)(gw.pack + nr * np);
+  }
+  double* dc = dr + np;
+  unsigned long long* bits = (unsigned long long*)(dc + np);
+  double* red = (double*)(bits + np);  // 8 scalars
+  int* isgn = (int*)(red + 8);
+  if (refine) {
+    gw.wts = red + 8;
+    gw.stat = gw.wts + nr * np;
+    gw.part = gw.stat + 4 * nr;
+    isgn = (int*)(gw.part + 64 * np);
+  }
+  int* dperm = isgn + np;
+  if (refine) {
+    gw.isgn = dperm + np;
+    gw.flag = gw.isgn + nr * np;
+  }
   LseWork w{st, red, di + 2};
   if ((rc = trsv_err_reset(st))) return rc;
   CK(cudaMemcpyAsync(dA, A, nn * es, cudaMemcpyHostToDevice, st));
@@ -727,14 +761,17 @@ static int solve_dropin(int32_t n, double* A, int32_t* ipiv, int32_t aodim, doub
     }
     S* dbc = refine ? (S*)cx->bc.p : nullptr;
     if (refine) CK(cudaMemcpyAsync(dbc, db, (size_t)n * n_rhs * es, cudaMemcpyDeviceToDevice, st));
-    if ((rc = getrs_batched<S>(st, dA, 0, n, n, dp, 0, db, n, n_rhs))) return rc;
+    // the interchanges as one permutation, for every solve of the call
+    const int* perm = nullptr;
+    if (perm_fits(n)) {
+      if ((rc = perm_run(st, dp, 0, n, 1, dperm))) return rc;
+      perm = dperm;
+    }
+    if ((rc = getrs_batched<S>(st, dA, 0, n, n, dp, 0, db, n, n_rhs, false, perm))) return rc;
     if (refine) {
       g_lse.ferr.assign(n_rhs, 0.0);
       g_lse.berr.assign(n_rhs, 0.0);
-      for (int j = 0; j < n_rhs; ++j)
-        if ((rc = gerfs1<S>(w, dAo, dA, dp, n, dbc + (size_t)j * n, db + (size_t)j * n, vR, vy, vv, isgn, wts, part,
-                            &g_lse.ferr[j], &g_lse.berr[j])))
-          return rc;
+      if ((rc = gerfs<S>(w, dAo, dA, dp, perm, n, n_rhs, dbc, db, gw, g_lse.ferr.data(), g_lse.berr.data()))) return rc;
     }
     if (scaling && (eq == 'C' || eq == 'B')) {
       k_rows_scale<S><<<152 * 4, 256, 0, st>>>(db, n, n_rhs, dc); ++g_launches;

@@ -960,10 +960,14 @@ __global__ void __launch_bounds__(128) k_panel_nopiv(S* A, long long sA, int lda
 // CTA that is already running: no co-residency is needed. Waits on flags are
 // bounded; a wait that gives up sets *err and the CTA publishes its block
 // anyway, so every other wait ends too.
-// LOWER: unit lower L, forward; else upper U with its diagonal, backward.
+// OP: unit lower L (forward), U (backward), or the conjugate-transposed factors
+// U^H (forward) and L^H (backward) of getrs 'C' and the norm estimates, read
+// with the roles of rows and columns exchanged (a thread's loads of a tile then
+// touch one column each; they are prefetched before the wait).
 // ready[b * nb + blk] must be 0 and *counter 0 on entry. Dynamic shared
 // memory: trsv_sf_smem<S>() bytes.
 // ---------------------------------------------------------------------------
+enum TrOp { TR_L = 0, TR_U = 1, TR_UH = 2, TR_LH = 3 };
 constexpr long long kTrsvSpin = 1LL << 22;
 template <typename S>
 constexpr size_t trsv_sf_smem() {
@@ -998,7 +1002,7 @@ __device__ __forceinline__ double2 ld_pinned(const double2* p) {
   asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
   return v;
 }
-template <typename S, bool LOWER>
+template <typename S, int OP>
 __global__ void __launch_bounds__(256) k_trsv_sf(const S* A, long long sA, int lda, int n, S* x, long long sx,
                                                  int batch, int nb, unsigned* counter, int* ready, int* err,
                                                  long long spin) {
@@ -1006,6 +1010,9 @@ __global__ void __launch_bounds__(256) k_trsv_sf(const S* A, long long sA, int l
   // xs [64] (the solved block being applied), rinv [64] (reciprocals of U's
   // diagonal, formed before the wait so that no division lies on the chain)
   extern __shared__ __align__(16) unsigned char sfraw[];
+  constexpr bool FWD = OP == TR_L || OP == TR_UH;    // order of the blocks
+  constexpr bool UNIT = OP == TR_L || OP == TR_LH;   // unit diagonal
+  constexpr bool CT = OP == TR_UH || OP == TR_LH;    // conjugate-transposed factor
   S* D = reinterpret_cast<S*>(sfraw);
   S (*part)[64] = reinterpret_cast<S (*)[64]>(D + 64 * 65);
   S* xs = D + 64 * 65 + 4 * 64;
@@ -1019,7 +1026,7 @@ __global__ void __launch_bounds__(256) k_trsv_sf(const S* A, long long sA, int l
     const int item = s_item;
     if (item >= nb * batch) break;
     const int b = item % batch, q = item / batch;
-    const int blk = LOWER ? q : nb - 1 - q;
+    const int blk = FWD ? q : nb - 1 - q;
     const int r0 = blk * 64, w = min(64, n - r0);
     const S* M = A + sA * b;
     S* xb = x + sx * b;
@@ -1029,27 +1036,34 @@ __global__ void __launch_bounds__(256) k_trsv_sf(const S* A, long long sA, int l
     // 64 values and 16 FMAs
     S mreg[16];
     auto load_tile = [&](int qq) {
-      const int jb = LOWER ? qq : nb - 1 - qq;
+      const int jb = FWD ? qq : nb - 1 - qq;
       const int c0 = jb * 64, wc = min(64, n - c0);
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         const int c = grp + 4 * i;
-        mreg[i] = (row < w && c < wc) ? ld_pinned(M + (size_t)(c0 + c) * lda + r0 + row) : Sc<S>::zero();
+        if (CT) mreg[i] = (row < w && c < wc) ? Sc<S>::conj(ld_pinned(M + (size_t)(r0 + row) * lda + c0 + c)) : Sc<S>::zero();
+        else mreg[i] = (row < w && c < wc) ? ld_pinned(M + (size_t)(c0 + c) * lda + r0 + row) : Sc<S>::zero();
       }
     };
     if (q > 0) load_tile(0);
-    // diagonal block into shared memory (used after the contributions); the
-    // upper triangle's rows scaled by the reciprocals of U's diagonal, so
-    // that the substitution chain below carries no multiplication by them
-    if (!LOWER) {
-      if (t < w) rinv[t] = Sc<S>::rcp(M[(size_t)(r0 + t) * lda + r0 + t]);
+    // diagonal block into shared memory (used after the contributions),
+    // transposed and conjugated for CT; without a unit diagonal its rows scaled
+    // by the reciprocals of the diagonal, so that the substitution chain below
+    // carries no multiplication by them
+    if (!UNIT) {
+      if (t < w) {
+        const S d = M[(size_t)(r0 + t) * lda + r0 + t];
+        rinv[t] = Sc<S>::rcp(CT ? Sc<S>::conj(d) : d);
+      }
       __syncthreads();
     }
     for (int e = t; e < 64 * 64; e += 256) {
       const int i = e & 63, j = e >> 6;
       if (i < w && j < w) {
+        // e & 63 runs along a column of the factor either way
         const S v = M[(size_t)(r0 + j) * lda + r0 + i];
-        D[j * 65 + i] = LOWER ? v : Sc<S>::mul(v, rinv[i]);
+        if (CT) D[i * 65 + j] = UNIT ? Sc<S>::conj(v) : Sc<S>::mul(Sc<S>::conj(v), rinv[j]);
+        else D[j * 65 + i] = UNIT ? v : Sc<S>::mul(v, rinv[i]);
       }
     }
     // contributions of the solved blocks, in the order they were solved:
@@ -1059,7 +1073,7 @@ __global__ void __launch_bounds__(256) k_trsv_sf(const S* A, long long sA, int l
     for (int done = 0; done < q;) {
       if (t == 0) {
         long long it = 0;
-        const int jb0 = LOWER ? done : nb - 1 - done;
+        const int jb0 = FWD ? done : nb - 1 - done;
         while (ld_acquire_s32(ready + (size_t)b * nb + jb0) == 0) {
           if (++it > lim) {
             atomicExch(err, 1);
@@ -1068,18 +1082,18 @@ __global__ void __launch_bounds__(256) k_trsv_sf(const S* A, long long sA, int l
           if (it > 64) __nanosleep(64);
         }
         int e = done + 1;
-        while (e < q && ld_acquire_s32(ready + (size_t)b * nb + (LOWER ? e : nb - 1 - e)) != 0) ++e;
+        while (e < q && ld_acquire_s32(ready + (size_t)b * nb + (FWD ? e : nb - 1 - e)) != 0) ++e;
         s_end = e;
       }
       __syncthreads();
       const int end = s_end;
       for (int qq = done; qq < end; ++qq) {
-        const int jb = LOWER ? qq : nb - 1 - qq;
+        const int jb = FWD ? qq : nb - 1 - qq;
         const int c0 = jb * 64, wc = min(64, n - c0);
         if (t < 64) xs[t] = t < wc ? __ldcg(xb + c0 + t) : Sc<S>::zero();
         __syncthreads();
 #pragma unroll
-        for (int i = 0; i < 16; ++i) acc = Sc<S>::add(acc, Sc<S>::mul(mreg[i], xs[grp + 4 * i]));
+        for (int i = 0; i < 16; ++i) acc = lu_fnma(mreg[i], xs[grp + 4 * i], acc);
         __syncthreads();
         if (qq + 1 < q) load_tile(qq + 1);
       }
@@ -1090,24 +1104,26 @@ __global__ void __launch_bounds__(256) k_trsv_sf(const S* A, long long sA, int l
     if (t < 32) {
       const int l = t;
       S x0 = Sc<S>::zero(), x1 = Sc<S>::zero();
-      if (l < w) x0 = Sc<S>::sub(xb[r0 + l], Sc<S>::add(Sc<S>::add(part[0][l], part[1][l]), Sc<S>::add(part[2][l], part[3][l])));
+      if (l < w) x0 = Sc<S>::add(xb[r0 + l], Sc<S>::add(Sc<S>::add(part[0][l], part[1][l]), Sc<S>::add(part[2][l], part[3][l])));
       if (l + 32 < w)
-        x1 = Sc<S>::sub(xb[r0 + l + 32], Sc<S>::add(Sc<S>::add(part[0][l + 32], part[1][l + 32]),
+        x1 = Sc<S>::add(xb[r0 + l + 32], Sc<S>::add(Sc<S>::add(part[0][l + 32], part[1][l + 32]),
                                                     Sc<S>::add(part[2][l + 32], part[3][l + 32])));
-      if (LOWER) {
-        for (int j = 0; j < w; ++j) {
-          const S xj = shfl_s(j < 32 ? x0 : x1, j & 31);
-          if (l > j && l < w) x0 = Sc<S>::sub(x0, Sc<S>::mul(D[j * 65 + l], xj));
-          if (l + 32 > j && l + 32 < w) x1 = Sc<S>::sub(x1, Sc<S>::mul(D[j * 65 + l + 32], xj));
-        }
-      } else {
-        // rows pre-scaled: x_l = y_l / u_ll - sum_{j > l} (u_lj / u_ll) x_j
+      if (!UNIT) {
+        // rows pre-scaled: x_l = y_l / d_l - sum_j (d_lj / d_l) x_j
         if (l < w) x0 = Sc<S>::mul(x0, rinv[l]);
         if (l + 32 < w) x1 = Sc<S>::mul(x1, rinv[l + 32]);
+      }
+      if (FWD) {
+        for (int j = 0; j < w; ++j) {
+          const S xj = shfl_s(j < 32 ? x0 : x1, j & 31);
+          if (l > j && l < w) x0 = lu_fnma(D[j * 65 + l], xj, x0);
+          if (l + 32 > j && l + 32 < w) x1 = lu_fnma(D[j * 65 + l + 32], xj, x1);
+        }
+      } else {
         for (int j = w - 1; j >= 0; --j) {
           const S xj = shfl_s(j < 32 ? x0 : x1, j & 31);
-          if (l < j) x0 = Sc<S>::sub(x0, Sc<S>::mul(D[j * 65 + l], xj));
-          if (l + 32 < j) x1 = Sc<S>::sub(x1, Sc<S>::mul(D[j * 65 + l + 32], xj));
+          if (l < j) x0 = lu_fnma(D[j * 65 + l], xj, x0);
+          if (l + 32 < j) x1 = lu_fnma(D[j * 65 + l + 32], xj, x1);
         }
       }
       if (l < w) xb[r0 + l] = x0;

@@ -739,10 +739,10 @@ __global__ void k_perm(const int* ipiv, long long sP, int n, int* perm) {
   for (int i = threadIdx.x; i < n; i += blockDim.x) perm[(size_t)n * bi + i] = pm[i];
 }
 template <typename S>
-__global__ void k_gather_perm(const S* x, long long sx, const int* perm, int n, S* out) {
+__global__ void k_gather_perm(const S* x, long long sx, const int* perm, int sperm, int n, S* out) {
   const int bi = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  out[(size_t)n * bi + i] = x[sx * bi + perm[(size_t)n * bi + i]];
+  out[(size_t)n * bi + i] = x[sx * bi + perm[(size_t)sperm * bi + i]];
 }
 template <typename S>
 __global__ void k_scatter_back(const S* tmp, int n, S* x, long long sx) {
@@ -773,56 +773,70 @@ static int trsv_err_check(cudaStream_t st) {
   return 0;
 }
 
+// one triangular solve (TrOp) of a batch in one launch: ready flags [batch][nb]
+// and a counter
+template <typename S, int OP>
+static int trsv_sf_run(cudaStream_t st, const S* A, long long sA, int lda, int n, S* b, long long sb, int batch) {
+  const int nb = (n + 63) / 64;
+  int rc = ensure(g_sf_ws, sizeof(int) * ((size_t)batch * nb + 1));
+  if (rc) return rc;
+  if (!g_sf_err.p) return fail(MFBEM_ECUDA, "triangular solve: error flag not set up");
+  int* ready = (int*)g_sf_ws.p;
+  unsigned* ctr = (unsigned*)(ready + (size_t)batch * nb);
+  int dev = 0, nsm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  const unsigned g = (unsigned)std::max(1, std::min(batch * nb, 2 * nsm));
+  if (raise_smem_limit((const void*)k_trsv_sf<S, OP>)) return fail(MFBEM_ECUDA, "shared-memory limit of the triangular solve");
+  CK(cudaMemsetAsync(g_sf_ws.p, 0, sizeof(int) * ((size_t)batch * nb + 1), st));
+  k_trsv_sf<S, OP><<<g, 256, trsv_sf_smem<S>(), st>>>(A, sA, lda, n, b, sb, batch, nb, ctr, ready, (int*)g_sf_err.p,
+                                                      g_spin_limit.load());
+  ++g_launches;
+  CK(cudaGetLastError());
+  return 0;
+}
+
+// the interchanges of each factorisation as one permutation (k_perm), where
+// its index array fits shared memory
+static bool perm_fits(int n) { return (size_t)n * sizeof(int) <= 200 * 1024; }
+static int perm_run(cudaStream_t st, const int* ipiv, long long sP, int n, int batch, int* perm) {
+  const size_t psm = (size_t)n * sizeof(int);
+  if (psm > 48 * 1024 && raise_smem_limit((const void*)k_perm)) return fail(MFBEM_ECUDA, "shared-memory limit of the row permutation");
+  k_perm<<<batch, 256, psm, st>>>(ipiv, sP, n, perm); ++g_launches;
+  CK(cudaGetLastError());
+  return 0;
+}
+
 // no_interchanges: the factors come from the unpivoted factorisation (ipiv is
-// the identity), so the permutation step is skipped
+// the identity), so the permutation step is skipped. perm (or null): the
+// permutation of perm_run for one factorisation that all systems share, so
+// that a caller with many solves forms it once (it is one thread's chain of n
+// exchanges, 97 us at n = 1999).
 template <typename S>
 static int getrs_batched(cudaStream_t st, const S* A, long long sA, int lda, int n, const int* ipiv, long long sP,
-                         S* b, long long sb, int batch, bool no_interchanges = false) {
-  // diagonal blocks of TB rows solved by one warp (k_trsv_diag64), the rows
-  // below / above updated by a GEMV over the solved block
-  const int TB = 64;
-  const size_t dsm = (size_t)TB * 65 * sizeof(S);
-  if (raise_smem_limit((const void*)k_trsv_diag64<S, true>) || raise_smem_limit((const void*)k_trsv_diag64<S, false>))
-    return fail(MFBEM_ECUDA, "shared-memory limit of the triangular solve");
-  const size_t psm = (size_t)n * sizeof(int);
+                         S* b, long long sb, int batch, bool no_interchanges = false, const int* perm1 = nullptr) {
   bool gathered = no_interchanges;
-  if (!gathered && psm <= 200 * 1024) {
+  if (!gathered && (perm1 || perm_fits(n))) {
     int rc = ensure(g_rs_ws, (size_t)batch * n * (sizeof(int) + sizeof(S)) + 256);
     if (rc) return rc;
-    if (psm > 48 * 1024 && raise_smem_limit((const void*)k_perm)) return fail(MFBEM_ECUDA, "shared-memory limit of the row permutation");
     int* perm = (int*)g_rs_ws.p;
     S* tmp = (S*)((char*)g_rs_ws.p + ((size_t)batch * n * sizeof(int) + 255) / 256 * 256);
-    k_perm<<<batch, 256, psm, st>>>(ipiv, sP, n, perm); ++g_launches;
-    k_gather_perm<S><<<dim3(nblk(n, 256), batch), 256, 0, st>>>(b, sb, perm, n, tmp); ++g_launches;
+    if (!perm1 && (rc = perm_run(st, ipiv, sP, n, batch, perm))) return rc;
+    k_gather_perm<S><<<dim3(nblk(n, 256), batch), 256, 0, st>>>(b, sb, perm1 ? perm1 : perm, perm1 ? 0 : n, n, tmp); ++g_launches;
     k_scatter_back<S><<<dim3(nblk(n, 256), batch), 256, 0, st>>>(tmp, n, b, sb); ++g_launches;
     gathered = true;
   }
   if (!gathered) { k_rhs_swap2<S><<<nblk(batch, 64), 64, 0, st>>>(b, sb, n, ipiv, sP, batch); ++g_launches; }
   if (trsv_sync_free()) {
-    // one launch per triangle (k_trsv_sf): ready flags [batch][nb] and a counter
-    const int nb = (n + 63) / 64;
-    int rc = ensure(g_sf_ws, sizeof(int) * ((size_t)batch * nb + 1));
-    if (rc) return rc;
-    if (!g_sf_err.p) return fail(MFBEM_ECUDA, "triangular solve: error flag not set up");
-    int* ready = (int*)g_sf_ws.p;
-    unsigned* ctr = (unsigned*)(ready + (size_t)batch * nb);
-    int* err = (int*)g_sf_err.p;
-    int dev = 0, nsm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const unsigned g = (unsigned)std::max(1, std::min(batch * nb, 2 * nsm));
-    constexpr size_t smem = trsv_sf_smem<S>();
-    if (raise_smem_limit((const void*)k_trsv_sf<S, true>) || raise_smem_limit((const void*)k_trsv_sf<S, false>))
-      return fail(MFBEM_ECUDA, "shared-memory limit of the triangular solve");
-    CK(cudaMemsetAsync(g_sf_ws.p, 0, sizeof(int) * ((size_t)batch * nb + 1), st));
-    k_trsv_sf<S, true><<<g, 256, smem, st>>>(A, sA, lda, n, b, sb, batch, nb, ctr, ready, err, g_spin_limit.load());
-    ++g_launches;
-    CK(cudaMemsetAsync(g_sf_ws.p, 0, sizeof(int) * ((size_t)batch * nb + 1), st));
-    k_trsv_sf<S, false><<<g, 256, smem, st>>>(A, sA, lda, n, b, sb, batch, nb, ctr, ready, err, g_spin_limit.load());
-    ++g_launches;
-    CK(cudaGetLastError());
-    return 0;
+    int rc = trsv_sf_run<S, TR_L>(st, A, sA, lda, n, b, sb, batch);
+    return rc ? rc : trsv_sf_run<S, TR_U>(st, A, sA, lda, n, b, sb, batch);
   }
+  // block by block: diagonal blocks of TB rows solved by one warp
+  // (k_trsv_diag64), the rows below / above updated by a GEMV over the solved block
+  const int TB = 64;
+  const size_t dsm = (size_t)TB * 65 * sizeof(S);
+  if (raise_smem_limit((const void*)k_trsv_diag64<S, true>) || raise_smem_limit((const void*)k_trsv_diag64<S, false>))
+    return fail(MFBEM_ECUDA, "shared-memory limit of the triangular solve");
   for (int r0 = 0; r0 < n; r0 += TB) {
     int w = std::min(TB, n - r0);
     k_trsv_diag64<S, true><<<batch, 128, dsm, st>>>(A, sA, lda, b, sb, r0, w); ++g_launches;
