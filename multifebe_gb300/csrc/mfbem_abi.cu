@@ -119,6 +119,7 @@ struct mfbem_handle {
   // radial tables of the last harmonic call and a bound of the distance
   // between any two points of the mesh's elements
   DevBuf rad;
+  DevBuf slc;  // copies of the system for the pair kernels' slices
   double rmax = 0.0;
   double box_lo[3] = {0, 0, 0}, box_hi[3] = {0, 0, 0};  // box that holds every element
   // work buffers of the internal points, in the order of their use (grown as
@@ -876,7 +877,7 @@ extern "C" int mfbem_mesh_release(mfbem_handle* h) {
     cudaDeviceSynchronize();
     for (auto& o : h->owned) pool_give(o.first, o.second, h->dev);
     for (DevBuf* b : {&h->A, &h->b, &h->A32, &h->x, &h->r, &h->work, &h->ipiv, &h->info, &h->par, &h->nu, &h->parf,
-                      &h->pphi_f, &h->geo_f, &h->gm, &h->parh, &h->rad})
+                      &h->pphi_f, &h->geo_f, &h->gm, &h->parh, &h->rad, &h->slc})
       pool_give(b->p, b->bytes, b->dev);
     for (DevBuf& b : h->ip_ws) pool_give(b.p, b.bytes, b.dev);
     if (h->st) {
@@ -1089,7 +1090,32 @@ static int launch_assembly(mfbem_handle* h, const POL& pol, const double* d_nu, 
                            const ff* sgf = nullptr, const ff* lgf = nullptr) {
   const DMesh& m = h->m;
   constexpr int WPB = 4;
-  long long nw = (long long)m.ndn * nf;
+  const long long nw0 = (long long)m.ndn * nf;
+  // slices per node (see Slices): up to 2432 warps -- 16 on each SM -- where the
+  // nodes alone give fewer than six on each, 8 slices at most, within 2 GB of
+  // copies. Static 870-unknown cube (290 nodes, 8 slices): regular pairs 1.35 ->
+  // 0.33 ms, singular pairs 1.18 -> 0.39; footing (225 nodes) 9.0 -> 1.7 ms in
+  // all; complex, 740 nodes: 5.0 -> 3.1. At 1154 nodes three slices lose (9.4 ->
+  // 10.4 ms): the binary64 pipe is full and the copies cost traffic.
+  constexpr bool kReal = std::is_same<POL, PolStatic>::value;
+  constexpr int W = kReal ? 1 : 2;
+  Slices z;
+  const size_t sysz = (size_t)m.ndof * m.ndof * W * nf;
+  if (nw0 > 0 && nw0 < 6 * 152) z.n = (int)std::min<long long>(8, (2432 + nw0 - 1) / nw0);
+  while (z.n > 1 && (z.n - 1) * sysz * sizeof(double) > ((size_t)2 << 30)) --z.n;
+  if (z.n > 1) {
+    const size_t bsz = (size_t)m.ndof * W * nf;
+    if (int rc = ensure(h->slc, (z.n - 1) * (sysz + bsz) * sizeof(double))) return rc;
+    z.A = (double*)h->slc.p;
+    z.lda = m.ndof;
+    z.astride = (size_t)m.ndof * m.ndof * W;
+    z.sstride = sysz;
+    z.b = z.A + (z.n - 1) * sysz;
+    z.bstride = (size_t)m.ndof * W;
+    z.sbstride = bsz;
+    CK(cudaMemsetAsync(z.A, 0, (z.n - 1) * (sysz + bsz) * sizeof(double), h->st));
+  }
+  const long long nw = nw0 * z.n;
   // the double-float kernels write rows 3 dn + il: a region with crack-like
   // boundaries (six rows per crack node) assembles in binary64 only
   if (h->has_crack) mixed = false;
@@ -1153,49 +1179,49 @@ static int launch_assembly(mfbem_handle* h, const POL& pol, const double* d_nu, 
     if constexpr (!kStatic) {
       if (mixed && pf && dsf) {
         k_mixed<MIX_REG, 2, kRad><<<nblk(nw, 2), 64, 0, h->st>>>(m, rt, pf, dsf, nullptr, nf, (double2*)A, lda,
-                                                               astride / 2, b, bstride);
+                                                               astride / 2, b, bstride, z);
       } else {
-        k_reg<POL, WPB><<<g, WPB * 32, 0, h->st>>>(m, pol, nf, A, lda, astride, b, bstride);
+        k_reg<POL, WPB><<<g, WPB * 32, 0, h->st>>>(m, pol, nf, A, lda, astride, b, bstride, z);
       }
     } else {
-      k_reg<POL, WPB><<<g, WPB * 32, 0, h->st>>>(m, pol, nf, A, lda, astride, b, bstride);
+      k_reg<POL, WPB><<<g, WPB * 32, 0, h->st>>>(m, pol, nf, A, lda, astride, b, bstride, z);
     }
     ++g_launches;
   }
   if constexpr (kStatic) {
     if (hs && mh.nreg > 0) {
-      k_reg<PolHsc, WPB><<<g, WPB * 32, 0, h->st>>>(mh, ph, nf, A, lda, astride, b, bstride);
+      k_reg<PolHsc, WPB><<<g, WPB * 32, 0, h->st>>>(mh, ph, nf, A, lda, astride, b, bstride, z);
       ++g_launches;
     }
   }
   if (bm && msv.nreg > 0) {
-    k_reg<POL, WPB><<<g, WPB * 32, 0, h->st>>>(msv, pol, nf, A, lda, astride, b, bstride);
+    k_reg<POL, WPB><<<g, WPB * 32, 0, h->st>>>(msv, pol, nf, A, lda, astride, b, bstride, z);
     ++g_launches;
   }
   if (hb && mb.nreg > 0) {
-    k_reg<PolH, WPB><<<g, WPB * 32, 0, h->st>>>(mb, phb, nf, A, lda, astride, b, bstride);
+    k_reg<PolH, WPB><<<g, WPB * 32, 0, h->st>>>(mb, phb, nf, A, lda, astride, b, bstride, z);
     ++g_launches;
   }
   if (tm) cudaEventRecord(tm->ev[1], h->st);
   if (m.nadp > 0) {
     if (mixed && lgf)
       k_mixed<MIX_ADP, 2, kRad><<<nblk(nw, 2), 64, 0, h->st>>>(m, rt, pf, dsf, lgf, nf, (double2*)A, lda, astride / 2, b,
-                                                             bstride);
-    else k_adp<POL, WPB><<<g, WPB * 32, 0, h->st>>>(m, pol, nf, A, lda, astride, b, bstride);
+                                                             bstride, z);
+    else k_adp<POL, WPB><<<g, WPB * 32, 0, h->st>>>(m, pol, nf, A, lda, astride, b, bstride, z);
     ++g_launches;
   }
   if constexpr (kStatic) {
     if (hs && mh.nadp > 0) {
-      k_adp<PolHsc, WPB><<<g, WPB * 32, 0, h->st>>>(mh, ph, nf, A, lda, astride, b, bstride);
+      k_adp<PolHsc, WPB><<<g, WPB * 32, 0, h->st>>>(mh, ph, nf, A, lda, astride, b, bstride, z);
       ++g_launches;
     }
   }
   if (bm && msv.nadp > 0) {
-    k_adp<POL, WPB><<<g, WPB * 32, 0, h->st>>>(msv, pol, nf, A, lda, astride, b, bstride);
+    k_adp<POL, WPB><<<g, WPB * 32, 0, h->st>>>(msv, pol, nf, A, lda, astride, b, bstride, z);
     ++g_launches;
   }
   if (hb && mb.nadp > 0) {
-    k_adp<PolH, WPB><<<g, WPB * 32, 0, h->st>>>(mb, phb, nf, A, lda, astride, b, bstride);
+    k_adp<PolH, WPB><<<g, WPB * 32, 0, h->st>>>(mb, phb, nf, A, lda, astride, b, bstride, z);
     ++g_launches;
   }
   if (tm) cudaEventRecord(tm->ev[2], h->st);
@@ -1203,30 +1229,35 @@ static int launch_assembly(mfbem_handle* h, const POL& pol, const double* d_nu, 
   if (m.nsing > 0) {
     if (mixed && sgf)
       k_mixed<MIX_SING, 2, kRad><<<nblk(nw, 2), 64, 0, h->st>>>(m, rt, pf, dsf, sgf, nf, (double2*)A, lda, astride / 2, b,
-                                                                bstride);
-    else k_sing<POL, 2><<<nblk(nw, 2), 64, 0, h->st>>>(m, pol, nf, A, lda, astride, b, bstride);
+                                                                bstride, z);
+    else k_sing<POL, 2><<<nblk(nw, 2), 64, 0, h->st>>>(m, pol, nf, A, lda, astride, b, bstride, z);
     ++g_launches;
   }
   if constexpr (kStatic) {
     if (hs && mh.nsing > 0) {
-      k_sing<PolHscSing, 2><<<nblk(nw, 2), 64, 0, h->st>>>(mh, phs, nf, A, lda, astride, b, bstride);
+      k_sing<PolHscSing, 2><<<nblk(nw, 2), 64, 0, h->st>>>(mh, phs, nf, A, lda, astride, b, bstride, z);
       ++g_launches;
     }
   }
   if (bm && msv.nsing > 0) {
-    k_sing<POL, 2><<<nblk(nw, 2), 64, 0, h->st>>>(msv, pol, nf, A, lda, astride, b, bstride);
+    k_sing<POL, 2><<<nblk(nw, 2), 64, 0, h->st>>>(msv, pol, nf, A, lda, astride, b, bstride, z);
     ++g_launches;
   }
   if (hb && mb.nsing > 0) {
-    k_hsing<HsK><<<(unsigned)nw, 32, 0, h->st>>>(mb, hsk, nf, A, lda, astride, b, bstride);
+    k_hsing<HsK><<<(unsigned)nw, 32, 0, h->st>>>(mb, hsk, nf, A, lda, astride, b, bstride, z);
+    ++g_launches;
+  }
+  if (z.n > 1) {
+    k_slice_sum<<<dim3(nblk((long long)m.ndof * W, 256), m.ndof, nf), 256, 0, h->st>>>(z, m.ndof, W, A, lda, astride, b,
+                                                                                      bstride);
     ++g_launches;
   }
   if (tm) cudaEventRecord(tm->ev[3], h->st);
-  k_free<POL><<<nblk(nw, 128), 128, 0, h->st>>>(m, pol, d_nu, nf, A, lda, astride, b, bstride, h->d_err); ++g_launches;
+  k_free<POL><<<nblk(nw0, 128), 128, 0, h->st>>>(m, pol, d_nu, nf, A, lda, astride, b, bstride, h->d_err); ++g_launches;
   if (hb) {
     const HarParH* pph = nullptr;
     if constexpr (!kStatic) pph = pol.ph;
-    k_hfree<typename POL::T><<<nblk(nw, 128), 128, 0, h->st>>>(mb, pph, nf, A, lda, astride, b, bstride);
+    k_hfree<typename POL::T><<<nblk(nw0, 128), 128, 0, h->st>>>(mb, pph, nf, A, lda, astride, b, bstride);
     ++g_launches;
   }
   if (tm) cudaEventRecord(tm->ev[4], h->st);

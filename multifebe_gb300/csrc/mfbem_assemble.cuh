@@ -286,6 +286,56 @@ __device__ __forceinline__ void flush_pair(const DMesh& m, const POL& pol, int f
   __syncwarp();
 }
 
+// A node's points can be dealt out to several warps (slices) when the nodes and
+// frequencies of a call do not fill the GPU. Slice 0 adds to the system itself,
+// slice s > 0 to a copy of its own (k_slice_sum adds the copies in order), so
+// no two warps add to the same entry and the result does not depend on timing.
+// A pair cut by a slice's end is flushed by both (its sums are linear; the
+// line-integral part of a singular pair goes with its first point).
+struct Slices {
+  int n = 1;
+  double* A = nullptr;
+  size_t lda = 0, astride = 0, sstride = 0;
+  double* b = nullptr;
+  size_t bstride = 0, sbstride = 0;
+};
+struct SliceRef {
+  int sl;
+  long long wid;  // dn + ndn f
+  __device__ SliceRef(const Slices& z, long long gw, long long nw, double*& A, size_t& lda, size_t& astride, double*& b,
+                      size_t& bstride) {
+    sl = (int)(gw / nw);
+    wid = gw - sl * nw;
+    if (sl > 0) {
+      A = z.A + (sl - 1) * z.sstride;
+      lda = z.lda;
+      astride = z.astride;
+      b = z.b + (sl - 1) * z.sbstride;
+      bstride = z.bstride;
+    }
+  }
+  // this slice's part [lo, hi) of Q points
+  __device__ void part(const Slices& z, long long Q, long long& lo, long long& hi) const {
+    lo = Q * sl / z.n;
+    hi = Q * (sl + 1) / z.n;
+  }
+};
+// A, b += the slices' copies (W doubles per entry: 1 real, 2 complex), in slice order
+__global__ void k_slice_sum(Slices z, int n, int W, double* A, size_t lda, size_t astride, double* b, size_t bstride) {
+  const int f = blockIdx.z, col = blockIdx.y;
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= n * W) return;
+  const double* s = z.A + z.astride * f + (size_t)col * z.lda * W + r;
+  double v = 0.0;
+  for (int i = 0; i < z.n - 1; ++i) v += s[(size_t)i * z.sstride];
+  A[astride * f + (size_t)col * lda * W + r] += v;
+  if (col == 0) {
+    double vb = 0.0;
+    for (int i = 0; i < z.n - 1; ++i) vb += z.b[(size_t)i * z.sbstride + z.bstride * f + r];
+    b[bstride * f + r] += vb;
+  }
+}
+
 template <typename T, int NG = 6>
 struct alignas(16) Combo {
   T fu[NG], ft[9];
@@ -342,26 +392,29 @@ __device__ __forceinline__ void accumulate(T* acc, const T* fug, const T* ft, co
 // ---------------------------------------------------------------- regular pairs
 template <class POL, int WPB>
 __global__ void __launch_bounds__(WPB * 32) k_reg(DMesh m, POL pol, int nf, double* A, size_t lda, size_t astride,
-                                                  double* b, size_t bstride) {
+                                                  double* b, size_t bstride, Slices z) {
   typedef typename POL::T T;
   constexpr int NG = POL::NG, NA = GOut<NG>::acc;
   __shared__ Combo<T, NG> sm[WPB][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x / 32;
   const long long gw = blockIdx.x * (long long)WPB + w;
-  if (gw >= (long long)m.ndn * nf) return;
-  const int dn = (int)(gw % m.ndn), f = (int)(gw / m.ndn);
+  if (gw >= (long long)m.ndn * nf * z.n) return;
+  const SliceRef zr(z, gw, (long long)m.ndn * nf, A, lda, astride, b, bstride);
+  const int dn = (int)(zr.wid % m.ndn), f = (int)(zr.wid / m.ndn);
   Combo<T, NG>* S = sm[w];
   for (int cp = m.dn_cp[dn]; cp < m.dn_cp[dn + 1]; ++cp) {
     const int s0 = m.reg_start[cp], s1 = m.reg_start[cp + 1];
     if (s0 == s1) continue;
     const double* xi = m.cpx + 3 * (size_t)cp;
     const long long P0 = m.reg_pt[s0], Q = m.reg_pt[s1] - P0;
+    long long lo, hi;
+    zr.part(z, Q, lo, hi);
     int cur = -1;
     T acc[NA];
     for (int j = 0; j < NA; ++j) acc[j] = VT<T>::zero();
-    for (long long base = 0; base < Q; base += 32) {
+    for (long long base = lo; base < hi; base += 32) {
       long long c = base + lane;
-      if (c < Q) {
+      if (c < hi) {
         int jp = find_le(m.reg_pt, s0, s1, P0 + c);
         int pr = m.reg_pair[jp];
         int e = pr & 0xFFFFFF, ps = pr >> 24;
@@ -375,7 +428,7 @@ __global__ void __launch_bounds__(WPB * 32) k_reg(DMesh m, POL pol, int nf, doub
         S[lane].pair = jp;
       }
       __syncwarp();
-      int nt = (int)min((long long)32, Q - base);
+      int nt = (int)min((long long)32, hi - base);
       for (int t = 0; t < nt; ++t) {
         int jp = S[t].pair;
         if (jp != cur) {
@@ -433,14 +486,15 @@ __device__ __forceinline__ void leaf_point(const DMesh& m, int l, int a, int k, 
 
 template <class POL, int WPB>
 __global__ void __launch_bounds__(WPB * 32) k_adp(DMesh m, POL pol, int nf, double* A, size_t lda, size_t astride,
-                                                  double* b, size_t bstride) {
+                                                  double* b, size_t bstride, Slices z) {
   typedef typename POL::T T;
   constexpr int NG = POL::NG, NA = GOut<NG>::acc;
   __shared__ Combo<T, NG> sm[WPB][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x / 32;
   const long long gw = blockIdx.x * (long long)WPB + w;
-  if (gw >= (long long)m.ndn * nf) return;
-  const int dn = (int)(gw % m.ndn), f = (int)(gw / m.ndn);
+  if (gw >= (long long)m.ndn * nf * z.n) return;
+  const SliceRef zr(z, gw, (long long)m.ndn * nf, A, lda, astride, b, bstride);
+  const int dn = (int)(zr.wid % m.ndn), f = (int)(zr.wid / m.ndn);
   Combo<T, NG>* S = sm[w];
   for (int cp = m.dn_cp[dn]; cp < m.dn_cp[dn + 1]; ++cp) {
     const int a0 = m.adp_start[cp], a1 = m.adp_start[cp + 1];
@@ -448,12 +502,14 @@ __global__ void __launch_bounds__(WPB * 32) k_adp(DMesh m, POL pol, int nf, doub
     const int l0 = m.adp_leaf[a0], l1 = m.adp_leaf[a1];
     const double* xi = m.cpx + 3 * (size_t)cp;
     const long long P0 = m.leaf_pt[l0], Q = m.leaf_pt[l1] - P0;
+    long long lo, hi;
+    zr.part(z, Q, lo, hi);
     int cur = -1;
     T acc[NA];
     for (int j = 0; j < NA; ++j) acc[j] = VT<T>::zero();
-    for (long long base = 0; base < Q; base += 32) {
+    for (long long base = lo; base < hi; base += 32) {
       long long c = base + lane;
-      if (c < Q) {
+      if (c < hi) {
         int l = find_le(m.leaf_pt, l0, l1, P0 + c);
         int a = m.leaf_pair[l];
         if (m.leaf_geo) {
@@ -476,7 +532,7 @@ __global__ void __launch_bounds__(WPB * 32) k_adp(DMesh m, POL pol, int nf, doub
         S[lane].pair = a;
       }
       __syncwarp();
-      int nt = (int)min((long long)32, Q - base);
+      int nt = (int)min((long long)32, hi - base);
       for (int t = 0; t < nt; ++t) {
         int a = S[t].pair;
         if (a != cur) {
@@ -565,26 +621,29 @@ __global__ void k_leaf_geo(DMesh m) {
 
 template <class POL, int WPB>
 __global__ void __launch_bounds__(WPB * 32) k_sing(DMesh m, POL pol, int nf, double* A, size_t lda, size_t astride,
-                                                   double* b, size_t bstride) {
+                                                   double* b, size_t bstride, Slices z) {
   typedef typename POL::T T;
   constexpr int NG = POL::NG, NA = GOut<NG>::acc;
   __shared__ ComboS<T, NG> sm[WPB][32];
   __shared__ double hp[WPB][17];  // hli[9], phi_i[8] of the pair being flushed
   const int lane = threadIdx.x & 31, w = threadIdx.x / 32;
   const long long gw = blockIdx.x * (long long)WPB + w;
-  if (gw >= (long long)m.ndn * nf) return;
-  const int dn = (int)(gw % m.ndn), f = (int)(gw / m.ndn);
+  if (gw >= (long long)m.ndn * nf * z.n) return;
+  const SliceRef zr(z, gw, (long long)m.ndn * nf, A, lda, astride, b, bstride);
+  const int dn = (int)(zr.wid % m.ndn), f = (int)(zr.wid / m.ndn);
   ComboS<T, NG>* S = sm[w];
   for (int cp = m.dn_cp[dn]; cp < m.dn_cp[dn + 1]; ++cp) {
     const int q0 = m.sing_start[cp], q1 = m.sing_start[cp + 1];
     if (q0 == q1) continue;
     const long long P0 = m.sing_pt[q0], Q = m.sing_pt[q1] - P0;
+    long long lo, hi;
+    zr.part(z, Q, lo, hi);
     int cur = -1;
     T acc[NA], acd[NA];
     for (int j = 0; j < NA; ++j) acc[j] = acd[j] = VT<T>::zero();
-    for (long long base = 0; base < Q; base += 32) {
+    for (long long base = lo; base < hi; base += 32) {
       long long c = base + lane;
-      if (c < Q) {
+      if (c < hi) {
         int q = find_le(m.sing_pt, q0, q1, P0 + c);
         double rv[3], n[3];
         if (m.sing_geo) {
@@ -605,13 +664,14 @@ __global__ void __launch_bounds__(WPB * 32) k_sing(DMesh m, POL pol, int nf, dou
         S[lane].pair = q;
       }
       __syncwarp();
-      int nt = (int)min((long long)32, Q - base);
+      int nt = (int)min((long long)32, hi - base);
       for (int t = 0; t < nt; ++t) {
         int q = S[t].pair;
         if (q != cur) {
           if (cur >= 0) {
             for (int j = 0; j < NA; ++j) acc[j] = acc[j] + acd[j];
-            flush_pair(m, pol, f, dn, m.sing_e[cur], acc, A, lda, astride, b, bstride, hp[w]);
+            flush_pair(m, pol, f, dn, m.sing_e[cur], acc, A, lda, astride, b, bstride,
+                       m.sing_pt[cur] >= P0 + lo ? hp[w] : nullptr);
           }
           cur = q;
           for (int j = 0; j < NA; ++j) acc[j] = acd[j] = VT<T>::zero();
@@ -636,7 +696,8 @@ __global__ void __launch_bounds__(WPB * 32) k_sing(DMesh m, POL pol, int nf, dou
     }
     if (cur >= 0) {
       for (int j = 0; j < NA; ++j) acc[j] = acc[j] + acd[j];
-      flush_pair(m, pol, f, dn, m.sing_e[cur], acc, A, lda, astride, b, bstride, hp[w]);
+      flush_pair(m, pol, f, dn, m.sing_e[cur], acc, A, lda, astride, b, bstride,
+                       m.sing_pt[cur] >= P0 + lo ? hp[w] : nullptr);
     }
   }
 }
@@ -1165,7 +1226,7 @@ enum MixKind { MIX_REG = 0, MIX_ADP = 1, MIX_SING = 2 };
 template <int KIND, int WPB, bool TAB>
 __global__ void __launch_bounds__(WPB * 32, KIND == MIX_SING ? 5 : 8) k_mixed(DMesh m, RadTab rt, const HarParF* pf, const ff* dsf,
                                                        const ff* gf, int nf, double2* Ac, size_t lda, size_t astride_e,
-                                                       double* b, size_t bstride) {
+                                                       double* b, size_t bstride, Slices z) {
   constexpr bool SG = KIND == MIX_SING;
   typedef PtRec<SG> R;
   __shared__ __align__(16) char sm[WPB][32 * R::kSize];
@@ -1173,14 +1234,17 @@ __global__ void __launch_bounds__(WPB * 32, KIND == MIX_SING ? 5 : 8) k_mixed(DM
   __shared__ ff hps[WPB][SG ? 17 : 1];
   const int lane = threadIdx.x & 31, w = threadIdx.x / 32;
   const long long gw = blockIdx.x * (long long)WPB + w;
-  if (gw >= (long long)m.ndn * nf) return;
-  const int dn = (int)(gw % m.ndn), f = (int)(gw / m.ndn);
+  if (gw >= (long long)m.ndn * nf * z.n) return;
+  double* Ad = reinterpret_cast<double*>(Ac);
+  size_t astride = 2 * astride_e;
+  const SliceRef zr(z, gw, (long long)m.ndn * nf, Ad, lda, astride, b, bstride);
+  const int dn = (int)(zr.wid % m.ndn), f = (int)(zr.wid / m.ndn);
   char* S = sm[w];
   char* my = S + lane * R::kSize;
   const ff* pphi_f = dsf;
   const ff* pn_f = dsf + 8LL * m.ne * m.ptot;
   const ff* dcv_f = pn_f + 3LL * m.ne * m.ptot;
-  double* Arow = reinterpret_cast<double*>(Ac + astride_e * f + 3 * (size_t)dn);
+  double* Arow = Ad + astride * f + 6 * (size_t)dn;
   // phase 2 layout: component comp (t* 0..8, u* 9..14; the 16th lane of a half
   // repeats the 15th) and nodes 4 half .. 4 half + 3
   const int half = lane >> 4, comp = min(lane & 15, 14);
@@ -1205,14 +1269,18 @@ __global__ void __launch_bounds__(WPB * 32, KIND == MIX_SING ? 5 : 8) k_mixed(DM
     if (s0 == s1) continue;
     const double* xi = m.cpx + 3 * (size_t)cp;
     const long long P0 = pts[s0];
-    const int Qn = (int)(pts[s1] - P0);
+    long long lo_, hi_;
+    zr.part(z, pts[s1] - P0, lo_, hi_);
+    const int lo = (int)lo_, Qn = (int)hi_;
+    if (lo == Qn) continue;
     int cur = -1;  // pair whose sums are open
     c2 acc[4], acd;
 #pragma unroll
     for (int k = 0; k < 4; ++k) acc[k] = c2_zero();
     acd = c2_zero();
-    int jw = s0;  // list entry of the batch's first point, before its own start bits
-    for (int base = 0; base < Qn; base += 32) {
+    // list entry of the batch's first point, before the start bits of the batch
+    int jw = lo == 0 ? s0 : find_le(pts, s0, s1, P0 + lo);
+    for (int base = lo; base < Qn; base += 32) {
       // starts of the list entries after jw inside this batch
       const int jn = jw + 1 + lane;
       const long long bd = jn < s1 ? pts[jn] - P0 - base : 32;
@@ -1274,7 +1342,7 @@ __global__ void __launch_bounds__(WPB * 32, KIND == MIX_SING ? 5 : 8) k_mixed(DM
         if (pr != cur) {
           if (cur >= 0) {
             const int e = KIND == MIX_REG ? (m.reg_pair[cur] & 0xFFFFFF) : (KIND == MIX_ADP ? m.adp_e[cur] : m.sing_e[cur]);
-            flush_pair_ff<SG>(m, cpv, dcv_f, e, acc, acd, Arow, lda, comp, half, cil, cik, bc0, bc1, stg[w], hps[w]);
+            flush_pair_ff<SG>(m, SG && m.sing_pt[cur] < P0 + lo ? cf_zero() : cpv, dcv_f, e, acc, acd, Arow, lda, comp, half, cil, cik, bc0, bc1, stg[w], hps[w]);
           }
           cur = pr;
 #pragma unroll

@@ -477,7 +477,7 @@ __device__ __forceinline__ void hsing_scatter(const DMesh& m, int dn, int e, int
 // o = lane + 32 j (m: o < 72, l: o >= 72) and the 36 pair sums P, Q.
 template <class HS>
 __global__ void __launch_bounds__(32) k_hsing(DMesh m, HS hs, int nf, double* A, size_t lda, size_t astride, double* b,
-                                              size_t bstride) {
+                                              size_t bstride, Slices z_) {
   typedef typename HS::T T;
   constexpr int NA = 5;  // 144 outputs over 32 lanes
   __shared__ ComboH<T> S[32];
@@ -485,8 +485,9 @@ __global__ void __launch_bounds__(32) k_hsing(DMesh m, HS hs, int nf, double* A,
   __shared__ double ex[8 + 24 + 3 + 52];  // phi_i, psi_i, n_i, line integrals of the pair being flushed
   const int lane = threadIdx.x & 31;
   const long long gw = blockIdx.x;
-  if (gw >= (long long)m.ndn * nf) return;
-  const int dn = (int)(gw % m.ndn), f = (int)(gw / m.ndn);
+  if (gw >= (long long)m.ndn * nf * z_.n) return;
+  const SliceRef zr(z_, gw, (long long)m.ndn * nf, A, lda, astride, b, bstride);
+  const int dn = (int)(zr.wid % m.ndn), f = (int)(zr.wid / m.ndn);
   const HsCoef<T> k = hs.coef(f);
   const T z = VT<T>::zero();
   double* Af = A + astride * f;
@@ -495,10 +496,13 @@ __global__ void __launch_bounds__(32) k_hsing(DMesh m, HS hs, int nf, double* A,
     if (q0 == q1) continue;
     const T beta = hbie_weighted(m.cp_kind[cp]) ? k.bm * m.cp_alpha[cp] : VT<T>::zero() + 1.0;
     const long long P0 = m.sing_pt[q0], Q = m.sing_pt[q1] - P0;
+    long long lo, hi;
+    zr.part(z_, Q, lo, hi);
     int cur = -1;
     T acc[NA], as0 = z, as1 = z;
     for (int j = 0; j < NA; ++j) acc[j] = z;
     auto flush = [&](int qp) {
+      const double one = m.sing_pt[qp] >= P0 + lo ? 1.0 : 0.0;  // line integrals: once per pair
       // pair sums + edge line integrals (bem_staela3d.f90:5308-5345), then scale and scatter
       const double* D = m.sing_d + (size_t)qp * SING_D;
       const double* X = m.hsing_x + (size_t)qp * HSING_X;
@@ -513,14 +517,14 @@ __global__ void __launch_bounds__(32) k_hsing(DMesh m, HS hs, int nf, double* A,
         if (s < 9) {
           const int il = s / 3, ik = s % 3;
           const double dk = il == ik ? 1.0 : 0.0;
-          v = v + k.S4s * (dk * L[HX_M1 - HX_LLI]) + k.S1s * L[HX_M3 - HX_LLI + s] +
-              k.S4s * (ni[ik] * L[HX_M4 - HX_LLI + il]) + k.S5s * (ni[il] * L[HX_M4 - HX_LLI + ik]);
+          v = v + one * (k.S4s * (dk * L[HX_M1 - HX_LLI]) + k.S1s * L[HX_M3 - HX_LLI + s] +
+                         k.S4s * (ni[ik] * L[HX_M4 - HX_LLI + il]) + k.S5s * (ni[il] * L[HX_M4 - HX_LLI + ik]));
         } else {
           const int qq = (s - 9) / 3, j = (s - 9) % 3, il = qq / 3, ik = qq % 3;
           const double dk = il == ik ? 1.0 : 0.0, djk = j == ik ? 1.0 : 0.0;
-          v = v + k.S4s * (dk * L[HX_M2 - HX_LLI + j]) +
-              S1o3 * (L[HX_M5 - HX_LLI + 9 * j + 3 * il + ik] + (dk + ni[il] * ni[ik]) * L[HX_M2 - HX_LLI + j] +
-                      (djk - ni[j] * ni[ik]) * L[HX_M2 - HX_LLI + il]);
+          v = v + one * (k.S4s * (dk * L[HX_M2 - HX_LLI + j]) +
+                         S1o3 * (L[HX_M5 - HX_LLI + 9 * j + 3 * il + ik] + (dk + ni[il] * ni[ik]) * L[HX_M2 - HX_LLI + j] +
+                                 (djk - ni[j] * ni[ik]) * L[HX_M2 - HX_LLI + il]));
         }
         pq[s] = v;
       }
@@ -540,7 +544,7 @@ __global__ void __launch_bounds__(32) k_hsing(DMesh m, HS hs, int nf, double* A,
           v = v * cs;
         } else {
           const int kn = (o - 72) / 9, qq = (o - 72) % 9;
-          v = v + ex[kn] * (k.T2s * L[qq]);  // L22
+          v = v + one * (ex[kn] * (k.T2s * L[qq]));  // L22
           v = v * cl;
           if (rev) v = -v;
         }
@@ -554,9 +558,9 @@ __global__ void __launch_bounds__(32) k_hsing(DMesh m, HS hs, int nf, double* A,
       }
       __syncwarp();
     };
-    for (long long base = 0; base < Q; base += 32) {
+    for (long long base = lo; base < hi; base += 32) {
       const long long c = base + lane;
-      if (c < Q) {
+      if (c < hi) {
         const int qp = find_le(m.sing_pt, q0, q1, P0 + c);
         double rv[3], n[3], w[8], wd[8];
         if (m.sing_geo) {
@@ -583,7 +587,7 @@ __global__ void __launch_bounds__(32) k_hsing(DMesh m, HS hs, int nf, double* A,
         S[lane].pair = qp;
       }
       __syncwarp();
-      const int nt = (int)min((long long)32, Q - base);
+      const int nt = (int)min((long long)32, hi - base);
       for (int t = 0; t < nt; ++t) {
         const int qp = S[t].pair;
         if (qp != cur) {
