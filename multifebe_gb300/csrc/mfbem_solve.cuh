@@ -35,9 +35,10 @@ __global__ void k_ipiv_identity(int* ipiv, int n) {
 }
 
 // Compute type of the single-precision trailing updates of the mixed LU:
-// 0 SIMT FP32 (k_gemm_simt), 1 tcgen05 TF32, one pass (TF32-accurate factors;
-// refinement in FP64 restores the accuracy and escalates to SIMT FP32 when it
-// stalls), 3 tcgen05 3xTF32 (FP32-accurate factors at tensor-core speed).
+// 0 SIMT FP32 (k_gemm_simt), 1 tcgen05, one pass of 11 bits (TF32-accurate
+// factors; refinement in FP64 restores the accuracy and escalates to SIMT FP32
+// when it stalls), 3 tcgen05 with both operands split in two 11-bit parts
+// (FP32-accurate factors at tensor-core speed).
 // The tensor-core kernels take the complex updates (tc_min_depth below); the
 // real ones run on SIMT FP32.
 // Default 3; MFBEM_FP32_GEMM=simt|tf32|tc3 overrides.
@@ -51,15 +52,16 @@ static int c32_default() {
 // updates; their timeout flag and pre-split operand tiles, per host thread
 static thread_local DevBuf g_tc_err, g_tc_ws;
 
-// C -= A B (complex64, batched): split A and B into pre-tiled hi / lo TF32
-// words once, then the bulk-copy / tcgen05 pipeline per 128 x 128 tile of C~.
+// C -= A B (complex64, batched): split A and B into pre-tiled hi / lo words
+// once, then the bulk-copy / tcgen05 pipeline per 128 x 128 tile of C~.
 static int tc_cgemm_run(cudaStream_t st, const float2* A, int lda, long long sA, const float2* B, int ldb,
                         long long sB, float2* C, int ldc, long long sC, int m, int n, int k, int batch, DevBuf& ws,
                         int* err, int passes = 3) {
-  const int nmt = (m + TC_BM / 2 - 1) / (TC_BM / 2), nnt = (n + TC_BN - 1) / TC_BN, nkc = (k + TQ / 2 - 1) / (TQ / 2);
+  const int nmt = (m + TC_BM / 2 - 1) / (TC_BM / 2), nnt = (n + TC_BN - 1) / TC_BN, nkc = (k + TQ - 1) / TQ;
   if (nmt == 0 || nnt == 0 || nkc == 0) return 0;
   const size_t wa = (size_t)batch * nmt * nkc * TQ_TW, wb = (size_t)batch * nnt * nkc * TQ_TW;
-  int rc = ensure(ws, sizeof(uint32_t) * 2 * (wa + wb));
+  const size_t na = (size_t)batch * nmt * (TC_BM / 2), nc = (size_t)batch * nnt * TC_BN;
+  int rc = ensure(ws, sizeof(uint32_t) * 2 * (wa + wb) + sizeof(float) * (na + nc));
   if (rc) return rc;
   // column tiles of 256 (M 128 x N 256 MMAs, two CTAs per SM) unless the
   // update is narrower; MFBEM_TC_BN=128 selects the 128-column tiles
@@ -74,17 +76,17 @@ static int tc_cgemm_run(cudaStream_t st, const float2* A, int lda, long long sA,
   uint32_t* alo = ahi + wa;
   uint32_t* bhi = alo + wa;
   uint32_t* blo = bhi + wb;
-  // one block per tile (wa / TQ_TW and wb / TQ_TW tiles)
-  k_tc_prep_a<<<(unsigned)(wa / TQ_TW), 256, 0, st>>>(A, lda, sA, m, k, nmt, nkc, batch, ahi, alo);
-  ++g_launches;
-  k_tc_prep_b<<<(unsigned)(wb / TQ_TW), 256, 0, st>>>(B, ldb, sB, k, n, nnt, nkc, batch, bhi, blo);
+  float* srow = (float*)(blo + wb);
+  float* scol = srow + na;
+  k_tc_split<<<dim3(nmt + nnt, batch), 256, 0, st>>>(A, lda, sA, m, B, ldb, sB, n, k, nmt, nnt, nkc, ahi, alo, srow, bhi,
+                                                     blo, scol);
   ++g_launches;
   if (wide)
     k_tc_cgemm_bulk<2><<<dim3(nmt, (nnt + 1) / 2, batch), 128, tc_smem_bulk<2>(), st>>>(
-        ahi, alo, bhi, blo, nmt, nnt, nkc, C, ldc, sC, m, n, err, g_spin_limit.load(), passes);
+        ahi, alo, bhi, blo, srow, scol, nmt, nnt, nkc, C, ldc, sC, m, n, err, g_spin_limit.load(), passes);
   else
-    k_tc_cgemm_bulk<1><<<dim3(nmt, nnt, batch), 128, tc_smem_bulk<1>(), st>>>(ahi, alo, bhi, blo, nmt, nnt, nkc, C, ldc,
-                                                                           sC, m, n, err, g_spin_limit.load(), passes);
+    k_tc_cgemm_bulk<1><<<dim3(nmt, nnt, batch), 128, tc_smem_bulk<1>(), st>>>(
+        ahi, alo, bhi, blo, srow, scol, nmt, nnt, nkc, C, ldc, sC, m, n, err, g_spin_limit.load(), passes);
   ++g_launches;
   CK(cudaGetLastError());
   return 0;

@@ -1,7 +1,7 @@
-// Complex64 GEMM update C -= A B on the 5th-generation tensor cores (tcgen05,
-// kind::tf32) with the 3xTF32 split (A_hi B_hi + A_hi B_lo + A_lo B_hi, each
-// operand x = hi + lo with hi = tf32(x)), i.e. FP32-level accuracy: the
-// trailing update of the mixed LU. Included into mfbem_abi.cu.
+// Complex64 GEMM update C -= A B on the 5th-generation tensor cores (tcgen05)
+// with each operand split x = hi + lo into two 11-bit parts (A_hi B_hi + A_hi
+// B_lo + A_lo B_hi, FP32 accumulation), i.e. FP32-level accuracy: the trailing
+// update of the mixed LU. Included into mfbem_abi.cu.
 //
 // The complex product is one real GEMM of the realified operands:
 //   C~ (2m x n)  = C viewed as real, column j = [re C0j, im C0j, re C1j, ...]
@@ -11,21 +11,23 @@
 // so C~ -= A~ B~ is C -= A B. Operand tiles live in shared memory in the
 // canonical K-major layout without swizzle (8-row x 16-byte core matrices,
 // 128 B apart along K, 1024 B apart along M/N); one thread issues
-// tcgen05.mma.cta_group::1.kind::tf32 (K 8) into a TMEM accumulator and
-// commits to an mbarrier; every warp then reads its 32 TMEM lanes
-// (tcgen05.ld 32x32b) and subtracts from C. Two kernels:
+// tcgen05.mma.cta_group::1 into a TMEM accumulator and commits to an mbarrier;
+// every warp then reads its 32 TMEM lanes (tcgen05.ld 32x32b) and subtracts
+// from C. Two kernels:
 //   k_tc_cgemm         each CTA splits and stages its own 128 x 128 tile's
-//                      operands (kept as the self-contained variant the
-//                      tests compare against);
+//                      operands in tf32 (kind::tf32, K 8; kept as the
+//                      self-contained variant the tests compare against);
 //   k_tc_cgemm_bulk<NH> the LU's trailing update: operands split once into
-//                      tf32 hi / lo tiles by k_tc_prep_a / k_tc_prep_b, copied
-//                      by cp.async.bulk into a two-stage pipeline; NH = 2 runs
-//                      one M 128 x N 256 MMA per K step (two 128-column
-//                      halves in 256 TMEM columns, two CTAs per SM).
+//                      scaled binary16 hi / lo tiles by k_tc_split (kind::f16,
+//                      K 16), copied by cp.async.bulk into a two-stage
+//                      pipeline; NH = 2 runs one M 128 x N 256 MMA per K step
+//                      (two 128-column halves in 256 TMEM columns, two CTAs
+//                      per SM).
 // Every wait is bounded: on a timeout the kernel sets *err, waits (bounded)
 // for its MMAs, frees its TMEM and returns.
 #pragma once
 #include <cstdint>
+#include <cuda_fp16.h>
 
 namespace mfb {
 
@@ -242,14 +244,23 @@ __global__ void __launch_bounds__(128, 1) k_tc_cgemm(const float2* A, int lda, l
 // ---------------------------------------------------------------------------
 // Pre-split operands + bulk-copy pipeline. The staging above converts every
 // element in every CTA that uses it; the LU's trailing update reuses the same
-// L panel (A) and U block (B) across all tiles, so they are split into
-// hi / lo TF32 once per update and written pre-tiled in the exact shared-
-// memory word order (one 16 KB tile per (row tile, K chunk) / (column tile,
-// K chunk)); the GEMM kernel then only streams tiles with cp.async.bulk into
-// two stages (mbarrier expect-tx) while the tensor cores work on the other.
+// L panel (A) and U block (B) across all tiles, so they are split once per
+// update and written pre-tiled in the exact shared-memory word order; the GEMM
+// kernel then only streams tiles with cp.async.bulk into two stages (mbarrier
+// expect-tx) while the tensor cores work on the other.
+//
+// Split: x 2^s = hi + lo in binary16, s per row of A~ and column of B~ so that
+// the largest entry lies in [2^14, 2^15). binary16 has tf32's 11 significant
+// bits, so hi and lo carry the same bits as a tf32 pair for every entry above
+// 2^-17 of its row's (column's) largest, and an absolute 2^-40 of that below;
+// kind::f16 runs at twice kind::tf32's rate and its words hold two entries, so
+// a chunk copied from L2 feeds twice the multiply-adds. FP32 accumulation as
+// before; the epilogue takes the powers of two back out. TCMEAS
 // ---------------------------------------------------------------------------
-// Tiles of the pipelined kernel: K chunk of TQ real K (16): 128 x 16 words,
-// core matrices 128 B apart along K and TQ / 4 * 128 B apart along rows.
+// Tiles of the pipelined kernel: K chunk of TQ words (2 binary16 each, 32 real
+// K): 128 x 16 words, core matrices 128 B apart along K and TQ / 4 * 128 B apart
+// along rows. Word (r, kw) holds real K 2 kw and 2 kw + 1 of the chunk, i.e. the
+// two components of complex index kw.
 constexpr int TQ = 16;
 constexpr int TQ_TW = TC_BM * TQ;                  // words per tile (2048)
 constexpr int TQ_TILE_BYTES = TQ_TW * 4;           // 8 KB
@@ -263,53 +274,115 @@ __device__ __forceinline__ uint64_t tq_desc(uint32_t addr) {
   d |= (uint64_t)1 << 46;
   return d;
 }
-// word w of a tile <-> element (row, k): core matrix w / 32 (TQ/4 along K per
-// 8-row group), row (w % 32) / 4 inside it, K offset w % 4
-__device__ __forceinline__ void tq_rk(int w, int& r, int& kk) {
-  const int cm = w >> 5;
-  r = (cm / (TQ / 4)) * 8 + ((w & 31) >> 2);
-  kk = (cm % (TQ / 4)) * 4 + (w & 3);
+// instruction descriptor, kind::f16: D f32, A and B f16, both K-major, N, M
+__host__ __device__ constexpr uint32_t tq_idesc(int m, int n) {
+  return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
-
-// A~ tiles: [batch][row tile][K chunk][word]. One 256-thread block per tile
-// (blockIdx.x = (b * nmt + mt) * nkc + kc), eight words per thread: the tile
-// coordinates are decoded once per block, not per word.
-__global__ void __launch_bounds__(256) k_tc_prep_a(const float2* A, int lda, long long sA, int m, int k, int nmt,
-                                                   int nkc, int batch, uint32_t* hi, uint32_t* lo) {
-  const int kc = (int)(blockIdx.x % nkc), tl = (int)(blockIdx.x / nkc), mt = tl % nmt, b = tl / nmt;
-  const float2* Ab = A + sA * b;
-  const size_t g0 = (size_t)blockIdx.x * TQ_TW;
-#pragma unroll 2
-  for (int w = threadIdx.x; w < TQ_TW; w += 256) {
-    int r, kk;
-    tq_rk(w, r, kk);
-    const int i = mt * (TC_BM / 2) + (r >> 1), l = kc * (TQ / 2) + (kk >> 1);
-    float2 a = make_float2(0.0f, 0.0f);
-    if (i < m && l < k) a = Ab[(size_t)l * lda + i];
-    const float v = (kk & 1) ? ((r & 1) ? a.x : -a.y) : ((r & 1) ? a.y : a.x);
-    const uint32_t h = f2tf32(v);
-    hi[g0 + w] = h;
-    lo[g0 + w] = f2tf32(v - __uint_as_float(h));
-  }
+// power of two p with p max in [2^14, 2^15) (exponent kept where p and 1 / p are
+// normal numbers; 2^14 for a zero row), and its inverse
+__device__ __forceinline__ void tq_scale(float mx, float& up, float& down) {
+  int e = (int)(__float_as_uint(mx) >> 23) - 127;
+  if (mx == 0.0f) e = 0;
+  e = min(max(e, -112), 127);
+  up = __uint_as_float((uint32_t)(14 - e + 127) << 23);
+  down = __uint_as_float((uint32_t)(e - 14 + 127) << 23);
 }
-// B~ tiles: [batch][column tile][K chunk][word]; element (jj, kk) is component
-// kk&1 of b(l, j). One block per tile as k_tc_prep_a.
-__global__ void __launch_bounds__(256) k_tc_prep_b(const float2* B, int ldb, long long sB, int k, int n, int nnt,
-                                                   int nkc, int batch, uint32_t* hi, uint32_t* lo) {
-  const int kc = (int)(blockIdx.x % nkc), tl = (int)(blockIdx.x / nkc), nt = tl % nnt, b = tl / nnt;
-  const float2* Bb = B + sB * b;
-  const size_t g0 = (size_t)blockIdx.x * TQ_TW;
-#pragma unroll 2
-  for (int w = threadIdx.x; w < TQ_TW; w += 256) {
-    int jj, kk;
-    tq_rk(w, jj, kk);
-    const int j = nt * TC_BN + jj, l = kc * (TQ / 2) + (kk >> 1);
-    float2 bv = make_float2(0.0f, 0.0f);
-    if (l < k && j < n) bv = Bb[(size_t)j * ldb + l];
-    const float v = (kk & 1) ? bv.y : bv.x;
-    const uint32_t h = f2tf32(v);
-    hi[g0 + w] = h;
-    lo[g0 + w] = f2tf32(v - __uint_as_float(h));
+// hi and lo words of the pair (x, y) (already scaled)
+__device__ __forceinline__ void tq_split(float x, float y, uint32_t& hi, uint32_t& lo) {
+  const __half hx = __float2half_rn(x), hy = __float2half_rn(y);
+  const __half lx = __float2half_rn(x - __half2float(hx)), ly = __float2half_rn(y - __half2float(hy));
+  hi = (uint32_t)__half_as_ushort(hx) | ((uint32_t)__half_as_ushort(hy) << 16);
+  lo = (uint32_t)__half_as_ushort(lx) | ((uint32_t)__half_as_ushort(ly) << 16);
+}
+// Both operands in one launch: blocks [0, nmt) row tiles of A (64 complex rows),
+// [nmt, nmt + nnt) column tiles of B; blockIdx.y the matrix. Tiles [batch][tile]
+// [K chunk][word]; a thread forms the four words of four complex K of one row
+// pair (A: rows 2i, (re, -im), and 2i + 1, (im, re)) or column (B: (re, im)), so
+// loads run along A's columns and B's columns and stores are 16 bytes.
+__global__ void __launch_bounds__(256) k_tc_split(const float2* A, int lda, long long sA, int m, const float2* B,
+                                                  int ldb, long long sB, int n, int k, int nmt, int nnt, int nkc,
+                                                  uint32_t* ahi, uint32_t* alo, float* srow, uint32_t* bhi,
+                                                  uint32_t* blo, float* scol) {
+  const int t = threadIdx.x, b = blockIdx.y;
+  if ((int)blockIdx.x < nmt) {
+    __shared__ float smax[4][64], sup[64];
+    const int mt = blockIdx.x, il = t & 63, part = t >> 6, i = mt * 64 + il;
+    const float2* Ab = A + sA * b + i;
+    float mx = 0.0f;
+    if (i < m) {
+#pragma unroll 4
+      for (int l = part; l < k; l += 4) {
+        const float2 v = Ab[(size_t)l * lda];
+        mx = fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y)));
+      }
+    }
+    smax[part][il] = mx;
+    __syncthreads();
+    if (t < 64) {
+      float up, down;
+      tq_scale(fmaxf(fmaxf(smax[0][t], smax[1][t]), fmaxf(smax[2][t], smax[3][t])), up, down);
+      sup[t] = up;
+      srow[((size_t)b * nmt + mt) * 64 + t] = down;
+    }
+    __syncthreads();
+    const float up = sup[il];
+    const size_t g0 = ((size_t)b * nmt + mt) * nkc * TQ_TW;
+    const int r = 2 * il, w0 = ((r >> 3) * (TQ / 4) + part) * 32 + (r & 7) * 4;
+    for (int kc = 0; kc < nkc; ++kc) {
+      uint32_t h0[4], l0[4], h1[4], l1[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int l = kc * TQ + 4 * part + q;
+        float2 v = make_float2(0.0f, 0.0f);
+        if (i < m && l < k) v = Ab[(size_t)l * lda];
+        v.x *= up;
+        v.y *= up;
+        tq_split(v.x, -v.y, h0[q], l0[q]);
+        tq_split(v.y, v.x, h1[q], l1[q]);
+      }
+      uint4* dh = reinterpret_cast<uint4*>(ahi + g0 + (size_t)kc * TQ_TW + w0);
+      uint4* dl = reinterpret_cast<uint4*>(alo + g0 + (size_t)kc * TQ_TW + w0);
+      dh[0] = make_uint4(h0[0], h0[1], h0[2], h0[3]);
+      dh[1] = make_uint4(h1[0], h1[1], h1[2], h1[3]);
+      dl[0] = make_uint4(l0[0], l0[1], l0[2], l0[3]);
+      dl[1] = make_uint4(l1[0], l1[1], l1[2], l1[3]);
+    }
+  } else {
+    __shared__ float cup[TC_BN];
+    const int nt = blockIdx.x - nmt, lane = t & 31, j0 = nt * TC_BN;
+    const float2* Bb = B + sB * b;
+    for (int c = t >> 5; c < TC_BN; c += 8) {
+      float mx = 0.0f;
+      if (j0 + c < n)
+        for (int l = lane; l < k; l += 32) {
+          const float2 v = Bb[(size_t)(j0 + c) * ldb + l];
+          mx = fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y)));
+        }
+      mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx)));
+      if (lane == 0) {
+        float up, down;
+        tq_scale(mx, up, down);
+        cup[c] = up;
+        scol[((size_t)b * nnt + nt) * TC_BN + c] = down;
+      }
+    }
+    __syncthreads();
+    const size_t g0 = ((size_t)b * nnt + nt) * nkc * TQ_TW;
+    for (int e = t; e < TC_BN * 4 * nkc; e += 256) {
+      const int g = e & 3, jj = (e >> 2) % TC_BN, kc = e / (4 * TC_BN);
+      const float up = cup[jj];
+      uint32_t h[4], lo[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int l = kc * TQ + 4 * g + q;
+        float2 v = make_float2(0.0f, 0.0f);
+        if (j0 + jj < n && l < k) v = Bb[(size_t)(j0 + jj) * ldb + l];
+        tq_split(v.x * up, v.y * up, h[q], lo[q]);
+      }
+      const size_t w = g0 + (size_t)kc * TQ_TW + ((jj >> 3) * (TQ / 4) + g) * 32 + (jj & 7) * 4;
+      *reinterpret_cast<uint4*>(bhi + w) = make_uint4(h[0], h[1], h[2], h[3]);
+      *reinterpret_cast<uint4*>(blo + w) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    }
   }
 }
 
@@ -322,8 +395,8 @@ __device__ __forceinline__ void tc_expect(uint32_t mbar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
 }
 
-// C -= A B from pre-split tiles (passes 3: the 3xTF32 products; 1: hi x hi
-// only, TF32-accurate); CTA (row tile, column tile of NH x 128 columns,
+// C -= A B from pre-split tiles (passes 3: hi hi + hi lo + lo hi; 1: hi x hi
+// only, 11 bits); CTA (row tile, column tile of NH x 128 columns,
 // batch); thread 0 runs the copy / MMA pipeline (stage s: the A hi / lo tiles
 // and NH B hi / lo tiles of 8 KB, "full" barrier fb[s] completed by the bulk
 // copies, "free" barrier mb[s] by the MMA commit), all four warps run the
@@ -339,7 +412,8 @@ __device__ __forceinline__ void tc_expect(uint32_t mbar, uint32_t bytes) {
 // (NH = 1: registers capped for three CTAs per SM, the shared-memory limit)
 template <int NH>
 __global__ void __launch_bounds__(128, NH == 1 ? 3 : 2) k_tc_cgemm_bulk(const uint32_t* Ahi, const uint32_t* Alo,
-                                                          const uint32_t* Bhi, const uint32_t* Blo, int nmt, int nnt,
+                                                          const uint32_t* Bhi, const uint32_t* Blo,
+                                                          const float* srow, const float* scol, int nmt, int nnt,
                                                           int nkc, float2* C, int ldc, long long sC, int m, int n,
                                                           int* err, long long spin, int passes) {
   constexpr int SB = (2 + 2 * NH) * TQ_TILE_BYTES;  // stage bytes
@@ -348,6 +422,7 @@ __global__ void __launch_bounds__(128, NH == 1 ? 3 : 2) k_tc_cgemm_bulk(const ui
   uint64_t* bars = reinterpret_cast<uint64_t*>(tsm + 2 * SB);  // fb[2], mb[2]
   uint32_t* tslot = reinterpret_cast<uint32_t*>(tsm + 2 * SB + 32);
   __shared__ int s_ok;
+  __shared__ float ssc[BN];  // the columns' scales
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const int mt = blockIdx.x, nt = blockIdx.y, bz = blockIdx.z;
   const int nh = min(NH, nnt - nt * NH);  // B halves present
@@ -363,6 +438,7 @@ __global__ void __launch_bounds__(128, NH == 1 ? 3 : 2) k_tc_cgemm_bulk(const ui
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     s_ok = 1;
   }
+  for (int c = t; c < nh * TC_BN; c += 128) ssc[c] = scol[((size_t)bz * nnt + (size_t)nt * NH) * TC_BN + c];
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)), "r"(BN)
                  : "memory");
@@ -372,7 +448,7 @@ __global__ void __launch_bounds__(128, NH == 1 ? 3 : 2) k_tc_cgemm_bulk(const ui
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tslot;
-  const uint32_t idesc = tc_idesc(TC_BM, BN);
+  const uint32_t idesc = tq_idesc(TC_BM, BN);
   int issued = 0;  // chunks whose MMAs were issued (the last commit covers all)
   int loaded = 0;  // chunks whose bulk copies were issued
   int landed = 0;  // chunks whose copies were waited for
@@ -404,19 +480,19 @@ __global__ void __launch_bounds__(128, NH == 1 ? 3 : 2) k_tc_cgemm_bulk(const ui
                      bl = ah + (2 + NH) * TQ_TILE_BYTES;
 #pragma unroll
       for (int ks = 0; ks < TQ / 8; ++ks) {
-        const uint32_t ko = ks * 256;  // 8 tf32 = two core matrices along K
+        const uint32_t ko = ks * 256;  // 16 binary16 = two core matrices along K
         const uint64_t dah = tq_desc(ah + ko), dal = tq_desc(al + ko), dbh = tq_desc(bh + ko), dbl = tq_desc(bl + ko);
         const uint32_t acc0 = (kc > 0 || ks > 0) ? 1u : 0u;
         asm volatile(
-            "{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}\n" ::"r"(
+            "{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(
                 tmem),
             "l"(dah), "l"(dbh), "r"(idesc), "r"(acc0)
             : "memory");
         if (passes == 3) {
-          asm volatile("tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, 1;" ::"r"(tmem), "l"(dah), "l"(dbl),
+          asm volatile("tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, 1;" ::"r"(tmem), "l"(dah), "l"(dbl),
                        "r"(idesc)
                        : "memory");
-          asm volatile("tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, 1;" ::"r"(tmem), "l"(dal), "l"(dbh),
+          asm volatile("tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, 1;" ::"r"(tmem), "l"(dal), "l"(dbh),
                        "r"(idesc)
                        : "memory");
         }
@@ -441,6 +517,7 @@ __global__ void __launch_bounds__(128, NH == 1 ? 3 : 2) k_tc_cgemm_bulk(const ui
   if (s_ok && nkc > 0) {
     const int r = 32 * warp + lane;
     const int i = mt * (TC_BM / 2) + (r >> 1), comp = r & 1;
+    const float sr = srow[((size_t)bz * nmt + mt) * (TC_BM / 2) + (r >> 1)];
     float2* Cb = C + sC * bz;
     for (int c0 = 0; c0 < nh * TC_BN; c0 += 32) {
       uint32_t v[32];
@@ -468,7 +545,7 @@ __global__ void __launch_bounds__(128, NH == 1 ? 3 : 2) k_tc_cgemm_bulk(const ui
 #pragma unroll
         for (int q = 0; q < 32; ++q) {
           const int j = nt * BN + c0 + q;
-          if (j < n) cr[2 * ((size_t)j * ldc + i) + comp] = cv[q] - __uint_as_float(v[q]);
+          if (j < n) cr[2 * ((size_t)j * ldc + i) + comp] = fmaf(-__uint_as_float(v[q]), sr * ssc[c0 + q], cv[q]);
         }
       }
     }
