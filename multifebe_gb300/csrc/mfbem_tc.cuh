@@ -533,19 +533,14 @@ __global__ void __launch_bounds__(128, NH == 1 ? 3 : 2) k_tc_cgemm_bulk(const ui
           : "memory");
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       if (i < m) {
-        // all loads first, then the stores (a load / store pair per element
-        // would serialise 32 global round trips)
+        // reductions at the L2: no wait for C (loading it took most of a tile's
+        // time at the depths of the LU; each entry gets one addition per
+        // update, so the result does not depend on their order)
         float* cr = reinterpret_cast<float*>(Cb);
-        float cv[32];
 #pragma unroll
         for (int q = 0; q < 32; ++q) {
           const int j = nt * BN + c0 + q;
-          cv[q] = j < n ? cr[2 * ((size_t)j * ldc + i) + comp] : 0.0f;
-        }
-#pragma unroll
-        for (int q = 0; q < 32; ++q) {
-          const int j = nt * BN + c0 + q;
-          if (j < n) cr[2 * ((size_t)j * ldc + i) + comp] = fmaf(-__uint_as_float(v[q]), sr * ssc[c0 + q], cv[q]);
+          if (j < n) atomicAdd(cr + 2 * ((size_t)j * ldc + i) + comp, -__uint_as_float(v[q]) * (sr * ssc[c0 + q]));
         }
       }
     }
