@@ -655,52 +655,92 @@ __global__ void __launch_bounds__(32) k_swap_trsm16(S* A, long long strideA, int
 // U12 = inv(L11) A12 of a whole outer block (w <= 128 rows from K, columns
 // [c0, c1)) in one launch: a CTA holds NC columns in shared memory and walks the
 // block in steps of 16 rows: a step's rows are solved (16 lanes per column,
-// shuffles), then all threads subtract their multiples from the rows below.
-// In place of a TRSM and a GEMM launch per 16 rows, each with a fixed cost
-// (copies, a tile of the SMs idle, for the tensor-core path an operand split).
+// shuffles), then the threads subtract their multiples from the rows below;
+// binary32: each thread CT columns of one row in four (a warp's lanes on
+// consecutive rows, so L's column is read without conflict and X's entries are
+// broadcasts), 4 + CT shared-memory loads for 4 CT multiply-adds. In place of a TRSM and a GEMM
+// launch per 16 or 32 rows, each with a fixed cost (copies, a tile of the SMs
+// idle, for the tensor-core paths an operand split).
 // ---------------------------------------------------------------------------
 template <typename S, int NC>
 __global__ void __launch_bounds__(256) k_trsm_block(S* A, long long strideA, int lda, int K, int w, int c0, int c1) {
+  constexpr int CT = NC >= 8 ? NC / 8 : 1, CG = NC / CT;  // columns per thread, column groups
+  constexpr int RT = 4;                                   // rows per thread (32 apart)
+  constexpr bool F64 = sizeof(typename Sc<S>::R) == 8;
   extern __shared__ __align__(16) unsigned char tbraw[];
   S* X = reinterpret_cast<S*>(tbraw);       // [NC][129]
   S* L = X + NC * 129;                      // [16][128 + 1]: the step's columns of L11
   S* M = A + strideA * blockIdx.y;
   const int cb = c0 + blockIdx.x * NC, nc = min(NC, c1 - cb), t = threadIdx.x;
-  for (int e = t; e < nc * w; e += 256) {
+  for (int e = t; e < NC * w; e += 256) {
     const int i = e % w, c = e / w;
-    X[c * 129 + i] = M[(size_t)(cb + c) * lda + K + i];
+    X[c * 129 + i] = c < nc ? M[(size_t)(cb + c) * lda + K + i] : Sc<S>::zero();
   }
   for (int s = 0; s < w; s += 16) {
     const int sb = min(16, w - s), rows = w - s;
     __syncthreads();  // X of the step before, and its reads of L, are done
-    for (int e = t; e < sb * rows; e += 256) {
+    for (int e = t; e < 16 * rows; e += 256) {
       const int i = e % rows, c = e / rows;
-      L[c * 129 + i] = M[(size_t)(K + s + c) * lda + K + s + i];
+      L[c * 129 + i] = c < sb ? M[(size_t)(K + s + c) * lda + K + s + i] : Sc<S>::zero();
     }
     __syncthreads();
     // 16 lanes per column, lane = row: one multiply-add per lane and step
-    if (t < 16 * NC) {
-      const int i = t & 15, c = t >> 4;
-      const bool on = i < sb && c < nc;
+    for (int u = t; u < 16 * NC; u += 256) {
+      const int i = u & 15, c = u >> 4;
+      const bool on = i < sb;
       S x = on ? X[c * 129 + s + i] : Sc<S>::zero();
 #pragma unroll
       for (int jj = 0; jj < 15; ++jj) {
-        const S l = on && jj < sb ? L[jj * 129 + i] : Sc<S>::zero();
-        const S xj = shfl_s(x, (t & 16) | jj);
+        const S l = on ? L[jj * 129 + i] : Sc<S>::zero();
+        const S xj = shfl_s(x, (u & 16) | jj);
         if (i > jj) x = lu_fnma(l, xj, x);
       }
       if (on) X[c * 129 + s + i] = x;
     }
     __syncthreads();
-    // rows below: thread -> (row, column), rows fastest
+    // rows below (none unless sb = 16)
     const int below = rows - sb;
-    for (int e = t; e < below * nc; e += 256) {
-      const int i = e % below, c = e / below;
-      S v = X[c * 129 + s + sb + i];
+    if constexpr (F64) {
+      // binary64: bound by its pipe, so one output per thread and all threads
+      for (int e = t; e < below * nc; e += 256) {
+        const int i = e % below, c = e / below;
+        S v = X[c * 129 + s + sb + i];
 #pragma unroll
-      for (int jj = 0; jj < 16; ++jj)
-        if (jj < sb) v = lu_fnma(L[jj * 129 + sb + i], X[c * 129 + s + jj], v);
-      X[c * 129 + s + sb + i] = v;
+        for (int jj = 0; jj < 16; ++jj) v = lu_fnma(L[jj * 129 + sb + i], X[c * 129 + s + jj], v);
+        X[c * 129 + s + sb + i] = v;
+      }
+      continue;
+    }
+    // 32 RT rows at a time
+    const int lane = t & 31, wid = t >> 5;
+    // warps over (column group, group of 32 RT rows)
+    for (int u = wid; u < CG * ((below + 32 * RT - 1) / (32 * RT)); u += 8) {
+      const int cg = u % CG, rb = (u / CG) * 32 * RT + lane;
+      S v[RT][CT];
+#pragma unroll
+      for (int r = 0; r < RT; ++r)
+#pragma unroll
+        for (int c = 0; c < CT; ++c)
+          if (rb + 32 * r < below) v[r][c] = X[(cg * CT + c) * 129 + s + sb + rb + 32 * r];
+#pragma unroll 4
+      for (int jj = 0; jj < 16; ++jj) {
+        S xj[CT];
+#pragma unroll
+        for (int c = 0; c < CT; ++c) xj[c] = X[(cg * CT + c) * 129 + s + jj];
+#pragma unroll
+        for (int r = 0; r < RT; ++r) {
+          if (rb + 32 * r < below) {
+            const S l = L[jj * 129 + sb + rb + 32 * r];
+#pragma unroll
+            for (int c = 0; c < CT; ++c) v[r][c] = lu_fnma(l, xj[c], v[r][c]);
+          }
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < RT; ++r)
+#pragma unroll
+        for (int c = 0; c < CT; ++c)
+          if (rb + 32 * r < below) X[(cg * CT + c) * 129 + s + sb + rb + 32 * r] = v[r][c];
     }
   }
   __syncthreads();

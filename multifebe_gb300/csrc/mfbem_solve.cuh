@@ -28,6 +28,10 @@ static int raise_smem_limit(const void* f) {
 // ---------------------------------------------------------------------------
 // GEMM dispatch for the trailing update A22 -= L21 U12 (plain library GEMM)
 // ---------------------------------------------------------------------------
+template <typename S> struct IsF64 { static const bool v = false; };
+template <> struct IsF64<double> { static const bool v = true; };
+template <> struct IsF64<double2> { static const bool v = true; };
+
 // ipiv[b][j] = j + 1
 __global__ void k_ipiv_identity(int* ipiv, int n) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -315,9 +319,6 @@ static int panel_nb_f64(int n) {
   return (v == 8 || v == 16) ? v : 32;
 }
 
-template <typename S> struct IsF64 { static const bool v = false; };
-template <> struct IsF64<double> { static const bool v = true; };
-template <> struct IsF64<double2> { static const bool v = true; };
 
 // U12 of an outer block by k_trsm_block: binary64 work on the FP64 pipe, w / 2
 // multiply-adds per row and column (four times that if complex) at two per
@@ -329,20 +330,39 @@ template <> struct IsF64<double2> { static const bool v = true; };
 // them, which takes half of that binary64 work to the tensor cores: 67.5 ->
 // 63.5 ms for four complex 3462-row systems, no difference for one below 4096.
 constexpr double kTrsmSplit = 4096.0;
-template <typename S>
-static int trsm_block_run(cudaStream_t st, S* A, long long sA, int lda, int K, int w, int c0, int c1, int batch) {
-  // columns per CTA: 4, then 8, until every SM has its CTA, then 16
-  const int nc = c1 - c0;
-  const int NC = (long long)nblk(nc, 4) * batch <= 304 ? 4 : ((long long)nblk(nc, 8) * batch <= 304 ? 8 : 16);
-  const size_t sm = sizeof(S) * (129 * (size_t)NC + 16 * 129);
-  const void* f = NC == 4 ? (const void*)k_trsm_block<S, 4>
-                          : (NC == 8 ? (const void*)k_trsm_block<S, 8> : (const void*)k_trsm_block<S, 16>);
-  if (raise_smem_limit(f)) return fail(MFBEM_ECUDA, "shared-memory limit of the block TRSM");
-  if (NC == 4) k_trsm_block<S, 4><<<dim3(nblk(nc, 4), batch), 256, sm, st>>>(A, sA, lda, K, w, c0, c1);
-  else if (NC == 8) k_trsm_block<S, 8><<<dim3(nblk(nc, 8), batch), 256, sm, st>>>(A, sA, lda, K, w, c0, c1);
-  else k_trsm_block<S, 16><<<dim3(nblk(nc, 16), batch), 256, sm, st>>>(A, sA, lda, K, w, c0, c1);
+template <typename S, int NC>
+static int trsm_block_launch(cudaStream_t st, S* A, long long sA, int lda, int K, int w, int c0, int c1, int batch) {
+  if (raise_smem_limit((const void*)k_trsm_block<S, NC>)) return fail(MFBEM_ECUDA, "shared-memory limit of the block TRSM");
+  k_trsm_block<S, NC><<<dim3(nblk(c1 - c0, NC), batch), 256, sizeof(S) * (129 * (size_t)NC + 16 * 129), st>>>(
+      A, sA, lda, K, w, c0, c1);
   ++g_launches;
   CK(cudaGetLastError());
+  return 0;
+}
+template <typename S>
+static int trsm_block_run(cudaStream_t st, S* A, long long sA, int lda, int K, int w, int c0, int c1, int batch) {
+  // columns per CTA: as many as leave every SM about two CTAs, 4 to 16 (binary32: 32)
+  const long long cols = (long long)(c1 - c0) * batch;
+  if (!IsF64<S>::v && cols >= 32 * 304) return trsm_block_launch<S, 32>(st, A, sA, lda, K, w, c0, c1, batch);
+  if (cols > 8 * 304) return trsm_block_launch<S, 16>(st, A, sA, lda, K, w, c0, c1, batch);
+  if (cols > 4 * 304) return trsm_block_launch<S, 8>(st, A, sA, lda, K, w, c0, c1, batch);
+  return trsm_block_launch<S, 4>(st, A, sA, lda, K, w, c0, c1, batch);
+}
+// inv(L11) A12 of an outer block of w <= 256 rows: halves of at most 128 rows
+// with an update between them (binary64: see kTrsmSplit)
+template <typename S>
+static int trsm_outer(cudaStream_t st, S* A, long long sA, int lda, int K, int w, int c0, int c1, int batch) {
+  const int nc = c1 - c0, cw = sizeof(S) / 8;
+  int h = w;
+  if (w > 128) h = 128;
+  else if (IsF64<S>::v && w == 128 && (double)nc * batch * cw >= kTrsmSplit) h = 64;
+  for (int s = 0; s < w; s += h) {
+    const int sb = std::min(h, w - s);
+    CKG(trsm_block_run<S>(st, A, sA, lda, K + s, sb, c0, c1, batch));
+    if (s + sb < w)
+      CKG(gemm_sb(st, w - s - sb, nc, sb, A + K + s + sb + (size_t)(K + s) * lda, lda, sA, A + K + s + (size_t)c0 * lda,
+                  lda, sA, A + K + s + sb + (size_t)c0 * lda, lda, sA, batch));
+  }
   return 0;
 }
 
@@ -588,24 +608,9 @@ static int getrf_batched(cudaStream_t st, S* A, long long sA, int lda, int n, in
       }
     }
     if (KE < n) {
-      // U12 of the outer block (rows [K, KE), columns [KE, n)), blocked by nb
+      // U12 of the outer block (rows [K, KE), columns [KE, n))
       const int nc = n - KE;
-      const bool one = IsF64<S>::v && KE - K <= 128;
-      if (one && KE - K == 128 && (double)nc * batch * cw >= kTrsmSplit) {
-        CKG(trsm_block_run<S>(st, A, sA, lda, K, 64, KE, n, batch));
-        CKG(gemm_sb(st, 64, nc, 64, A + K + 64 + (size_t)K * lda, lda, sA, A + K + (size_t)KE * lda, lda, sA,
-                    A + (K + 64) + (size_t)KE * lda, lda, sA, batch));
-        CKG(trsm_block_run<S>(st, A, sA, lda, K + 64, 64, KE, n, batch));
-      } else if (one) {
-        CKG(trsm_block_run<S>(st, A, sA, lda, K, KE - K, KE, n, batch));
-      }
-      for (int k = K; k < KE && !one; k += nb) {
-        const int kb = std::min(nb, KE - k);
-        CKG(trsm(k, kb, KE, n));
-        if (k + kb < KE)
-          CKG(gemm_sb(st, KE - k - kb, nc, kb, A + k + kb + (size_t)k * lda, lda, sA, A + k + (size_t)KE * lda, lda, sA,
-                      A + (k + kb) + (size_t)KE * lda, lda, sA, batch));
-      }
+      CKG(trsm_outer<S>(st, A, sA, lda, K, KE - K, KE, n, batch));
       // trailing update of depth KE - K
       CKG(gemm_sb(st, nc, nc, KE - K, A + KE + (size_t)K * lda, lda, sA, A + K + (size_t)KE * lda, lda, sA,
                   A + KE + (size_t)KE * lda, lda, sA, batch));
