@@ -923,66 +923,88 @@ __global__ void __launch_bounds__(128) k_trsv_diag64(const S* A, long long strid
 // pivot sets info and leaves the rows as they are.
 // Grid: (max(1, ceil((r1 - r0) / 128)), batch).
 // ---------------------------------------------------------------------------
+// The diagonal block sits in registers, warp g holding the columns g + 4 q of
+// row = lane: a step takes one reciprocal, one exchange of the column of
+// multipliers through shared memory with one barrier, and shuffles of the
+// pivot row inside each warp (a copy in shared memory with two barriers and an
+// index division per element took twice as long). The rows of L21 update to the
+// right, so their multiply-adds are independent. PNMEAS
+__device__ __forceinline__ float diag_rcp(float d) { return 1.0f / d; }
+__device__ __forceinline__ float2 diag_rcp(float2 d) {
+  const float q = fmaf(d.x, d.x, d.y * d.y);
+  if (!(q > 1e-30f && q < 1e30f)) return Sc<float2>::rcp(d);
+  const float r = 1.0f / q;
+  return make_float2(d.x * r, -d.y * r);
+}
 template <typename S>
 __global__ void __launch_bounds__(128) k_panel_nopiv(S* A, long long sA, int lda, int k, int kb, int r0, int r1,
                                                      int* info, int* cnt) {
   __shared__ S D[32 * 33];
   __shared__ S ur[32];  // reciprocals of U11's diagonal: the row chains multiply, no division
+  __shared__ S lc[2][32];  // multipliers of the step's column, by step parity
   __shared__ int s_bad, s_last;
-  const int b = blockIdx.y, t = threadIdx.x;
+  const int b = blockIdx.y, t = threadIdx.x, lane = t & 31, g = t >> 5;
   S* M = A + sA * b;
-  for (int e = t; e < kb * kb; e += 128) {
-    const int i = e % kb, c = e / kb;
-    D[c * 33 + i] = M[(size_t)(k + c) * lda + k + i];
+  // entries beyond kb: those of the identity
+  S v[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int c = g + 4 * q;
+    v[q] = lane < kb && c < kb ? M[(size_t)(k + c) * lda + k + lane] : (lane == c ? Sc<S>::one() : Sc<S>::zero());
   }
   if (t == 0) s_bad = 0;
   __syncthreads();
   if (t == 0) s_last = atomicAdd(cnt + b, 1) == (int)gridDim.x - 1;
-  for (int j = 0; j < kb; ++j) {
-    const S d = D[j * 33 + j];
-    const float m = (float)Sc<S>::abs1(d);
-    if (!(m > 0.0f) || !isfinite(m)) {
-      if (t == 0) {
-        s_bad = 1;
-        if (s_last && info[b] == 0) info[b] = k + j + 1;
+#pragma unroll
+  for (int j = 0; j < 32; ++j) {
+    if (g == (j & 3)) {
+      const S d = shfl_s(v[j >> 2], j);
+      const float m = (float)Sc<S>::abs1(d);
+      const bool bad = !(m > 0.0f) || !isfinite(m);
+      const S rc = diag_rcp(d);
+      const S l = Sc<S>::mul(v[j >> 2], rc);
+      if (lane > j) v[j >> 2] = l;
+      lc[j & 1][lane] = l;
+      if (lane == 0) {
+        ur[j] = rc;
+        if (bad && s_bad == 0) s_bad = j + 1;
       }
-      break;
-    }
-    const S rcp = Sc<S>::rcp(d);
-    for (int i = j + 1 + t; i < kb; i += 128) D[j * 33 + i] = Sc<S>::mul(D[j * 33 + i], rcp);
-    __syncthreads();
-    const int w = kb - j - 1;
-    for (int e = t; e < w * w; e += 128) {
-      const int i = j + 1 + e % w, c = j + 1 + e / w;
-      D[c * 33 + i] = Sc<S>::sub(D[c * 33 + i], Sc<S>::mul(D[j * 33 + i], D[c * 33 + j]));
     }
     __syncthreads();
+    const S l = lc[j & 1][lane];
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (4 * q + 3 > j) {
+        const S u = shfl_s(v[q], j);
+        if (lane > j && g + 4 * q > j) v[q] = lu_fnma(l, u, v[q]);
+      }
   }
+#pragma unroll
+  for (int q = 0; q < 8; ++q) D[(g + 4 * q) * 33 + lane] = v[q];
   __syncthreads();
+  // a zero or non-finite pivot at column s_bad - 1: nothing is written back
   if (s_last) {
-    for (int e = t; e < kb * kb; e += 128) {
-      const int i = e % kb, c = e / kb;
-      M[(size_t)(k + c) * lda + k + i] = D[c * 33 + i];
+    if (s_bad) {
+      if (t == 0 && info[b] == 0) info[b] = k + s_bad;
+    } else {
+      for (int e = t; e < 1024; e += 128) {
+        const int i = e & 31, c = e >> 5;
+        if (i < kb && c < kb) M[(size_t)(k + c) * lda + k + i] = D[c * 33 + i];
+      }
     }
     if (t == 0) cnt[b] = 0;
   }
   if (s_bad) return;
-  if (t < kb) ur[t] = Sc<S>::rcp(D[t * 33 + t]);
-  __syncthreads();
   const int row = r0 + blockIdx.x * 128 + t;
   if (row >= r1) return;
   S x[32];
 #pragma unroll
-  for (int j = 0; j < 32; ++j)
-    if (j < kb) x[j] = M[(size_t)(k + j) * lda + row];
+  for (int j = 0; j < 32; ++j) x[j] = j < kb ? M[(size_t)(k + j) * lda + row] : Sc<S>::zero();
 #pragma unroll
   for (int j = 0; j < 32; ++j) {
-    if (j < kb) {
-      S v = x[j];
+    x[j] = Sc<S>::mul(x[j], ur[j]);
 #pragma unroll
-      for (int c = 0; c < j; ++c) v = Sc<S>::sub(v, Sc<S>::mul(x[c], D[j * 33 + c]));
-      x[j] = Sc<S>::mul(v, ur[j]);
-    }
+    for (int c = j + 1; c < 32; ++c) x[c] = lu_fnma(x[j], D[c * 33 + j], x[c]);
   }
 #pragma unroll
   for (int j = 0; j < 32; ++j)

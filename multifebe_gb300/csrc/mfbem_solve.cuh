@@ -348,8 +348,8 @@ static int trsm_block_run(cudaStream_t st, S* A, long long sA, int lda, int K, i
   if (cols > 4 * 304) return trsm_block_launch<S, 8>(st, A, sA, lda, K, w, c0, c1, batch);
   return trsm_block_launch<S, 4>(st, A, sA, lda, K, w, c0, c1, batch);
 }
-// inv(L11) A12 of an outer block of w <= 256 rows: halves of at most 128 rows
-// with an update between them (binary64: see kTrsmSplit)
+// inv(L11) A12 of an outer block of w rows: blocks of at most 128 rows with
+// updates between them (binary64: see kTrsmSplit)
 template <typename S>
 static int trsm_outer(cudaStream_t st, S* A, long long sA, int lda, int K, int w, int c0, int c1, int batch) {
   const int nc = c1 - c0, cw = sizeof(S) / 8;
@@ -540,18 +540,24 @@ static int getrf_batched(cudaStream_t st, S* A, long long sA, int lda, int n, in
     ++g_launches;
     return 0;
   };
-  // Two-level blocking: outer blocks of NBO columns are factorised with inner
-  // panels of nb columns (updates restricted to the outer block), then one
-  // trailing GEMM of depth NBO updates the rest of the matrix.
+  // Three levels: outer blocks of NBO columns consist of blocks of at most 128,
+  // factorised with inner panels of nb columns whose updates stay inside the
+  // block; a finished block updates the rest of its outer block at depth 128,
+  // and one trailing GEMM of depth NBO the rest of the matrix. The trailing
+  // update moves the whole remaining matrix through memory once per outer
+  // block (a 14883-row system: 20 ms of traffic in all at NBO = 128, 5 at 512),
+  // so deep outer blocks pay where the inner updates are cheap. NBMEAS
   const int NBO = std::max(nb, nbo);
-  for (int K = 0; K < n; K += NBO) {
-    const int KE = std::min(n, K + NBO);
+  // the columns [K, KE) of all rows from K, updates inside the block only
+  auto factor_block = [&](int K, int KE) -> int {
     for (int k = K; k < KE; k += nb) {
       const int kb = std::min(nb, KE - k);
       if (nopiv) {
-        const unsigned gr = std::max(1u, nblk(n - k - kb, 128));
-        k_panel_nopiv<S><<<dim3(gr, batch), 128, 0, st>>>(A, sA, lda, k, kb, k + kb, n, info, pn_cnt);
-        ++g_launches;
+        if constexpr (!IsF64<S>::v) {
+          const unsigned gr = std::max(1u, nblk(n - k - kb, 128));
+          k_panel_nopiv<S><<<dim3(gr, batch), 128, 0, st>>>(A, sA, lda, k, kb, k + kb, n, info, pn_cnt);
+          ++g_launches;
+        }
       } else if (use_cl) {
         const int chunk = (n - k + GC - 1) / GC;
         cudaLaunchConfig_t cfg = {};
@@ -600,21 +606,29 @@ static int getrf_batched(cudaStream_t st, S* A, long long sA, int lda, int n, in
         k_swap_trsm16<S><<<dim3(nblk(nout, 32), batch), 32, 0, st>>>(A, sA, lda, n, k, kb, KE, ipiv); ++g_launches;
       } else if (nout > 0 && !nopiv) { k_laswp<S><<<dim3(nblk(nout, 128), batch), 128, 0, st>>>(A, sA, lda, n, k, kb, ipiv); ++g_launches; }
       if (k + kb < KE) {
-        // inside the outer block: U12 and the update of columns [k+kb, KE)
+        // inside the block: U12 and the update of columns [k+kb, KE)
         const int nc = KE - k - kb;
         if (!fused) CKG(trsm(k, kb, k + kb, KE));
         CKG(gemm_sb(st, n - k - kb, nc, kb, A + k + kb + (size_t)k * lda, lda, sA, A + k + (size_t)(k + kb) * lda, lda,
                     sA, A + (k + kb) + (size_t)(k + kb) * lda, lda, sA, batch));
       }
     }
-    if (KE < n) {
-      // U12 of the outer block (rows [K, KE), columns [KE, n))
-      const int nc = n - KE;
-      CKG(trsm_outer<S>(st, A, sA, lda, K, KE - K, KE, n, batch));
-      // trailing update of depth KE - K
-      CKG(gemm_sb(st, nc, nc, KE - K, A + KE + (size_t)K * lda, lda, sA, A + K + (size_t)KE * lda, lda, sA,
-                  A + KE + (size_t)KE * lda, lda, sA, batch));
+    return 0;
+  };
+  // U12 of rows [K, KE) and columns [c0, c1), then those columns' update below
+  auto update_block = [&](int K, int KE, int c0, int c1) -> int {
+    CKG(trsm_outer<S>(st, A, sA, lda, K, KE - K, c0, c1, batch));
+    return gemm_sb(st, n - KE, c1 - c0, KE - K, A + KE + (size_t)K * lda, lda, sA, A + K + (size_t)c0 * lda, lda, sA,
+                   A + KE + (size_t)c0 * lda, lda, sA, batch);
+  };
+  for (int KO = 0; KO < n; KO += NBO) {
+    const int KOE = std::min(n, KO + NBO);
+    for (int K = KO; K < KOE; K += 128) {
+      const int KE = std::min(KOE, K + 128);
+      CKG(factor_block(K, KE));
+      if (KE < KOE) CKG(update_block(K, KE, KE, KOE));
     }
+    if (KOE < n) CKG(update_block(KO, KOE, KOE, n));
   }
   CK(cudaGetLastError());
   if (coop) {
@@ -637,7 +651,7 @@ static int getrf_batched(cudaStream_t st, S* A, long long sA, int lda, int n, in
 }
 
 // ---------------------------------------------------------------------------
-// Autotuner of the mixed LU's outer block width (64, 128 or 256 columns: the
+// Autotuner of the mixed LU's outer block width (64 to 512 columns: the
 // depth of the trailing GEMMs against the number of panel steps), per scalar
 // type, size class (n rounded up to 512), batch and GEMM compute type. The
 // first factorisation of a class times the candidates on a seeded random
@@ -684,10 +698,10 @@ static int tuned_nbo(cudaStream_t st, int n, int batch, int* ipiv, int* info, in
   cudaEvent_t t0, t1;
   cudaEventCreate(&t0);
   cudaEventCreate(&t1);
-  const int cand[3] = {64, 128, 256};
+  const int cand[4] = {64, 128, 256, 512};
   float best = 1e30f;
   int bn = 128, rc = 0;
-  for (int c = 0; c < 3 && !rc; ++c) {
+  for (int c = 0; c < 4 && !rc; ++c) {
     k_tune_fill<S><<<152 * 8, 256, 0, st>>>(T, nn * batch); ++g_launches;
     cudaEventRecord(t0, st);
     rc = getrf_batched<S>(st, T, nn, n, n, batch, ipiv, info, cand[c]);
