@@ -546,7 +546,9 @@ static int getrf_batched(cudaStream_t st, S* A, long long sA, int lda, int n, in
   // and one trailing GEMM of depth NBO the rest of the matrix. The trailing
   // update moves the whole remaining matrix through memory once per outer
   // block (a 14883-row system: 20 ms of traffic in all at NBO = 128, 5 at 512),
-  // so deep outer blocks pay where the inner updates are cheap. NBMEAS
+  // so deep outer blocks pay where the inner updates are cheap. Measured with the
+  // register panel: 58.5 -> 53.2 ms at 14883 unknowns, 20.9 -> 20.4 ms for the
+  // 20 systems of 3462.
   const int NBO = std::max(nb, nbo);
   // the columns [K, KE) of all rows from K, updates inside the block only
   auto factor_block = [&](int K, int KE) -> int {
