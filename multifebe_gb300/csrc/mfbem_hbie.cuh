@@ -406,9 +406,9 @@ __device__ __forceinline__ void hsing_point(const HS& hs, int f, const HsCoef<ty
     S1 = c.S1; S2 = c.S2; S3 = c.S3; S4 = c.S4; S5 = c.S5;
   }
   const T S1o3 = k.S1s * (1.0 / 3.0);
-#pragma unroll 1
+#pragma unroll
   for (int il = 0; il < 3; ++il)
-#pragma unroll 1
+#pragma unroll
     for (int ik = 0; ik < 3; ++ik) {
       const int q = 3 * il + ik;
       const double dk = il == ik ? 1.0 : 0.0;
@@ -447,6 +447,14 @@ __device__ __forceinline__ void hsing_point(const HS& hs, int f, const HsCoef<ty
     }
 }
 
+// bc[i] += v without indexing the registers
+template <typename T>
+__device__ __forceinline__ void bc_add(T bc[3], int i, T v) {
+  if (i == 0) bc[0] = bc[0] + v;
+  else if (i == 1) bc[1] = bc[1] + v;
+  else bc[2] = bc[2] + v;
+}
+
 // Scatter one HBIE singular pair (final m, l of this lane's outputs) into A, b.
 // On a crack-like element face 2 takes -m and l at the next column.
 template <typename T>
@@ -458,7 +466,7 @@ __device__ __forceinline__ void hsing_scatter(const DMesh& m, int dn, int e, int
     for (int fc = 0; fc <= ck; ++fc, v = -v) {
       const int dof = m.edof[8 * e + kn] + (ik << ck) + fc;
       if (m.dct[dof] == 1) addA(Af, (size_t)dof * lda + row, v);
-      else bc[il] = bc[il] - v * cval(m.dcv, dof, v);
+      else bc_add(bc, il, -(v * cval(m.dcv, dof, v)));
     }
   } else {
     const int q = o - 72, kn = q / 9, il = (q % 9) / 3, ik = q % 3;
@@ -466,7 +474,7 @@ __device__ __forceinline__ void hsing_scatter(const DMesh& m, int dn, int e, int
     for (int fc = 0; fc <= ck; ++fc) {
       const int dof = m.edof[8 * e + kn] + (ik << ck) + fc;
       if (m.dct[dof] == 0) addA(Af, (size_t)dof * lda + row, -v);
-      else bc[il] = bc[il] + v * cval(m.dcv, dof, v);
+      else bc_add(bc, il, v * cval(m.dcv, dof, v));
     }
   }
 }
@@ -474,7 +482,12 @@ __device__ __forceinline__ void hsing_scatter(const DMesh& m, int dn, int e, int
 // One warp per (dnode, frequency) walks the HBIE singular pairs of the node's
 // collocation points (one per point: the element holding it). Phase 1: one
 // lane per polar point forms ComboH; phase 2: lanes own the outputs
-// o = lane + 32 j (m: o < 72, l: o >= 72) and the 36 pair sums P, Q.
+// o = lane + 32 j (m: o < 72, l: o >= 72) and the 36 pair sums P, Q. The loops
+// over accumulators and components are unrolled, so that these are registers
+// and not local memory: Burton-Miller cube of 5 x 5 elements per face, two
+// frequencies, singular pairs 38 -> 34.8 ms (the sums of the SBIE pairs
+// included). The same in the SBIE pair kernels spilled and lost: static singular
+// pairs 0.37 -> 0.47 ms, a slab's assembly 18.2 -> 19.9.
 template <class HS>
 __global__ void __launch_bounds__(32) k_hsing(DMesh m, HS hs, int nf, double* A, size_t lda, size_t astride, double* b,
                                               size_t bstride, Slices z_) {
@@ -500,6 +513,7 @@ __global__ void __launch_bounds__(32) k_hsing(DMesh m, HS hs, int nf, double* A,
     zr.part(z_, Q, lo, hi);
     int cur = -1;
     T acc[NA], as0 = z, as1 = z;
+#pragma unroll
     for (int j = 0; j < NA; ++j) acc[j] = z;
     auto flush = [&](int qp) {
       const double one = m.sing_pt[qp] >= P0 + lo ? 1.0 : 0.0;  // line integrals: once per pair
@@ -533,9 +547,10 @@ __global__ void __launch_bounds__(32) k_hsing(DMesh m, HS hs, int nf, double* A,
       const bool rev = (m.rev[e] & 1) != 0;
       const T cs = k.cte_s * beta, cl = k.cte_d * beta;
       T bc[3] = {z, z, z};
+#pragma unroll
       for (int j = 0; j < NA; ++j) {
         const int o = lane + 32 * j;
-        if (o >= 144) break;
+        if (o >= 144) continue;
         T v = acc[j];
         if (o < 72) {
           const int kn = o / 9, qq = o % 9;
@@ -550,6 +565,7 @@ __global__ void __launch_bounds__(32) k_hsing(DMesh m, HS hs, int nf, double* A,
         }
         hsing_scatter(m, dn, e, o, v, Af, lda, bc);
       }
+#pragma unroll
       for (int il = 0; il < 3; ++il)
         for (int o = 16; o > 0; o >>= 1) bc[il] = bc[il] + shfl_x(bc[il], o);
       if (lane == 0) {
@@ -593,6 +609,7 @@ __global__ void __launch_bounds__(32) k_hsing(DMesh m, HS hs, int nf, double* A,
         if (qp != cur) {
           if (cur >= 0) flush(cur);
           cur = qp;
+#pragma unroll
           for (int j = 0; j < NA; ++j) acc[j] = z;
           as0 = as1 = z;
         }
