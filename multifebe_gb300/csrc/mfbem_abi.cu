@@ -280,6 +280,12 @@ static int ensure(DevBuf& b, size_t bytes) {
   b.dev = dev;
   return 0;
 }
+// ensure() for work space that a call can do without: false if there is no memory for it
+static bool try_ensure(DevBuf& b, size_t bytes) {
+  if (!ensure(b, bytes)) return true;
+  cudaGetLastError();
+  return false;
+}
 // calls on a handle run on the device it was uploaded on
 static int check_dev(const mfbem_handle* h) {
   const int d = cur_dev();
@@ -1041,7 +1047,7 @@ struct AsmTimes {
 // device parameter blocks (dparh: HBIE points only), mixed: the double-float
 // rows too. t->n = 0 (the kernels evaluate E_n directly) where the tables do
 // not apply: a wavenumber of zero or not finite, or more intervals than
-// kRadMaxN.
+// kRadMaxN, more than 4 GB (many frequencies on a small mesh) or no memory.
 static int radial_prepare(mfbem_handle* h, double rmax, const double* q, int nf, const HarParD* dpar, const HarParH* dparh,
                           bool mixed, RadTab* t) {
   *t = RadTab();
@@ -1061,8 +1067,8 @@ static int radial_prepare(mfbem_handle* h, double rmax, const double* q, int nf,
   const int n = (int)std::ceil(most) + 1, nfun = dparh ? 10 : 5;
   const size_t rows = (size_t)nf * n, bc = rows * nfun * kRadC * sizeof(double2),
                bf = mixed ? rows * 5 * kRadRowF * sizeof(float4) : 0, bs = sizeof(RadF) * nf, bsf = sizeof(RadFF) * nf;
-  int rc;
-  if ((rc = ensure(h->rad, bc + bf + bs + bsf + sizeof(double) * nf))) return rc;
+  const size_t bytes = bc + bf + bs + bsf + sizeof(double) * nf;
+  if (bytes > ((size_t)4 << 30) || !try_ensure(h->rad, bytes)) return 0;
   char* p = (char*)h->rad.p;
   double2* c = (double2*)p;
   float4* cf4 = mixed ? (float4*)(p + bc) : nullptr;
@@ -1103,9 +1109,9 @@ static int launch_assembly(mfbem_handle* h, const POL& pol, const double* d_nu, 
   const size_t sysz = (size_t)m.ndof * m.ndof * W * nf;
   if (nw0 > 0 && nw0 < 6 * 152) z.n = (int)std::min<long long>(8, (2432 + nw0 - 1) / nw0);
   while (z.n > 1 && (z.n - 1) * sysz * sizeof(double) > ((size_t)2 << 30)) --z.n;
+  const size_t bsz = (size_t)m.ndof * W * nf;
+  if (z.n > 1 && !try_ensure(h->slc, (z.n - 1) * (sysz + bsz) * sizeof(double))) z.n = 1;
   if (z.n > 1) {
-    const size_t bsz = (size_t)m.ndof * W * nf;
-    if (int rc = ensure(h->slc, (z.n - 1) * (sysz + bsz) * sizeof(double))) return rc;
     z.A = (double*)h->slc.p;
     z.lda = m.ndof;
     z.astride = (size_t)m.ndof * m.ndof * W;

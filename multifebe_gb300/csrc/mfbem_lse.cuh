@@ -525,6 +525,7 @@ static int gecon1(const LseWork& w, const S* Ao, const S* LU, int n, S* x, S* v,
 // in step, so a triangular solve -- a chain of n / 64 blocks whatever their
 // number -- serves all that need it. Work per right-hand side: R, y, v, p (n
 // each), wts (n), isgn (n ints), stat (4), flag; part (64 n) shared.
+constexpr int kRefineRhs = 64;  // right-hand sides in step at most: bounds the work space
 template <typename S>
 struct GerfsWork {
   S *R, *y, *v, *pack;
@@ -673,11 +674,11 @@ static int solve_dropin(int32_t n, double* A, int32_t* ipiv, int32_t aodim, doub
   const size_t es = sizeof(S), nn = (size_t)n * n, nr = (size_t)std::max(1, n_rhs);
   const bool keep_ao = condition || refine;
   // vector work: x, v (n S each), r, c (n doubles), bits (n u64), isgn, perm (n
-  // ints), scalars; refine, per right-hand side: R, y, v, pack (n S), wts (n
-  // doubles), stat (4), isgn (n ints), flag; part (64 n doubles)
-  const size_t np = (size_t)n;
+  // ints), scalars; refine, per right-hand side in step: R, y, v, pack (n S),
+  // wts (n doubles), stat (4), isgn (n ints), flag; part (64 n doubles)
+  const size_t np = (size_t)n, nw = std::min<size_t>(nr, kRefineRhs);
   const size_t wbytes = 2 * np * es + 3 * np * 8 + 2 * np * 4 + 256 +
-                        (refine ? nr * (4 * np * es + np * 8 + 4 * 8 + np * 4 + 4) + 64 * np * 8 + 64 : 0);
+                        (refine ? nw * (4 * np * es + np * 8 + 4 * 8 + np * 4 + 4) + 64 * np * 8 + 64 : 0);
   if ((rc = ensure(cx->A, nn * es)) || (rc = ensure(cx->b, (size_t)n * nr * es)) ||
       (rc = ensure(cx->ipiv, sizeof(int) * n)) || (rc = ensure(cx->info, sizeof(int) * 4)) ||
       (rc = ensure(cx->wv, wbytes)) || (keep_ao && (rc = ensure(cx->Ao, nn * es))) ||
@@ -696,10 +697,10 @@ static int solve_dropin(int32_t n, double* A, int32_t* ipiv, int32_t aodim, doub
   double* dr = (double*)(vv + np);
   if (refine) {
     gw.R = vv + np;
-    gw.y = gw.R + nr * np;
-    gw.v = gw.y + nr * np;
-    gw.pack = gw.v + nr * np;
-    dr = (double*)(gw.pack + nr * np);
+    gw.y = gw.R + nw * np;
+    gw.v = gw.y + nw * np;
+    gw.pack = gw.v + nw * np;
+    dr = (double*)(gw.pack + nw * np);
   }
   double* dc = dr + np;
   unsigned long long* bits = (unsigned long long*)(dc + np);
@@ -707,14 +708,14 @@ static int solve_dropin(int32_t n, double* A, int32_t* ipiv, int32_t aodim, doub
   int* isgn = (int*)(red + 8);
   if (refine) {
     gw.wts = red + 8;
-    gw.stat = gw.wts + nr * np;
-    gw.part = gw.stat + 4 * nr;
+    gw.stat = gw.wts + nw * np;
+    gw.part = gw.stat + 4 * nw;
     isgn = (int*)(gw.part + 64 * np);
   }
   int* dperm = isgn + np;
   if (refine) {
     gw.isgn = dperm + np;
-    gw.flag = gw.isgn + nr * np;
+    gw.flag = gw.isgn + nw * np;
   }
   LseWork w{st, red, di + 2};
   if ((rc = trsv_err_reset(st))) return rc;
@@ -771,7 +772,10 @@ static int solve_dropin(int32_t n, double* A, int32_t* ipiv, int32_t aodim, doub
     if (refine) {
       g_lse.ferr.assign(n_rhs, 0.0);
       g_lse.berr.assign(n_rhs, 0.0);
-      if ((rc = gerfs<S>(w, dAo, dA, dp, perm, n, n_rhs, dbc, db, gw, g_lse.ferr.data(), g_lse.berr.data()))) return rc;
+      for (int j = 0; j < n_rhs; j += kRefineRhs)
+        if ((rc = gerfs<S>(w, dAo, dA, dp, perm, n, std::min(kRefineRhs, n_rhs - j), dbc + (size_t)j * n,
+                           db + (size_t)j * n, gw, g_lse.ferr.data() + j, g_lse.berr.data() + j)))
+          return rc;
     }
     if (scaling && (eq == 'C' || eq == 'B')) {
       k_rows_scale<S><<<152 * 4, 256, 0, st>>>(db, n, n_rhs, dc); ++g_launches;
