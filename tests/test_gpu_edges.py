@@ -1,0 +1,117 @@
+"""Sizes at which the kernels of the solve, the mixed updates, the assembly and
+the internal points change tile, path or remainder."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from multifebe_gb300 import BemRegion, _abi, solve_lse
+from multifebe_gb300 import meshgen as M
+
+pytestmark = pytest.mark.gpu
+EPS = 2.0 ** -53
+
+
+def rel(a, b):
+    return np.abs(a - b).max() / max(np.abs(b).max(), 1e-300)
+
+
+# panel widths 16 and 32, outer blocks of 64 and 128, 16-CTA panels (above 1200
+# complex, 2400 real), the split block TRSM (4096 real columns to the right)
+@pytest.mark.parametrize("cplx", [False, True], ids=["real", "complex"])
+@pytest.mark.parametrize("n", [1, 2, 15, 16, 17, 31, 33, 127, 128, 129, 257, 1199, 1201, 2305, 2403])
+def test_lu_and_solve(n, cplx):
+    """Backward errors of the factorisation and of the solve. Each entry of
+    L U sums n products, each operation within 2 eps (4 eps complex): n times
+    that of max(|L| |U|), and the same for each of the two triangular solves."""
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((n, n)) + (1j * rng.standard_normal((n, n)) if cplx else 0)
+    b = rng.standard_normal((n, 3)) + (1j * rng.standard_normal((n, 3)) if cplx else 0)
+    F, x = np.array(A, order="F", copy=True), np.array(b, order="F", copy=True)
+    _, ipiv = solve_lse(F, x)
+    L, U = np.tril(F, -1) + np.eye(n), np.triu(F)
+    p = np.arange(n)
+    for k in range(n):
+        j = ipiv[k] - 1
+        assert k <= j < n
+        p[[k, j]] = p[[j, k]]
+    u = (4 if cplx else 2) * EPS
+    size = np.abs(L) @ np.abs(U)
+    assert np.abs(A[p] - L @ U).max() <= n * u * size.max()
+    # multipliers of the |re| + |im| pivot
+    assert np.abs(L).max() <= (np.sqrt(2) if cplx else 1.0) * (1 + 8 * EPS)
+    assert (np.abs(A @ x - b) <= 3 * n * u * (size @ np.abs(x)).max(0)).all()
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (63, 127, 15), (65, 129, 17), (130, 257, 33), (200, 300, 128)])
+def test_binary16_split_of_uneven_rows_and_columns(m, n, k):
+    """Rows of A and columns of B scaled over 2^+-20, one row and one column
+    zero, entries down to 2^-24 of their row's largest. Split: each factor to
+    2^-22 of itself and 2^-39 of its row's largest, lo lo left out (2^-22); FP32
+    sums: three passes over ceil(2 k / 16) steps, each within 2^-22 of the sum
+    of moduli; the last subtraction 2^-23 of C and the sum."""
+    rng = np.random.default_rng(m + n + k)
+
+    def cplx(r, c):
+        x = rng.standard_normal((r, c)) + 1j * rng.standard_normal((r, c))
+        return x * 2.0 ** rng.integers(-24, 1, size=(r, c))
+    A = cplx(m, k) * 2.0 ** rng.integers(-20, 21, size=(m, 1))
+    B = cplx(k, n) * 2.0 ** rng.integers(-20, 21, size=(1, n))
+    A[m // 2], B[:, n // 2] = 0, 0
+    if m == n == 1:
+        A[0, 0], B[0, 0] = 3.0 + 1j, 2.0 - 5j
+    C = rng.standard_normal((m, n)) + 1j * rng.standard_normal((m, n))
+    A, B, C = (np.asfortranarray(v, dtype=np.complex64) for v in (A, B, C))
+    L = _abi.load()
+    L.mfbem_internal_tc_cgemm.argtypes = [ctypes.c_int32] * 3 + [ctypes.c_void_p] * 3 + [ctypes.c_int32]
+    G = C.copy(order="F")
+    _abi.check(L.mfbem_internal_tc_cgemm(m, n, k, A.ctypes.data, B.ctypes.data, G.ctypes.data, 0))
+    A, B, C, G = (v.astype(np.complex128) for v in (A, B, C, G))
+    a1, b1 = np.abs(A.real) + np.abs(A.imag), np.abs(B.real) + np.abs(B.imag)
+    S = a1 @ b1
+    top = a1.max(1)[:, None] * b1.max(0)[None, :]
+    tol = (3 * 2.0 ** -22 + 3 * -(-2 * k // 16) * 2.0 ** -22) * S + 4 * k * 2.0 ** -39 * top + 2.0 ** -23 * (np.abs(C) + S)
+    assert (np.abs(G - (C - A @ B)) <= tol).all()
+
+
+@pytest.mark.parametrize("divs", [(1, 1, 1), (2, 1, 1), (3, 2, 1), (5, 3, 2), (7, 5, 3), (9, 6, 4)])
+def test_mixed_solve_of_odd_sizes(divs):
+    """Unpivoted panels, their remainders and the outer blocks: the mixed
+    solution against the binary64 one (the bound of the mixed solves: 1e-9)."""
+    d = M.box((1.0, 0.8, 0.6), divs)
+    z = d.nodes[:, 2]
+    d.ctype[z < 1e-9] = 0
+    d.cvalue[z > 0.6 - 1e-9] = (0.0, 0.3, -1.0)
+    R = BemRegion(d)
+    xp = R.solve_staela(1.0, 0.25, precision="plain")
+    xm = R.solve_staela(1.0, 0.25, precision="mixed")
+    R.close()
+    assert rel(xm, xp) < 1e-9
+
+
+# 20, 56, 884 and 1154 nodes: 8 slices of a node's points, 3, and none (from 912)
+@pytest.mark.parametrize("n", [1, 2, 7, 8])
+def test_slices_of_a_nodes_points(oracle, n):
+    d = M.cube_clamped_top_traction(n)
+    R = BemRegion(d)
+    A, b = R.build_lse_staela(1.0, 0.25)
+    Ao, bo = oracle.Problem(d).assemble_staela(1.0, 0.25)
+    R.close()
+    assert rel(A, Ao) < 1e-11 and rel(b, bo) < 1e-11
+
+
+# element groups of 32: 6, 24, 54 and 96 elements; 1 point, and so many that a
+# warp takes several groups
+@pytest.mark.parametrize("n,nip", [(1, 1), (2, 7), (3, 33), (4, 5000)])
+def test_groups_of_elements_at_internal_points(oracle, n, nip):
+    d = M.cube_confined_kat(n)
+    rng = np.random.default_rng(nip)
+    P = oracle.Problem(d)
+    X = 0.4 + 0.2 * rng.random((nip, 3))
+    A, b = P.assemble_staela(0.4, 0.25)
+    u, t = P.solution(oracle.lu_solve(A, b))
+    R = BemRegion(d)
+    ui, si = R.internal_points(X, u, t, mu=0.4, nu=0.25)
+    uo, so = P.internal_points(X, u, t, mu=0.4, nu=0.25)
+    R.close()
+    assert rel(ui, uo) < 1e-11 and rel(si, so) < 1e-11
