@@ -5,7 +5,7 @@ a0 = 0.1..2.0, bottom face clamped, uniform harmonic t_z=-1 on the top face.
 
 One step = one full frequency sweep on the device = 20 solves, mixed precision:
 double-float assembly of the 20 systems (binary64 results), complex64 LU with
-TF32 tensor-core trailing updates, FP64 iterative refinement to a 1e-12
+binary16-split tensor-core trailing updates, FP64 iterative refinement to a 1e-12
 backward error (solutions within 1e-8 of the FP64 oracle's). value: device time
 (CUDA events inside the library) with the mesh resident in HBM; inputs (20 x
 192 MB systems) exceed L2. e2e: the same sweep through the public C-ABI from
@@ -56,15 +56,15 @@ FLOPS_PER_REGULAR_POINT = 1280
 # formulation of the same kernel could at best run at this rate
 FP64_NOMINAL_TFLOPS = 1.25
 # DRAM bytes per frequency of that kernel from ncu (dram__bytes_read.sum +
-# dram__bytes_write.sum of one launch of the 2-frequency profile case, 453.4 +
-# 392.9 MB, divided by 2; profiles/k_mixed_cube8x2freq.md): A written once
-# and read back once (the flush adds into the zeroed system). Traffic grows in
+# dram__bytes_write.sum of one launch of the 2-frequency profile case, 449.6 +
+# 394.1 MB, divided by 2; profiles/k_mixed_cube8x2freq.md): A written once
+# and read once (the pair sums are added to the zeroed system at the L2). Traffic grows in
 # proportion to the frequencies (one system per frequency).
-REG_TRAFFIC_PER_FREQ = 423.2e6
-# Pipe utilisation of the same launch (ncu --set full, same small case and
+REG_TRAFFIC_PER_FREQ = 421.9e6
+# Pipe utilisation of the same launch (ncu, same small case and
 # file): the kernel is bound by instruction issue on the FP32 pipe
 # (double-float arithmetic), not by HBM.
-REG_NCU_PIPES = {"issue_slots_busy_pct": 61.4, "fp32_fma_pipe_pct": 40.0, "fp64_pipe_pct": 26.3,
+REG_NCU_PIPES = {"issue_slots_busy_pct": 53.2, "fp32_fma_pipe_pct": 28.0, "fp64_pipe_pct": 34.9,
                  "source": "profiles/k_mixed_cube8x2freq.md"}
 
 
@@ -269,7 +269,7 @@ def run_gpu(args):
     line = {"metric": METRIC, "value": value, "unit": "solves/s", "n_gpus": ws, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": per_step_ms, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None,
-            "dtype": "double-float assembly (binary64 x - x_i) into binary64 systems / complex64 LU with 3xTF32 "
+            "dtype": "double-float assembly (binary64 x - x_i) into binary64 systems / complex64 LU with binary16 hi/lo "
                      "tensor-core updates + FP64 refinement",
             "data": "synthetic",
             "config": bench_config(n, nf),
