@@ -918,9 +918,14 @@ __global__ void __launch_bounds__(128) k_trsv_diag64(const S* A, long long strid
 // column and no launch between the diagonal block and its rows (a separate
 // diagonal kernel cost one dependent launch per 32 columns). The factorised
 // block goes back in place only after every CTA has read the original: each
-// CTA takes a ticket from cnt[b] after its load, and the last one writes and
-// resets the counter (zero on entry, zero on exit). A zero or non-finite
-// pivot sets info and leaves the rows as they are.
+// CTA takes a ticket from cnt[b], and the last one writes and resets the
+// counter (zero on entry, zero on exit). The ticket is taken once the factors
+// are in shared memory: they are computed from the loaded entries, so all of
+// the CTA's loads have returned before the barrier that precedes it (a barrier
+// alone does not wait for loads whose registers nothing has read), and fences
+// on both sides of the counter order them before the last CTA's stores. The
+// counter's round trip is hidden behind the CTA's own rows. A zero or
+// non-finite pivot sets info and leaves the block and the rows as they are.
 // Grid: (max(1, ceil((r1 - r0) / 128)), batch).
 // ---------------------------------------------------------------------------
 // The diagonal block sits in registers, warp g holding the columns g + 4 q of
@@ -956,7 +961,6 @@ __global__ void __launch_bounds__(128) k_panel_nopiv(S* A, long long sA, int lda
   }
   if (t == 0) s_bad = 0;
   __syncthreads();
-  if (t == 0) s_last = atomicAdd(cnt + b, 1) == (int)gridDim.x - 1;
 #pragma unroll
   for (int j = 0; j < 32; ++j) {
     if (g == (j & 3)) {
@@ -984,6 +988,31 @@ __global__ void __launch_bounds__(128) k_panel_nopiv(S* A, long long sA, int lda
 #pragma unroll
   for (int q = 0; q < 8; ++q) D[(g + 4 * q) * 33 + lane] = v[q];
   __syncthreads();
+  int ticket = 0;
+  if (t == 0) {
+    __threadfence();
+    ticket = atomicAdd(cnt + b, 1);
+  }
+  const int row = r0 + blockIdx.x * 128 + t;
+  if (!s_bad && row < r1) {
+    S x[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) x[j] = j < kb ? M[(size_t)(k + j) * lda + row] : Sc<S>::zero();
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      x[j] = Sc<S>::mul(x[j], ur[j]);
+#pragma unroll
+      for (int c = j + 1; c < 32; ++c) x[c] = lu_fnma(x[j], D[c * 33 + j], x[c]);
+    }
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+      if (j < kb) M[(size_t)(k + j) * lda + row] = x[j];
+  }
+  if (t == 0) {
+    s_last = ticket == (int)gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
   // a zero or non-finite pivot at column s_bad - 1: nothing is written back
   if (s_last) {
     if (s_bad) {
@@ -996,21 +1025,6 @@ __global__ void __launch_bounds__(128) k_panel_nopiv(S* A, long long sA, int lda
     }
     if (t == 0) cnt[b] = 0;
   }
-  if (s_bad) return;
-  const int row = r0 + blockIdx.x * 128 + t;
-  if (row >= r1) return;
-  S x[32];
-#pragma unroll
-  for (int j = 0; j < 32; ++j) x[j] = j < kb ? M[(size_t)(k + j) * lda + row] : Sc<S>::zero();
-#pragma unroll
-  for (int j = 0; j < 32; ++j) {
-    x[j] = Sc<S>::mul(x[j], ur[j]);
-#pragma unroll
-    for (int c = j + 1; c < 32; ++c) x[c] = lu_fnma(x[j], D[c * 33 + j], x[c]);
-  }
-#pragma unroll
-  for (int j = 0; j < 32; ++j)
-    if (j < kb) M[(size_t)(k + j) * lda + row] = x[j];
 }
 
 // ---------------------------------------------------------------------------

@@ -89,6 +89,21 @@ def test_mixed_solve_of_odd_sizes(divs):
     assert rel(xm, xp) < 1e-9
 
 
+@pytest.mark.parametrize("harmonic", [False, True], ids=["static", "harmonic"])
+def test_mixed_solves_repeat_bitwise(harmonic):
+    """The unpivoted panel's diagonal block is read by up to 28 CTAs and written
+    back by one of them (3462 rows): the same solve gives the same bits."""
+    d = M.cube_clamped_top_traction(8)
+    mat = M.viscoelastic(1.0, 0.3, 1.0, 0.05)
+    R = BemRegion(d)
+    x = [R.sweep_harela(mat, M.omega_from_a0([0.4, 1.1], mat), precision="mixed") if harmonic else
+         R.solve_staela(1.0, 0.25, precision="mixed") for _ in range(4)]
+    refactorizations = R.last_stats["refactorizations"]
+    R.close()
+    assert refactorizations == 0
+    assert all((v == x[0]).all() for v in x[1:])
+
+
 # 20, 56, 884 and 1154 nodes: 8 slices of a node's points, 3, and none (from 912)
 @pytest.mark.parametrize("n", [1, 2, 7, 8])
 def test_slices_of_a_nodes_points(oracle, n):
