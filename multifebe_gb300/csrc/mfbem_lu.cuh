@@ -98,6 +98,13 @@ template <> struct Sc<float2> {
   __device__ static float re(float2 a) { return a.x; }
 };
 
+// biased exponent of the larger component's modulus; 0 for zero and subnormal
+// values, and for non-finite ones, which stay so under any scale
+__device__ __forceinline__ int tq_exp(float2 v) {
+  const int x = (__float_as_uint(v.x) >> 23) & 255, y = (__float_as_uint(v.y) >> 23) & 255;
+  return max(x == 255 ? 0 : x, y == 255 ? 0 : y);
+}
+
 // a value of another lane
 template <typename S> __device__ __forceinline__ S shfl_s(S v, int src);
 template <> __device__ __forceinline__ float2 shfl_s(float2 v, int src) {
@@ -660,10 +667,11 @@ __global__ void __launch_bounds__(32) k_swap_trsm16(S* A, long long strideA, int
 // consecutive rows, so L's column is read without conflict and X's entries are
 // broadcasts), 4 + CT shared-memory loads for 4 CT multiply-adds. In place of a TRSM and a GEMM
 // launch per 16 or 32 rows, each with a fixed cost (copies, a tile of the SMs
-// idle, for the tensor-core paths an operand split).
+// idle, for the tensor-core paths an operand split). kexp: as in k_trsm_cols.
 // ---------------------------------------------------------------------------
 template <typename S, int NC>
-__global__ void __launch_bounds__(256) k_trsm_block(S* A, long long strideA, int lda, int K, int w, int c0, int c1) {
+__global__ void __launch_bounds__(256) k_trsm_block(S* A, long long strideA, int lda, int K, int w, int c0, int c1,
+                                                    int* kexp, int kst) {
   constexpr int CT = NC >= 8 ? NC / 8 : 1, CG = NC / CT;  // columns per thread, column groups
   constexpr int RT = 4;                                   // rows per thread (32 apart)
   constexpr bool F64 = sizeof(typename Sc<S>::R) == 8;
@@ -748,6 +756,13 @@ __global__ void __launch_bounds__(256) k_trsm_block(S* A, long long strideA, int
     const int i = e % w, c = e / w;
     M[(size_t)(cb + c) * lda + K + i] = X[c * 129 + i];
   }
+  if constexpr (std::is_same<S, float2>::value) {
+    if (kexp && t < w) {
+      int e = 0;
+      for (int c = 0; c < nc; ++c) e = max(e, tq_exp(X[c * 129 + t]));
+      atomicMax(kexp + (size_t)kst * blockIdx.y + K + t, e);
+    }
+  }
 }
 
 // Apply the panel interchanges (rows k..k+nb-1 with ipiv) to the columns
@@ -799,11 +814,15 @@ __global__ void k_trsm_llu(S* A, long long strideA, int lda, int n, int k, int n
 // U12 = L11^{-1} A12 for the columns [c0, c1) (L11 unit lower, w x w at (k,k),
 // w <= 32). A CTA of trsm_cols<S>() threads stages a 32-row tile of as many
 // columns (coalesced along each column), thread t solves column t in shared
-// memory, and the tile is written back.
+// memory, and the tile is written back. kexp (complex64, else null): [batch][kst]
+// by absolute row, raised to the largest exponent in each solved row; the
+// operand split of the updates balances its scales with it (mfbem_tc.cuh), and
+// a row of U gets its parts by several solves, so the maxima gather over one
+// factorisation.
 template <typename S> __host__ __device__ constexpr int trsm_cols() { return sizeof(S) > 8 ? 32 : 64; }
 template <typename S>
 __global__ void __launch_bounds__(trsm_cols<S>()) k_trsm_cols(S* A, long long strideA, int lda, int k, int w, int c0,
-                                                              int c1) {
+                                                              int c1, int* kexp, int kst) {
   constexpr int NC = trsm_cols<S>();
   const int bidx = blockIdx.y;
   S* M = A + strideA * bidx;
@@ -847,6 +866,13 @@ __global__ void __launch_bounds__(trsm_cols<S>()) k_trsm_cols(S* A, long long st
   for (int t = threadIdx.x; t < 32 * ncol; t += NC) {
     const int i = t & 31, cc = t >> 5;
     if (i < w) M[(size_t)(cb + cc) * lda + k + i] = T[cc * 33 + i];
+  }
+  if constexpr (std::is_same<S, float2>::value) {
+    if (kexp && (int)threadIdx.x < w) {
+      int e = 0;
+      for (int q = 0; q < ncol; ++q) e = max(e, tq_exp(T[q * 33 + threadIdx.x]));
+      atomicMax(kexp + (size_t)kst * bidx + k + threadIdx.x, e);
+    }
   }
 }
 

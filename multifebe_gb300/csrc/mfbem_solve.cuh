@@ -56,16 +56,26 @@ static int c32_default() {
 // updates; their timeout flag and pre-split operand tiles, per host thread
 static thread_local DevBuf g_tc_err, g_tc_ws;
 
+// exponents of U's rows for the split's balance (k_trsm_cols): [batch][n] of the
+// factorisation under way
+static thread_local DevBuf g_tc_kexp;
+
+// bytes of the operand split of a complex64 update (m x n, depth k)
+static size_t tc_ws_bytes(int m, int n, int k, int batch) {
+  const size_t nmt = (m + TC_BM / 2 - 1) / (TC_BM / 2), nnt = (n + TC_BN - 1) / TC_BN, nkc = (k + TQ - 1) / TQ;
+  return batch * (8 * (nmt + nnt) * nkc * TQ_TW + 4 * (nmt * (TC_BM / 2) + nnt * TC_BN + k));
+}
+
 // C -= A B (complex64, batched): split A and B into pre-tiled hi / lo words
 // once, then the bulk-copy / tcgen05 pipeline per 128 x 128 tile of C~.
 static int tc_cgemm_run(cudaStream_t st, const float2* A, int lda, long long sA, const float2* B, int ldb,
                         long long sB, float2* C, int ldc, long long sC, int m, int n, int k, int batch, DevBuf& ws,
-                        int* err, int passes = 3) {
+                        int* err, int passes = 3, const int* kexp = nullptr, int kst = 0) {
   const int nmt = (m + TC_BM / 2 - 1) / (TC_BM / 2), nnt = (n + TC_BN - 1) / TC_BN, nkc = (k + TQ - 1) / TQ;
   if (nmt == 0 || nnt == 0 || nkc == 0) return 0;
   const size_t wa = (size_t)batch * nmt * nkc * TQ_TW, wb = (size_t)batch * nnt * nkc * TQ_TW;
   const size_t na = (size_t)batch * nmt * (TC_BM / 2), nc = (size_t)batch * nnt * TC_BN;
-  int rc = ensure(ws, sizeof(uint32_t) * 2 * (wa + wb) + sizeof(float) * (na + nc));
+  int rc = ensure(ws, tc_ws_bytes(m, n, k, batch));
   if (rc) return rc;
   // column tiles of 256 (M 128 x N 256 MMAs, two CTAs per SM) unless the
   // update is narrower; MFBEM_TC_BN=128 selects the 128-column tiles
@@ -82,8 +92,16 @@ static int tc_cgemm_run(cudaStream_t st, const float2* A, int lda, long long sA,
   uint32_t* blo = bhi + wb;
   float* srow = (float*)(blo + wb);
   float* scol = srow + na;
-  k_tc_split<<<dim3(nmt + nnt, batch), 256, 0, st>>>(A, lda, sA, m, B, ldb, sB, n, k, nmt, nnt, nkc, ahi, alo, srow, bhi,
-                                                     blo, scol);
+  if (!kexp) {
+    int* own = (int*)(scol + nc);
+    kst = k;
+    CK(cudaMemsetAsync(own, 0, sizeof(int) * (size_t)batch * k, st));
+    k_tc_kexp<<<dim3(nblk(k, 32), nblk(n, 128), batch), 256, 0, st>>>(B, ldb, sB, n, k, kst, own);
+    ++g_launches;
+    kexp = own;
+  }
+  k_tc_split<<<dim3(nmt + nnt, batch), 256, 0, st>>>(A, lda, sA, m, B, ldb, sB, n, k, nmt, nnt, nkc, kexp, kst, ahi,
+                                                     alo, srow, bhi, blo, scol);
   ++g_launches;
   if (wide)
     k_tc_cgemm_bulk<2><<<dim3(nmt, (nnt + 1) / 2, batch), 128, tc_smem_bulk<2>(), st>>>(
@@ -277,23 +295,27 @@ static int tc_min_depth(int batch) {
 // C -= A B (batched) in the scalar type of the factorisation, as configured
 // above: FP64 (plain LU) or FP32 (mixed LU)
 static int gemm_sb(cudaStream_t st, int m, int n, int k, const double* A, int lda, long long sA, const double* B,
-                   int ldb, long long sB, double* C, int ldc, long long sC, int batch) {
+                   int ldb, long long sB, double* C, int ldc, long long sC, int batch,
+                   const int* = nullptr, int = 0) {
   return f64_gemm<double>(st, m, n, k, A, lda, sA, B, ldb, sB, C, ldc, sC, batch);
 }
 static int gemm_sb(cudaStream_t st, int m, int n, int k, const double2* A, int lda, long long sA, const double2* B,
-                   int ldb, long long sB, double2* C, int ldc, long long sC, int batch) {
+                   int ldb, long long sB, double2* C, int ldc, long long sC, int batch,
+                   const int* = nullptr, int = 0) {
   return f64_gemm<double2>(st, m, n, k, A, lda, sA, B, ldb, sB, C, ldc, sC, batch);
 }
 static int gemm_sb(cudaStream_t st, int m, int n, int k, const float* A, int lda, long long sA, const float* B,
-                   int ldb, long long sB, float* C, int ldc, long long sC, int batch) {
+                   int ldb, long long sB, float* C, int ldc, long long sC, int batch,
+                   const int* = nullptr, int = 0) {
   return gemm_simt<float>(st, m, n, k, A, lda, sA, B, ldb, sB, C, ldc, sC, batch);
 }
 static int gemm_sb(cudaStream_t st, int m, int n, int k, const float2* A, int lda, long long sA, const float2* B,
-                   int ldb, long long sB, float2* C, int ldc, long long sC, int batch) {
+                   int ldb, long long sB, float2* C, int ldc, long long sC, int batch,
+                   const int* kexp = nullptr, int kst = 0) {
   const int mode = g_c32_mode;
   if ((mode == 3 || mode == 1) && g_tc_err.p && k >= tc_min_depth(batch))
     return tc_cgemm_run(st, A, lda, sA, B, ldb, sB, C, ldc, sC, m, n, k, batch, g_tc_ws, (int*)g_tc_err.p,
-                        mode == 3 ? 3 : 1);
+                        mode == 3 ? 3 : 1, kexp, kst);
   return gemm_simt<float2>(st, m, n, k, A, lda, sA, B, ldb, sB, C, ldc, sC, batch);
 }
 
@@ -331,37 +353,40 @@ static int panel_nb_f64(int n) {
 // 63.5 ms for four complex 3462-row systems, no difference for one below 4096.
 constexpr double kTrsmSplit = 4096.0;
 template <typename S, int NC>
-static int trsm_block_launch(cudaStream_t st, S* A, long long sA, int lda, int K, int w, int c0, int c1, int batch) {
+static int trsm_block_launch(cudaStream_t st, S* A, long long sA, int lda, int K, int w, int c0, int c1, int batch,
+                             int* kx, int kst) {
   if (raise_smem_limit((const void*)k_trsm_block<S, NC>)) return fail(MFBEM_ECUDA, "shared-memory limit of the block TRSM");
   k_trsm_block<S, NC><<<dim3(nblk(c1 - c0, NC), batch), 256, sizeof(S) * (129 * (size_t)NC + 16 * 129), st>>>(
-      A, sA, lda, K, w, c0, c1);
+      A, sA, lda, K, w, c0, c1, kx, kst);
   ++g_launches;
   CK(cudaGetLastError());
   return 0;
 }
 template <typename S>
-static int trsm_block_run(cudaStream_t st, S* A, long long sA, int lda, int K, int w, int c0, int c1, int batch) {
+static int trsm_block_run(cudaStream_t st, S* A, long long sA, int lda, int K, int w, int c0, int c1, int batch, int* kx,
+                          int kst) {
   // columns per CTA: as many as leave every SM about two CTAs, 4 to 16 (binary32: 32)
   const long long cols = (long long)(c1 - c0) * batch;
-  if (!IsF64<S>::v && cols >= 32 * 304) return trsm_block_launch<S, 32>(st, A, sA, lda, K, w, c0, c1, batch);
-  if (cols > 8 * 304) return trsm_block_launch<S, 16>(st, A, sA, lda, K, w, c0, c1, batch);
-  if (cols > 4 * 304) return trsm_block_launch<S, 8>(st, A, sA, lda, K, w, c0, c1, batch);
-  return trsm_block_launch<S, 4>(st, A, sA, lda, K, w, c0, c1, batch);
+  if (!IsF64<S>::v && cols >= 32 * 304) return trsm_block_launch<S, 32>(st, A, sA, lda, K, w, c0, c1, batch, kx, kst);
+  if (cols > 8 * 304) return trsm_block_launch<S, 16>(st, A, sA, lda, K, w, c0, c1, batch, kx, kst);
+  if (cols > 4 * 304) return trsm_block_launch<S, 8>(st, A, sA, lda, K, w, c0, c1, batch, kx, kst);
+  return trsm_block_launch<S, 4>(st, A, sA, lda, K, w, c0, c1, batch, kx, kst);
 }
 // inv(L11) A12 of an outer block of w rows: blocks of at most 128 rows with
-// updates between them (binary64: see kTrsmSplit)
+// updates between them (binary64: see kTrsmSplit). kx: k_trsm_cols' kexp
 template <typename S>
-static int trsm_outer(cudaStream_t st, S* A, long long sA, int lda, int K, int w, int c0, int c1, int batch) {
+static int trsm_outer(cudaStream_t st, S* A, long long sA, int lda, int K, int w, int c0, int c1, int batch, int* kx,
+                      int kst) {
   const int nc = c1 - c0, cw = sizeof(S) / 8;
   int h = w;
   if (w > 128) h = 128;
   else if (IsF64<S>::v && w == 128 && (double)nc * batch * cw >= kTrsmSplit) h = 64;
   for (int s = 0; s < w; s += h) {
     const int sb = std::min(h, w - s);
-    CKG(trsm_block_run<S>(st, A, sA, lda, K + s, sb, c0, c1, batch));
+    CKG(trsm_block_run<S>(st, A, sA, lda, K + s, sb, c0, c1, batch, kx, kst));
     if (s + sb < w)
       CKG(gemm_sb(st, w - s - sb, nc, sb, A + K + s + sb + (size_t)(K + s) * lda, lda, sA, A + K + s + (size_t)c0 * lda,
-                  lda, sA, A + K + s + sb + (size_t)c0 * lda, lda, sA, batch));
+                  lda, sA, A + K + s + sb + (size_t)c0 * lda, lda, sA, batch, kx ? kx + K + s : nullptr, kst));
   }
   return 0;
 }
@@ -457,6 +482,13 @@ static int getrf_batched(cudaStream_t st, S* A, long long sA, int lda, int n, in
   k_ipiv_identity<<<dim3(nblk(n, 256), batch), 256, 0, st>>>(ipiv, n); ++g_launches;
   typedef typename Sc<S>::R R;
   const bool tc = (g_c32_mode == 3 || g_c32_mode == 1) && std::is_same<S, float2>::value;
+  int* kx = nullptr;  // exponents of U's rows (k_trsm_cols)
+  if (tc) {
+    int rc = ensure(g_tc_kexp, sizeof(int) * (size_t)n * batch);
+    if (rc) return rc;
+    kx = (int*)g_tc_kexp.p;
+    CK(cudaMemsetAsync(kx, 0, sizeof(int) * (size_t)n * batch, st));
+  }
   // single precision only: the mixed path's unpivoted first attempt
   const bool nopiv = g_nopiv && !IsF64<S>::v;
   int* pn_cnt = nullptr;  // tickets of k_panel_nopiv, one per matrix
@@ -536,7 +568,8 @@ static int getrf_batched(cudaStream_t st, S* A, long long sA, int lda, int n, in
   auto trsm = [&](int k, int kb, int c0, int c1) -> int {
     const int nc = c1 - c0;
     if (nc <= 0) return 0;
-    k_trsm_cols<S><<<dim3(nblk(nc, trsm_cols<S>()), batch), trsm_cols<S>(), 0, st>>>(A, sA, lda, k, kb, c0, c1);
+    k_trsm_cols<S><<<dim3(nblk(nc, trsm_cols<S>()), batch), trsm_cols<S>(), 0, st>>>(A, sA, lda, k, kb, c0, c1,
+                                                                                              kx, n);
     ++g_launches;
     return 0;
   };
@@ -612,16 +645,16 @@ static int getrf_batched(cudaStream_t st, S* A, long long sA, int lda, int n, in
         const int nc = KE - k - kb;
         if (!fused) CKG(trsm(k, kb, k + kb, KE));
         CKG(gemm_sb(st, n - k - kb, nc, kb, A + k + kb + (size_t)k * lda, lda, sA, A + k + (size_t)(k + kb) * lda, lda,
-                    sA, A + (k + kb) + (size_t)(k + kb) * lda, lda, sA, batch));
+                    sA, A + (k + kb) + (size_t)(k + kb) * lda, lda, sA, batch, kx ? kx + k : nullptr, n));
       }
     }
     return 0;
   };
   // U12 of rows [K, KE) and columns [c0, c1), then those columns' update below
   auto update_block = [&](int K, int KE, int c0, int c1) -> int {
-    CKG(trsm_outer<S>(st, A, sA, lda, K, KE - K, c0, c1, batch));
+    CKG(trsm_outer<S>(st, A, sA, lda, K, KE - K, c0, c1, batch, kx, n));
     return gemm_sb(st, n - KE, c1 - c0, KE - K, A + KE + (size_t)K * lda, lda, sA, A + K + (size_t)c0 * lda, lda, sA,
-                   A + KE + (size_t)c0 * lda, lda, sA, batch);
+                   A + KE + (size_t)c0 * lda, lda, sA, batch, kx ? kx + K : nullptr, n);
   };
   for (int KO = 0; KO < n; KO += NBO) {
     const int KOE = std::min(n, KO + NBO);

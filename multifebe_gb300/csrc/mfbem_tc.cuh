@@ -252,7 +252,15 @@ __global__ void __launch_bounds__(128, 1) k_tc_cgemm(const float2* A, int lda, l
 // Split: x 2^s = hi + lo in binary16, s per row of A~ and column of B~ so that
 // the largest entry lies in [2^14, 2^15). binary16 has tf32's 11 significant
 // bits, so hi and lo carry the same bits as a tf32 pair for every entry above
-// 2^-17 of its row's (column's) largest, and an absolute 2^-40 of that below;
+// 2^-17 of its row's (column's) largest, and an absolute 2^-40 of that below.
+// For that to lose nothing the entries of a row have to be of one scale, which
+// the units decide: in L21 U12 row l of U has the scale of equation l and column
+// l of L its inverse, and the SBIE and HBIE rows of one region differ by the
+// shear modulus (2^36 in Pa). So a power of two per index l goes from B to A
+// first (tq_bal, exact): A's column l is multiplied by the one below the largest
+// entry of B's row l, B's row l divided by it. A region with mixed SBIE / HBIE
+// rows then takes 2 or 3 corrections at moduli from 1e-6 to 1e13, as with tf32
+// pairs; without the balance it did not converge at 8e10.
 // kind::f16 runs at twice kind::tf32's rate and its words hold two entries, so
 // a chunk copied from L2 feeds twice the multiply-adds. FP32 accumulation as
 // before; the epilogue takes the powers of two back out. Updates of 20
@@ -289,6 +297,40 @@ __device__ __forceinline__ void tq_scale(float mx, float& up, float& down) {
   up = __uint_as_float((uint32_t)(14 - e + 127) << 23);
   down = __uint_as_float((uint32_t)(e - 14 + 127) << 23);
 }
+// largest exponent of each row of B, kexp[b][l] (zeroed by the caller), for an
+// operand whose producer has not left it (the LU's triangular solves do): grid
+// (k / 32, columns / 128, batch), lane = l
+__global__ void __launch_bounds__(256) k_tc_kexp(const float2* B, int ldb, long long sB, int n, int k, int kst,
+                                                 int* kexp) {
+  __shared__ int s[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, b = blockIdx.z;
+  const int l = blockIdx.x * 32 + lane, j0 = blockIdx.y * 128, j1 = min(n, j0 + 128);
+  int e = 0;
+  if (l < k) {
+    const float2* Bb = B + sB * b + l;
+#pragma unroll 8
+    for (int j = j0 + w; j < j1; j += 8) e = max(e, tq_exp(Bb[(size_t)j * ldb]));
+  }
+  s[w][lane] = e;
+  __syncthreads();
+  if (w == 0 && l < k) {
+#pragma unroll
+    for (int q = 1; q < 8; ++q) e = max(e, s[q][lane]);
+    atomicMax(kexp + (size_t)b * kst + l, e);
+  }
+}
+// power of two that moves from B's row l to A's column l, and its inverse (both
+// normal numbers; 1 for a row without a normal entry)
+__device__ __forceinline__ int tq_bal_exp(const int* kexp, int l) {
+  const int e = __ldg(kexp + l);
+  return e == 0 ? 127 : min(e, 253);
+}
+__device__ __forceinline__ float tq_bal(const int* kexp, int l) {
+  return __uint_as_float((uint32_t)tq_bal_exp(kexp, l) << 23);
+}
+__device__ __forceinline__ float tq_bal_inv(const int* kexp, int l) {
+  return __uint_as_float((uint32_t)(254 - tq_bal_exp(kexp, l)) << 23);
+}
 // hi and lo words of the pair (x, y) (already scaled)
 __device__ __forceinline__ void tq_split(float x, float y, uint32_t& hi, uint32_t& lo) {
   const __half hx = __float2half_rn(x), hy = __float2half_rn(y);
@@ -303,9 +345,10 @@ __device__ __forceinline__ void tq_split(float x, float y, uint32_t& hi, uint32_
 // loads run along A's columns and B's columns and stores are 16 bytes.
 __global__ void __launch_bounds__(256) k_tc_split(const float2* A, int lda, long long sA, int m, const float2* B,
                                                   int ldb, long long sB, int n, int k, int nmt, int nnt, int nkc,
-                                                  uint32_t* ahi, uint32_t* alo, float* srow, uint32_t* bhi,
+                                                  const int* kexp, int kst, uint32_t* ahi, uint32_t* alo, float* srow, uint32_t* bhi,
                                                   uint32_t* blo, float* scol) {
   const int t = threadIdx.x, b = blockIdx.y;
+  kexp += (size_t)b * kst;
   if ((int)blockIdx.x < nmt) {
     __shared__ float smax[4][64], sup[64];
     const int mt = blockIdx.x, il = t & 63, part = t >> 6, i = mt * 64 + il;
@@ -315,7 +358,7 @@ __global__ void __launch_bounds__(256) k_tc_split(const float2* A, int lda, long
 #pragma unroll 4
       for (int l = part; l < k; l += 4) {
         const float2 v = Ab[(size_t)l * lda];
-        mx = fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y)));
+        mx = fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y)) * tq_bal(kexp, l));
       }
     }
     smax[part][il] = mx;
@@ -336,9 +379,12 @@ __global__ void __launch_bounds__(256) k_tc_split(const float2* A, int lda, long
       for (int q = 0; q < 4; ++q) {
         const int l = kc * TQ + 4 * part + q;
         float2 v = make_float2(0.0f, 0.0f);
-        if (i < m && l < k) v = Ab[(size_t)l * lda];
-        v.x *= up;
-        v.y *= up;
+        if (i < m && l < k) {
+          v = Ab[(size_t)l * lda];
+          const float bal = tq_bal(kexp, l);
+          v.x = v.x * bal * up;
+          v.y = v.y * bal * up;
+        }
         tq_split(v.x, -v.y, h0[q], l0[q]);
         tq_split(v.y, v.x, h1[q], l1[q]);
       }
@@ -358,7 +404,7 @@ __global__ void __launch_bounds__(256) k_tc_split(const float2* A, int lda, long
       if (j0 + c < n)
         for (int l = lane; l < k; l += 32) {
           const float2 v = Bb[(size_t)(j0 + c) * ldb + l];
-          mx = fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y)));
+          mx = fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y)) * tq_bal_inv(kexp, l));
         }
       mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx)));
       if (lane == 0) {
@@ -378,8 +424,13 @@ __global__ void __launch_bounds__(256) k_tc_split(const float2* A, int lda, long
       for (int q = 0; q < 4; ++q) {
         const int l = kc * TQ + 4 * g + q;
         float2 v = make_float2(0.0f, 0.0f);
-        if (j0 + jj < n && l < k) v = Bb[(size_t)(j0 + jj) * ldb + l];
-        tq_split(v.x * up, v.y * up, h[q], lo[q]);
+        if (j0 + jj < n && l < k) {
+          v = Bb[(size_t)(j0 + jj) * ldb + l];
+          const float bal = tq_bal_inv(kexp, l);
+          v.x = v.x * bal * up;
+          v.y = v.y * bal * up;
+        }
+        tq_split(v.x, v.y, h[q], lo[q]);
       }
       const size_t w = g0 + (size_t)kc * TQ_TW + ((jj >> 3) * (TQ / 4) + g) * 32 + (jj & 7) * 4;
       *reinterpret_cast<uint4*>(bhi + w) = make_uint4(h[0], h[1], h[2], h[3]);
@@ -542,7 +593,7 @@ __global__ void __launch_bounds__(128, NH == 1 ? 3 : 2) k_tc_cgemm_bulk(const ui
 #pragma unroll
         for (int q = 0; q < 32; ++q) {
           const int j = nt * BN + c0 + q;
-          if (j < n) atomicAdd(cr + 2 * ((size_t)j * ldc + i) + comp, -__uint_as_float(v[q]) * (sr * ssc[c0 + q]));
+          if (j < n) atomicAdd(cr + 2 * ((size_t)j * ldc + i) + comp, -__uint_as_float(v[q]) * ssc[c0 + q] * sr);
         }
       }
     }

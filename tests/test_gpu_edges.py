@@ -104,6 +104,73 @@ def test_mixed_solves_repeat_bitwise(harmonic):
     assert all((v == x[0]).all() for v in x[1:])
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 2, 1), (63, 127, 31), (65, 129, 33), (130, 300, 128), (200, 257, 300)])
+def test_binary16_split_of_factors_in_units(m, n, k):
+    """The factors of an LU with equations in units: index l carries 2^p_l in A
+    and 2^-p_l in B (p over +-40), so their products are of one size. Split and
+    sums as in the test above, top of the factors without the units (a power of
+    two per l moves between A and B, and the split's choice of it differs from
+    p by the spread of B's row maxima, 2^3 at most here)."""
+    rng = np.random.default_rng(m + n + k)
+    A, B = (rng.standard_normal(v) + 1j * rng.standard_normal(v) for v in ((m, k), (k, n)))
+    C = rng.standard_normal((m, n)) + 1j * rng.standard_normal((m, n))
+    top = np.abs(A).max() * np.abs(B).max()
+    u = 2.0 ** rng.integers(-40, 41, size=k)
+    A, B, C = (np.asfortranarray(v, dtype=np.complex64) for v in (A * u, B / u[:, None], C))
+    L = _abi.load()
+    L.mfbem_internal_tc_cgemm.argtypes = [ctypes.c_int32] * 3 + [ctypes.c_void_p] * 3 + [ctypes.c_int32]
+    G = C.copy(order="F")
+    _abi.check(L.mfbem_internal_tc_cgemm(m, n, k, A.ctypes.data, B.ctypes.data, G.ctypes.data, 0))
+    A, B, C, G = (v.astype(np.complex128) for v in (A, B, C, G))
+    S = (np.abs(A.real) + np.abs(A.imag)) @ (np.abs(B.real) + np.abs(B.imag))
+    tol = (3 * 2.0 ** -22 + 3 * -(-2 * k // 16) * 2.0 ** -22) * S + 8 * 4 * k * 2.0 ** -39 * top + \
+        2.0 ** -23 * (np.abs(C) + S)
+    assert (np.abs(G - (C - A @ B)) <= tol).all()
+
+
+def scaled_solution(A, b):
+    """x of A x = b: rows and columns scaled by powers of two to maxima near 1,
+    refined with residuals in extended precision (the equations mix units, and
+    a plain solution loses as many digits as they differ)."""
+    p2 = lambda v: 2.0 ** -np.frexp(v)[1].astype(float)
+    r = p2(np.abs(A).max(1))
+    c = p2(np.abs(A * r[:, None]).max(0))
+    S, sb = A * r[:, None] * c, b * r
+    inv = np.linalg.inv(S)
+    x = np.zeros(len(b), np.clongdouble)
+    for _ in range(6):
+        x = x + inv @ (sb - S.astype(np.clongdouble) @ x).astype(complex)
+    return x.astype(complex) * c
+
+
+@pytest.mark.parametrize("E", [1.0, 1e6, 8e10])
+@pytest.mark.parametrize("region", ["crack", "codes"])
+def test_mixed_sweep_of_sbie_and_hbie_rows_in_real_units(region, E):
+    """SBIE and HBIE rows of one region differ by the shear modulus: the mixed
+    sweep takes as many corrections in Pa as with a modulus of 1, and reaches
+    the system's solution to the bound of the mixed sweeps (1e-8)."""
+    if region == "crack":
+        d, crack = M.penny_crack_in_box(1.0, 2, 1, 2.0, 2)
+        R = BemRegion(d, crack=crack)
+    else:
+        d = M.cube_clamped_top_traction(4)
+        f = np.full(d.n_nodes, 2, dtype=np.int32)
+        f[d.nodes[:, 2] > 0.99] = 1
+        f[d.nodes[:, 1] < 0.01] = 3
+        f[d.nodes[:, 0] < 0.01] = 0
+        R = BemRegion(d, formulation=f)
+    mat = M.viscoelastic(E, 0.25, 1.0, 0.05)
+    om = [float(M.omega_from_a0(a, mat)) for a in (0.4, 0.9)]
+    X = R.sweep_harela(mat, om, precision="mixed")
+    st = R.last_stats
+    ref = [scaled_solution(*R.build_lse_harela(mat, w)) for w in om]
+    R.close()
+    # the counter is of all systems together, which go in step
+    assert st["refactorizations"] == 0 and st["gmres_iterations"] == 0 and st["refinement_iterations"] <= 3, st
+    for x, xr in zip(X, ref):
+        assert rel(x, xr) < 1e-8
+
+
 # 20, 56, 884 and 1154 nodes: 8 slices of a node's points, 3, and none (from 912)
 @pytest.mark.parametrize("n", [1, 2, 7, 8])
 def test_slices_of_a_nodes_points(oracle, n):
