@@ -99,6 +99,16 @@ __device__ __forceinline__ void oz_digits(double v, int e, int d[OZ_S]) {
   d[OZ_S - 1] = (int)R;
 }
 
+// 2^s, a normal number
+__device__ __forceinline__ double oz_pow2(int s) { return __hiloint2double((s + 1023) << 20, 0); }
+// v 2^s where 2^s need not be a number (|s| beyond 2040: zero or infinity):
+// two factors, so that the one rounding is that of a subnormal result
+__device__ __forceinline__ double oz_scale2(double v, int s) {
+  s = s < -2040 ? -2040 : (s > 2040 ? 2040 : s);
+  const int h = s >> 1;
+  return v * oz_pow2(h) * oz_pow2(s - h);
+}
+
 // bf16 pair (lo: d0 2^(-8p), hi: d1 2^(-8p)) as one word
 __device__ __forceinline__ uint32_t oz_pack(int d0, int d1, int p) {
   const float sc = __int_as_float((127 - 8 * p) << 23);  // 2^(-8p)
@@ -388,12 +398,13 @@ __global__ void __launch_bounds__(128, 1) k_oz_gemm(const uint32_t* At, const ui
           const long long i4 = (long long)__float2int_rn(__uint_as_float(v[4][q]) * 0x1p32f);
           const long long i5 = (long long)__float2int_rn(__uint_as_float(v[5][q]) * 0x1p42f);
           const long long V = (i0 << 42) + (i1 << 34) + (i2 << 26) + (i3 << 18) + (i4 << 10) + i5;
-          int s = er + sfc[c0 + q] - 56;
-          s = s < -1022 ? -1022 : (s > 1023 ? 1023 : s);
-          const double scale = __hiloint2double((s + 1023) << 20, 0);
+          const int s = er + sfc[c0 + q] - 56;
+          double r = (double)V;
+          if (s >= -1022 && s <= 1023) r *= oz_pow2(s);
+          else r = oz_scale2(r, s);  // operands near the ends of the exponent range
           const int j = nt * OZ_BN + c0 + q;
           // a reduction at the L2: no wait for C; one addition per entry and update
-          if (j < n) atomicAdd(Cb + (size_t)j * ldc + row, -((double)V * scale));
+          if (j < n) atomicAdd(Cb + (size_t)j * ldc + row, -r);
         }
       }
     }

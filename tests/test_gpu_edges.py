@@ -43,6 +43,23 @@ def test_lu_and_solve(n, cplx):
     assert (np.abs(A @ x - b) <= 3 * n * u * (size @ np.abs(x)).max(0)).all()
 
 
+@pytest.mark.parametrize("cplx", [False, True], ids=["real", "complex"])
+@pytest.mark.parametrize("e", [-980, 900])
+def test_solve_of_tiny_and_huge_entries(e, cplx):
+    """A and b times 2^e, large enough for updates on the tensor cores: the
+    backward error of the solve as above (subnormal parts of an entry are 2^-90
+    of the largest)."""
+    n, s = 1100, 2.0 ** e
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((n, n)) + (1j * rng.standard_normal((n, n)) if cplx else 0)
+    b = rng.standard_normal((n, 2)) + (1j * rng.standard_normal((n, 2)) if cplx else 0)
+    F, x = np.array(A * s, order="F", copy=True), np.array(b * s, order="F", copy=True)
+    solve_lse(F, x)
+    size = np.abs(np.tril(F, -1) + np.eye(n)) @ np.abs(np.triu(F) / s)
+    u = (4 if cplx else 2) * EPS
+    assert (np.abs(A @ x - b) <= 3 * n * u * (size @ np.abs(x)).max(0)).all()
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 1, 1), (63, 127, 15), (65, 129, 17), (130, 257, 33), (200, 300, 128)])
 def test_binary16_split_of_uneven_rows_and_columns(m, n, k):
     """Rows of A and columns of B scaled over 2^+-20, one row and one column

@@ -120,3 +120,21 @@ def test_zero_rows_columns_and_wide_exponent_range():
     bound = 2.0 ** -50 * (np.abs(C) + 2 * k * np.outer(ra, cb))
     for g, e in zip((Cg.real, Cg.imag), ex):
         assert np.all(np.abs(g.astype(np.longdouble) - e) <= bound)
+
+
+@pytest.mark.parametrize("cplx", [True, False], ids=["complex", "real"])
+@pytest.mark.parametrize("ea,eb", [(-300, -300), (-480, -486), (-500, -490), (0, -990), (500, 490)])
+def test_scales_to_the_ends_of_the_exponent_range(ea, eb, cplx):
+    """A 2^ea and B 2^eb with C 2^(ea + eb): the same update, to the bit where
+    the result's last place is above the smallest subnormal number."""
+    rng = np.random.default_rng(5)
+    m, n, k = 130, 85, 40
+    A = np.asfortranarray(_mat(rng, m, k, cplx, 0))
+    B = np.asfortranarray(_mat(rng, k, n, cplx, 0))
+    C = np.asfortranarray(_mat(rng, m, n, cplx, 0))
+    G = _run(A, B, C, 0)
+    s = 2.0 ** (ea + eb)
+    H = _run(A * 2.0 ** ea, B * 2.0 ** eb, C * s, 0)
+    for g, h in ((G.real, H.real), (G.imag, H.imag)):
+        on = np.abs(g) > 2.0 ** -8
+        assert np.array_equal((g * s)[on], h[on]) and np.abs(g * s - h).max() <= 2.0 ** -60 * s
