@@ -21,11 +21,12 @@
 // level t holds it exactly; levels 5..6 (13 products, 2^-40 and smaller) share
 // a sixth accumulator, whose FP32 accumulation (rounded or truncated by the
 // tensor core) stays near 2^-53 of the result. The epilogue rebuilds the
-// exact integer sum of levels 0..4 in int64 in units of 2^-42 (below 2^63), adds
-// the tail rounded to that unit, converts it once to binary64, scales it by
-// 2^(e_r + f_j - 56) and subtracts it from C by a reduction at the L2 (two
-// binary64 operations per output, at two lanes per cycle and SM, and no wait
-// for C; four and a wait before).
+// exact integer sum of levels 0..4 in int64 (below 2^53 in units of 2^-32),
+// converts it to binary64, adds the tail with one FMA that applies the scale
+// 2^(e_r + f_j - 14) too, and subtracts the result from C by a reduction at the
+// L2: two binary64 operations per output (at two lanes per cycle and SM) and no
+// wait for C. The scaled tail is put together from the bits of the FP32 one; the
+// FMA rounds sum + tail once, as the scale is a power of two.
 //
 // Complex: C~ (2m x n real) -= A~ (2m x 2k) B~ (2k x n) with A~ realified in
 // 2 x 2 blocks [[re, -im], [im, re]] and B~, C~ the complex arrays viewed as
@@ -387,21 +388,23 @@ __global__ void __launch_bounds__(128, 1) k_oz_gemm(const uint32_t* At, const ui
       if (live) {
 #pragma unroll
         for (int q = 0; q < 16; ++q) {
-          // exact integer sum of levels 0..4 in units of 2^-32 (|V| < 2^53), then
-          // of 2^-42 (|V| < 2^63) with the tail rounded to that unit -- 2^-45 rms
-          // against 2^-42 and more of the levels left out -- and one conversion
-          // and one multiplication of binary64 instead of two and two
+          // exact integer sum of levels 0..4 in units of 2^-32 (|V| < 2^53)
           const long long i0 = (long long)__float2int_rn(__uint_as_float(v[0][q]));
           const long long i1 = (long long)__float2int_rn(__uint_as_float(v[1][q]) * 0x1p8f);
           const long long i2 = (long long)__float2int_rn(__uint_as_float(v[2][q]) * 0x1p16f);
           const long long i3 = (long long)__float2int_rn(__uint_as_float(v[3][q]) * 0x1p24f);
           const long long i4 = (long long)__float2int_rn(__uint_as_float(v[4][q]) * 0x1p32f);
-          const long long i5 = (long long)__float2int_rn(__uint_as_float(v[5][q]) * 0x1p42f);
-          const long long V = (i0 << 42) + (i1 << 34) + (i2 << 26) + (i3 << 18) + (i4 << 10) + i5;
-          const int s = er + sfc[c0 + q] - 56;
-          double r = (double)V;
-          if (s >= -1022 && s <= 1023) r *= oz_pow2(s);
-          else r = oz_scale2(r, s);  // operands near the ends of the exponent range
+          const long long V = (i0 << 32) + (i1 << 24) + (i2 << 16) + (i3 << 8) + i4;
+          const int s = er + sfc[c0 + q] - 14;
+          double r;
+          if (s >= -960 && s <= 1000) {
+            // the tail is a multiple of 2^-48 (its products are) or zero
+            const uint32_t te = (v[5][q] >> 23) & 255;
+            const int hi = (int)((v[5][q] & 0x80000000u) | ((te + (uint32_t)(s + 896)) << 20) | ((v[5][q] >> 3) & 0xFFFFFu));
+            r = fma((double)V, oz_pow2(s - 32), te ? __hiloint2double(hi, (int)(v[5][q] << 29)) : 0.0);
+          } else {  // operands near the ends of the exponent range
+            r = oz_scale2(fma((double)V, 0x1p-32, (double)__uint_as_float(v[5][q])), s);
+          }
           const int j = nt * OZ_BN + c0 + q;
           // a reduction at the L2: no wait for C; one addition per entry and update
           if (j < n) atomicAdd(Cb + (size_t)j * ldc + row, -r);

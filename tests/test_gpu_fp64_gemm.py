@@ -138,3 +138,13 @@ def test_scales_to_the_ends_of_the_exponent_range(ea, eb, cplx):
     for g, h in ((G.real, H.real), (G.imag, H.imag)):
         on = np.abs(g) > 2.0 ** -8
         assert np.array_equal((g * s)[on], h[on]) and np.abs(g * s - h).max() <= 2.0 ** -60 * s
+
+
+def test_tail_levels_keep_their_bits():
+    """A product whose only bit below 2^-52 of the row and column scales is one
+    of the last level's: exact in the FP32 tail, so the update is exact."""
+    A = np.array([[1.0, 2.0 ** -5], [1.0, -(2.0 ** -5)]], order="F")
+    B = np.array([[0.0, 0.0], [1.0 + 2.0 ** -52, 1.0 + 2.0 ** -51]], order="F")
+    C = np.array([[1.0, 1.0], [-1.0, -1.0]], order="F") * 2.0 ** -5
+    exact = np.array([[-1.0, -2.0], [1.0, 2.0]]) * 2.0 ** -57
+    assert np.array_equal(_run(A, B, C, 0), exact)
