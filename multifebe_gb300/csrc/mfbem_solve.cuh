@@ -1331,9 +1331,16 @@ static int refine_classical(MixCtx<SD, SF>& c, int* conv) {
 }
 
 // GMRES-IR: up to 10 outer corrections, each a GMRES(m) solve of
-// M^-1 A d = M^-1 r to 1e-6 relative (preconditioned residual).
+// M^-1 A d = M^-1 r to 1e-6 relative (preconditioned residual). It stops on the
+// backward error alone, unless a classical stage has failed before (stalled):
+// the normwise backward error says nothing about the rows of a region whose
+// equations differ in size (SBIE and HBIE rows by the shear modulus), where an x
+// that has diverged passes it. M^-1 r then has to be small against x too: down
+// to kFwdTol, or no longer falling by 4 and below kFwdDiv, the floor of an
+// ill-conditioned system (cond eps) staying admissible up to there.
+constexpr double kFwdDiv = 1e-2;
 template <typename SD, typename SF>
-static int refine_gmres(MixCtx<SD, SF>& c, int* conv) {
+static int refine_gmres(MixCtx<SD, SF>& c, int* conv, bool stalled = false) {
   typedef std::complex<double> C;
   cudaStream_t st = c.h->st;
   const int n = c.n, batch = c.batch, m = 20;
@@ -1360,14 +1367,36 @@ static int refine_gmres(MixCtx<SD, SF>& c, int* conv) {
     else return v.real();
   };
   *conv = 0;
-  c.dx.assign(batch, 0.0);  // GMRES-IR stops on the backward error alone
+  c.dx.assign(batch, 0.0);
+  std::vector<int> acc(batch, 0);
+  std::vector<double> fwd(batch, HUGE_VAL);
+  // stalled: acc[b] = system b is accepted (w: M^-1 r); active = the others
+  auto accept = [&](bool last) -> int {
+    k_vecmax<SD><<<batch, 256, 0, st>>>(w, n, n, c.nrm, 5, 8); ++g_launches;
+    k_vecmax<SD><<<batch, 256, 0, st>>>(c.x, n, n, c.nrm, 6, 8); ++g_launches;
+    std::vector<double> hn(8 * (size_t)batch);
+    CK(cudaMemcpyAsync(hn.data(), c.nrm, sizeof(double) * 8 * batch, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    std::vector<int> hact(batch);
+    for (int bi = 0; bi < batch; ++bi) {
+      const double f = hn[8 * bi + 5] / hn[8 * bi + 6];
+      acc[bi] = c.be[bi] <= c.tol && (f <= kFwdTol || (f <= kFwdDiv && (last || f > 0.25 * fwd[bi])));
+      fwd[bi] = f;
+      hact[bi] = !acc[bi];
+    }
+    CK(cudaMemcpyAsync(c.active, hact.data(), sizeof(int) * batch, cudaMemcpyHostToDevice, st));
+    CK(cudaStreamSynchronize(st));
+    *conv = std::all_of(acc.begin(), acc.end(), [](int a) { return a != 0; });
+    return 0;
+  };
   for (int outer = 0; outer < 10; ++outer) {
     bool all;
     if ((rc = residual_check(c, c.fresh, &all))) return rc;
-    if (all) { *conv = 1; return 0; }
-    ++c.it;
+    if (all && !stalled) { *conv = 1; return 0; }
     // z = M^-1 r -> V_0 = z / beta
     if ((rc = precond(c, c.r, w))) return rc;
+    if (stalled && ((rc = accept(false)) || *conv)) return rc;
+    ++c.it;
     k_bdot<SD><<<dim3(1, batch), 256, 0, st>>>(w, n, 1, w, n, n, hc, m + 1); ++g_launches;
     CK(cudaMemcpyAsync(hh.data(), hc, cbytes, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
@@ -1378,7 +1407,7 @@ static int refine_gmres(MixCtx<SD, SF>& c, int* conv) {
     std::vector<std::vector<C>> sn(batch, std::vector<C>(m));
     for (int bi = 0; bi < batch; ++bi) {
       beta[bi] = std::sqrt(std::max(0.0, toC(hh[(size_t)(m + 1) * bi]).real()));
-      done[bi] = !(c.be[bi] > c.tol) || beta[bi] == 0.0;
+      done[bi] = (stalled ? acc[bi] != 0 : !(c.be[bi] > c.tol)) || beta[bi] == 0.0;
       hs[bi] = beta[bi] > 0.0 ? 1.0 / beta[bi] : 0.0;
       g[bi][0] = beta[bi];
     }
@@ -1459,6 +1488,7 @@ static int refine_gmres(MixCtx<SD, SF>& c, int* conv) {
   }
   bool all;
   if ((rc = residual_check(c, false, &all))) return rc;
+  if (stalled) return (rc = precond(c, c.r, w)) ? rc : accept(true);
   *conv = all ? 1 : 0;
   return 0;
 }
@@ -1610,7 +1640,9 @@ static int solve_batch(mfbem_handle* h, SD* A, int n, int batch, const SD* b, SD
         if ((rc = refine_classical(c, &conv))) return rc;
       }
       if (!conv) {
-        if ((rc = refine_gmres(c, &conv))) return rc;
+        // a correction as large as x: x has diverged and is not worth starting from
+        const bool diverged = std::any_of(c.dxraw.begin(), c.dxraw.end(), [](double d) { return !(d <= 0.25); });
+        if ((diverged && (rc = restart())) || (rc = refine_gmres(c, &conv, true))) return rc;
       }
     }
     cudaEventRecord(e2, st);

@@ -5,7 +5,7 @@ import ctypes
 import numpy as np
 import pytest
 
-from multifebe_gb300 import BemRegion, _abi, solve_lse
+from multifebe_gb300 import BemRegion, MfbemError, _abi, solve_lse
 from multifebe_gb300 import meshgen as M
 
 pytestmark = pytest.mark.gpu
@@ -186,6 +186,32 @@ def test_mixed_sweep_of_sbie_and_hbie_rows_in_real_units(region, E):
     assert st["refactorizations"] == 0 and st["gmres_iterations"] == 0 and st["refinement_iterations"] <= 3, st
     for x, xr in zip(X, ref):
         assert rel(x, xr) < 1e-8
+
+
+@pytest.mark.parametrize("E", [1e6, 1e9, 8e10])
+@pytest.mark.parametrize("region", ["codes", "halves"])
+def test_refinement_accepts_no_diverged_solution(region, E, monkeypatch):
+    """FP32 factors with partial pivoting of SBIE / HBIE rows in Pa are no good
+    preconditioner: whatever the refinement returns is a solution (its estimate
+    of the error is below 1e-2, and a diverged x is off by its own size)."""
+    monkeypatch.setenv("MFBEM_PIVOT", "partial")
+    d = M.cube_clamped_top_traction(4)
+    f = np.full(d.n_nodes, 2, dtype=np.int32)
+    f[d.nodes[:, 2] > 0.99] = 1
+    f[d.nodes[:, 1] < 0.01] = 3
+    f[d.nodes[:, 0] < 0.01] = 0
+    if region == "halves":
+        f = (d.nodes[:, 0] > 0.4).astype(np.int32)
+    R = BemRegion(d, formulation=f)
+    mat = M.viscoelastic(E, 0.25, 1.0, 0.05)
+    om = float(M.omega_from_a0(0.7, mat))
+    ref = scaled_solution(*R.build_lse_harela(mat, om))
+    try:
+        x = R.sweep_harela(mat, [om], precision="mixed")[0]
+    except MfbemError:
+        x = None
+    R.close()
+    assert x is None or rel(x, ref) < 0.1
 
 
 # 20, 56, 884 and 1154 nodes: 8 slices of a node's points, 3, and none (from 912)
