@@ -25,6 +25,66 @@
 
 namespace mfb {
 
+// ---------------------------------------------------------------------------
+// Conjugate-transposed triangular solves with the LU factors, U^H forward
+// (lower, non-unit) and L^H backward (upper, unit), block by block: two launches
+// per 64 rows, for MFBEM_TRSV=blocked (no CTA waits for another).
+// ---------------------------------------------------------------------------
+template <typename S, bool LH>
+__global__ void __launch_bounds__(128) k_trsv_diag64_h(const S* A, long long strideA, int lda, S* b,
+                                                       long long strideb, int r0, int w) {
+  const S* M = A + strideA * blockIdx.x;
+  S* xg = b + strideb * blockIdx.x;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  S* D = reinterpret_cast<S*>(smraw);  // D[col * 65 + row] = A(r0 + row, r0 + col)
+  stage_diag64(M, lda, r0, w, D);
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  const int l = threadIdx.x;
+  S x0 = l < w ? xg[r0 + l] : Sc<S>::zero();
+  S x1 = l + 32 < w ? xg[r0 + l + 32] : Sc<S>::zero();
+  if (!LH) {
+    // x_j /= conj(U_jj); x_i -= conj(U_ji) x_j for i > j (U_ji = D[i * 65 + j])
+    for (int j = 0; j < w; ++j) {
+      if (j < 32) { if (l == j) x0 = Sc<S>::div(x0, Sc<S>::conj(D[j * 65 + j])); }
+      else { if (l + 32 == j) x1 = Sc<S>::div(x1, Sc<S>::conj(D[j * 65 + j])); }
+      const S xj = shfl_s(j < 32 ? x0 : x1, j & 31);
+      if (l > j && l < w) x0 = Sc<S>::sub(x0, Sc<S>::mul(Sc<S>::conj(D[l * 65 + j]), xj));
+      if (l + 32 > j && l + 32 < w) x1 = Sc<S>::sub(x1, Sc<S>::mul(Sc<S>::conj(D[(l + 32) * 65 + j]), xj));
+    }
+  } else {
+    // unit diagonal; x_i -= conj(L_ji) x_j for i < j
+    for (int j = w - 1; j >= 0; --j) {
+      const S xj = shfl_s(j < 32 ? x0 : x1, j & 31);
+      if (l < j) x0 = Sc<S>::sub(x0, Sc<S>::mul(Sc<S>::conj(D[l * 65 + j]), xj));
+      if (l + 32 < j) x1 = Sc<S>::sub(x1, Sc<S>::mul(Sc<S>::conj(D[(l + 32) * 65 + j]), xj));
+    }
+  }
+  if (l < w) xg[r0 + l] = x0;
+  if (l + 32 < w) xg[r0 + l + 32] = x1;
+}
+
+// rows [i0, i1): x_i -= sum_j conj(A(r0 + j, i)) x_{r0 + j}; one warp per row,
+// reading column i's block rows contiguously
+template <typename S>
+__global__ void k_trsv_update_h(const S* A, long long strideA, int lda, S* b, long long strideb, int r0, int w,
+                                int i0, int i1) {
+  const S* M = A + strideA * blockIdx.y;
+  S* x = b + strideb * blockIdx.y;
+  __shared__ S xs[64];
+  if ((int)threadIdx.x < w) xs[threadIdx.x] = x[r0 + threadIdx.x];
+  __syncthreads();
+  const int l = threadIdx.x & 31;
+  const int i = i0 + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (i >= i1) return;
+  const S* col = M + (size_t)i * lda + r0;
+  S acc = Sc<S>::zero();
+  if (l < w) acc = Sc<S>::mul(Sc<S>::conj(col[l]), xs[l]);
+  if (l + 32 < w) acc = Sc<S>::add(acc, Sc<S>::mul(Sc<S>::conj(col[l + 32]), xs[l + 32]));
+  for (int o = 16; o > 0; o >>= 1) acc = Sc<S>::add(acc, shfl_s(acc, l ^ o));
+  if (l == 0) x[i] = Sc<S>::sub(x[i], acc);
+}
+
 // inverse of the getrs row permutation: out[perm[i]] = x[i]
 template <typename S>
 __global__ void k_scatter_perm(const S* x, long long sx, const int* perm, int n, S* out) {
@@ -50,10 +110,40 @@ __global__ void k_rhs_swap_rev(S* b, long long sb, int n, const int* ipiv, long 
   }
 }
 
+// block by block (MFBEM_TRSV=blocked)
+template <typename S>
+static int trsv_blocked(cudaStream_t st, const S* A, int lda, int n, S* b, long long sb, int batch, int op) {
+  const int TB = 64, last = ((n - 1) / TB) * TB;
+  const size_t dsm = (size_t)TB * 65 * sizeof(S);
+  const void* kd = op == TR_L ? (const void*)k_trsv_diag64<S, true>
+                   : op == TR_U ? (const void*)k_trsv_diag64<S, false>
+                   : op == TR_UH ? (const void*)k_trsv_diag64_h<S, false> : (const void*)k_trsv_diag64_h<S, true>;
+  if (raise_smem_limit(kd)) return fail(MFBEM_ECUDA, "shared-memory limit of the triangular solve");
+  const bool fwd = op == TR_L || op == TR_UH;
+  for (int k = 0; k < n; k += TB) {
+    const int r0 = fwd ? k : last - k, w = std::min(TB, n - r0);
+    const int i0 = fwd ? r0 + w : 0, i1 = fwd ? n : r0;
+    switch (op) {
+      case TR_L: k_trsv_diag64<S, true><<<batch, 128, dsm, st>>>(A, 0, lda, b, sb, r0, w); break;
+      case TR_U: k_trsv_diag64<S, false><<<batch, 128, dsm, st>>>(A, 0, lda, b, sb, r0, w); break;
+      case TR_UH: k_trsv_diag64_h<S, false><<<batch, 128, dsm, st>>>(A, 0, lda, b, sb, r0, w); break;
+      default: k_trsv_diag64_h<S, true><<<batch, 128, dsm, st>>>(A, 0, lda, b, sb, r0, w); break;
+    }
+    ++g_launches;
+    if (i1 > i0) {
+      if (op <= TR_U) k_trsv_update<S><<<dim3(nblk(i1 - i0, 256), batch), 256, 0, st>>>(A, 0, lda, b, sb, r0, w, i0, i1);
+      else k_trsv_update_h<S><<<dim3(nblk(i1 - i0, 8), batch), 256, 0, st>>>(A, 0, lda, b, sb, r0, w, i0, i1);
+      ++g_launches;
+    }
+  }
+  CK(cudaGetLastError());
+  return 0;
+}
 // one triangular solve with the factors in A (no permutation), batch
 // right-hand sides of one matrix
 template <typename S>
 static int trsv_op(cudaStream_t st, const S* A, int lda, int n, S* b, long long sb, int batch, int op) {
+  if (!trsv_sync_free()) return trsv_blocked<S>(st, A, lda, n, b, sb, batch, op);
   switch (op) {
     case TR_L: return trsv_sf_run<S, TR_L>(st, A, 0, lda, n, b, sb, batch);
     case TR_U: return trsv_sf_run<S, TR_U>(st, A, 0, lda, n, b, sb, batch);

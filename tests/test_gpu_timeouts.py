@@ -16,7 +16,7 @@ import numpy as np
 import pytest
 import scipy.linalg as sl
 
-from multifebe_gb300 import _abi, meshgen as M, BemRegion, solve_lse, MfbemError
+from multifebe_gb300 import _abi, meshgen as M, BemRegion, solve_lse, LseState, MfbemError
 
 pytestmark = pytest.mark.gpu
 
@@ -121,3 +121,27 @@ def test_mixed_sweep_reports_the_timeout_then_recovers(short_waits, oracle):
         xo = oracle.lu_solve(Ao, bo)
         assert np.abs(X[i] - xo).max() / np.abs(xo).max() < 1e-8
     R.close()
+
+
+@pytest.mark.parametrize("cplx", [False, True], ids=["real", "complex"])
+def test_blocked_triangular_solves_wait_for_nothing(short_waits, monkeypatch, cplx):
+    """MFBEM_TRSV=blocked: every triangular solve of a call with all options
+    (conjugate-transposed ones of the norm estimates too) runs launch by launch,
+    so that no limit on waits touches it; same results as by the waiting form to
+    the tolerances of test_gpu_lse.py."""
+    rng = np.random.default_rng(4)
+    n = 300
+    A = rng.standard_normal((n, n)) + (1j * rng.standard_normal((n, n)) if cplx else 0)
+    b = rng.standard_normal((n, 2)) + (1j * rng.standard_normal((n, 2)) if cplx else 0)
+    out = []
+    for blocked in (False, True):
+        if blocked:
+            monkeypatch.setenv("MFBEM_TRSV", "blocked")
+            short_waits.mfbem_internal_set_spin_limit(1)
+        st, x = LseState(), np.array(b, order="F")
+        solve_lse(np.array(A, order="F"), x, scaling=True, condition=True, refine=True, state=st)
+        out.append((x, st))
+    (x0, s0), (x1, s1) = out
+    assert np.abs(x1 - x0).max() <= 20 * 2.0 ** -53 / s0.rcond * np.abs(x0).max()
+    assert abs(s1.rcond / s0.rcond - 1) < 1e-8
+    assert np.all(np.abs(np.log(s1.ferr / s0.ferr)) < np.log(4.0)) and np.all(s1.berr <= 4 * 2.0 ** -53)
