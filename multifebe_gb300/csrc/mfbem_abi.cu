@@ -116,10 +116,10 @@ struct mfbem_handle {
   bool ms_built[2] = {false, false};
   long long mb_pts[3] = {0, 0, 0}, ms_pts[2][3] = {{0, 0, 0}, {0, 0, 0}};
   DevBuf parh;  // HarParH per frequency of the last harmonic assembly
-  // radial tables of the last harmonic call and a bound of the distance
-  // between any two points of the mesh's elements
-  DevBuf rad;
-  DevBuf slc;  // copies of the system for the pair kernels' slices
+  // work space of the assembly that a call can do without: radial tables,
+  // copies of the system for the pair kernels' slices
+  DevBuf rad, slc;
+  // bound of the distance between any two points of the mesh's elements
   double rmax = 0.0;
   double box_lo[3] = {0, 0, 0}, box_hi[3] = {0, 0, 0};  // box that holds every element
   // work buffers of the internal points, in the order of their use (grown as
@@ -280,11 +280,28 @@ static int ensure(DevBuf& b, size_t bytes) {
   b.dev = dev;
   return 0;
 }
-// ensure() for work space that a call can do without: false if there is no memory for it
+// ensure() for work space that a call can do without: false if there is no
+// memory for it. Taken after the buffers that the call needs, as far as these are
+// known, and handed to idle() once used.
 static bool try_ensure(DevBuf& b, size_t bytes) {
+  const std::string msg = g_err;
   if (!ensure(b, bytes)) return true;
   cudaGetLastError();
+  g_err = msg;
   return false;
+}
+// b is not used any more and its work has been waited for: its memory goes to
+// the cache of idle buffers, from where the next call takes it and any
+// allocation that finds no memory drops it. Small buffers, and those the cache
+// has no room for, stay.
+static void idle(DevBuf& b) {
+  if (b.bytes < (1u << 20)) return;
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  auto cap = g_pool_cap.find(b.dev);
+  if (cap == g_pool_cap.end() || g_pool_bytes[b.dev] + b.bytes > (size_t)cap->second) return;
+  g_pool.emplace(b.bytes, std::make_pair(b.dev, b.p));
+  g_pool_bytes[b.dev] += b.bytes;
+  b = DevBuf();
 }
 // calls on a handle run on the device it was uploaded on
 static int check_dev(const mfbem_handle* h) {
@@ -1336,6 +1353,8 @@ static int assemble_common(mfbem_handle* h, const POL& pol, const double* nu_hos
     CK(cudaMemcpyAsync(b, db, n * es, cudaMemcpyDeviceToHost, h->st));
   }
   rc = check_err(h);
+  idle(h->rad);
+  idle(h->slc);
   float ms = 0;
   cudaEventElapsedTime(&ms, e0, e1);
   cudaEventDestroy(e0);
@@ -1385,6 +1404,8 @@ extern "C" int mfbem_assemble_harela(mfbem_handle* h, const double lambda[2], co
   CK(cudaMemcpyAsync(dq, q, sizeof(q), cudaMemcpyHostToDevice, h->st));
   k_harpar<<<1, 32, 0, h->st>>>(dq, 1, (HarParD*)h->par.p, zexp_thresholds()); ++g_launches;
   if ((rc = bm_prepare(h, 1))) return rc;
+  const size_t n = h->ndof;
+  if (!(flags & MFBEM_DEVICE_PTRS) && ((rc = ensure(h->A, 16 * n * n)) || (rc = ensure(h->b, 16 * n)))) return rc;
   PolHarmonicRad pr;
   pr.p = (const HarParD*)h->par.p;
   if ((rc = hbie_params(h, dq, 1, &pr.ph)) || (rc = radial_prepare(h, h->rmax, q, 1, pr.p, pr.ph, false, &pr.t))) return rc;

@@ -1716,14 +1716,6 @@ extern "C" int mfbem_sweep_harela(mfbem_handle* h, const double lambda[2], const
   CK(cudaMemsetAsync(A, 0, sizeof(double2) * nn * n_freq, h->st));
   CK(cudaMemsetAsync(b, 0, sizeof(double2) * (size_t)n * n_freq, h->st));
   if ((rc = bm_prepare(h, 1))) return rc;
-  PolHarmonicRad pr;
-  pr.p = dpar;
-  if ((rc = hbie_params(h, dq, n_freq, &pr.ph)) ||
-      (rc = radial_prepare(h, h->rmax, q.data(), n_freq, dpar, pr.ph, precision >= 1, &pr.t)))
-    return rc;
-  PolHarmonic pol;
-  pol.p = dpar;
-  pol.ph = pr.ph;
   AsmTimes tm;
   long long l0 = g_launches;
   const HarParF* pf = nullptr;
@@ -1755,6 +1747,14 @@ extern "C" int mfbem_sweep_harela(mfbem_handle* h, const double lambda[2], const
     pf = (const HarParF*)h->parf.p;
     dsf = (const ff*)h->pphi_f.p;
   }
+  PolHarmonicRad pr;
+  pr.p = dpar;
+  if ((rc = hbie_params(h, dq, n_freq, &pr.ph)) ||
+      (rc = radial_prepare(h, h->rmax, q.data(), n_freq, dpar, pr.ph, precision >= 1, &pr.t)))
+    return rc;
+  PolHarmonic pol;
+  pol.p = dpar;
+  pol.ph = pr.ph;
   rc = pr.t.n > 0 ? launch_assembly(h, pr, dnu, n_freq, (double*)A, n, 2 * nn, (double*)b, 2 * (size_t)n, &tm, pf, dsf,
                                     precision >= 1, sgf, lgf)
                   : launch_assembly(h, pol, dnu, n_freq, (double*)A, n, 2 * nn, (double*)b, 2 * (size_t)n, &tm, pf, dsf,
@@ -1762,6 +1762,8 @@ extern "C" int mfbem_sweep_harela(mfbem_handle* h, const double lambda[2], const
   if (rc) return rc;
   cudaEventRecord(a1, h->st);
   if ((rc = check_err(h))) return rc;
+  idle(h->rad);
+  idle(h->slc);
   float ams = 0;
   cudaEventElapsedTime(&ams, a0, a1);
   cudaEventDestroy(a0);
@@ -1815,6 +1817,7 @@ extern "C" int mfbem_solve_staela(mfbem_handle* h, double mu, double nu, int32_t
   long long l0 = g_launches;
   if ((rc = launch_assembly(h, pol, (const double*)h->nu.p, 1, A, n, 0, b, 0, &tm))) return rc;
   if ((rc = check_err(h))) return rc;
+  idle(h->slc);
   tm.read(&s);
   rc = solve_batch<double, float>(h, A, n, 1, b, x, precision, rel_tol, &s);
   s.kernel_launches = g_launches - l0;

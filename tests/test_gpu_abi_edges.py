@@ -13,6 +13,13 @@ from multifebe_gb300 import BemRegion, MfbemError, meshgen as M, _abi
 pytestmark = pytest.mark.gpu
 
 
+def _dll(name):
+    try:
+        return ctypes.CDLL(name)
+    except OSError:
+        return None
+
+
 def _harela_args(mat):
     lam = np.array([complex(mat["lambda"]).real, complex(mat["lambda"]).imag])
     mu = np.array([complex(mat["mu"]).real, complex(mat["mu"]).imag])
@@ -147,3 +154,39 @@ def test_released_device_memory_is_reused_safely():
     X = R.sweep_harela(mat, M.omega_from_a0(np.linspace(0.2, 1.6, 4), mat), precision="mixed")
     R.close()
     assert np.abs(X - first[3]).max() <= 1e-12 * np.abs(first[3]).max()
+
+
+def test_optional_work_space_gives_way_to_what_a_call_needs():
+    """With 200 MB of device memory left a mixed sweep of 2220 unknowns still gets
+    the 290 MB that it needs: the slices' copies of an earlier call (two systems
+    and more, 176 MB) are dropped for them. A call that succeeds leaves no message."""
+    rt = next(v for v in (_dll(n) for n in ("libcudart.so.13", "libcudart.so")) if v)
+    rt.cudaMalloc.argtypes = [ctypes.POINTER(ctypes.c_void_p), ctypes.c_size_t]
+    rt.cudaFree.argtypes = [ctypes.c_void_p]
+    L = _abi.load()
+    L.mfbem_last_error.restype = ctypes.c_char_p
+    mat = M.viscoelastic(1.0, 0.25, 1.0, 0.05)
+    om = [float(M.omega_from_a0(0.7, mat))]
+    assert L.mfbem_trim_device_cache() == 0
+    R = BemRegion(M.cube_clamped_top_traction(6))
+    xp = R.sweep_harela(mat, om, precision="plain")[0]
+    held = []
+    try:
+        fr, tot = ctypes.c_size_t(), ctypes.c_size_t()
+        step = 1 << 40
+        while step >= 8 << 20:
+            assert rt.cudaMemGetInfo(ctypes.byref(fr), ctypes.byref(tot)) == 0
+            size = min(step, fr.value - (200 << 20))
+            p = ctypes.c_void_p()
+            if size >= 8 << 20 and rt.cudaMalloc(ctypes.byref(p), size) == 0:
+                held.append(p)
+            else:
+                rt.cudaGetLastError()
+                step = min(step, fr.value) // 2
+        xm = R.sweep_harela(mat, om, precision="mixed")[0]
+        msg = L.mfbem_last_error()
+    finally:
+        for p in held:
+            rt.cudaFree(p)
+    R.close()
+    assert np.abs(xm - xp).max() <= 1e-9 * np.abs(xp).max() and msg == b""
