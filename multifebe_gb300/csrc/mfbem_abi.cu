@@ -1419,11 +1419,17 @@ extern "C" int mfbem_assemble_harela(mfbem_handle* h, const double lambda[2], co
 // ---------------------------------------------------------------------------
 // Internal points (calculate_internal_points_mechanics_bem_{staela,harela})
 // ---------------------------------------------------------------------------
-// work buffers of one call: the handle's ip_ws in order of use
+// work buffers of one call: the handle's ip_ws in order of use (they grow with
+// points x elements, so large ones go back to the cache after the call)
 struct TmpBufs {
   mfbem_handle* h;
   size_t used = 0;
   explicit TmpBufs(mfbem_handle* h_) : h(h_) {}
+  ~TmpBufs() {
+    cudaStreamSynchronize(h->st);
+    for (DevBuf& b : h->ip_ws) idle(b);
+    idle(h->rad);
+  }
   int get(void** p, size_t bytes) {
     if (used == h->ip_ws.size()) h->ip_ws.emplace_back();
     DevBuf& b = h->ip_ws[used++];

@@ -7,6 +7,8 @@ Tolerances (max-norm relative to the largest value): displacement and stress
 <= 1e-11 against the oracle (FP64 on both sides; FMA contraction and the
 device's transcendental functions); <= 1e-9 where quasi-singular subdivision
 dominates (thin slab)."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -14,6 +16,13 @@ from multifebe_gb300 import MfbemError, BemRegion, meshgen as M, _abi
 from test_oracle_kat import INTERIOR, _p_wave_column
 
 pytestmark = pytest.mark.gpu
+
+
+def _loads(name):
+    try:
+        return bool(ctypes.CDLL(name))
+    except OSError:
+        return False
 
 
 def rel(a, b):
@@ -88,3 +97,27 @@ def test_internal_points_at_nodes_and_on_elements():
         R.internal_points(np.vstack([INTERIOR[:1], xm[None, :]]), u, t, mu=mat["mu"], nu=mat["nu"])
     assert ex.value.code == _abi.MFBEM_EUNSUPPORTED
     R.close()
+
+
+def test_work_buffers_go_back_after_the_call():
+    """Points x elements decide the work space of a call; once it is over,
+    mfbem_trim_device_cache gives all of the large buffers back."""
+    L = _abi.load()
+    rt = next(ctypes.CDLL(n) for n in ("libcudart.so.13", "libcudart.so") if _loads(n))
+    d = M.cube_clamped_top_traction(5)
+    n = d.n_nodes
+    X = np.random.default_rng(1).random((40000, 3)) * 0.2 + 0.4
+    R = BemRegion(d)
+    R.internal_points(X[:10], np.zeros((n, 3)), np.ones((n, 3)), mu=0.4, nu=0.25)
+
+    def free():
+        assert L.mfbem_trim_device_cache() == 0
+        fr, tot = ctypes.c_size_t(), ctypes.c_size_t()
+        assert rt.cudaMemGetInfo(ctypes.byref(fr), ctypes.byref(tot)) == 0
+        return fr.value
+    before = free()
+    R.internal_points(X, np.zeros((n, 3)), np.ones((n, 3)), mu=0.4, nu=0.25)
+    left = before - free()
+    R.close()
+    # classes alone take 12 MB; buffers below 1 MB may stay with the handle
+    assert left <= 8 << 20, left
