@@ -369,7 +369,8 @@ struct IpArgs {
   int* err;              // first point (1-based) on an element away from its nodes, 0 if none
   void* slot;            // [nf][npairs][9] T: u (3), sigma (6)
   int npairs;
-  void* uw;              // [nf][ne ptot][6] T: u_w, t_w at the dataset points
+  int e0, nec;           // elements of this launch (e0 a multiple of 32)
+  void* uw;              // [nf][nec ptot][6] T: u_w, t_w at the dataset points
   void* part;            // [nf][nip][nch][9] T: partial sums of gpc groups of 32 elements each
   int nch, gpc;
   void* out;             // [nf][nip][12] T: u(3), then sigma(:, kc) for kc = 0..2
@@ -620,13 +621,13 @@ __global__ void k_ip_adp(DMesh m, IpArgs a, POL pol, const QsCurves* __restrict_
   for (int c = 0; c < 6; ++c) sl[3 + c] = sg[c];
 }
 
-// u_w, t_w at every dataset point (all precalculated rules) of every element
+// u_w, t_w at every dataset point (all precalculated rules) of the launch's elements
 template <typename T>
 __global__ void k_ip_weights(DMesh m, IpArgs a) {
-  const long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x, np = (long long)m.ne * m.ptot;
+  const long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x, np = (long long)a.nec * m.ptot;
   if (id >= np * a.nf) return;
   const int f = (int)(id / np);
-  const long long pt = id - f * np;
+  const long long pt = id - f * np + (long long)a.e0 * m.ptot;
   const int e = (int)(pt / m.ptot);
   const T* uv = (const T*)a.uval + (size_t)f * a.nn * 3;
   const T* tv = (const T*)a.tval + (size_t)f * a.nn * 3;
@@ -647,7 +648,8 @@ __global__ void k_ip_weights(DMesh m, IpArgs a) {
 }
 
 // One warp per (gpc groups of 32 elements, point, frequency): the
-// precalculated-rule pairs. gpc is 1 until the points alone fill the GPU.
+// precalculated-rule pairs of the launch's elements, added to the sums of the
+// launches before. gpc is 1 until the points alone fill the GPU.
 // A lane looks up one element's rule; a scan of the point counts then deals the
 // quadrature points of all 32 out to the lanes.
 template <class POL, int WPB>
@@ -661,13 +663,14 @@ __global__ void __launch_bounds__(WPB * 32) k_ip_reg(DMesh m, IpArgs a, POL pol)
   const double* xi = a.xip + 3 * (size_t)ip;
   double xr[3];
   ip_ref(a, xi, xr);
-  const T* uw = (const T*)a.uw + (size_t)f * m.ne * m.ptot * 6;
+  const T* uw = (const T*)a.uw + (size_t)f * a.nec * m.ptot * 6;
+  const size_t pt0 = (size_t)a.e0 * m.ptot;
   T du[3], sg[6];
   for (int c = 0; c < 3; ++c) du[c] = VT<T>::zero();
   for (int c = 0; c < 6; ++c) sg[c] = VT<T>::zero();
   unsigned revs = 0;
   int cls_s = CLS_SING, cls_h = CLS_SING, e = 0;
-  const int g0 = ch * a.gpc, g1 = min(g0 + a.gpc, (m.ne + 31) / 32);
+  const int g0 = ch * a.gpc, g1 = min(g0 + a.gpc, (a.nec + 31) / 32);
 #pragma unroll 1
   for (int hg = 2 * g0; hg < 2 * g1; ++hg) {
     const int h = hg & 1;
@@ -675,11 +678,11 @@ __global__ void __launch_bounds__(WPB * 32) k_ip_reg(DMesh m, IpArgs a, POL pol)
       e = 16 * hg + lane;
       int rev = 0;
       cls_s = cls_h = CLS_SING;
-      if (e < m.ne) {
-        const size_t cid = (size_t)ip * m.ne + e;
+      if (e < a.nec) {
+        const size_t cid = (size_t)ip * m.ne + a.e0 + e;
         cls_s = a.cls_s[cid];
         cls_h = a.cls_h[cid];
-        rev = m.rev[e] & 1;
+        rev = m.rev[a.e0 + e] & 1;
         if (cls_s == CLS_SING || cls_h == CLS_SING) cls_s = cls_h = CLS_SING;
       }
       revs = __ballot_sync(0xffffffffu, rev);
@@ -692,7 +695,8 @@ __global__ void __launch_bounds__(WPB * 32) k_ip_reg(DMesh m, IpArgs a, POL pol)
       if (lane >= o) end += v;
     }
     const int total = __shfl_sync(0xffffffffu, end, 31);
-    // dataset index of scan position q of this lane's element: first + q
+    // dataset index, from the launch's first element, of scan position q of this
+    // lane's element: first + q
     const int first = P > 0 ? e * m.ptot + m.ps_off[c] - (end - P) : 0;
 #pragma unroll 1
     for (int base = 0; base < total; base += 32) {
@@ -705,8 +709,10 @@ __global__ void __launch_bounds__(WPB * 32) k_ip_reg(DMesh m, IpArgs a, POL pol)
       const int pt = __shfl_sync(0xffffffffu, first, j) + q;
       if (q < total) {
         const double rs = (revs >> j) & 1 ? -1.0 : 1.0;
-        const double rv[3] = {m.px[3 * (size_t)pt] - xr[0], m.px[3 * (size_t)pt + 1] - xr[1], m.px[3 * (size_t)pt + 2] - xr[2]};
-        const double n[3] = {m.pn[3 * (size_t)pt], m.pn[3 * (size_t)pt + 1], m.pn[3 * (size_t)pt + 2]};
+        const double* px = m.px + 3 * (pt0 + pt);
+        const double* pn = m.pn + 3 * (pt0 + pt);
+        const double rv[3] = {px[0] - xr[0], px[1] - xr[1], px[2] - xr[2]};
+        const double n[3] = {pn[0], pn[1], pn[2]};
         const T* v = uw + 6 * (size_t)pt;
         const T uu[3] = {v[0], v[1], v[2]}, ut[3] = {v[3], v[4], v[5]};
         if (h) pol.hbie(f, xi, rv, n, ut, uu, rs, sg);
@@ -719,7 +725,7 @@ __global__ void __launch_bounds__(WPB * 32) k_ip_reg(DMesh m, IpArgs a, POL pol)
   for (int j = 0; j < 9; ++j) {
     T v = j < 3 ? du[j < 3 ? j : 0] : sg[j < 3 ? 0 : j - 3];
     for (int off = 16; off > 0; off >>= 1) v = v + shfl_x(v, off);
-    if (lane == 0) o[j] = v;
+    if (lane == 0) o[j] = a.e0 > 0 ? o[j] + v : v;
   }
 }
 

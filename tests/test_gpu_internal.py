@@ -99,6 +99,26 @@ def test_internal_points_at_nodes_and_on_elements():
     R.close()
 
 
+def test_points_of_a_mesh_in_several_launches(oracle):
+    """Sixteen precalculated rules up to the largest (9944 points an element): the
+    294 elements of a harmonic region go through in launches of 256 and 38, the
+    second adding to the sums of the first."""
+    gl = tuple(range(17, 33))
+    d = M.cube_clamped_top_traction(7)
+    mat = M.viscoelastic(1.0, 0.25, 1.0, 0.05)
+    om = float(M.omega_from_a0(0.7, mat))
+    rng = np.random.default_rng(6)
+    X = 0.1 + 0.8 * rng.random((40, 3))
+    X[0] = d.nodes[3]
+    u, t = (rng.standard_normal((d.n_nodes, 3)) + 1j * rng.standard_normal((d.n_nodes, 3)) for _ in range(2))
+    P = oracle.Problem(d, ps_gln=gl)
+    R = BemRegion(d, precalset_gln=gl)
+    ui, si = R.internal_points(X, u, t, mat=mat, omega=om)
+    uo, so = P.internal_points(X, u, t, mat=mat, omega=om)
+    R.close()
+    assert rel(ui, uo) < 1e-11 and rel(si, so) < 1e-11
+
+
 def test_work_buffers_go_back_after_the_call():
     """Points x elements decide the work space of a call; once it is over,
     mfbem_trim_device_cache gives all of the large buffers back."""
