@@ -691,8 +691,13 @@ static int getrf_batched(cudaStream_t st, S* A, long long sA, int lda, int n, in
 // type, size class (n rounded up to 512), batch and GEMM compute type. The
 // first factorisation of a class times the candidates on a seeded random
 // batch of that size (partial pivoting; the operation count is what is timed)
-// and caches the fastest.
-// MFBEM_AUTOTUNE=0 keeps 128.
+// and caches the fastest. The candidates differ by a tenth at most, so nothing
+// else may enter their times: the split workspace is grown to the largest
+// candidate's need before (0.5 GB at 14883 unknowns, which 512 columns, timed
+// last, would pay for), the first candidate runs once untimed where loading the
+// kernels would count (2^24 entries and fewer: a few ms), and one host thread
+// tunes at a time.
+// MFBEM_AUTOTUNE=0 keeps 128, 64, 128, 256 and 512 keep that width.
 // ---------------------------------------------------------------------------
 template <typename S> __device__ __forceinline__ S rnd_val(unsigned long long h);
 template <> __device__ __forceinline__ float rnd_val<float>(unsigned long long h) {
@@ -711,48 +716,67 @@ __global__ void k_tune_fill(S* A, long long total) {
     A[i] = rnd_val<S>(z);
   }
 }
-static std::mutex g_tune_mu;
+static std::mutex g_tune_mu, g_tune_run_mu;
 static std::map<std::tuple<int, int, int, int>, int> g_tune;
 template <typename S>
 static int tuned_nbo(cudaStream_t st, int n, int batch, int* ipiv, int* info, int* out) {
   *out = 128;
   const char* e = getenv("MFBEM_AUTOTUNE");
   if (e && std::string(e) == "0") return 0;
+  const int cand[4] = {64, 128, 256, 512};
+  for (int c : cand)
+    if (e && std::to_string(c) == e) { *out = c; return 0; }
   const auto key = std::make_tuple((int)sizeof(S), (n + 511) / 512, batch, g_c32_mode * 2 + (g_nopiv ? 1 : 0));
-  {
+  auto known = [&]() {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune.find(key);
-    if (it != g_tune.end()) { *out = it->second; return 0; }
-  }
+    if (it != g_tune.end()) *out = it->second;
+    return it != g_tune.end();
+  };
+  if (known()) return 0;
+  std::lock_guard<std::mutex> run(g_tune_run_mu);
+  if (known()) return 0;
   const long long nn = (long long)n * n;
   S* T = nullptr;
   if (cudaMalloc(&T, sizeof(S) * nn * batch) != cudaSuccess) {
     cudaGetLastError();
     return 0;  // no room to tune: keep the default
   }
+  if (sizeof(S) == sizeof(float2) && g_c32_mode != 0) {
+    size_t wb = 0;
+    for (int c : cand)
+      if (n > c) wb = std::max(wb, tc_ws_bytes(n - c, n - c, c, batch));
+    if (wb) try_ensure(g_tc_ws, wb);
+  }
   cudaEvent_t t0, t1;
   cudaEventCreate(&t0);
   cudaEventCreate(&t1);
-  const int cand[4] = {64, 128, 256, 512};
   float best = 1e30f;
   int bn = 128, rc = 0;
-  for (int c = 0; c < 4 && !rc; ++c) {
+  for (int c = nn * batch <= (1 << 24) ? -1 : 0; c < 4 && !rc; ++c) {
     k_tune_fill<S><<<152 * 8, 256, 0, st>>>(T, nn * batch); ++g_launches;
     cudaEventRecord(t0, st);
-    rc = getrf_batched<S>(st, T, nn, n, n, batch, ipiv, info, cand[c]);
+    rc = getrf_batched<S>(st, T, nn, n, n, batch, ipiv, info, cand[std::max(c, 0)]);
     cudaEventRecord(t1, st);
     cudaEventSynchronize(t1);
     float ms = 0.0f;
     cudaEventElapsedTime(&ms, t0, t1);
-    if (!rc && ms < best) { best = ms; bn = cand[c]; }
+    if (!rc && c >= 0 && ms < best) { best = ms; bn = cand[c]; }
+  }
+  // no memory for a width's workspace: the ones before it stand, for this call
+  const bool part = rc == MFBEM_ENOMEM;
+  if (part) {
+    rc = 0;
+    g_err.clear();
   }
   cudaEventDestroy(t0);
   cudaEventDestroy(t1);
   cudaFree(T);
   if (rc) return rc;
+  *out = bn;
+  if (part) return 0;
   std::lock_guard<std::mutex> lk(g_tune_mu);
   g_tune[key] = bn;
-  *out = bn;
   return 0;
 }
 

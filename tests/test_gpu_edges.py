@@ -106,6 +106,30 @@ def test_mixed_solve_of_odd_sizes(divs):
     assert rel(xm, xp) < 1e-9
 
 
+# 2220 unknowns: 172 columns beyond a multiple of 512, 44 of 128
+@pytest.mark.parametrize("harmonic", [False, True], ids=["static", "harmonic"])
+@pytest.mark.parametrize("width", [64, 128, 256, 512])
+def test_mixed_solve_at_each_outer_block_width(width, harmonic, monkeypatch):
+    """Outer blocks of one to four 128-column blocks, with interchanges and
+    without: the mixed solution against the binary64 one (the bound of the mixed
+    solves: 1e-9)."""
+    monkeypatch.setenv("MFBEM_AUTOTUNE", str(width))
+    d = M.cube_clamped_top_traction(6)
+    mat = M.viscoelastic(1.0, 0.3, 1.0, 0.05)
+    om = M.omega_from_a0([0.4, 1.1], mat)
+    R = BemRegion(d)
+
+    def run(precision):
+        return R.sweep_harela(mat, om, precision=precision) if harmonic else \
+            R.solve_staela(1.0, 0.25, precision=precision)
+    xp = run("plain")
+    for pivot in ("none", "partial"):
+        monkeypatch.setenv("MFBEM_PIVOT", pivot)
+        assert rel(run("mixed"), xp) < 1e-9
+        assert R.last_stats["refactorizations"] == 0 and R.last_stats["gmres_iterations"] == 0
+    R.close()
+
+
 @pytest.mark.parametrize("harmonic", [False, True], ids=["static", "harmonic"])
 def test_mixed_solves_repeat_bitwise(harmonic):
     """The unpivoted panel's diagonal block is read by up to 28 CTAs and written
