@@ -44,6 +44,22 @@ def test_lu_and_solve(n, cplx):
 
 
 @pytest.mark.parametrize("cplx", [False, True], ids=["real", "complex"])
+def test_pivot_reciprocal_is_rounded_once(cplx):
+    """The multiplier of an entry 1 is the pivot's reciprocal: each of its parts
+    within half a unit in the last place, 2^-53 of |1 / d| in all."""
+    rng = np.random.default_rng(11)
+    for k in range(300):
+        d = (1.0 + rng.random()) * 2.0 ** rng.integers(1, 30)
+        if cplx:
+            d = d * np.exp(2j * np.pi * rng.random())
+        F = np.array([[d, 0.5], [1.0, 1.0]], dtype=np.complex128 if cplx else np.float64, order="F")
+        solve_lse(F, np.ones((2, 1), dtype=F.dtype, order="F"))
+        dl = np.clongdouble(d)
+        exact = dl.conjugate() / (dl.real * dl.real + dl.imag * dl.imag)
+        assert F[0, 0] == d and abs(np.clongdouble(F[1, 0]) - exact) <= 1.001 * EPS * abs(exact)
+
+
+@pytest.mark.parametrize("cplx", [False, True], ids=["real", "complex"])
 @pytest.mark.parametrize("e", [-980, 900])
 def test_solve_of_tiny_and_huge_entries(e, cplx):
     """A and b times 2^e, large enough for updates on the tensor cores: the
