@@ -108,6 +108,37 @@ template <> __device__ __forceinline__ double2 shfl_s(double2 v, int src) {
 template <> __device__ __forceinline__ float shfl_s(float v, int src) { return __shfl_sync(0xffffffffu, v, src); }
 template <> __device__ __forceinline__ double shfl_s(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
 
+// 1 / d by two Newton steps from the binary32 reciprocal (2^-23 -> 2^-46 -> the
+// rounding of the last step: half a unit in the last place, as a division) where
+// d and 1 / d are well inside binary32's range: on the chain of every column,
+// where a dependent binary64 operation takes 63 cycles and more
+__device__ __forceinline__ double piv_rcp(double d) {
+  const float f = fabsf((float)d);
+  if (!(f > 1e-36f && f < 1e36f)) return 1.0 / d;
+  double y = (double)__frcp_rn((float)d);
+  y = fma(y, fma(-d, y, 1.0), y);
+  return fma(y, fma(-d, y, 1.0), y);
+}
+// conj(d) / |d|^2 where |d|^2 stays within that range, else Smith's form. |d|^2 as
+// q + lo, lo the rounding errors of the squares and of their sum (formed while the
+// first step runs), and the second step's correction c applied to the products,
+// so that each part is rounded once: 0.44 x 2^-53 of |1 / d| rms, 1.0 at most, over
+// 2e7 values (Smith's form 0.61 and 1.6; without lo and c 0.79 and 3.0)
+__device__ __forceinline__ double2 piv_rcp(double2 d) {
+  const bool xm = fabs(d.x) >= fabs(d.y);
+  const double a = xm ? d.x : d.y, b = xm ? d.y : d.x;  // |a| >= |b|: aa - q is exact
+  const double aa = a * a, q = fma(b, b, aa);
+  const float f = (float)q;
+  if (!(f > 1e-36f && f < 1e36f)) return Sc<double2>::rcp(d);
+  const double lo = fma(b, b, aa - q) + fma(a, a, -aa);
+  double y = (double)__frcp_rn(f);
+  y = fma(y, fma(-q, y, 1.0), y);
+  const double c = y * fma(-lo, y, fma(-q, y, 1.0));
+  return make_double2(fma(d.x, y, d.x * c), -fma(d.y, y, d.y * c));
+}
+__device__ __forceinline__ float piv_rcp(float d) { return 1.0f / d; }
+__device__ __forceinline__ float2 piv_rcp(float2 d) { return Sc<float2>::rcp(d); }
+
 // ---------------------------------------------------------------------------
 // Panel factorisation, one CTA per matrix (used where the panel's arithmetic
 // is cheap relative to synchronisation: FP32 and small FP64 problems).
@@ -388,7 +419,7 @@ __global__ void __launch_bounds__(NT) k_panel_coop(S* A, long long strideA, int 
     __syncthreads();
     const S dj = prow[j];
     if (!Sc<S>::iszero(dj)) {
-      const S rcp = Sc<S>::rcp(dj);
+      const S rcp = piv_rcp(dj);
       for (int i = max(jj + 1, r0) - r0 + threadIdx.x; i < nr; i += NT) {
         const S l = Sc<S>::mul(pan[(size_t)j * chunk + i], rcp);
         pan[(size_t)j * chunk + i] = l;
@@ -445,36 +476,6 @@ __device__ __forceinline__ void piv_reduce(unsigned long long& key1, unsigned& r
   row = __reduce_min_sync(0xffffffffu, hi == mh && lo == ml ? row : 0xffffffffu);
   key1 = ((unsigned long long)mh << 32) | ml;
 }
-// 1 / d by two Newton steps from the binary32 reciprocal (2^-23 -> 2^-46 -> the
-// rounding of the last step: half a unit in the last place, as a division) where
-// d and 1 / d are well inside binary32's range: on the chain of every column,
-// where a dependent binary64 operation takes 63 cycles and more
-__device__ __forceinline__ double piv_rcp(double d) {
-  const float f = fabsf((float)d);
-  if (!(f > 1e-36f && f < 1e36f)) return 1.0 / d;
-  double y = (double)__frcp_rn((float)d);
-  y = fma(y, fma(-d, y, 1.0), y);
-  return fma(y, fma(-d, y, 1.0), y);
-}
-// conj(d) / |d|^2 where |d|^2 stays within that range, else Smith's form. |d|^2 as
-// q + lo, lo the rounding errors of the squares and of their sum (formed while the
-// first step runs), and the second step's correction c applied to the products,
-// so that each part is rounded once: 0.44 x 2^-53 of |1 / d| rms, 1.0 at most, over
-// 2e7 values (Smith's form 0.61 and 1.6; without lo and c 0.79 and 3.0)
-__device__ __forceinline__ double2 piv_rcp(double2 d) {
-  const bool xm = fabs(d.x) >= fabs(d.y);
-  const double a = xm ? d.x : d.y, b = xm ? d.y : d.x;  // |a| >= |b|: aa - q is exact
-  const double aa = a * a, q = fma(b, b, aa);
-  const float f = (float)q;
-  if (!(f > 1e-36f && f < 1e36f)) return Sc<double2>::rcp(d);
-  const double lo = fma(b, b, aa - q) + fma(a, a, -aa);
-  double y = (double)__frcp_rn(f);
-  y = fma(y, fma(-q, y, 1.0), y);
-  const double c = y * fma(-lo, y, fma(-q, y, 1.0));
-  return make_double2(fma(d.x, y, d.x * c), -fma(d.y, y, d.y * c));
-}
-__device__ __forceinline__ float piv_rcp(float d) { return 1.0f / d; }
-__device__ __forceinline__ float2 piv_rcp(float2 d) { return Sc<float2>::rcp(d); }
 // a - l p
 __device__ __forceinline__ double lu_fnma(double l, double p, double a) { return fma(-l, p, a); }
 __device__ __forceinline__ float lu_fnma(float l, float p, float a) { return fmaf(-l, p, a); }
