@@ -48,12 +48,13 @@ WORKLOAD_P = "harela surface patch 40x40 quad8 (20x20), 14883 complex DOF, a0=0.
 # Algorithmic work of the regular-pair assembly kernel (the dominant kernel):
 # bytes = the complex system A (n^2) and b (n) written once per frequency;
 # flops = FLOPS_PER_REGULAR_POINT real flops per regular quadrature point of the
-# time-harmonic kernel, counted on the binary64 formulation: distance and
-# powers 13, E_2..E_5 for both wavenumbers 272, psi/chi/TT1..TT3 320, 1/r
-# scalings and dr 24, u*/t* components 168, 120 complex accumulations 480.
-FLOPS_PER_REGULAR_POINT = 1280
+# time-harmonic kernel, counted on the binary64 formulation with the radial
+# functions from the call's table: distance, 1/r and interval 16, five complex
+# Horner sums of degree 7 with their singular parts 160, dr, dr/dn and the
+# products with it 12, u*/t* components 108, 120 complex accumulations 480.
+FLOPS_PER_REGULAR_POINT = 776
 # GB300 FP64 rate (nominal; not in the measured peaks): the binary64
-# formulation of the same kernel could at best run at this rate
+# formulation of the same kernel (the plain path's) could at best run at this rate
 FP64_NOMINAL_TFLOPS = 1.25
 # DRAM bytes per frequency of that kernel from ncu (dram__bytes_read.sum +
 # dram__bytes_write.sum of one launch of the 2-frequency profile case, 449.6 +
@@ -359,9 +360,9 @@ def roofline(st, n, nf):
                         "fp64_nominal_peak_tflops": FP64_NOMINAL_TFLOPS,
                         "frac_of_fp64_nominal": tfl / FP64_NOMINAL_TFLOPS,
                         "ncu_pipes_of_active_cycles": REG_NCU_PIPES,
-                        "note": "SIMT-issue bound (double-float on the FP32 pipe, binary64 only for x - x_i): "
-                                "FP64-equivalent flops above the GPU's whole FP64 rate; HBM and tensor pipes "
-                                "are not the limit of this kernel"}}
+                        "note": "SIMT-issue bound (double-float on the FP32 pipe, binary64 for x - x_i and the "
+                                "pair sums' last addition): FP64-equivalent flops of the tabulated formulation; "
+                                "HBM and tensor pipes are not the limit of this kernel"}}
 
 
 def batching_form():

@@ -330,9 +330,11 @@ int mfbem_solve_report(double* rcond, int32_t n_rhs, double* ferr, double* berr)
                 backward error (the FP64 residual r = b - A x is evaluated with
                 the FP64 matrix) and until the last correction is below 1e-10
                 of x. The LU's trailing updates run on the tensor cores
-                (tcgen05, 3xTF32: FP32-accurate factors); classical refinement
-                x += LU^-1 r follows, GMRES-based refinement (FP64 GMRES
-                preconditioned by the LU factors) when it stalls. With
+                (tcgen05, operands split in two 11-bit parts: FP32-accurate
+                factors); classical refinement x += LU^-1 r follows,
+                GMRES-based refinement (FP64 GMRES preconditioned by the LU
+                factors) when it stalls, accepted only where the preconditioned
+                residual is small against x too (else MFBEM_ENOCONV). With
                 MFBEM_FP32_GEMM=tf32 (single-pass TF32 updates) a stall first
                 redoes the LU with SIMT FP32 updates.
    precision 2: GMRES-based refinement from the start.

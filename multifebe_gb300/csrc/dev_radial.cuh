@@ -30,9 +30,10 @@ constexpr int kRadD = 7;             // polynomial degree
 constexpr int kRadC = kRadD + 1;
 constexpr int kRadDF = 4;            // double-float path: terms up to this degree in df64, the rest in FP32
 constexpr int kRadRowF = kRadDF + 3; // float4 per function and interval of the double-float table
-// intervals per frequency at most: 64 Ki of 128 Ki * 16 B rows. Beyond it
-// (|k| times the mesh's extent above 8192, 1300 wavelengths across) the
-// kernels evaluate E_n directly.
+// intervals per frequency at most: rows of 640 B (1280 with S1..S5, and 560 more
+// for the double-float ones), 40 to 120 MB per frequency. Beyond it (|k| times the
+// mesh's extent above 8192, 1300 wavelengths across) the kernels evaluate E_n
+// directly.
 constexpr int kRadMaxN = 65536;
 
 // singular coefficients (scaled) and the interval of one frequency

@@ -1808,9 +1808,9 @@ extern "C" int mfbem_internal_radial(const double* q, double rmax, int32_t n, co
 #include "mfbem_learned.cuh"
 
 // Test hook (not part of the reference interface): C -= A B for complex64
-// column-major A (m x k), B (k x n), C (m x n) with the tcgen05 3xTF32
-// kernels: pre-split tiles + bulk-copy pipeline (staged = 0) or the
-// self-staging kernel (staged = 1).
+// column-major A (m x k), B (k x n), C (m x n) with the tcgen05
+// kernels: pre-split binary16 hi / lo tiles + bulk-copy pipeline (staged = 0) or
+// the self-staging kernel with tf32 pairs (staged = 1).
 extern "C" int mfbem_internal_tc_cgemm(int32_t m, int32_t n, int32_t k, const float* A, const float* B, float* C,
                                        int32_t staged) {
   g_err.clear();

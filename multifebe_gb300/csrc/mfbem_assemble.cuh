@@ -3,8 +3,10 @@
 // points and their pair lists in element order, and adds the integrated
 // (kn, il, ik) blocks into A and b with the scatter of
 // assemble_bem_{staela,harela}_equation (ordinary BE boundary,
-// src/assemble_bem_staela_equation.f90:69-98). Rows are owned by exactly one
-// warp, so no atomics are used and the summation order is fixed.
+// src/assemble_bem_staela_equation.f90:69-98). Entries are added by reductions at
+// the L2 (addA); rows -- of the system, or of the copy that a slice of a small
+// system's points adds to (Slices) -- belong to exactly one warp, so the
+// summation order is fixed.
 //
 // Each kernel runs in two phases per batch of 32 quadrature points:
 //   phase 1: one lane per point evaluates geometry and the fundamental
@@ -764,13 +766,13 @@ __global__ void k_free(DMesh m, POL pol, const double* nu /* complex, per freque
 }
 
 // ============================================================================
-// Mixed-precision regular pairs (time-harmonic). Only x - x_i is formed in
-// binary64; the distance, the decomposed exponentials E_n of both wavenumbers,
-// the linear combinations forming psi, chi, TT1..TT3, the fundamental solutions
-// and the quadrature sums run in double-float arithmetic (dev_df64.cuh) on the
-// FP32 pipe. Used by the mixed sweep only: regular (far-field) pairs have smooth
-// integrands, and double-float keeps them at ~1e-14 relative; singular and
-// quasi-singular pairs stay FP64.
+// Mixed-precision pairs (time-harmonic): regular, quasi-singular and singular
+// ones of the SBIE. Only x - x_i (for the hoisted points of the latter two their
+// geometry) is formed in binary64; the distance, psi, chi, TT1..TT3 (from the
+// call's radial table, or the decomposed exponentials E_n of both wavenumbers and
+// their linear combinations), the fundamental solutions and the quadrature sums
+// run in double-float arithmetic (dev_df64.cuh) on the FP32 pipe, which keeps
+// the entries at ~1e-14 relative. Used by the mixed sweep only.
 // ============================================================================
 
 // Coefficients of one frequency in double-float. The five combinations
@@ -1218,11 +1220,12 @@ enum MixKind { MIX_REG = 0, MIX_ADP = 1, MIX_SING = 2 };
 // a component and a weight for each). Flush: the sums go through shared memory
 // so that the 144 reals of A's 24 columns x 3 rows, whose binary64 conversions
 // and additions run at two lanes per cycle, fill the warp.
-// Bound by issue slots and latency (45 % of slots, FP64 pipe 34 %, FP32 pipe
-// 24 % at 2 frequencies of the 8x8 cube; 174 warp instructions a regular
+// Bound by issue slots and latency (53 % of slots, FP64 pipe 35 %, FP32 pipe
+// 28 % at 2 frequencies of the 8x8 cube; 174 warp instructions a regular
 // point). Against direct E_n evaluation with scalar double-float and outputs
-// dealt out 32 at a time (497 instructions a point), the 20-frequency sweep of
-// the cube: regular pairs 73 -> 35 ms, singular pairs 26 -> 11.3 ms.
+// dealt out 32 at a time (497 instructions a point) and a flush that reads A, the
+// 20-frequency sweep of the cube: regular pairs 73 -> 25 ms, singular pairs 26 ->
+// 11.2 ms.
 template <int KIND, int WPB, bool TAB>
 __global__ void __launch_bounds__(WPB * 32, KIND == MIX_SING ? 5 : 8) k_mixed(DMesh m, RadTab rt, const HarParF* pf, const ff* dsf,
                                                        const ff* gf, int nf, double2* Ac, size_t lda, size_t astride_e,

@@ -261,6 +261,7 @@ static int oz_err_check(cudaStream_t st) {
 // kernel even in mode 0: the Ozaki path's fixed cost (operand split, TMEM
 // allocation, binary64 epilogue; about 30-40 µs) exceeds the SIMT kernel's
 // time there (small static systems, the depth-16 updates inside an outer block).
+// Measured with 64-wide SIMT tiles alone, before the 32- and 16-wide ones.
 constexpr double kOzMinMacs = 16777216.0;  // 2^24
 // smallest update depth taken by the Ozaki scheme (MFBEM_OZ_MIN_K; 0, the
 // default: any depth above the size threshold). Sending the depth-16 and
